@@ -78,6 +78,13 @@ def lib_path() -> str:
     return _build.LIB
 
 
+def torch_front():
+    """The native front end for torch tensors (``csrc/ws_torch.cpp``)."""
+    load()
+    from . import _ws_torch  # built beside libws_tp.so by build.build()
+    return _ws_torch
+
+
 def load(build_if_missing: bool = True) -> C.CDLL:
     """Load the CUDA library, building it in-tree first when it is absent or stale."""
     global _lib
