@@ -15,6 +15,7 @@
 #include "../../include/ws_tp.h"
 #include "ws_device.cuh"
 #include "ws_fp8_kernel.cuh"
+#include "ws_fp8_gemv_kernel.cuh"
 #include "ws_fp8_bs_kernel.cuh"
 #include "ws_misc_kernels.cuh"
 #include "ws_moe_kernel.cuh"
@@ -295,8 +296,11 @@ ws_status_t ws_tp_create(int32_t world, int32_t rank, int32_t device, const ws_t
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(WS_ERR_CUDA);
     tp->peers[rank] = tp->sym;
     if (world == 1) tp->connected = true;
-    if (set_smem(tp, moe_gemv_kernel) != WS_OK || set_smem(tp, fp8_rowpar_kernel<0>) != WS_OK || set_smem(tp, fp8_rowpar_kernel<1>) != WS_OK ||
-        set_smem(tp, fp8_rowpar_kernel<2>) != WS_OK || set_smem(tp, moe_down_kernel) != WS_OK ||
+    if (set_smem(tp, moe_gemv_kernel) != WS_OK || set_smem(tp, fp8_rowpar_kernel) != WS_OK ||
+        set_smem(tp, fp8_gemv_kernel<1, 1>) != WS_OK || set_smem(tp, fp8_gemv_kernel<1, 2>) != WS_OK ||
+        set_smem(tp, fp8_gemv_kernel<1, 4>) != WS_OK || set_smem(tp, fp8_gemv_kernel<1, 8>) != WS_OK ||
+        set_smem(tp, fp8_gemv_kernel<2, 1>) != WS_OK || set_smem(tp, fp8_gemv_kernel<2, 2>) != WS_OK ||
+        set_smem(tp, fp8_gemv_kernel<2, 4>) != WS_OK || set_smem(tp, moe_down_kernel) != WS_OK ||
         set_smem(tp, fp8_bs_kernel<16>) != WS_OK || set_smem(tp, fp8_bs_kernel<32>) != WS_OK ||
         set_smem(tp, fp8_bs_kernel<64>) != WS_OK || set_smem(tp, fp8_bs_kernel<128>) != WS_OK || set_smem(tp, moe_bs_kernel) != WS_OK ||
         cudaFuncSetAttribute(moe_bs_prep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
@@ -628,10 +632,112 @@ static int fp8_rows_per_launch(const ws_tp *t0, const ws_fp8_gemm_args_t &a, int
     const int skb = (int)((a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
     for (int mp = std::min(64, (rem + 7) / 8 * 8); mp > 8; mp -= 8) {
         const int m = std::min(rem, mp);
-        const Fp8Smem fixed = fp8_smem_layout(0, kbox, mp, (Gm * kGroupRows) / a.block_n + 4, skb, m, (Gm + 2) * kGroupRows, 0);
+        const Fp8Smem fixed = fp8_smem_layout(0, kbox, mp, (Gm * kGroupRows) / a.block_n + 4, skb, m, (Gm + 2) * kGroupRows);
         if ((kSmemBudget - fixed.total) / (fp8_stage_boxes(kbox) * kBoxBytes) >= 3) return m;
     }
     return 8;
+}
+
+// A lone rank that holds only a shard of the vocabulary: the rows nobody computes read as zero.
+static ws_status_t zero_lone_shard(ws_tp *const *ranks, int n, const ws_lm_head_args_t *lm, int m0, int mt, void *const *streams) {
+    if (!lm || n != 1 || ranks[0]->world != 1 || !lm[0].logits || lm[0].g.n >= lm[0].vocab) return WS_OK;
+    WS_CUDA(ranks[0], cudaSetDevice(ranks[0]->device));
+    WS_CUDA(ranks[0], cudaMemsetAsync(lm[0].logits + (size_t)m0 * lm[0].vocab, 0, (size_t)mt * lm[0].vocab * sizeof(float),
+                                      static_cast<cudaStream_t>(streams ? streams[0] : nullptr)));
+    return WS_OK;
+}
+
+// Plan of the one- and two-row CUDA-core kernel; ok = false when the shape does not fit it.
+struct GemvPlan {
+    bool ok;
+    int chunks, slices, rows_per_stage, stage_bytes, nstages, nslot_max, rows_max;
+    size_t smem;
+};
+static GemvPlan gemv_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta) {
+    GemvPlan u{};
+    if (mt > 2) return u;
+    // A lane keeps C 16-byte chunks of K of every token in registers: as many as fit beside the loads in
+    // flight with two CTAs per SM, more only when eight slices do not cover K.
+    const int q = (a.k + 511) / 512;  // 512 bytes: one chunk of every lane
+    u.chunks = 1;
+    while (u.chunks < q && u.chunks * mt < 4) u.chunks *= 2;
+    while ((q + u.chunks - 1) / u.chunks > kGemvMaxSlices) u.chunks *= 2;
+    if (u.chunks * mt > 8) return u;
+    u.slices = (q + u.chunks - 1) / u.chunks;
+    const int groups = kConsumerWarps / u.slices;
+    u.rows_max = (a.n + ncta - 1) / ncta;
+    const int target = getenv("X2") ? atoi(getenv("X2")) * 1024 : 32 * 1024;
+    const int per = 2 * groups;  // rows one turn of every warp takes
+    u.rows_per_stage = std::min(32, std::max(1, target / a.k));
+    if (u.rows_per_stage > per) u.rows_per_stage = u.rows_per_stage / per * per;
+    u.rows_per_stage = std::min(u.rows_per_stage, u.rows_max);
+    u.stage_bytes = (int)align_up((int64_t)u.rows_per_stage * a.k, 128);
+    u.nslot_max = (u.rows_max + a.block_n - 2) / a.block_n + 1;
+    const int items = (u.rows_max + u.rows_per_stage - 1) / u.rows_per_stage;
+    auto total = [&](int ns) { return fp8_gemv_smem(ns, u.stage_bytes, u.nslot_max, skb, mt, u.slices, u.rows_max).total; };
+    const int budget = getenv("X1") && atoi(getenv("X1")) ? kHalfSmemBudget : kSmemBudget;
+    int ns = std::min((int)kMaxStages, items);
+    while (ns >= 2 && total(ns) > budget) --ns;
+    u.nstages = ns;
+    u.ok = (ns >= 2 || ns == items) && total(ns) <= budget;
+    u.smem = (size_t)total(ns);
+    return u;
+}
+
+static ws_status_t gemv_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t *args, const ws_lm_head_args_t *lm, int m0, int mt,
+                             void *const *streams, int ncta, bool same_device, const GemvPlan &u, int skb, bool last) {
+    ws_tp *t0 = ranks[0];
+    const ws_fp8_gemm_args_t &a0 = lm ? lm[0].g : args[0];
+    Fp8GemvParams p{};
+    p.m = mt; p.n = a0.n; p.k = a0.k; p.x_dtype = a0.x_dtype; p.scale_kind = a0.scale_kind; p.world = t0->world;
+    p.mode = lm ? kModeLmHead : kModeAllReduce;
+    p.vocab = lm ? lm[0].vocab : 0;
+    for (p.bk_shift = 0; (1 << p.bk_shift) < a0.block_k; ++p.bk_shift) {}
+    for (p.bn_shift = 0; (1 << p.bn_shift) < a0.block_n; ++p.bn_shift) {}
+    p.nslot_max = u.nslot_max; p.skb = skb; p.slices = u.slices; p.rows_per_stage = u.rows_per_stage; p.nstages = u.nstages;
+    p.rows_max = u.rows_max; p.stage_bytes = u.stage_bytes;
+    p.timeout_ns = t0->timeout_ns;
+    p.lay = t0->lay;
+    for (int i = 0; i < n; ++i) {
+        const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
+        if ((reinterpret_cast<uintptr_t>(a.w) & 15) || (a.ldw & 15))
+            return fail(t0, WS_ERR_INVALID, "weight base and row stride must be multiples of 16 bytes");
+        Fp8RankArgs &r = p.r[i];
+        r.x = static_cast<const char *>(a.x) + (size_t)m0 * a.ldx * (a.x_dtype == WS_ACT_BF16 ? 2 : 4);
+        r.scales = a.scales;
+        r.out = lm ? nullptr : a.out + (size_t)m0 * a.n;
+        r.logits = lm && lm[i].logits ? lm[i].logits + (size_t)m0 * lm[i].vocab : nullptr;
+        if (r.logits) p.gather_logits = 1;
+        r.argmax = lm && lm[i].argmax ? lm[i].argmax + m0 : nullptr;
+        r.ldx = a.ldx; r.scale_ld = a.scale_ld; r.row0 = a.row0; r.k0 = a.k0;
+        r.vocab_row0 = lm ? lm[i].vocab_row0 : 0;
+        r.ctx = make_ctx(ranks[i]);
+        if (last) r.ctx.host_done = ranks[i]->host_done_arm;
+        p.w[i] = a.w;
+        p.ldw[i] = a.ldw;
+    }
+    for (int i = 0; i < n; ++i) ranks[i]->step++;
+    void (*const kernel)(Fp8GemvParams) = mt == 1 ? (u.chunks == 1   ? fp8_gemv_kernel<1, 1>
+                                                     : u.chunks == 2 ? fp8_gemv_kernel<1, 2>
+                                                     : u.chunks == 4 ? fp8_gemv_kernel<1, 4>
+                                                                     : fp8_gemv_kernel<1, 8>)
+                                                  : (u.chunks == 1   ? fp8_gemv_kernel<2, 1>
+                                                     : u.chunks == 2 ? fp8_gemv_kernel<2, 2>
+                                                                     : fp8_gemv_kernel<2, 4>);
+    ws_status_t s = zero_lone_shard(ranks, n, lm, m0, mt, streams);
+    for (int i = 0; i < (same_device ? 1 : n) && s == WS_OK; ++i) {
+        Fp8GemvParams q = p;
+        if (!same_device) {  // one launch per device, each sees itself as virtual rank 0
+            q.r[0] = p.r[i];
+            q.w[0] = p.w[i];
+            q.ldw[0] = p.ldw[i];
+        }
+        WS_CUDA(ranks[i], cudaSetDevice(ranks[i]->device));
+        s = launch(ranks[i], kernel, q, ncta, same_device ? n : 1, kThreads, u.smem, static_cast<cudaStream_t>(streams ? streams[i] : nullptr),
+                   t0->pdl != 0);
+        if (s != WS_OK) t0->err = ranks[i]->err;
+    }
+    return s;
 }
 
 // One fused step over the activation rows [m0, m0 + mt) (mt from fp8_rows_per_launch).
@@ -649,6 +755,15 @@ static ws_status_t fp8_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t
         }
         const BsPlan u = bs_plan(a0, mt, (int)skb_u, ncta, n == 1);  // CTA pairs need a cluster launch, virtual ranks a cooperative one
         if (u.ok) return bs_step(ranks, n, args, lm, m0, mt, streams, ncta, same_device, u, (int)skb_u, last);
+    }
+    if (t0->kernel_sel != 1 && mt <= 2) {  // one or two activation rows: CUDA-core dot products
+        int64_t skb_u = 1;
+        for (int i = 0; i < n; ++i) {
+            const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
+            skb_u = std::max<int64_t>(skb_u, (a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
+        }
+        const GemvPlan u = gemv_plan(a0, mt, (int)skb_u, ncta);
+        if (u.ok) return gemv_step(ranks, n, args, lm, m0, mt, streams, ncta, same_device, u, (int)skb_u, last);
     }
     Fp8Params p{};
     p.m = mt; p.n = a0.n; p.k = a0.k; p.x_dtype = a0.x_dtype; p.scale_kind = a0.scale_kind;
@@ -676,16 +791,13 @@ static ws_status_t fp8_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t
     p.gran = ragged_granularity(p.n, ncta);
     p.nslot_max = (Gm * kGroupRows) / p.bn + 2 + 2;
     p.part_rows = (Gm + 2) * kGroupRows;  // whole tiles + at most two ragged tiles
-    // One or two activation rows: CUDA-core dot products; more: the tensor-core MMA.
-    const int gt = (t0->kernel_sel != 1 && mt <= 2) ? mt : 0;
-    void (*const kernel)(Fp8Params) = gt == 1 ? fp8_rowpar_kernel<1> : gt == 2 ? fp8_rowpar_kernel<2> : fp8_rowpar_kernel<0>;
-    const Fp8Smem fixed = fp8_smem_layout(0, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows, gt);
+    const Fp8Smem fixed = fp8_smem_layout(0, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows);
     p.stage_bytes = fp8_stage_boxes(kbox) * kBoxBytes;
     int ns = (kSmemBudget - fixed.total) / p.stage_bytes;
     if (ns > kMaxStages) ns = kMaxStages;
     if (ns < 2) return fail(t0, WS_ERR_CAPACITY, "shapes m=%d n=%d k=%d leave no room for the weight stage ring", p.m, p.n, p.k);
     p.nstages = ns;
-    const size_t smem = (size_t)fp8_smem_layout(ns, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows, gt).total + 1024;
+    const size_t smem = (size_t)fp8_smem_layout(ns, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows).total + 1024;
 
     for (int i = 0; i < n; ++i) {
         ws_tp *t = ranks[i];
@@ -706,26 +818,21 @@ static ws_status_t fp8_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t
         r.vocab_row0 = lm ? lm[i].vocab_row0 : 0;
         r.ctx = make_ctx(t);
         if (last) r.ctx.host_done = t->host_done_arm;
-        p.w[i] = a.w;
-        p.ldw[i] = a.ldw;
     }
-    // as in the tensor-memory path: only when a second CTA can be resident beside the predecessor's
-    p.l2_prefetch = (2 * smem <= (size_t)227 * 1024 && (size_t)p.n * p.k <= ((size_t)64 << 20)) ? 1 : 0;
+    zero_lone_shard(ranks, n, lm, m0, mt, streams);
     // every endpoint advances by one step
     for (int i = 0; i < n; ++i) ranks[i]->step++;
     if (same_device) {
         WS_CUDA(t0, cudaSetDevice(t0->device));
-        return launch(t0, kernel, p, ncta, n, fp8_threads(gt), smem, static_cast<cudaStream_t>(streams ? streams[0] : nullptr), t0->pdl != 0);
+        return launch(t0, fp8_rowpar_kernel, p, ncta, n, kThreads, smem, static_cast<cudaStream_t>(streams ? streams[0] : nullptr), t0->pdl != 0);
     }
     for (int i = 0; i < n; ++i) {  // one launch per device, each sees itself as virtual rank 0
         Fp8Params q = p;
         q.r[0] = p.r[i];
         q.tmap[0][0] = p.tmap[i][0];
         q.tmap[0][1] = p.tmap[i][1];
-        q.w[0] = p.w[i];
-        q.ldw[0] = p.ldw[i];
         WS_CUDA(ranks[i], cudaSetDevice(ranks[i]->device));
-        ws_status_t s = launch(ranks[i], kernel, q, ncta, 1, fp8_threads(gt), smem,
+        ws_status_t s = launch(ranks[i], fp8_rowpar_kernel, q, ncta, 1, kThreads, smem,
                                static_cast<cudaStream_t>(streams ? streams[i] : nullptr), t0->pdl != 0);
         if (s != WS_OK) { t0->err = ranks[i]->err; return s; }
     }
@@ -1423,7 +1530,7 @@ ws_status_t ws_fp8_gemm_static_scratch(const ws_fp8_gemm_args_t *a, int32_t devi
             }
             int sms = 0;
             ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-            if (ce == cudaSuccess) ce = cudaFuncSetAttribute(fp8_rowpar_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            if (ce == cudaSuccess) ce = cudaFuncSetAttribute(fp8_rowpar_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (ce != cudaSuccess) { set_err(err, err_len, "device set-up: %s", cudaGetErrorString(ce)); return WS_ERR_CUDA; }
             g_static_sm_count[device] = sms;
             g_static_scratch_addr[device] = static_cast<unsigned char *>(ptr);
@@ -1450,12 +1557,12 @@ ws_status_t ws_fp8_gemm_static_scratch(const ws_fp8_gemm_args_t *a, int32_t devi
     p.ragged = Gm < 8 ? 1 : 0;
     p.gran = ragged_granularity(p.n, ncta);
     p.part_rows = (Gm + 2) * kGroupRows;
-    const Fp8Smem fixed = fp8_smem_layout(0, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows, 0);
+    const Fp8Smem fixed = fp8_smem_layout(0, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows);
     p.stage_bytes = fp8_stage_boxes(kbox) * kBoxBytes;
     int ns = std::min((kSmemBudget - fixed.total) / p.stage_bytes, (int)kMaxStages);
     if (ns < 2) { set_err(err, err_len, "shapes m=%d n=%d k=%d leave no room for the weight stage ring", p.m, p.n, p.k); return WS_ERR_CAPACITY; }
     p.nstages = ns;
-    const size_t smem = (size_t)fp8_smem_layout(ns, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows, 0).total + 1024;
+    const size_t smem = (size_t)fp8_smem_layout(ns, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows).total + 1024;
     Fp8RankArgs &r = p.r[0];
     for (int b = 0; b < 2; ++b) {
         st = make_tmap(&probe_err, &p.tmap[0][b], a->w, (uint64_t)a->n, (uint64_t)a->k, (uint64_t)a->ldw,
@@ -1468,7 +1575,7 @@ ws_status_t ws_fp8_gemm_static_scratch(const ws_fp8_gemm_args_t *a, int32_t devi
     r.ctx.status = r.ctx.counters + kMaxShared;
     r.ctx.step_ctr = r.ctx.counters + kMaxShared + 2;
     r.ctx.rank = 0;
-    fp8_rowpar_kernel<0><<<dim3((unsigned)ncta, 1, 1), kThreads, smem, cs>>>(p);
+    fp8_rowpar_kernel<<<dim3((unsigned)ncta, 1, 1), kThreads, smem, cs>>>(p);
     ce = cudaGetLastError();
     if (ce != cudaSuccess) { set_err(err, err_len, "kernel launch: %s", cudaGetErrorString(ce)); return WS_ERR_CUDA; }
     return WS_OK;

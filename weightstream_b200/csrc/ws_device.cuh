@@ -146,6 +146,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
+// Untiled bulk copy global -> shared (16-byte aligned addresses and size), completion on an mbarrier.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t &r0, uint32_t &r1,
                                             uint32_t &r2, uint32_t &r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -414,6 +420,11 @@ __device__ __forceinline__ float pow2_f32(int e) {  // 2^e for any e: inf above 
     if (e > 127) return __uint_as_float(0x7F800000u);
     if (e >= -126) return __uint_as_float((uint32_t)(e + 127) << 23);
     return e >= -149 ? __uint_as_float(1u << (e + 149)) : 0.0f;
+}
+// UE8M0 byte -> 2^(b - 127); 255 is NaN.
+__device__ __forceinline__ float e8m0_f32(uint32_t b) {
+    return (b == 0xFFu) ? __uint_as_float(0x7FC00000u)
+                        : (b == 0u ? __uint_as_float(0x00400000u) : __uint_as_float(b << 23));
 }
 // Two floats -> two E4M3 bytes (lo = a, hi = b), RNE, saturating, NaN -> 0x7F.
 __device__ __forceinline__ uint32_t cvt_e4m3x2(float a, float b) {

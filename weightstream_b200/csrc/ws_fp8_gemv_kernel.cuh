@@ -1,0 +1,246 @@
+// FP8 E4M3 row-parallel decode step for one or two activation rows on CUDA cores, fused with its
+// exchange (sm_100a).  One persistent CTA per SM (two where they fit: the next step's CTA then fills its
+// ring while this one finishes).
+//
+// A CTA owns a contiguous range of output rows, floor or ceil of n / ncta, so all SMs stream the same
+// bytes to within a row.  One producer warp brings whole rows in by bulk copy, R rows per stage.  The
+// eight consumer warps are S slices of K times G row groups; a lane owns the same C 16-byte chunks of K
+// in every row its warp visits, and holds that K's activations in registers as f16 pairs: it quantises
+// them itself, straight from memory, exactly as the reference does
+// (crates/weightstream-ref/src/actquant.rs:21-57), so no shared memory, barrier or other warp stands
+// between the predecessor's end and the first product.  Per row and chunk: one conflict-free 128-bit
+// shared load, 8 conversions to f16 pairs, 16 mixed-precision FMAs with exact products
+// (fma.rn.f32.f16), one FMA with the product of the block scales; two rows' sums are folded over the
+// lanes by five shuffles.  Slices meet once, after the last row, in slice order.
+//
+// Bound: HBM for large shards, the dependency latency between steps for small ones.
+#pragma once
+
+#include <math.h>
+
+#include "ws_device.cuh"
+#include "ws_fp8_kernel.cuh"
+
+namespace ws {
+
+constexpr int kGemvMaxSlices = kConsumerWarps;
+
+struct alignas(64) Fp8GemvParams {
+    int32_t m, n, k, x_dtype, scale_kind, world, mode, vocab;
+    int32_t bk_shift, bn_shift, nslot_max, skb;
+    int32_t slices, rows_per_stage, nstages, rows_max, stage_bytes, gather_logits;
+    uint64_t timeout_ns;
+    SymLayout lay;
+    Fp8RankArgs r[WS_MAX_WORLD];
+    const uint8_t *w[WS_MAX_WORLD];
+    int64_t ldw[WS_MAX_WORLD];
+};
+
+struct Fp8GemvSmem {
+    int32_t stages, sw, part, bars, total;
+};
+__host__ __device__ inline Fp8GemvSmem fp8_gemv_smem(int nstages, int stage_bytes, int nslot_max, int skb, int m, int slices, int rows_max) {
+    Fp8GemvSmem s{};
+    int o = 0;
+    s.stages = o; o += nstages * stage_bytes;
+    s.sw = o;     o += (nslot_max * skb * 4 + 15) / 16 * 16;
+    s.part = o;   o += (m * slices * rows_max * 4 + 15) / 16 * 16;  // [token][slice][row of the CTA]
+    s.bars = o;   o += 2 * kMaxStages * 8;
+    s.total = o;
+    return s;
+}
+
+template <int GT, int C>
+__device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    constexpr int CW = kConsumerWarps, CT = kConsumerThreads;
+    const int vr = blockIdx.y, cta = blockIdx.x, ncta = gridDim.x;
+    const Fp8RankArgs &A = p.r[vr];
+    const RankCtx &X = A.ctx;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row_a = (int)((int64_t)p.n * cta / ncta), rows = (int)((int64_t)p.n * (cta + 1) / ncta) - row_a;
+    const int R = p.rows_per_stage, NS = p.nstages, items = (rows + R - 1) / R;
+
+    const Fp8GemvSmem L = fp8_gemv_smem(NS, p.stage_bytes, p.nslot_max, p.skb, GT, p.slices, p.rows_max);
+    float *sw_s = reinterpret_cast<float *>(smem + L.sw), *part_s = reinterpret_cast<float *>(smem + L.part);
+    const uint32_t stage0 = smem_u32(smem + L.stages);
+    const uint32_t full0 = smem_u32(smem + L.bars), empty0 = full0 + kMaxStages * 8;
+    if (tid == CT) {  // the producer's first lane
+        for (int s = 0; s < NS; ++s) {
+            mbar_init(full0 + s * 8, 1);
+            mbar_init(empty0 + s * 8, CW);
+        }
+        mbar_fence_init();
+    }
+    __syncthreads();
+    // Let the next kernel on the stream begin (it only streams weights until its own wait).
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    if (warp == CW) {
+        // ------------------------------------------------------------ producer warp
+        const uint8_t *w = p.w[vr] + (int64_t)row_a * p.ldw[vr];
+        const bool dense = p.ldw[vr] == p.k;
+        RingPos rp;
+        for (int it = 0; it < items; ++it, rp.next(NS)) {
+            const int s = rp.s, r0 = it * R, nr = min(R, rows - r0);
+            if (!mbar_wait(empty0 + s * 8, rp.ph ^ 1u, X.status)) return;  // a wait gave up: stop streaming
+            if (lane == 0) mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)(nr * p.k));
+            __syncwarp();
+            const uint32_t dst = stage0 + s * p.stage_bytes;
+            if (dense ? lane == 0 : lane < nr)  // adjacent rows of a dense shard are one copy
+                bulk_load(dst + lane * p.k, w + (int64_t)(r0 + lane) * p.ldw[vr], (uint32_t)(dense ? nr * p.k : p.k), full0 + s * 8);
+        }
+        return;
+    }
+
+    // ---------------------------------------------------------------- consumer warps
+    const int S = p.slices, G = CW / S;
+    const int slice = warp % S, grp = warp / S;  // warps beyond S * G only keep the barriers moving
+    const int64_t kcol0 = A.k0 >> p.bk_shift, srow_lo = (A.row0 + row_a) >> p.bn_shift;
+    {   // weight scales of this CTA's rows: static, so fetched before the wait on the predecessor
+        const int ncols = (int)(((A.k0 + p.k - 1) >> p.bk_shift) - kcol0 + 1);
+        const int nslot = rows > 0 ? (int)(((A.row0 + row_a + rows - 1) >> p.bn_shift) - srow_lo + 1) : 0;
+        for (int i = tid; i < nslot * ncols; i += CT) {
+            const int sl = i / ncols, c = i - sl * ncols;
+            const int64_t idx = (srow_lo + sl) * A.scale_ld + kcol0 + c;
+            float v;
+            if (p.scale_kind == WS_SCALE_UE8M0) v = e8m0_f32(__ldg(static_cast<const uint8_t *>(A.scales) + idx));
+            else v = __ldg(static_cast<const float *>(A.scales) + idx);
+            sw_s[sl * p.skb + c] = v;
+        }
+    }
+    consumer_bar();
+    // Everything below may read what the previous kernel on the stream wrote (activations, the step
+    // sequence, exchange slots).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint32_t xh[GT][C][8];  // this lane's quantised activations
+    float sa[GT][C];        // and their block scales 2^e
+    int swc[C];             // column of each chunk in sw_s
+    bool live[C];
+    {
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            const int k = ((slice * C + i) * 32 + lane) * 16;
+            live[i] = k < p.k && grp < G;
+            swc[i] = live[i] ? (int)(((A.k0 + k) >> p.bk_shift) - kcol0) : 0;
+        }
+        float v[GT][C][16];
+#pragma unroll
+        for (int t = 0; t < GT; ++t)
+#pragma unroll
+            for (int i = 0; i < C; ++i) {
+                const int k = ((slice * C + i) * 32 + lane) * 16;
+                load_act8(A.x, p.x_dtype, (int64_t)t * A.ldx + k, live[i], *reinterpret_cast<float(*)[8]>(v[t][i]));
+                load_act8(A.x, p.x_dtype, (int64_t)t * A.ldx + k + 8, live[i], *reinterpret_cast<float(*)[8]>(v[t][i] + 8));
+            }
+#pragma unroll
+        for (int t = 0; t < GT; ++t)
+#pragma unroll
+            for (int i = 0; i < C; ++i) {
+                float amax = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[t][i][j]));
+                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));  // a 32-block is two adjacent lanes
+                const int e = act_scale_exp(amax);
+                const float inv = e > 127 ? 0.0f : pow2_f32(-e);  // an infinite block scale divides everything to zero
+                sa[t][i] = live[i] ? pow2_f32(e) : 0.0f;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    xh[t][i][j] = live[i] ? e4m3x2_to_f16x2(cvt_e4m3x2(v[t][i][2 * j] * inv, v[t][i][2 * j + 1] * inv)) : 0u;
+            }
+    }
+    const bool solo = p.mode == kModeAllReduce && p.world == 1;
+    const uint32_t seq = solo ? 0u : step_begin(X);
+
+    float f[GT][C];
+    int blk = -1;  // scale row the factors f are for
+    auto factors = [&](int row) {
+        const int b = (int)(((A.row0 + row_a + row) >> p.bn_shift) - srow_lo);
+        if (b == blk) return;
+        blk = b;
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            const float sw = sw_s[b * p.skb + swc[i]];
+#pragma unroll
+            for (int t = 0; t < GT; ++t) f[t][i] = sa[t][i] * sw;
+        }
+    };
+    auto dot = [&](const uint4 (&w)[C], float (&acc)[GT]) {
+#pragma unroll
+        for (int t = 0; t < GT; ++t) acc[t] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+            uint32_t h[8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                h[2 * q] = e4m3x2_half_to_f16x2<0>(ww[q]);
+                h[2 * q + 1] = e4m3x2_half_to_f16x2<1>(ww[q]);
+            }
+#pragma unroll
+            for (int t = 0; t < GT; ++t) {
+                float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    fma2_f16(s0, h[2 * q], xh[t][i][2 * q]);
+                    fma2_f16(s1, h[2 * q + 1], xh[t][i][2 * q + 1]);
+                }
+                acc[t] = fmaf(s0 + s1, f[t][i], acc[t]);
+            }
+        }
+    };
+    const uint32_t lane_off = (uint32_t)((slice * C * 32 + lane) * 16);
+    auto load_row = [&](uint32_t rbase, uint4 (&w)[C]) {
+#pragma unroll
+        for (int i = 0; i < C; ++i) w[i] = live[i] ? lds_u128(rbase + lane_off + i * 512) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    const bool hi = (lane & 16) != 0;
+    RingPos rp;
+    for (int it = 0; it < items; ++it, rp.next(NS)) {
+        const int s = rp.s, r0 = it * R, nr = min(R, rows - r0);
+        const bool landed = mbar_wait(full0 + s * 8, rp.ph, X.status);  // false: a wait gave up, the step is void
+        const uint32_t sbase = stage0 + s * p.stage_bytes;
+        if (landed && grp < G) {
+            for (int r = grp; r < nr; r += 2 * G) {  // two rows at a time
+                const int r2 = r + G;
+                const bool two = r2 < nr;  // warp-uniform
+                uint4 wa[C], wb[C];
+                load_row(sbase + r * p.k, wa);
+                load_row(sbase + (two ? r2 : r) * p.k, wb);
+                float va[GT], vb[GT];
+                factors(r0 + r);
+                dot(wa, va);
+                if (two) factors(r0 + r2);
+                dot(wb, vb);
+#pragma unroll
+                for (int t = 0; t < GT; ++t) {  // lanes 0-15 end with row r, lanes 16-31 with row r2
+                    float v = (hi ? vb[t] : va[t]) + __shfl_xor_sync(0xffffffffu, hi ? va[t] : vb[t], 16);
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    if ((lane & 15) == 0 && (!hi || two)) part_s[(t * S + slice) * p.rows_max + r0 + (hi ? r2 : r)] = v;
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty0 + s * 8);
+    }
+    consumer_bar();  // part_s complete
+
+    auto value = [&](int tok, int r) {
+        const float *q = part_s + (size_t)tok * S * p.rows_max + r;
+        float v = q[0];
+        for (int s = 1; s < S; ++s) v += q[s * p.rows_max];
+        return v;
+    };
+    fp8_finish<CT>(p, A, X, seq, tid, rows, [&](int i) { return row_a + i; }, value);
+}
+
+template <int GT, int C>
+__global__ void __launch_bounds__(kThreads, GT * C <= 4 ? 2 : 1) fp8_gemv_kernel(const __grid_constant__ Fp8GemvParams p) {
+    const RankCtx &X = p.r[blockIdx.y].ctx;
+    fp8_gemv_body<GT, C>(p);
+    if (p.world > 1 || p.mode == kModeLmHead) step_end(X, step_begin(X), gridDim.x);  // a lone all-reduce rank exchanges nothing
+    host_done_signal(X, gridDim.x);
+}
+
+}  // namespace ws

@@ -6,15 +6,10 @@
 // across CTAs.  Weight tiles arrive by TMA into a ring of 32 KB stages filled by one producer
 // warp: 16-row x 128-byte boxes for whole tiles, 8/4/2/1-row boxes for the ragged rows, all
 // 128B-swizzled.  The prologue quantises the activations exactly as the reference does; eight
-// consumer warps then multiply the staged rows with them and apply the activation- and
-// weight-block scales per 32-wide K block in fp32.  Two formulations of that product:
-//   GT = 1, 2 (one or two activation rows): CUDA cores.  A lane owns 16 bytes of a row
-//     (128-bit shared load), converts them to f16 pairs and accumulates exact products in fp32
-//     (fma.rn.f32.f16); the eight lanes of a row are combined by shuffles at the end of a tile.
-//     About 1.5 lane-instructions per weight byte, so HBM, not issue, bounds it.
-//   GT = 0 (three to eight rows): the FP8 tensor-core MMA m16n8k32, one per 32-wide K block.
-//     Its issue rate caps streaming near 70 % of HBM bandwidth, which is why it is not used
-//     for the narrow cases.
+// consumer warps then multiply the staged rows with them by the FP8 tensor-core MMA m16n8k32, one per
+// 32-wide K block, and apply the activation- and weight-block scales in fp32.  Its issue rate caps
+// streaming near 70 % of HBM bandwidth: it serves the shapes neither the one- and two-row kernel
+// (ws_fp8_gemv_kernel.cuh) nor the tensor-memory kernel (ws_fp8_bs_kernel.cuh) takes.
 //
 // Exchange (world > 1): a thread stores its rows' fp32 partials into slot [my rank] of every
 // peer's exchange memory as 64-bit {step, value} words and then adds the same rows' words of all
@@ -53,28 +48,16 @@ struct alignas(64) Fp8Params {
     int32_t gather_logits, ragged;   // ragged = 0: leftover tiles go whole to the first CTAs
     int32_t bk_shift, bn_shift;      // log2 of the scale block edges
     int32_t part_rows, gran;         // partial rows reserved per token; row granularity (1,2,4,8) of the ragged share
-    int32_t stage_bytes, l2_prefetch;  // bytes of one weight stage: a whole number of 2 KB boxes (fp8_stage_boxes); see below
+    int32_t stage_bytes, pad0;         // bytes of one weight stage: a whole number of 2 KB boxes (fp8_stage_boxes)
     uint64_t timeout_ns;
     SymLayout lay;
     Fp8RankArgs r[WS_MAX_WORLD];
-    // l2_prefetch: once the stage ring is full for the first time, the producer asks L2 for the rest
-    // of this CTA's rows (weights are static), so that HBM keeps streaming while the predecessor on
-    // the stream finishes and this kernel quantises its activations.  Needs the plain addresses:
-    const uint8_t *w[WS_MAX_WORLD];
-    int64_t ldw[WS_MAX_WORLD];
 };
-
-// Consumer warps per CTA.  Sixteen warps instead of eight changed neither formulation's time by
-// more than 2 % on B200, so both run eight.
-__host__ __device__ constexpr int fp8_consumer_warps(int) { return kConsumerWarps; }
-__host__ __device__ constexpr int fp8_threads(int gt) { return (fp8_consumer_warps(gt) + 1) * 32; }  // + the TMA producer warp
 
 struct Fp8Smem {  // byte offsets from the 1024-aligned base
     int32_t stages, q, sa, sw, red, part, bars, misc, total;
 };
 
-// gt: 0 for the MMA formulation (activations kept as E4M3 bytes, [kb][tok][32]), else the number
-// of activation rows of the CUDA-core formulation (kept as f16, [tok][kbox*128]).
 // Boxes (16 rows x 128 bytes) per stage: a tile's kbox boxes are cut into equal stages of at most
 // kBoxesPerStage, so that no stage travels half empty (7168 columns = 56 boxes: four stages of 14
 // instead of 16 + 16 + 16 + 8).
@@ -84,14 +67,14 @@ __host__ __device__ inline int fp8_stage_boxes(int kbox) {
 }
 
 __host__ __device__ inline Fp8Smem fp8_smem_layout(int nstages, int kbox, int mp, int nslot_max, int skb,
-                                                   int m, int part_rows, int gt) {
+                                                   int m, int part_rows) {
     Fp8Smem s{};
     int o = 0;
     s.stages = o; o += nstages * fp8_stage_boxes(kbox) * kBoxBytes;
-    s.q = o;      o += gt > 0 ? kbox * 128 * 2 * gt : kbox * 4 * mp * 32;
+    s.q = o;      o += kbox * 4 * mp * 32;  // E4M3 bytes, [kb][tok][32]
     s.sa = o;     o += kbox * 4 * (mp > 8 ? mp : 8) * 4;
     s.sw = o;     o += ((nslot_max * skb * 4 + 15) / 16) * 16;
-    s.red = o;    o += 2 * fp8_consumer_warps(gt) * 128 * 4;
+    s.red = o;    o += 2 * kConsumerWarps * 128 * 4;
     s.part = o;   o += ((m * part_rows * 4 + 15) / 16) * 16;
     s.bars = o;   o += 2 * kMaxStages * 8;
     s.misc = o;   o += 128;
@@ -127,13 +110,128 @@ __device__ __forceinline__ bool cand_better(float v, uint32_t i, float bv, uint3
     return v > bv || (v == bv && i < bi);
 }
 
-template <int GT>
+// What follows a CTA's finished rows, in both decode kernels: the output, the all-reduce exchange, or the
+// lm_head's logits and argmax.  The CTA holds `count` row slots; row_of(i) is the global row of slot i
+// (negative: none), value(tok, i) its finished sum.  Called by the CT consumer threads.
+template <int CT, typename P, typename RowOf, typename Value>
+__device__ __forceinline__ void fp8_finish(const P &p, const Fp8RankArgs &A, const RankCtx &X, uint32_t seq, int tid, int count,
+                                           RowOf row_of, Value value) {
+    constexpr int CW = CT / 32;
+    const int cta = blockIdx.x, ncta = gridDim.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t bank = seq & 1u;
+    auto for_rows = [&](auto fn) {  // fn(tok, global row, slot)
+        for (int j = tid; j < p.m * count; j += CT) {
+            const int tok = j / count, i = j - tok * count, row = row_of(i);
+            if (row >= 0) fn(tok, row, i);
+        }
+    };
+    if (p.mode == kModeAllReduce && p.world == 1) {
+        for_rows([&](int tok, int row, int i) { A.out[(size_t)tok * p.n + row] = value(tok, i); });
+        return;
+    }
+    const int nflag = kMaxCtas + kMaxShared;
+    const uint32_t *myflags = reinterpret_cast<const uint32_t *>(X.sym[X.rank] + p.lay.flags_off) +
+                              (size_t)bank * p.world * nflag;
+
+    if (p.mode == kModeAllReduce) {
+        // every thread sends its rows' partials to all ranks as tagged words, then folds the same
+        // rows in rank order as the ranks' words arrive: no barrier, fence or flag in between
+        const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
+        for (int pr = 0; pr < p.world; ++pr) {
+            uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride;
+            for_rows([&](int tok, int row, int i) { st_word_sys(dst + (size_t)tok * p.n + row, seq, value(tok, i)); });
+        }
+        const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) +
+                                (size_t)bank * p.world * astride;
+        for_rows([&](int tok, int row, int) {
+            const size_t off = (size_t)tok * p.n + row;
+            A.out[off] = fold_words(slots, astride, off, p.world, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
+        });
+        return;
+    }
+
+    // ---- lm_head: gather rows, publish candidates, final argmax
+    const bool gathers = p.gather_logits && p.world > 1;
+    if (gathers) {
+        for (int pr = 0; pr < p.world; ++pr) {
+            float *dst = reinterpret_cast<float *>(X.sym[pr] + p.lay.gather_off) +
+                         (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab;
+            for_rows([&](int tok, int row, int i) { dst[(size_t)tok * p.lay.max_vocab + A.vocab_row0 + row] = value(tok, i); });
+        }
+    } else if (A.logits != nullptr) {  // a lone rank's rows are final where they are
+        for_rows([&](int tok, int row, int i) { A.logits[(size_t)tok * p.vocab + A.vocab_row0 + row] = value(tok, i); });
+    }
+    for (int tok = warp; tok < p.m; tok += CW) {  // a warp per token
+        float bv = -INFINITY;
+        uint32_t bi = 0xFFFFFFFFu;
+        for (int i = lane; i < count; i += 32) {
+            if (row_of(i) < 0) continue;
+            const float v = value(tok, i);
+            const uint32_t idx = (uint32_t)(A.vocab_row0 + row_of(i));
+            if (v > -INFINITY && cand_better(v, idx, bv, bi)) { bv = v; bi = idx; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+            if (cand_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+        }
+        if (lane < p.world) {
+            uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[lane] + p.lay.pairs_off) +
+                            (((size_t)bank * p.world + X.rank) * kMaxCtas + cta) * p.lay.max_m + tok;
+            *dst = ((uint64_t)__float_as_uint(bv) << 32) | bi;
+        }
+    }
+    consumer_bar_n<CT>();  // the st.release.sys below is cumulative over the stores this barrier ordered
+    if (tid < p.world) {
+        uint32_t *f = reinterpret_cast<uint32_t *>(X.sym[tid] + p.lay.flags_off) +
+                      ((size_t)bank * p.world + X.rank) * nflag;
+        st_release_sys(f + cta, seq);
+    }
+    const bool copies = gathers && A.logits != nullptr;
+    if (!copies && cta != 0) return;
+    // every CTA of every rank has published (its flag follows all of its stores)
+    for (int i = tid; i < p.world * ncta; i += CT)
+        wait_flag(myflags + (size_t)(i / ncta) * nflag + (i % ncta), seq, p.timeout_ns, X.status, kStatTimeoutGather);
+    consumer_bar_n<CT>();
+    if (copies) {
+        const float *gl = reinterpret_cast<const float *>(X.sym[X.rank] + p.lay.gather_off) +
+                          (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab;
+        const int64_t per = ((int64_t)p.vocab + ncta - 1) / ncta;
+        const int64_t v0 = (int64_t)cta * per, v1 = min((int64_t)p.vocab, v0 + per);
+        for (int tok = 0; tok < p.m; ++tok)
+            for (int64_t v = v0 + tid; v < v1; v += CT)
+                A.logits[(size_t)tok * p.vocab + v] = __ldcg(gl + (size_t)tok * p.lay.max_vocab + v);
+    }
+    if (cta == 0 && A.argmax != nullptr) {
+        const uint64_t *pairs = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.pairs_off) +
+                                (size_t)bank * p.world * kMaxCtas * p.lay.max_m;
+        for (int tok = warp; tok < p.m; tok += CW) {
+            float bv = -INFINITY;
+            uint32_t bi = 0xFFFFFFFFu;
+            for (int i = lane; i < p.world * ncta; i += 32) {
+                const uint64_t pr = ld_volatile_u64(pairs + ((size_t)(i / ncta) * kMaxCtas + (i % ncta)) * p.lay.max_m + tok);
+                const float v = __uint_as_float((uint32_t)(pr >> 32));
+                const uint32_t idx = (uint32_t)pr;
+                if (cand_better(v, idx, bv, bi)) { bv = v; bi = idx; }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+                const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (cand_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+            }
+            if (lane == 0) A.argmax[tok] = (bi == 0xFFFFFFFFu) ? 0u : bi;
+        }
+    }
+}
+
 __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
 
-    constexpr int CW = fp8_consumer_warps(GT), CT = CW * 32;  // consumer warps / threads of this formulation
+    constexpr int CW = kConsumerWarps, CT = kConsumerThreads;
     const int vr = blockIdx.y, cta = blockIdx.x, ncta = gridDim.x;
     const Fp8RankArgs &A = p.r[vr];
     const RankCtx &X = A.ctx;
@@ -154,7 +252,7 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
     // stage always carries 16-32 KB: one box column = tpad rows x 128 bytes.
     auto tpad = [](int cnt) { return cnt > 8 ? 16 : cnt > 4 ? 8 : cnt > 2 ? 4 : cnt > 1 ? 2 : 1; };
 
-    const Fp8Smem S = fp8_smem_layout(p.nstages, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows, GT);
+    const Fp8Smem S = fp8_smem_layout(p.nstages, kbox, p.mp, p.nslot_max, p.skb, p.m, p.part_rows);
     uint8_t *q_s = smem + S.q;
     float *sa_s = reinterpret_cast<float *>(smem + S.sa);
     float *sw_s = reinterpret_cast<float *>(smem + S.sw);
@@ -173,22 +271,12 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
     }
     __syncthreads();
 
-    const int nflag = kMaxCtas + kMaxShared;
     // Let the next kernel on the stream begin (it only prefetches weights until its own wait).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp == CW) {
         // ------------------------------------------------------------ TMA producer warp
         RingPos rp;
-        int issued = 0;
-        bool prefetched = !p.l2_prefetch;
-        auto prefetch_rest = [&]() {  // every row of this CTA after its first tile, one request per row
-            for (int t = 1; t < ntile; ++t)
-                for (int r = lane; r < tcnt(t); r += 32)
-                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
-                                 ::"l"(p.w[vr] + (size_t)(trow(t) + r) * (size_t)p.ldw[vr]), "r"((uint32_t)(p.k & ~15)) : "memory");
-            prefetched = true;
-        };
         for (int t = 0; t < ntile; ++t) {
             const int r0 = trow(t), cnt = tcnt(t);
             const int pad = tpad(cnt), cols = p.stage_bytes / (pad * 128);  // box columns one stage holds
@@ -208,10 +296,8 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
                     }
                 }
                 rp.next(NS);
-                if (!prefetched && ++issued >= NS) prefetch_rest();
             }
         }
-        if (!prefetched) prefetch_rest();
         return;
     }
 
@@ -221,7 +307,6 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
     // which are static, and does not wait.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t seq = step_begin(X);
-    const uint32_t bank = seq & 1u;
     // Prologue: weight scales of the rows this CTA touches (loads issued first, stored last, so
     // their latency overlaps the activation loads), then the activation quantisation.
     // q_s[kb][tok][32] holds E4M3 bytes, sa_s[kb][tok(sast)] the block scale 2^e.
@@ -279,16 +364,8 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
                 act_quant8(v[u], e, lo, hi);
                 if (c < total) {
                     const int kb = ch[u] >> 2;
-                    if constexpr (GT > 0) {  // f16 copies of the quantised values (exact)
-                        uint4 hv = make_uint4(0u, 0u, 0u, 0u);
-                        if (valid[u])
-                            hv = make_uint4(e4m3x2_to_f16x2(lo), e4m3x2_to_f16x2(lo >> 16), e4m3x2_to_f16x2(hi),
-                                            e4m3x2_to_f16x2(hi >> 16));
-                        *reinterpret_cast<uint4 *>(q_s + ((size_t)tok[u] * chunks_per_row + ch[u]) * 16) = hv;
-                    } else {
-                        *reinterpret_cast<uint2 *>(q_s + ((size_t)(kb * p.mp + tok[u]) * 32 + (ch[u] & 3) * 8)) =
-                            valid[u] ? make_uint2(lo, hi) : make_uint2(0u, 0u);
-                    }
+                    *reinterpret_cast<uint2 *>(q_s + ((size_t)(kb * p.mp + tok[u]) * 32 + (ch[u] & 3) * 8)) =
+                        valid[u] ? make_uint2(lo, hi) : make_uint2(0u, 0u);
                     if ((ch[u] & 3) == 0) sa_s[kb * sast + tok[u]] = valid[u] ? pow2_f32(e) : 0.0f;
                 }
             }
@@ -306,7 +383,6 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
     const int lm_row = (lane & 7) + ((lane >> 3) & 1) * 8;  // ldmatrix source row of this lane
     const int lm_hi = lane >> 4;                            // 0: k 0..15 of the block, 1: k 16..31
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    int item = 0;
     RingPos rp;
     int redbuf = 0;
 
@@ -365,7 +441,6 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(empty0 + s * 8);
-        ++item;
         rp.next(NS);
     };
     // Sum the consumer warps' accumulators in warp order; thread t < 128 ends with
@@ -388,248 +463,39 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
         return v;
     };
 
-    // ---- CUDA-core formulation.  Lane = (row 4j + rsub of the tile, 16-byte chunk cch of the box);
-    // accv[tok][j] collects this lane's share of row 4j + rsub over every box its warp visits.
-    // Weights become f16 pairs, the activations are kept as f16 pairs, their exact products are
-    // summed in fp32 by mixed-precision FMAs (measured: 45 weight bytes per clock and SM, against
-    // 31 with conversions to f32 and packed fp32 FMAs), and the block scale multiplies each
-    // 16-element partial sum.
-    constexpr int GTn = GT > 0 ? GT : 1;
-    float accv[GTn][4];
-    const int rsub = lane >> 3, cch = lane & 7;
-    // whole tiles: row 4j + rsub sits at j * 512 + its swizzled chunk; the swizzle phase (row & 7)
-    // only depends on the parity of j
-    const uint32_t off_e = (uint32_t)(rsub * 128 + ((cch ^ rsub) << 4));
-    const uint32_t off_o = (uint32_t)((rsub + 4) * 128 + ((cch ^ rsub ^ 4) << 4));
-    auto dot16 = [&](const uint4 w, const uint32_t (&xh)[GTn][8], const float (&f)[GTn], int j) {
-        const uint32_t h0 = e4m3x2_half_to_f16x2<0>(w.x), h1 = e4m3x2_half_to_f16x2<1>(w.x);
-        const uint32_t h2 = e4m3x2_half_to_f16x2<0>(w.y), h3 = e4m3x2_half_to_f16x2<1>(w.y);
-        const uint32_t h4 = e4m3x2_half_to_f16x2<0>(w.z), h5 = e4m3x2_half_to_f16x2<1>(w.z);
-        const uint32_t h6 = e4m3x2_half_to_f16x2<0>(w.w), h7 = e4m3x2_half_to_f16x2<1>(w.w);
-#pragma unroll
-        for (int tk = 0; tk < GTn; ++tk) {
-            float s0 = 0.0f, s1 = 0.0f;
-            fma2_f16(s0, h0, xh[tk][0]); fma2_f16(s1, h1, xh[tk][1]);
-            fma2_f16(s0, h2, xh[tk][2]); fma2_f16(s1, h3, xh[tk][3]);
-            fma2_f16(s0, h4, xh[tk][4]); fma2_f16(s1, h5, xh[tk][5]);
-            fma2_f16(s0, h6, xh[tk][6]); fma2_f16(s1, h7, xh[tk][7]);
-            accv[tk][j] = fmaf(s0 + s1, f[tk], accv[tk][j]);
-        }
-    };
-    auto run_item_gemv = [&](int b0, int nb, int slot, int pad) {
-        const int s = rp.s;
-        const bool landed = mbar_wait(full0 + s * 8, rp.ph, X.status);  // false: a wait gave up, the step is void
-        const uint32_t sbase = stage0 + s * p.stage_bytes;
-        const uint32_t swrow = smem_u32(sw_s) + (uint32_t)(slot * p.skb * 4);
-        const uint32_t xbase = smem_u32(q_s) + (uint32_t)(cch * 32);
-        for (int bi = warp; bi < nb && landed; bi += CW) {
-            const int box = b0 + bi;
-            const int kb = box * 4 + (cch >> 1);  // the 32-wide K block of this lane's chunk
-            const float sw = kb < kb32 ? lds_f32(swrow + (uint32_t)(((kofs + kb * 32) >> p.bk_shift) * 4)) : 0.0f;
-            uint32_t xh[GTn][8];
-            float f[GTn];
-#pragma unroll
-            for (int tk = 0; tk < GTn; ++tk) {
-                const uint32_t xa = xbase + (uint32_t)((tk * kbox + box) * 256);
-                const uint4 x0 = lds_u128(xa), x1 = lds_u128(xa + 16);
-                xh[tk][0] = x0.x; xh[tk][1] = x0.y; xh[tk][2] = x0.z; xh[tk][3] = x0.w;
-                xh[tk][4] = x1.x; xh[tk][5] = x1.y; xh[tk][6] = x1.z; xh[tk][7] = x1.w;
-                f[tk] = kb < kb32 ? lds_f32(smem_u32(sa_s) + (uint32_t)((kb * sast + tk) * 4)) * sw : 0.0f;
-            }
-            const uint32_t bbase = sbase + bi * pad * 128;
-            if (pad == kGroupRows) {  // whole tile: four rows per lane, straight-line
-                const uint4 wa = lds_u128(bbase + off_e), wb = lds_u128(bbase + off_o);
-                const uint4 wc = lds_u128(bbase + 1024 + off_e), wd = lds_u128(bbase + 1024 + off_o);
-                dot16(wa, xh, f, 0);
-                dot16(wb, xh, f, 1);
-                dot16(wc, xh, f, 2);
-                dot16(wd, xh, f, 3);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (4 * j < pad) {  // warp-uniform: rows the stage holds
-                        const int r = 4 * j + rsub;
-                        dot16(lds_u128(bbase + r * 128 + ((uint32_t)(cch ^ ((bi * pad + r) & 7)) << 4)), xh, f, j);
-                    }
-                }
-            }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(empty0 + s * 8);
-        ++item;
-        rp.next(NS);
-    };
-    // Combine the eight lanes of each row, then the warps in warp order (same result layout as
-    // reduce_warps: thread t < 128 ends with row t & 15 of token t >> 4).
-    auto reduce_gemv = [&]() -> float {
-        float *rb = red_s + (redbuf * CW + warp) * 128;
-#pragma unroll
-        for (int tk = 0; tk < GTn; ++tk)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float v = accv[tk][j];
-                v += __shfl_xor_sync(0xffffffffu, v, 1);
-                v += __shfl_xor_sync(0xffffffffu, v, 2);
-                v += __shfl_xor_sync(0xffffffffu, v, 4);
-                if (cch == 0) rb[tk * 16 + 4 * j + rsub] = v;
-            }
-        consumer_bar_n<CT>();
-        float v = 0.0f;
-        if (tid < 16 * GTn) {
-            const float *r0 = red_s + redbuf * CW * 128 + tid;
-            v = r0[0];
-#pragma unroll
-            for (int w = 1; w < CW; ++w) v += r0[w * 128];
-        }
-        redbuf ^= 1;
-        return v;
-    };
-
     const int row_t = tid & 15, tok_t = tid >> 4;  // meaningful for tid < 128
-    const bool solo = (p.mode == kModeAllReduce && p.world == 1);
     const int PR = p.part_rows;
 
     for (int t = 0; t < ntile; ++t) {
         const int slot = slot_of(t);
         const int pad = tpad(tcnt(t)), cols = p.stage_bytes / (pad * 128);
-        float v;
-        if constexpr (GT > 0) {
-#pragma unroll
-            for (int tk = 0; tk < GTn; ++tk) accv[tk][0] = accv[tk][1] = accv[tk][2] = accv[tk][3] = 0.0f;
-            for (int b0 = 0; b0 < kbox; b0 += cols) run_item_gemv(b0, min(cols, kbox - b0), slot, pad);
-            v = reduce_gemv();
-        } else {
-            acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
-            for (int b0 = 0; b0 < kbox; b0 += cols) run_item(b0, min(cols, kbox - b0), slot, pad);
-            if (wide) {  // the accumulator fragment is final: rows g, g + 8 x tokens 8 tg + 2 tq, + 1
-                const int tk0 = tg * 8 + 2 * tq;
-                if (tk0 < p.m) {
-                    part_s[tk0 * PR + t * kGroupRows + g] = acc[0];
-                    part_s[tk0 * PR + t * kGroupRows + g + 8] = acc[2];
-                }
-                if (tk0 + 1 < p.m) {
-                    part_s[(tk0 + 1) * PR + t * kGroupRows + g] = acc[1];
-                    part_s[(tk0 + 1) * PR + t * kGroupRows + g + 8] = acc[3];
-                }
-                continue;
+        acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
+        for (int b0 = 0; b0 < kbox; b0 += cols) run_item(b0, min(cols, kbox - b0), slot, pad);
+        if (wide) {  // the accumulator fragment is final: rows g, g + 8 x tokens 8 tg + 2 tq, + 1
+            const int tk0 = tg * 8 + 2 * tq;
+            if (tk0 < p.m) {
+                part_s[tk0 * PR + t * kGroupRows + g] = acc[0];
+                part_s[tk0 * PR + t * kGroupRows + g + 8] = acc[2];
             }
-            v = reduce_warps();
+            if (tk0 + 1 < p.m) {
+                part_s[(tk0 + 1) * PR + t * kGroupRows + g] = acc[1];
+                part_s[(tk0 + 1) * PR + t * kGroupRows + g + 8] = acc[3];
+            }
+            continue;
         }
+        const float v = reduce_warps();
         if (tid < 128 && tok_t < p.m) part_s[tok_t * PR + t * kGroupRows + row_t] = v;
     }
     consumer_bar_n<CT>();  // part_s complete
 
-    // Visit every (token, valid row) of this CTA: fn(tok, global row, value index in part_s).
-    auto for_rows = [&](auto fn) {
-        for (int i = tid; i < ntile * p.m * kGroupRows; i += CT) {
-            const int t = i / (p.m * kGroupRows), j = i - t * (p.m * kGroupRows);
-            const int tok = j >> 4, r = j & 15;
-            if (r < tcnt(t)) fn(tok, trow(t) + r, tok * PR + t * kGroupRows + r);
-        }
-    };
-
-    if (solo) {
-        for_rows([&](int tok, int row, int pi) { A.out[(size_t)tok * p.n + row] = part_s[pi]; });
-        return;
-    }
-    const uint32_t *myflags = reinterpret_cast<const uint32_t *>(X.sym[X.rank] + p.lay.flags_off) +
-                              (size_t)bank * p.world * nflag;
-
-    if (p.mode == kModeAllReduce) {
-        // every thread sends its rows' partials to all ranks as tagged words, then folds the same
-        // rows in rank order as the ranks' words arrive: no barrier, fence or flag in between
-        const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
-        for (int pr = 0; pr < p.world; ++pr) {
-            uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride;
-            for_rows([&](int tok, int row, int pi) { st_word_sys(dst + (size_t)tok * p.n + row, seq, part_s[pi]); });
-        }
-        const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) +
-                                (size_t)bank * p.world * astride;
-        for_rows([&](int tok, int row, int) {
-            const size_t off = (size_t)tok * p.n + row;
-            A.out[off] = fold_words(slots, astride, off, p.world, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
-        });
-        return;
-    }
-
-    // ---- lm_head: gather rows, publish candidates, final argmax
-    if (p.gather_logits) {
-        for (int pr = 0; pr < p.world; ++pr) {
-            float *dst = reinterpret_cast<float *>(X.sym[pr] + p.lay.gather_off) +
-                         (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab;
-            for_rows([&](int tok, int row, int pi) { dst[(size_t)tok * p.lay.max_vocab + A.vocab_row0 + row] = part_s[pi]; });
-        }
-    }
-    for (int tok = warp; tok < p.m; tok += CW) {  // a warp per token
-        float bv = -INFINITY;
-        uint32_t bi = 0xFFFFFFFFu;
-        for (int i = lane; i < ntile * kGroupRows; i += 32) {
-            const int t = i >> 4, r = i & 15;
-            if (r >= tcnt(t)) continue;
-            const float v = part_s[tok * PR + i];
-            const uint32_t idx = (uint32_t)(A.vocab_row0 + trow(t) + r);
-            if (v > -INFINITY && cand_better(v, idx, bv, bi)) { bv = v; bi = idx; }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (cand_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-        }
-        if (lane < p.world) {
-            uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[lane] + p.lay.pairs_off) +
-                            (((size_t)bank * p.world + X.rank) * kMaxCtas + cta) * p.lay.max_m + tok;
-            *dst = ((uint64_t)__float_as_uint(bv) << 32) | bi;
-        }
-    }
-    consumer_bar_n<CT>();  // the st.release.sys below is cumulative over the stores this barrier ordered
-    if (tid < p.world) {
-        uint32_t *f = reinterpret_cast<uint32_t *>(X.sym[tid] + p.lay.flags_off) +
-                      ((size_t)bank * p.world + X.rank) * nflag;
-        st_release_sys(f + cta, seq);
-    }
-    const bool copies = p.gather_logits && A.logits != nullptr;
-    if (!copies && cta != 0) return;
-    // every CTA of every rank has published (its flag follows all of its stores)
-    for (int i = tid; i < p.world * ncta; i += CT)
-        wait_flag(myflags + (size_t)(i / ncta) * nflag + (i % ncta), seq, p.timeout_ns, X.status, kStatTimeoutGather);
-    consumer_bar_n<CT>();
-    if (copies) {
-        const float *gl = reinterpret_cast<const float *>(X.sym[X.rank] + p.lay.gather_off) +
-                          (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab;
-        const int64_t per = ((int64_t)p.vocab + ncta - 1) / ncta;
-        const int64_t v0 = (int64_t)cta * per, v1 = min((int64_t)p.vocab, v0 + per);
-        for (int tok = 0; tok < p.m; ++tok)
-            for (int64_t v = v0 + tid; v < v1; v += CT)
-                A.logits[(size_t)tok * p.vocab + v] = __ldcg(gl + (size_t)tok * p.lay.max_vocab + v);
-    }
-    if (cta == 0 && A.argmax != nullptr) {
-        const uint64_t *pairs = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.pairs_off) +
-                                (size_t)bank * p.world * kMaxCtas * p.lay.max_m;
-        for (int tok = warp; tok < p.m; tok += CW) {
-            float bv = -INFINITY;
-            uint32_t bi = 0xFFFFFFFFu;
-            for (int i = lane; i < p.world * ncta; i += 32) {
-                const uint64_t pr = ld_volatile_u64(pairs + ((size_t)(i / ncta) * kMaxCtas + (i % ncta)) * p.lay.max_m + tok);
-                const float v = __uint_as_float((uint32_t)(pr >> 32));
-                const uint32_t idx = (uint32_t)pr;
-                if (cand_better(v, idx, bv, bi)) { bv = v; bi = idx; }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (cand_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-            }
-            if (lane == 0) A.argmax[tok] = (bi == 0xFFFFFFFFu) ? 0u : bi;
-        }
-    }
+    fp8_finish<CT>(p, A, X, seq, tid, ntile * kGroupRows,
+                   [&](int i) { const int t = i >> 4, r = i & 15; return r < tcnt(t) ? trow(t) + r : -1; },
+                   [&](int tok, int i) { return part_s[tok * PR + i]; });
 }
 
-template <int GT>
-__global__ void __launch_bounds__(fp8_threads(GT), 1) fp8_rowpar_kernel(const __grid_constant__ Fp8Params p) {
+__global__ void __launch_bounds__(kThreads, 1) fp8_rowpar_kernel(const __grid_constant__ Fp8Params p) {
     const RankCtx &X = p.r[blockIdx.y].ctx;
-    fp8_rowpar_kernel_body<GT>(p);
+    fp8_rowpar_kernel_body(p);
     if (p.world > 1 || p.mode == kModeLmHead) {  // a lone all-reduce rank exchanges nothing
         // step_begin again: the value is unchanged until the last CTA publishes the next one below
         step_end(X, step_begin(X), gridDim.x);

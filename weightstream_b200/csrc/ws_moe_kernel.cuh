@@ -85,11 +85,6 @@ __device__ __forceinline__ void fp4x8_to_e4m3(uint32_t w, uint32_t &even, uint32
     even = ((w << 2) & 0x1C1C1C1Cu) | ((w << 4) & 0x80808080u);
     odd = ((w >> 2) & 0x1C1C1C1Cu) | (w & 0x80808080u);
 }
-__device__ __forceinline__ float e8m0_f32(uint32_t b) {
-    return (b == 0xFFu) ? __uint_as_float(0x7FC00000u)
-                        : (b == 0u ? __uint_as_float(0x00400000u) : __uint_as_float(b << 23));
-}
-
 __device__ __forceinline__ void moe_down_body(const MoeParams &p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
