@@ -656,31 +656,34 @@ struct GemvPlan {
 static GemvPlan gemv_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta) {
     GemvPlan u{};
     if (mt > 2) return u;
-    // A lane keeps C 16-byte chunks of K of every token in registers: as many as fit beside the loads in
-    // flight with two CTAs per SM, more only when eight slices do not cover K.
+    // A lane keeps C 16-byte chunks of K of every token in registers: one, unless eight slices do not cover K
+    // (K/rank 1024 and 2048: 3.9 and 5.8 us per step with one chunk, 4.4 and 6.2 with two).
     const int q = (a.k + 511) / 512;  // 512 bytes: one chunk of every lane
     u.chunks = 1;
-    while (u.chunks < q && u.chunks * mt < 4) u.chunks *= 2;
     while ((q + u.chunks - 1) / u.chunks > kGemvMaxSlices) u.chunks *= 2;
     if (u.chunks * mt > 8) return u;
     u.slices = (q + u.chunks - 1) / u.chunks;
     const int groups = kConsumerWarps / u.slices;
     u.rows_max = (a.n + ncta - 1) / ncta;
-    const int target = getenv("X2") ? atoi(getenv("X2")) * 1024 : 32 * 1024;
-    const int per = 2 * groups;  // rows one turn of every warp takes
-    u.rows_per_stage = std::min(32, std::max(1, target / a.k));
+    const int per = 4 * groups;  // rows one turn of every warp takes
+    u.rows_per_stage = std::min(32, std::max(1, 32 * 1024 / a.k));
     if (u.rows_per_stage > per) u.rows_per_stage = u.rows_per_stage / per * per;
     u.rows_per_stage = std::min(u.rows_per_stage, u.rows_max);
     u.stage_bytes = (int)align_up((int64_t)u.rows_per_stage * a.k, 128);
     u.nslot_max = (u.rows_max + a.block_n - 2) / a.block_n + 1;
     const int items = (u.rows_max + u.rows_per_stage - 1) / u.rows_per_stage;
     auto total = [&](int ns) { return fp8_gemv_smem(ns, u.stage_bytes, u.nslot_max, skb, mt, u.slices, u.rows_max).total; };
-    const int budget = getenv("X1") && atoi(getenv("X1")) ? kHalfSmemBudget : kSmemBudget;
-    int ns = std::min((int)kMaxStages, items);
-    while (ns >= 2 && total(ns) > budget) --ns;
-    u.nstages = ns;
-    u.ok = (ns >= 2 || ns == items) && total(ns) <= budget;
-    u.smem = (size_t)total(ns);
+    // Half an SM whenever that holds three stages: the next step's CTA is then resident beside this one and
+    // its ring is full when this one ends (K/rank 8192, one row: 13.2 us per step and 22.9 alone; with the
+    // whole SM 13.7 and 25.9).
+    for (int half = 1; half >= 0; --half) {
+        const int budget = half ? kHalfSmemBudget : kSmemBudget;
+        u.nstages = std::min((int)kMaxStages, items);
+        while (u.nstages > 1 && total(u.nstages) > budget) --u.nstages;
+        u.ok = (u.nstages >= (half ? 3 : 2) || u.nstages == items) && total(u.nstages) <= budget;
+        if (u.ok) break;
+    }
+    u.smem = (size_t)total(u.nstages);
     return u;
 }
 

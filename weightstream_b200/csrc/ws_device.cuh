@@ -250,6 +250,21 @@ __device__ __forceinline__ void fma2_f16(float &s, uint32_t a, uint32_t b) {
         : "+f"(s) : "r"(a), "r"(b));
 }
 
+// Four per-lane partial sums (one per row) -> their 32-lane sums: lanes are folded 4 -> 2 -> 1
+// values per lane, then three plain steps (6 shuffles instead of 20).  The lane with
+// (lane & 7) == 0 ends with the sum of row 2 * bit4(lane) + bit3(lane).
+__device__ __forceinline__ float fold4(const float (&v)[4], bool hi16, bool hi8) {
+    float k0 = hi16 ? v[2] : v[0], k1 = hi16 ? v[3] : v[1];
+    k0 += __shfl_xor_sync(0xffffffffu, hi16 ? v[0] : v[2], 16);
+    k1 += __shfl_xor_sync(0xffffffffu, hi16 ? v[1] : v[3], 16);
+    float k = hi8 ? k1 : k0;
+    k += __shfl_xor_sync(0xffffffffu, hi8 ? k0 : k1, 8);
+    k += __shfl_xor_sync(0xffffffffu, k, 4);
+    k += __shfl_xor_sync(0xffffffffu, k, 2);
+    k += __shfl_xor_sync(0xffffffffu, k, 1);
+    return k;
+}
+
 template <int N>
 __device__ __forceinline__ void consumer_bar_n() {  // the N consumer threads only
     asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory");

@@ -10,8 +10,8 @@
 // (crates/weightstream-ref/src/actquant.rs:21-57), so no shared memory, barrier or other warp stands
 // between the predecessor's end and the first product.  Per row and chunk: one conflict-free 128-bit
 // shared load, 8 conversions to f16 pairs, 16 mixed-precision FMAs with exact products
-// (fma.rn.f32.f16), one FMA with the product of the block scales; two rows' sums are folded over the
-// lanes by five shuffles.  Slices meet once, after the last row, in slice order.
+// (fma.rn.f32.f16), one FMA with the product of the block scales; four rows are in flight at a time and
+// their sums are folded over the lanes by six shuffles.  Slices meet once, after the last row, in slice order.
 //
 // Bound: HBM for large shards, the dependency latency between steps for small ones.
 #pragma once
@@ -152,72 +152,66 @@ __device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
     const bool solo = p.mode == kModeAllReduce && p.world == 1;
     const uint32_t seq = solo ? 0u : step_begin(X);
 
+    // byte offset of each chunk inside a row; lanes past the end of K read the row's first chunk and multiply
+    // it by zero (a NaN there is in the row's sum anyway)
+    uint32_t off[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) off[i] = live[i] ? (uint32_t)(((slice * C + i) * 32 + lane) * 16) : 0u;
+    const bool hi16 = (lane & 16) != 0, hi8 = (lane & 8) != 0;
+    const int jrow = (hi16 ? 2 : 0) + (hi8 ? 1 : 0);  // the row of four whose sum fold4 leaves on this lane
+    auto block_of = [&](int row) { return (int)(((A.row0 + row_a + row) >> p.bn_shift) - srow_lo); };
     float f[GT][C];
     int blk = -1;  // scale row the factors f are for
-    auto factors = [&](int row) {
-        const int b = (int)(((A.row0 + row_a + row) >> p.bn_shift) - srow_lo);
-        if (b == blk) return;
-        blk = b;
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            const float sw = sw_s[b * p.skb + swc[i]];
-#pragma unroll
-            for (int t = 0; t < GT; ++t) f[t][i] = sa[t][i] * sw;
-        }
-    };
-    auto dot = [&](const uint4 (&w)[C], float (&acc)[GT]) {
-#pragma unroll
-        for (int t = 0; t < GT; ++t) acc[t] = 0.0f;
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
-            uint32_t h[8];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                h[2 * q] = e4m3x2_half_to_f16x2<0>(ww[q]);
-                h[2 * q + 1] = e4m3x2_half_to_f16x2<1>(ww[q]);
-            }
-#pragma unroll
-            for (int t = 0; t < GT; ++t) {
-                float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    fma2_f16(s0, h[2 * q], xh[t][i][2 * q]);
-                    fma2_f16(s1, h[2 * q + 1], xh[t][i][2 * q + 1]);
-                }
-                acc[t] = fmaf(s0 + s1, f[t][i], acc[t]);
-            }
-        }
-    };
-    const uint32_t lane_off = (uint32_t)((slice * C * 32 + lane) * 16);
-    auto load_row = [&](uint32_t rbase, uint4 (&w)[C]) {
-#pragma unroll
-        for (int i = 0; i < C; ++i) w[i] = live[i] ? lds_u128(rbase + lane_off + i * 512) : make_uint4(0u, 0u, 0u, 0u);
-    };
-    const bool hi = (lane & 16) != 0;
     RingPos rp;
     for (int it = 0; it < items; ++it, rp.next(NS)) {
         const int s = rp.s, r0 = it * R, nr = min(R, rows - r0);
         const bool landed = mbar_wait(full0 + s * 8, rp.ph, X.status);  // false: a wait gave up, the step is void
         const uint32_t sbase = stage0 + s * p.stage_bytes;
-        if (landed && grp < G) {
-            for (int r = grp; r < nr; r += 2 * G) {  // two rows at a time
-                const int r2 = r + G;
-                const bool two = r2 < nr;  // warp-uniform
-                uint4 wa[C], wb[C];
-                load_row(sbase + r * p.k, wa);
-                load_row(sbase + (two ? r2 : r) * p.k, wb);
-                float va[GT], vb[GT];
-                factors(r0 + r);
-                dot(wa, va);
-                if (two) factors(r0 + r2);
-                dot(wb, vb);
+        for (int r = grp; r < nr && landed && grp < G; r += 4 * G) {  // four rows at a time: r, r + G, r + 2G, r + 3G
+            uint32_t ra[4];
 #pragma unroll
-                for (int t = 0; t < GT; ++t) {  // lanes 0-15 end with row r, lanes 16-31 with row r2
-                    float v = (hi ? vb[t] : va[t]) + __shfl_xor_sync(0xffffffffu, hi ? va[t] : vb[t], 16);
+            for (int j = 0; j < 4; ++j) ra[j] = sbase + min(r + j * G, nr - 1) * p.k;
+            const int mine = r + jrow * G, b_last = block_of(r0 + min(r + 3 * G, nr - 1));
+            // once, or once more for each further scale row that the four rows reach into
+            for (int b = block_of(r0 + r); b <= b_last; ++b) {
+                if (b != blk) {
+                    blk = b;
 #pragma unroll
-                    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                    if ((lane & 15) == 0 && (!hi || two)) part_s[(t * S + slice) * p.rows_max + r0 + (hi ? r2 : r)] = v;
+                    for (int i = 0; i < C; ++i) {
+                        const float sw = sw_s[b * p.skb + swc[i]];
+#pragma unroll
+                        for (int t = 0; t < GT; ++t) f[t][i] = sa[t][i] * sw;
+                    }
+                }
+                float acc[GT][4];
+#pragma unroll
+                for (int i = 0; i < C; ++i) {
+                    uint4 w[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) w[j] = lds_u128(ra[j] + off[i]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t ww[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
+                        float s0[GT], s1[GT];
+#pragma unroll
+                        for (int t = 0; t < GT; ++t) s0[t] = s1[t] = 0.0f;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const uint32_t h0 = e4m3x2_half_to_f16x2<0>(ww[q]), h1 = e4m3x2_half_to_f16x2<1>(ww[q]);
+#pragma unroll
+                            for (int t = 0; t < GT; ++t) {
+                                fma2_f16(s0[t], h0, xh[t][i][2 * q]);
+                                fma2_f16(s1[t], h1, xh[t][i][2 * q + 1]);
+                            }
+                        }
+#pragma unroll
+                        for (int t = 0; t < GT; ++t) acc[t][j] = i == 0 ? (s0[t] + s1[t]) * f[t][i] : fmaf(s0[t] + s1[t], f[t][i], acc[t][j]);
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < GT; ++t) {
+                    const float v = fold4(acc[t], hi16, hi8);
+                    if ((lane & 7) == 0 && mine < nr && block_of(r0 + mine) == b) part_s[(t * S + slice) * p.rows_max + r0 + mine] = v;
                 }
             }
         }

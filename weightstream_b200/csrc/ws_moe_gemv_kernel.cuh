@@ -245,21 +245,6 @@ __device__ __forceinline__ void dot32_e2m1(const uint4 w, const uint32_t (&xa)[1
     db = b0 + b1;
 }
 
-// Four per-lane partial sums (one per row) -> their 32-lane sums: lanes are folded 4 -> 2 -> 1
-// values per lane, then three plain steps (6 shuffles instead of 20).  The lane with
-// (lane & 7) == 0 ends with the sum of row 2 * bit4(lane) + bit3(lane).
-__device__ __forceinline__ float fold4(const float (&v)[4], bool hi16, bool hi8) {
-    float k0 = hi16 ? v[2] : v[0], k1 = hi16 ? v[3] : v[1];
-    k0 += __shfl_xor_sync(0xffffffffu, hi16 ? v[0] : v[2], 16);
-    k1 += __shfl_xor_sync(0xffffffffu, hi16 ? v[1] : v[3], 16);
-    float k = hi8 ? k1 : k0;
-    k += __shfl_xor_sync(0xffffffffu, hi8 ? k0 : k1, 8);
-    k += __shfl_xor_sync(0xffffffffu, k, 4);
-    k += __shfl_xor_sync(0xffffffffu, k, 2);
-    k += __shfl_xor_sync(0xffffffffu, k, 1);
-    return k;
-}
-
 __device__ __forceinline__ void moe_gemv_body(const MoeGemvParams &p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
