@@ -128,6 +128,25 @@ ws_status_t make_tmap(ws_tp *tp, CUtensorMap *map, const void *base, uint64_t ro
     return WS_OK;
 }
 
+// The same matrix as [whole 128-byte slabs of K][rows][128 bytes]: one box carries `slabs` slabs of box_rows rows,
+// slab after slab, each in the layout of make_tmap's box (box_rows a multiple of 8 keeps the swizzle's phase).
+ws_status_t make_tmap_slabs(ws_tp *tp, CUtensorMap *map, const void *base, uint64_t rows, uint64_t whole_slabs, uint64_t ld,
+                            uint32_t box_rows, uint32_t slabs) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return fail(tp, WS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld & 15))
+        return fail(tp, WS_ERR_INVALID, "weight base and row stride must be multiples of 16 bytes");
+    cuuint64_t dims[3] = {128, rows, whole_slabs};
+    cuuint64_t strides[2] = {ld, 128};
+    cuuint32_t box[3] = {128, box_rows, slabs};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(tp, WS_ERR_CUDA, "cuTensorMapEncodeTiled (slabs) failed (%d)", (int)r);
+    return WS_OK;
+}
+
 // Expert slab [experts][rows][k] of packed 4-bit codes (row stride k/2 bytes), boxes of 128 codes x
 // box_rows x 1 expert; the copy unpacks 16 codes (8 bytes) into 16 bytes of shared memory, the form
 // tcgen05.mma.kind::mxf8f6f4 reads 4-bit operands in; 128B swizzle.
@@ -301,8 +320,8 @@ ws_status_t ws_tp_create(int32_t world, int32_t rank, int32_t device, const ws_t
         set_smem(tp, fp8_gemv_kernel<1, 4>) != WS_OK || set_smem(tp, fp8_gemv_kernel<1, 8>) != WS_OK ||
         set_smem(tp, fp8_gemv_kernel<2, 1>) != WS_OK || set_smem(tp, fp8_gemv_kernel<2, 2>) != WS_OK ||
         set_smem(tp, fp8_gemv_kernel<2, 4>) != WS_OK || set_smem(tp, moe_down_kernel) != WS_OK ||
-        set_smem(tp, fp8_bs_kernel<16>) != WS_OK || set_smem(tp, fp8_bs_kernel<32>) != WS_OK ||
-        set_smem(tp, fp8_bs_kernel<64>) != WS_OK || set_smem(tp, fp8_bs_kernel<128>) != WS_OK || set_smem(tp, moe_bs_kernel) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<16, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<64, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, false>) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<16, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<64, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, true>) != WS_OK || set_smem(tp, moe_bs_kernel) != WS_OK ||
         cudaFuncSetAttribute(moe_bs_prep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         // The prep kernel uses no shared memory, but a main-kernel CTA (which needs almost all of an SM's)
         // cannot move onto an SM whose L1/shared split must first change, and that has to wait for the prep
@@ -440,10 +459,11 @@ static ws_status_t validate_fp8(ws_tp *tp, const ws_fp8_gemm_args_t &a, bool lm_
 }
 
 // Plan of the block-scaled tcgen05 path for one fused step; ok = false when the shape does not fit it
-// (it needs fp32 weight scales whose K blocks are whole 128-wide slabs, and k a multiple of 128).
+// (fp32 weight scales need K blocks of whole 128-wide slabs and k a multiple of 128; UE8M0 scales need
+// neither: a 32-wide scale block is the MMA's own).
 struct BsPlan {
-    bool ok;
-    int mp, tile_rows, ntiles, a_pitch, b_pitch, slabs_per_stage, nstages, nslot_max, nacc;
+    bool ok, wue;
+    int mp, ks, tile_rows, ntiles, a_pitch, x_pitch, slabs_per_stage, nstages, nslot_max, nacc;
     int csize;  // 2: CTA pairs share a tile, each CTA streams half of K (tiles of a lone CTA would fill under half of the MMA's rows)
     int ncta;   // CTAs the plan is for (even with pairs)
     int tmem_cols;  // tensor-memory columns the CTA allocates (a power of two)
@@ -451,29 +471,29 @@ struct BsPlan {
 };
 static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bool pairs_allowed) {
     BsPlan u{};
-    if (a.scale_kind != WS_SCALE_F32 || a.block_k % 128 || a.k % 128 || mt > kBsMaxTokens) return u;
+    u.wue = a.scale_kind == WS_SCALE_UE8M0;
+    if (mt > kBsMaxTokens || (!u.wue && (a.block_k % 128 || a.k % 128))) return u;
     u.mp = mt <= 16 ? 16 : mt <= 32 ? 32 : mt <= 64 ? 64 : 128;
-    // tiles of equal height that deal out evenly: a CTA's share of the rows, cut into as few pieces
-    // of at most 128 rows as possible
-    const int kslabs = a.k / 128;
+    u.ks = (a.k + 127) / 128;
     // The tensor pipe spends the same time on an MMA however few of its 128 rows are real.  When a
     // CTA's share of the rows fills under half of them, two CTAs share a tile and split K instead.
-    u.csize = (pairs_allowed && ncta >= 2 && kslabs >= 2 && (a.n + ncta - 1) / ncta <= kBsMmaRows / 2) ? 2 : 1;
+    u.csize = (pairs_allowed && ncta >= 2 && u.ks >= 2 && (a.n + ncta - 1) / ncta <= kBsMmaRows / 2) ? 2 : 1;
     u.ncta = u.csize == 2 ? ncta & ~1 : ncta;
     const int nparts = u.ncta / u.csize;
+    // tiles of equal height that deal out evenly: a CTA's share of the rows, cut into as few pieces of at
+    // most 128 rows as possible; multiples of 8, so that the slabs of one TMA box keep the swizzle's phase
     const int crmax = (a.n + nparts - 1) / nparts;
     const int pieces = (crmax + kBsMmaRows - 1) / kBsMmaRows;
-    u.tile_rows = (crmax + pieces - 1) / pieces;
+    u.tile_rows = std::min((int)kBsMmaRows, ((crmax + pieces - 1) / pieces + 7) / 8 * 8);
     u.ntiles = (a.n + u.tile_rows - 1) / u.tile_rows;
     const int tiles_per_cta = (u.ntiles + nparts - 1) / nparts;
-    u.a_pitch = (u.tile_rows + 7) / 8 * 8 * 128;
-    u.b_pitch = u.mp * 128;
-    const int slab_bytes = u.a_pitch + u.b_pitch + kBsAtomBytes;
-    // slabs per stage: one MMA commit (a ~160 ns stall of the issuing thread) per stage, so several
-    // slabs share it; bounded by the stage size and by tensor memory (each slab has its own
-    // accumulator buffer: groups x slabs x (mp + 4) + 8 columns of 512, at least two groups)
+    u.a_pitch = u.tile_rows * 128;
+    const int x_slab = u.mp * 128 + kBsAtomBytes, slab_bytes = u.a_pitch + x_slab + (u.wue ? kBsAtomBytes : 0);
+    // slabs per stage: one MMA commit (a ~160 ns stall of the issuing thread) and two copies (~100 ns each)
+    // per stage, so several slabs share it; bounded by the stage size and by tensor memory (fp32 scales: each
+    // slab has its own accumulator buffer, groups x slabs x (mp + 4) + 8 columns of 512, at least two groups)
     u.nslot_max = (tiles_per_cta * u.tile_rows) / a.block_n + 2;
-    const int rx_rows = u.csize == 2 ? mt : 0;
+    const int rx_rows = u.csize == 2 ? mt : 0, kcta = (u.ks + u.csize - 1) / u.csize;
     // Half an SM (shared memory and tensor memory) when the tokens are few and the CTA's whole share of
     // the weights fits such a ring (TP-8 shards): the next step's CTA is then resident beside this one
     // (one CTA per SM and step) and loads all of its weights under this step's exchange and exit.
@@ -483,21 +503,28 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     for (int half = small ? 1 : 0; half >= 0; --half) {
         const int budget = half ? kHalfSmemBudget : kSmemBudget, tmem = half ? 256 : 512;
         const int stage_target = half ? 32 * 1024 : 56 * 1024;
-        u.slabs_per_stage = std::max(1, std::min({4, stage_target / slab_bytes, (tmem - 8) / (2 * (u.mp + 4)), kslabs}));
-        u.nacc = std::min((int)kBsMaxAcc, (tmem - 8) / (u.slabs_per_stage * (u.mp + 4)));
+        u.slabs_per_stage = std::max(1, std::min({4, stage_target / slab_bytes, kcta, u.wue ? 4 : (tmem - 8) / (2 * (u.mp + 4))}));
+        const int groups = (kcta + u.slabs_per_stage - 1) / u.slabs_per_stage;
+        u.slabs_per_stage = (kcta + groups - 1) / groups;  // groups of equal size, so that few slabs travel outside whole boxes
+        u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * x_slab, 1024);
+        u.nacc = u.wue ? std::min(2, std::max(1, (tmem - 8 - 2 * u.slabs_per_stage * 8) / u.mp))
+                       : std::min((int)kBsMaxAcc, (tmem - 8) / (u.slabs_per_stage * (u.mp + 4)));
+        auto total = [&](int ns) {
+            return bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, u.nslot_max, skb, u.mp, rx_rows, u.wue).total + 1024;
+        };
         int ns = kMaxStages;  // the most stages whose layout fits
-        while (ns >= 2 && bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.b_pitch, u.nslot_max, skb, u.mp, rx_rows).total + 1024 > budget) --ns;
-        const int items = tiles_per_cta * ((kslabs / u.csize + u.slabs_per_stage - 1) / u.slabs_per_stage);
-        ns = std::min(ns, std::min((int)kMaxStages, std::max(2, items)));
+        while (ns >= 2 && total(ns) > budget) --ns;
+        const int items = tiles_per_cta * groups;
+        ns = std::min(ns, std::max(2, items));
         u.nstages = ns;
-        // the epilogue and the producer wait on the same per-stage barrier: the MMA thread must not get a
-        // whole lap of the stage ring ahead of the epilogue, which holds when groups <= stages
-        u.nacc = std::max(1, std::min(u.nacc, ns));
+        // fp32 scales: the epilogue and the producer wait on the same per-stage barrier: the MMA thread must not
+        // get a whole lap of the stage ring ahead of the epilogue, which holds when groups <= stages
+        if (!u.wue) u.nacc = std::max(1, std::min(u.nacc, ns));
         u.ok = ns >= 2;
         if (!u.ok || (half && items > ns)) continue;  // half an SM only when the CTA's whole share of the weights fits the ring
-        u.smem = (size_t)bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.b_pitch, u.nslot_max, skb, u.mp, rx_rows).total + 1024;
+        u.smem = (size_t)total(ns);
         int cols = 32;
-        while (cols < u.nacc * u.slabs_per_stage * (u.mp + 4) + 4) cols *= 2;
+        while (cols < (u.wue ? u.nacc * u.mp + 2 * u.slabs_per_stage * 8 : u.nacc * u.slabs_per_stage * (u.mp + 4) + 4)) cols *= 2;
         u.tmem_cols = half ? std::min(cols, 256) : 512;
         break;
     }
@@ -521,97 +548,97 @@ static ws_status_t ensure_bs_scratch(ws_tp *tp, size_t bytes) {
     return WS_OK;
 }
 
-// A tensor map over a row-major byte matrix with boxes of 128 bytes x box_rows, 128B swizzle (see make_tmap).
-// One fused step over at most 64 activation rows on the block-scaled tcgen05 path: the prep
+// A lone rank that holds only a shard of the vocabulary: the rows nobody computes read as zero.
+static ws_status_t zero_lone_shard(ws_tp *const *ranks, int n, const ws_lm_head_args_t *lm, int m0, int mt, void *const *streams) {
+    if (!lm || n != 1 || ranks[0]->world != 1 || !lm[0].logits || lm[0].g.n >= lm[0].vocab) return WS_OK;
+    WS_CUDA(ranks[0], cudaSetDevice(ranks[0]->device));
+    WS_CUDA(ranks[0], cudaMemsetAsync(lm[0].logits + (size_t)m0 * lm[0].vocab, 0, (size_t)mt * lm[0].vocab * sizeof(float),
+                                      static_cast<cudaStream_t>(streams ? streams[0] : nullptr)));
+    return WS_OK;
+}
+
+// One fused step over at most kBsMaxTokens activation rows on the block-scaled tcgen05 path: the prep
 // kernel (activation quantisation once per step) followed by the persistent MMA kernel.
 static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t *args, const ws_lm_head_args_t *lm,
-                           int m0, int mt, void *const *streams, int ncta, bool same_device, const BsPlan &u, int skb, bool last) {
+                           int m0, int mt, void *const *streams, bool same_device, const BsPlan &u, int skb, bool last) {
     ws_tp *t0 = ranks[0];
     const ws_fp8_gemm_args_t &a0 = lm ? lm[0].g : args[0];
     BsParams p{};
-    p.m = mt; p.mp = u.mp; p.n = a0.n; p.k = a0.k; p.world = t0->world;
+    p.m = mt; p.mp = u.mp; p.n = a0.n; p.k = a0.k; p.ks = u.ks; p.world = t0->world;
     for (p.bk_shift = 0; (1 << p.bk_shift) < a0.block_k; ++p.bk_shift) {}
     for (p.bn_shift = 0; (1 << p.bn_shift) < a0.block_n; ++p.bn_shift) {}
     p.mode = lm ? kModeLmHead : kModeAllReduce;
     p.vocab = lm ? lm[0].vocab : 0;
-    p.tile_rows = u.tile_rows; p.ntiles = u.ntiles; p.a_pitch = u.a_pitch; p.b_pitch = u.b_pitch;
+    p.tile_rows = u.tile_rows; p.ntiles = u.ntiles; p.a_pitch = u.a_pitch; p.x_pitch = u.x_pitch;
     p.slabs_per_stage = u.slabs_per_stage; p.nstages = u.nstages; p.nslot_max = u.nslot_max; p.skb = skb; p.nacc = u.nacc;
     p.csize = u.csize;
     p.tmem_cols = u.tmem_cols;
     // 32 rows and more on four ranks and more: all-to-all of every partial sum costs more link time than the second hop
     p.owner_reduce = (t0->world >= 4 && u.mp >= 32) ? 1 : 0;
-    ncta = u.ncta;
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
     ActPrepParams q{};
-    q.m = mt; q.mp = u.mp; q.k = a0.k; q.x_dtype = a0.x_dtype;
-    // scratch of one endpoint: quantised activations and their scale atoms
-    const size_t xq_bytes = align_up((int64_t)kBsMaxTokens * a0.k, 256), sf_bytes = (size_t)(a0.k / 128) * kBsAtomBytes;
+    q.m = mt; q.mp = u.mp; q.k = a0.k; q.x_dtype = a0.x_dtype; q.ks = u.ks; q.csize = u.csize; q.sl = u.slabs_per_stage;
+    // scratch of one endpoint: the activation image
+    const size_t img_bytes = (size_t)u.ks * (kBsMaxTokens * 128 + kBsAtomBytes);
 
     for (int i = 0; i < n; ++i) {
         ws_tp *t = ranks[i];
         const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
-        ws_status_t s = ensure_bs_scratch(t, xq_bytes + sf_bytes);
-        if (s == WS_OK) s = make_tmap(t, &p.tmap_w[i], a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, (uint32_t)u.tile_rows);
-        uint8_t *const xq = t->bs_work;
-        if (s == WS_OK) s = make_tmap(t, &p.tmap_x[i], xq, (uint64_t)u.mp, (uint64_t)a.k, (uint64_t)a.k, (uint32_t)u.mp);
+        ws_status_t s = ensure_bs_scratch(t, img_bytes);
+        if (s == WS_OK)  // (with less than one whole slab only the second map is used)
+            s = make_tmap_slabs(t, &p.tmap_w[i], a.w, (uint64_t)a.n, (uint64_t)std::max(1, a.k / 128), (uint64_t)a.ldw, (uint32_t)u.tile_rows,
+                                (uint32_t)u.slabs_per_stage);
+        if (s == WS_OK) s = make_tmap(t, &p.tmap_t[i], a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, (uint32_t)u.tile_rows);
         if (s != WS_OK) { t0->err = t->err; return s; }
         Fp8RankArgs &r = p.r[i];
-        const size_t xes = a.x_dtype == WS_ACT_BF16 ? 2 : 4;
         r.x = nullptr;
         r.scales = a.scales;
         r.out = lm ? nullptr : a.out + (size_t)m0 * a.n;
-        r.logits = nullptr;
+        r.logits = lm && lm[i].logits ? lm[i].logits + (size_t)m0 * lm[i].vocab : nullptr;
+        if (r.logits) p.gather_logits = 1;
         r.argmax = lm && lm[i].argmax ? lm[i].argmax + m0 : nullptr;
         r.ldx = a.ldx; r.scale_ld = a.scale_ld; r.row0 = a.row0; r.k0 = a.k0;
         r.vocab_row0 = lm ? lm[i].vocab_row0 : 0;
         r.ctx = make_ctx(t);
         if (last) r.ctx.host_done = t->host_done_arm;
-        p.sfb[i] = xq + xq_bytes;
-        q.r[i].x = static_cast<const char *>(a.x) + (size_t)m0 * a.ldx * xes;
-        q.r[i].xq = xq;
-        q.r[i].sfb = xq + xq_bytes;
+        p.img[i] = t->bs_work;
+        q.r[i].x = static_cast<const char *>(a.x) + (size_t)m0 * a.ldx * (a.x_dtype == WS_ACT_BF16 ? 2 : 4);
+        q.r[i].img = t->bs_work;
         q.r[i].ldx = a.ldx;
     }
     for (int i = 0; i < n; ++i) ranks[i]->step++;
-    void (*const kernel)(BsParams) = u.mp == 16 ? fp8_bs_kernel<16> : u.mp == 32 ? fp8_bs_kernel<32>
-                                     : u.mp == 64 ? fp8_bs_kernel<64> : fp8_bs_kernel<128>;
-    const int prep_blocks = (int)(((int64_t)u.mp * (a0.k / 8) + 255) / 256);
-    if (same_device) {
-        WS_CUDA(t0, cudaSetDevice(t0->device));
-        cudaStream_t cs = static_cast<cudaStream_t>(streams ? streams[0] : nullptr);
-        ws_status_t s = launch(t0, act_prep_kernel, q, prep_blocks, n, 256, 0, cs, t0->pdl != 0, false);
-        if (s != WS_OK) return s;
-        return launch(t0, kernel, p, ncta, n, bs_threads(u.mp), u.smem, cs, t0->pdl != 0, true, u.csize);
-    }
-    for (int i = 0; i < n; ++i) {
-        BsParams pi = p;
-        pi.r[0] = p.r[i];
-        pi.tmap_w[0] = p.tmap_w[i];
-        pi.tmap_x[0] = p.tmap_x[i];
-        pi.sfb[0] = p.sfb[i];
-        ActPrepParams qi = q;
-        qi.r[0] = q.r[i];
+    void (*kernel)(BsParams);
+    if (u.wue) kernel = u.mp == 16 ? fp8_bs_kernel<16, true> : u.mp == 32 ? fp8_bs_kernel<32, true> : u.mp == 64 ? fp8_bs_kernel<64, true> : fp8_bs_kernel<128, true>;
+    else kernel = u.mp == 16 ? fp8_bs_kernel<16, false> : u.mp == 32 ? fp8_bs_kernel<32, false> : u.mp == 64 ? fp8_bs_kernel<64, false> : fp8_bs_kernel<128, false>;
+    const int prep_blocks = (int)(((int64_t)mt * u.ks * 16 + 255) / 256);
+    ws_status_t s = zero_lone_shard(ranks, n, lm, m0, mt, streams);
+    for (int i = 0; i < (same_device ? 1 : n) && s == WS_OK; ++i) {
+        if (i > 0) {  // one launch per device, each sees itself as virtual rank 0
+            p.r[0] = p.r[i];
+            p.tmap_w[0] = p.tmap_w[i];
+            p.tmap_t[0] = p.tmap_t[i];
+            p.img[0] = p.img[i];
+            q.r[0] = q.r[i];
+        }
+        const int nvr = same_device ? n : 1;
         WS_CUDA(ranks[i], cudaSetDevice(ranks[i]->device));
         cudaStream_t cs = static_cast<cudaStream_t>(streams ? streams[i] : nullptr);
-        ws_status_t s = launch(ranks[i], act_prep_kernel, qi, prep_blocks, 1, 256, 0, cs, t0->pdl != 0, false);
-        if (s == WS_OK) s = launch(ranks[i], kernel, pi, ncta, 1, bs_threads(u.mp), u.smem, cs, t0->pdl != 0, true, u.csize);
-        if (s != WS_OK) { t0->err = ranks[i]->err; return s; }
+        s = launch(ranks[i], act_prep_kernel, q, prep_blocks, nvr, 256, 0, cs, t0->pdl != 0, false);
+        if (s == WS_OK) s = launch(ranks[i], kernel, p, u.ncta, nvr, bs_threads(u.mp, u.wue), u.smem, cs, t0->pdl != 0, true, u.csize);
+        if (s != WS_OK) t0->err = ranks[i]->err;
     }
-    return WS_OK;
+    return s;
 }
 
 // Whether rows [.., +mt) of this step go to the block-scaled tcgen05 path: always when the caller
 // selected it; by default from three rows up, and for one or two rows when the shard is large enough
 // for its streaming rate to outweigh the second launch (measured on B200, M=1: 927 MB 153 against
 // 208 us on CUDA cores; 58.7 MB 17.7 against 17.2 us, 14.7 MB 8.8 against 6.8 us, 7.3 MB 12.8 against 5.9 us).
-// A step that also gathers the logits stays on the CUDA-core kernel: the tensor-memory kernel leaves
-// only the argmax candidates (the decode loop's form of the call).
-static bool bs_wanted(const ws_tp *t0, int mt, const ws_fp8_gemm_args_t &a, bool gathers_logits, bool lm_head = false) {
-    if (gathers_logits) return false;
+static bool bs_wanted(const ws_tp *t0, int mt, const ws_fp8_gemm_args_t &a, bool lm_head = false) {
     if (t0->kernel_sel == 2) return true;
     if (t0->kernel_sel != 0) return false;
-    // an argmax-only lm_head step also saves the exchange of one candidate per CTA (this kernel sends one per rank)
+    // an lm_head step also saves the exchange of one candidate per CTA (this kernel sends one per rank)
     // two rows: the CUDA-core kernel needs 23 us for a 58.7 MB shard, this one 17.8 (it is the same for 2 to 8 rows)
     if (mt == 2 && (int64_t)a.n * a.k >= ((int64_t)32 << 20)) return true;
     return mt >= 3 || (int64_t)a.n * a.k >= ((int64_t)(lm_head ? 32 : 128) << 20);
@@ -620,11 +647,11 @@ static bool bs_wanted(const ws_tp *t0, int mt, const ws_fp8_gemm_args_t &a, bool
 // Activation rows the next launch takes: up to 64 when their quantised copies fit in shared
 // memory beside at least three weight stages (the weights are then streamed once for all of
 // them), else 8.
-static int fp8_rows_per_launch(const ws_tp *t0, const ws_fp8_gemm_args_t &a, int ncta, int rem, bool gathers_logits, bool lm_head = false) {
-    {   // the tensor-memory path streams the weights once for up to 64 rows
+static int fp8_rows_per_launch(const ws_tp *t0, const ws_fp8_gemm_args_t &a, int ncta, int rem, bool lm_head = false) {
+    {   // the tensor-memory path streams the weights once for up to kBsMaxTokens rows
         const int mt = std::min(rem, (int)kBsMaxTokens);
         const int skb = (int)((a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
-        if (bs_wanted(t0, mt, a, gathers_logits, lm_head) && bs_plan(a, mt, skb, ncta, false).ok) return mt;
+        if (bs_wanted(t0, mt, a, lm_head) && bs_plan(a, mt, skb, ncta, false).ok) return mt;
     }
     if (rem <= 8) return rem;
     const int kbox = (a.k + 127) / 128;
@@ -636,15 +663,6 @@ static int fp8_rows_per_launch(const ws_tp *t0, const ws_fp8_gemm_args_t &a, int
         if ((kSmemBudget - fixed.total) / (fp8_stage_boxes(kbox) * kBoxBytes) >= 3) return m;
     }
     return 8;
-}
-
-// A lone rank that holds only a shard of the vocabulary: the rows nobody computes read as zero.
-static ws_status_t zero_lone_shard(ws_tp *const *ranks, int n, const ws_lm_head_args_t *lm, int m0, int mt, void *const *streams) {
-    if (!lm || n != 1 || ranks[0]->world != 1 || !lm[0].logits || lm[0].g.n >= lm[0].vocab) return WS_OK;
-    WS_CUDA(ranks[0], cudaSetDevice(ranks[0]->device));
-    WS_CUDA(ranks[0], cudaMemsetAsync(lm[0].logits + (size_t)m0 * lm[0].vocab, 0, (size_t)mt * lm[0].vocab * sizeof(float),
-                                      static_cast<cudaStream_t>(streams ? streams[0] : nullptr)));
-    return WS_OK;
 }
 
 // Plan of the one- and two-row CUDA-core kernel; ok = false when the shape does not fit it.
@@ -748,16 +766,16 @@ static ws_status_t fp8_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t
                             int m0, int mt, void *const *streams, int ncta, bool same_device, bool last) {
     ws_tp *t0 = ranks[0];
     const ws_fp8_gemm_args_t &a0 = lm ? lm[0].g : args[0];
-    bool gathers_logits = false;
-    for (int i = 0; lm && i < n; ++i) gathers_logits |= lm[i].logits != nullptr;
-    if (bs_wanted(t0, mt, a0, gathers_logits, lm != nullptr)) {  // tensor-memory path whenever the shape fits it
+    if (bs_wanted(t0, mt, a0, lm != nullptr)) {  // tensor-memory path whenever the shape fits it
         int64_t skb_u = 1;
+        bool slabs_fit = true;
         for (int i = 0; i < n; ++i) {
             const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
             skb_u = std::max<int64_t>(skb_u, (a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
+            slabs_fit &= a.scale_kind == WS_SCALE_UE8M0 || a.k0 % 128 == 0;  // a slab reads one scale column
         }
         const BsPlan u = bs_plan(a0, mt, (int)skb_u, ncta, n == 1);  // CTA pairs need a cluster launch, virtual ranks a cooperative one
-        if (u.ok) return bs_step(ranks, n, args, lm, m0, mt, streams, ncta, same_device, u, (int)skb_u, last);
+        if (u.ok && slabs_fit) return bs_step(ranks, n, args, lm, m0, mt, streams, same_device, u, (int)skb_u, last);
     }
     if (t0->kernel_sel != 1 && mt <= 2) {  // one or two activation rows: CUDA-core dot products
         int64_t skb_u = 1;
@@ -862,7 +880,7 @@ ws_status_t ws_fp8_rowpar_gemm_allreduce_group(ws_tp_t *const *ranks, int32_t n,
         return fail(t0, WS_ERR_CAPACITY, "m=%d n=%d exceed the endpoint's max_m=%d max_n=%d", args[0].m, args[0].n,
                     t0->cfg.max_m, t0->cfg.max_n);
     for (int m0 = 0; m0 < args[0].m;) {
-        const int mt = fp8_rows_per_launch(t0, args[0], ncta, args[0].m - m0, false);
+        const int mt = fp8_rows_per_launch(t0, args[0], ncta, args[0].m - m0);
         s = fp8_step(ranks, n, args, nullptr, m0, mt, streams, ncta, same, m0 + mt >= args[0].m);
         if (s != WS_OK) return s;
         m0 += mt;
@@ -901,7 +919,7 @@ ws_status_t ws_lm_head_allgather_argmax_group(ws_tp_t *const *ranks, int32_t n, 
     if (any_logits && args[0].vocab > t0->cfg.max_vocab)
         return fail(t0, WS_ERR_CAPACITY, "vocab=%d exceeds the endpoint's max_vocab=%d", args[0].vocab, t0->cfg.max_vocab);
     for (int m0 = 0; m0 < args[0].g.m;) {
-        const int mt = fp8_rows_per_launch(t0, args[0].g, ncta, args[0].g.m - m0, any_logits, true);
+        const int mt = fp8_rows_per_launch(t0, args[0].g, ncta, args[0].g.m - m0, true);
         s = fp8_step(ranks, n, nullptr, args, m0, mt, streams, ncta, same, m0 + mt >= args[0].g.m);
         if (s != WS_OK) return s;
         m0 += mt;
@@ -1376,9 +1394,9 @@ ws_status_t ws_fp8_rowpar_gemm_allreduce_host(ws_tp_t *tp, const ws_fp8_gemm_arg
         ws_tp *self[1] = {tp};
         if (validate_fp8(tp, a, false) == WS_OK && group_prelude(self, 1, &ncta, &same) == WS_OK) {
             const int skb = (int)((dw->k0 + dw->k - 1) / dw->block_k - dw->k0 / dw->block_k + 1);
-            const int mt = fp8_rows_per_launch(tp, a, ncta, a.m, false);
+            const int mt = fp8_rows_per_launch(tp, a, ncta, a.m);
             direct = true;
-            stage = !(bs_wanted(tp, mt, a, false) && bs_plan(a, mt, skb, ncta, true).ok);
+            stage = !(bs_wanted(tp, mt, a) && bs_plan(a, mt, skb, ncta, true).ok);
             if (!stage) a.x = pin;
         }
     }

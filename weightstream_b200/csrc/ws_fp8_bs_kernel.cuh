@@ -1,37 +1,37 @@
 // FP8 E4M3 row-parallel GEMM on the 5th-generation tensor cores with block scaling
 // (tcgen05.mma.kind::mxf8f6f4.block_scale, accumulators in tensor memory), fused with its
-// exchange (sm_100a).  One pass over the weights for up to 64 activation rows.
-//
-// Two kernels per step:
+// exchange (sm_100a).  One pass over the weights for up to 128 activation rows.
 //
 //   act_prep_kernel   quantises the activations once per step exactly as the reference does
-//                     (crates/weightstream-ref/src/actquant.rs:21-57): E4M3 bytes [mp][k] and the
-//                     per-32 UE8M0 exponents in the layout the MMA's scale operand wants (one 512-byte
-//                     atom per 128-wide K slab: byte (t & 31) * 16 + (t >> 5) * 4 + j holds the exponent
-//                     of token t, K block 4 * slab + j).  Both stay in L2 for the main kernel.
+//                     (crates/weightstream-ref/src/actquant.rs:21-57) into an image of what the main
+//                     kernel's stages hold, so that one bulk copy fills a stage's share of it.
 //   fp8_bs_kernel     persistent, one CTA per SM.  The rows are cut into tiles of at most 128 rows (the
-//                     M of the MMA) that deal out evenly, and a CTA streams the weights of its tiles over
-//                     the whole local K, so every output is a complete dot product inside one CTA.  Per
-//                     128-byte K slab the producer warp lands, in one stage of a shared-memory ring: the
-//                     tile's weight rows (TMA box, 128B swizzle), the quantised activations of all
-//                     tokens (TMA box from the prep kernel's buffer) and their scale atom (bulk copy).
-//                     One thread copies the atom into tensor memory (tcgen05.cp) and issues four MMAs
-//                     (M=128, N=tokens, K=32): the activations' per-32 scales ride the MMA's scale
-//                     operand, the weight operand's scale is 2^0, and the four K blocks accumulate in
-//                     tensor memory.  The weights' own scales are fp32 per (block_n x block_k) block,
-//                     which no MMA scale format can carry, so every slab gets its own accumulator
-//                     buffer and four epilogue warps read a stage's buffers back (tcgen05.ld) and add
-//                     them, times the fp32 weight scale, to their registers while the next stages'
-//                     MMAs run into the other buffers.
+//                     M of the MMA), dealt out whole; a CTA (or a CTA pair, each CTA one half of K)
+//                     streams the weights of its tiles, so every output is a complete dot product inside
+//                     one CTA pair and nothing is combined through global memory.  A stage of the ring
+//                     holds SL K slabs of 128: their weight rows (ONE 3-D TMA box, 128B swizzle) and their
+//                     activation image (SL tiles of tokens x 128 bytes, swizzled alike, then SL 512-byte
+//                     scale atoms: byte (t & 31) * 16 + (t >> 5) * 4 + j = exponent of token t, K block j).
+//                     One thread copies the atoms into tensor memory (tcgen05.cp) and issues four MMAs per
+//                     slab (M=128, N=tokens, K=32): the activations' per-32 scales ride the MMA's scale
+//                     operand.
+//   Weight scales     fp32 per (block_n x block_k) fit no MMA scale format: the weight operand's scale is
+//                     2^0, every slab has its own accumulator buffer, and the epilogue warps read a stage's
+//                     buffers back (tcgen05.ld) and add them x the fp32 scale while later MMAs run.
+//                     UE8M0 (WUE): they ARE an MMA scale operand.  Four auxiliary warps lay the tile's scale
+//                     bytes out as atoms in the stage, a tile accumulates over all of its K in tensor
+//                     memory and is read back once.
 //
-// Measured on B200 and kept in mind above: the tensor pipe needs 30-45 ns per K=32 MMA at M=128 however
-// few of the rows are real (M=64 is not available with block scaling); a tcgen05.commit stalls the
-// issuing thread for ~160 ns; handing partial sums from one CTA to another through L2 (a split of K
-// across CTAs) costs 3-5 us, more than it saves on these shapes.
+// Measured on B200 and kept in mind above: every TMA or bulk copy costs its issuing thread ~100 ns, so a
+// stage is two copies (one box, one image) and not three per slab; the tensor pipe needs 30-45 ns per K=32
+// MMA at M=128 however few of the rows are real (M=64 is not available with block scaling); a
+// tcgen05.commit stalls the issuing thread for ~160 ns; handing partial sums from one CTA to another
+// through L2 (a split of K across CTAs) costs 3-5 us, more than it saves on these shapes.
 //
 // MMA rows past a tile's end are computed on whatever follows in shared memory and never read back.
-// Exchange and lm_head mode are those of the decode kernel (ws_fp8_kernel.cuh): tagged 64-bit
-// words stored into every peer's slots and folded in rank order, or argmax candidates merged per rank.
+// Exchange and lm_head mode are those of the decode kernels (ws_fp8_kernel.cuh): tagged 64-bit
+// words stored into every peer's slots and folded in rank order, or logits gathered and argmax candidates
+// merged per rank.
 #pragma once
 
 #include <math.h>
@@ -45,91 +45,105 @@ namespace ws {
 // epilogue warps: four (one per 32-lane quarter of the tensor memory, all token columns) for up to 32
 // tokens, eight (two per quarter, half of the token columns each) for 64, where reading the
 // accumulators back is what a stage waits for (measured on B200, 64 rows: lm_head 324 -> 249 us;
-// with 32 rows eight warps were 3 % slower than four).
+// with 32 rows eight warps were 3 % slower than four); then, for UE8M0 weight scales, four auxiliary warps.
 __host__ __device__ constexpr int bs_epi_warps(int mp) { return mp >= 64 ? 8 : 4; }
-__host__ __device__ constexpr int bs_threads(int mp) { return 64 + 32 * bs_epi_warps(mp); }
+constexpr int kBsAuxWarps = 4;
+__host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 * (bs_epi_warps(mp) + (wue ? kBsAuxWarps : 0)); }
 constexpr int kBsMaxAcc = 8;         // accumulator groups in tensor memory (a group = one stage's slabs)
 constexpr int kBsMaxTokens = 128;    // activation rows one launch takes (16, 32, 64 or 128 MMA columns)
 constexpr int kBsAtomBytes = 512;    // one scale atom: 128 rows x 4 K blocks
 constexpr int kBsMmaRows = 128;      // M of the MMA; a tile of output rows holds at most as many
 
+// The activation image of a step: the slabs in order, grouped as the CTAs' stages take them.  CTA half h
+// of K owns slabs [h * ks / csize, (h + 1) * ks / csize), in groups of at most sl; a group is its tiles
+// [mp tokens x 128 bytes, 16-byte chunk c of token t at c ^ (t & 7)], then its atoms.
+struct BsImage {
+    int32_t tile, atom;  // byte offsets of the slab's tile and atom inside the image
+};
+__host__ __device__ inline BsImage bs_image_at(int slab, int ks, int csize, int sl, int mp) {
+    int lo = 0, hi = ks;
+    if (csize == 2) {
+        if (slab >= ks / 2) lo = ks / 2;
+        else hi = ks / 2;
+    }
+    const int g0 = lo + (slab - lo) / sl * sl, n = sl < hi - g0 ? sl : hi - g0, base = g0 * (mp * 128 + kBsAtomBytes);
+    return BsImage{base + (slab - g0) * mp * 128, base + n * mp * 128 + (slab - g0) * kBsAtomBytes};
+}
+
 // ---------------------------------------------------------------- activation prep
 struct ActPrepRank {
     const void *x;
-    uint8_t *xq;   // [mp][k] E4M3
-    uint8_t *sfb;  // [k / 128][512] scale atoms
+    uint8_t *img;  // see BsImage
     int64_t ldx;
 };
 struct ActPrepParams {
-    int32_t m, mp, k, x_dtype;
+    int32_t m, mp, k, x_dtype, ks, csize, sl, pad0;
     ActPrepRank r[WS_MAX_WORLD];
 };
 
+// Thread = 8 values of one token; tokens the step does not carry are left out (their MMA columns are
+// never read), the K tail of the last slab is written as zeros.
 __global__ void __launch_bounds__(256) act_prep_kernel(const __grid_constant__ ActPrepParams p) {
     // The step that follows may become resident at once (it streams weights until its own wait);
     // the activations come from earlier work on the stream.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const ActPrepRank &A = p.r[blockIdx.y];
-    const int chunks_per_row = p.k >> 3;
-    const int64_t total = (int64_t)p.mp * chunks_per_row;
+    const int chunks_per_row = p.ks << 4;
+    const int64_t total = (int64_t)p.m * chunks_per_row;
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = c < total;
     const int tok = in ? (int)(c / chunks_per_row) : 0;
     const int ch = in ? (int)(c - (int64_t)tok * chunks_per_row) : 0;
-    const bool valid = in && tok < p.m;
+    const bool valid = in && ch * 8 < p.k;
     float v[8];
     load_act8(A.x, p.x_dtype, (int64_t)tok * A.ldx + ch * 8, valid, v);
     int e;
     uint32_t lo, hi;
     act_quant8(v, e, lo, hi);  // the four lanes of a 32-block are adjacent threads of one warp
     if (in) {
-        *reinterpret_cast<uint2 *>(A.xq + (int64_t)tok * p.k + ch * 8) = valid ? make_uint2(lo, hi) : make_uint2(0u, 0u);
-        if ((ch & 3) == 0) {
-            const int kb = ch >> 2;
-            const int eb = valid ? min(max(e + 127, 0), 255) : 127;
-            A.sfb[(size_t)(kb >> 2) * kBsAtomBytes + (tok & 31) * 16 + (tok >> 5) * 4 + (kb & 3)] = (uint8_t)eb;
-        }
+        const BsImage o = bs_image_at(ch >> 4, p.ks, p.csize, p.sl, p.mp);
+        *reinterpret_cast<uint2 *>(A.img + o.tile + tok * 128 + ((((ch >> 1) & 7) ^ (tok & 7)) << 4) + (ch & 1) * 8) = make_uint2(lo, hi);
+        if ((ch & 3) == 0)
+            A.img[o.atom + (tok & 31) * 16 + (tok >> 5) * 4 + ((ch >> 2) & 3)] = (uint8_t)min(max(e + 127, 0), 255);
     }
 }
 
 // ---------------------------------------------------------------- main kernel
 struct alignas(64) BsParams {
-    CUtensorMap tmap_w[WS_MAX_WORLD];  // weight shard [n][k bytes], box 128 bytes x tile_rows, 128B swizzle
-    CUtensorMap tmap_x[WS_MAX_WORLD];  // quantised activations [mp][k bytes], box 128 bytes x mp, 128B swizzle
-    int32_t m, mp, n, k, bn_shift, bk_shift;
+    CUtensorMap tmap_w[WS_MAX_WORLD];  // weight shard as [whole slabs][n][128 bytes]: box SL slabs x tile_rows x 128 bytes, 128B swizzle
+    CUtensorMap tmap_t[WS_MAX_WORLD];  // weight shard as [n][k bytes], box tile_rows x 128 bytes: slabs of a group that is not whole
+    int32_t m, mp, n, k, ks, bn_shift, bk_shift;
     int32_t world, mode, vocab, tmem_cols;  // tmem_cols: tensor-memory columns to allocate (512, or at most 256 when two CTAs share an SM)
     int32_t owner_reduce;              // all-reduce by owners: tile t is folded by rank t % world, which sends the sums back
     int32_t csize;                     // 1, or 2: CTA pairs (a cluster) share a tile, each streams half of K
-    int32_t tile_rows, ntiles;         // output rows per tile (<= 128) and tiles of the shard
+    int32_t tile_rows, ntiles;         // output rows per tile (a multiple of 8, <= 128) and tiles of the shard
     int32_t slabs_per_stage, nstages;
-    int32_t a_pitch, b_pitch;          // bytes one slab's weights / activations occupy in a stage (multiples of 1024)
-    int32_t skb, nslot_max, nacc;
+    int32_t a_pitch, x_pitch;          // bytes one slab's weights / one stage's activation image occupy (multiples of 1024)
+    int32_t skb, nslot_max, nacc, gather_logits;
     uint64_t timeout_ns;
     SymLayout lay;
-    Fp8RankArgs r[WS_MAX_WORLD];       // x is unused here; scales/out/logits/argmax/row0/k0/ctx as in the decode kernel
-    const uint8_t *sfb[WS_MAX_WORLD];  // the prep kernel's scale atoms
+    Fp8RankArgs r[WS_MAX_WORLD];       // x is unused here; scales/out/logits/argmax/row0/k0/ctx as in the decode kernels
+    const uint8_t *img[WS_MAX_WORLD];  // the prep kernel's activation image
 };
 
 struct BsSmem {
-    int32_t a, b, sf, sfa, sw, cand, rx, bars, misc, total;
+    int32_t a, x, wsf, sw, cand, rx, bars, misc, total;
 };
-__host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stage, int a_pitch, int b_pitch, int nslot_max,
-                                                 int skb, int mp, int rx_rows) {
+__host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stage, int a_pitch, int x_pitch, int nslot_max,
+                                                 int skb, int mp, int rx_rows, bool wue) {
     BsSmem s{};
     const int nsl = nstages * slabs_per_stage;
-    const int b_bytes = nsl * b_pitch;
     int o = 0;
     s.a = o;    o += nsl * a_pitch;
-    s.b = o;    o += b_bytes;
+    s.x = o;    o += nstages * x_pitch;
     // an MMA reads 128 rows of its weight slab however many the tile holds: keep 16 KB readable behind the last one
-    if (b_bytes < kBsMmaRows * 128) o += kBsMmaRows * 128 - b_bytes;
-    s.sf = o;   o += nsl * kBsAtomBytes;
-    s.sfa = o;  o += kBsAtomBytes;
-    s.sw = o;   o += (int)align_up((int64_t)nslot_max * skb * 4, 16);
+    if (nstages * x_pitch < kBsMmaRows * 128) o += kBsMmaRows * 128 - nstages * x_pitch;
+    s.wsf = o;  o += wue ? nsl * kBsAtomBytes : kBsAtomBytes;  // the weights' scale atoms (fp32 scales: one atom of 2^0)
+    s.sw = o;   o += wue ? 0 : (int)align_up((int64_t)nslot_max * skb * 4, 16);
     s.cand = o; o += bs_epi_warps(mp) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
     s.rx = o;   o += rx_rows * kBsMmaRows * 4;           // CTA pairs: the partner's partial sums of one tile, [token][row]
-    s.bars = o; o += (2 * kMaxStages + kBsMaxAcc + 2) * 8;
+    s.bars = o; o += (2 * kMaxStages + 2 * kBsMaxAcc + 2) * 8;
     s.misc = o; o += 64;
     s.total = o;
     return s;
@@ -260,6 +274,12 @@ __device__ __forceinline__ void bs_epi_bar_n() {  // the epilogue warps
     asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
 }
 
+// 3-D TMA tile load, completion on an mbarrier.
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+
 // The sequence of stage items of one CTA.  The shard's rows are cut into tiles of tile_rows rows
 // (at most 128, the M of the MMA; chosen so that the tiles deal out evenly) and CTA c takes tiles
 // [c * T / ncta, (c + 1) * T / ncta) whole, so every output row is a complete dot product inside one
@@ -289,8 +309,15 @@ struct BsWalk {
     }
 };
 
-template <int MP>
-__global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_constant__ BsParams p) {
+// Floats in an order that unsigned comparison keeps; everything that is not above -inf is 0.
+__device__ __forceinline__ uint32_t order_key(float v) {
+    if (!(v > -INFINITY)) return 0u;
+    const uint32_t b = __float_as_uint(v + 0.0f);  // -0 and +0 are equal
+    return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);
+}
+
+template <int MP, bool WUE>
+__global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_kernel(const __grid_constant__ BsParams p) {
     constexpr int EW = bs_epi_warps(MP), ET = EW * 32;  // epilogue warps / threads
     constexpr int CP = MP * 4 / EW;                      // token columns one epilogue thread holds
     auto bs_epi_bar = [] { bs_epi_bar_n<ET>(); };
@@ -303,7 +330,7 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
     const RankCtx &X = A.ctx;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    const int KS = p.k >> 7;                                // slabs per tile
+    const int KS = p.ks;                                    // slabs per tile
     // CTA pairs: which half of K is this CTA's, and which pair of how many it belongs to
     uint32_t crank = 0;
     if (p.csize == 2) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
@@ -312,25 +339,29 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
     const int SL = p.slabs_per_stage, NS = p.nstages, NB = p.nacc;
     const int ntiles = p.ntiles, TR = p.tile_rows;
 
-    const BsSmem S = bs_smem_layout(NS, SL, p.a_pitch, p.b_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? p.m : 0);
+    const BsSmem S = bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? p.m : 0, WUE);
     float *sw_s = reinterpret_cast<float *>(smem + S.sw);
     uint32_t *misc_s = reinterpret_cast<uint32_t *>(smem + S.misc);
-    const uint32_t a0 = smem_u32(smem + S.a), b0 = smem_u32(smem + S.b), sf0 = smem_u32(smem + S.sf);
-    // full[s]: the stage's bytes landed.  done[s]: every MMA that reads the stage has completed (ONE
-    // tcgen05.commit per stage: a commit stalls the issuing thread for ~160 ns, so it is not spent per
-    // slab) -- the producer reads it as "stage free", the epilogue as "this stage's accumulators are
-    // ready".  A stage's slabs accumulate into the SL buffers of accumulator group g = item mod NB;
-    // accempty[g]: the group has been read back.
+    const uint32_t a0 = smem_u32(smem + S.a), x0 = smem_u32(smem + S.x), wsf0 = smem_u32(smem + S.wsf);
+    // full[s]: the stage's bytes landed (UE8M0: and the auxiliary warps have written its weight scales).
+    // done[s]: every MMA that reads the stage has completed (ONE tcgen05.commit per stage: a commit stalls
+    // the issuing thread for ~160 ns, so it is not spent per slab).  fp32 weight scales: a stage's slabs
+    // accumulate into the SL buffers of accumulator group g = item mod NB, done[s] also tells the epilogue
+    // that they are ready, accempty[g] that the group has been read back.  UE8M0: a tile accumulates into
+    // buffer (tile mod NB), accfull / accempty hand it over.
     const uint32_t full0 = smem_u32(smem + S.bars), done0 = full0 + kMaxStages * 8;
-    const uint32_t accempty0 = done0 + kMaxStages * 8;
-    const uint32_t rxfull = accempty0 + kBsMaxAcc * 8, rxempty = rxfull + 8;  // CTA pairs: the partner's sums of a tile have arrived / been read
+    const uint32_t accempty0 = done0 + kMaxStages * 8, accfull0 = accempty0 + kBsMaxAcc * 8;
+    const uint32_t rxfull = accfull0 + kBsMaxAcc * 8, rxempty = rxfull + 8;  // CTA pairs: the partner's sums of a tile have arrived / been read
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
-            mbar_init(full0 + s * 8, 1);
+            mbar_init(full0 + s * 8, WUE ? 1 + kBsAuxWarps : 1);
             mbar_init(done0 + s * 8, 1);
         }
-        for (int b = 0; b < kBsMaxAcc; ++b) mbar_init(accempty0 + b * 8, EW);  // one arrival per epilogue warp
+        for (int b = 0; b < kBsMaxAcc; ++b) {
+            mbar_init(accempty0 + b * 8, EW);  // one arrival per epilogue warp
+            mbar_init(accfull0 + b * 8, 1);
+        }
         mbar_init(rxfull, ET);   // every epilogue thread of the partner arrives after its stores
         mbar_init(rxempty, ET);
         mbar_fence_init();
@@ -339,9 +370,8 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
         tmem_alloc(smem_u32(misc_s), (uint32_t)p.tmem_cols);
         tmem_relinquish();
     }
-    if (warp >= 2 && warp < 6) {  // the weight operand's scale atom: 2^0 everywhere (128 threads x 4 bytes)
-        uint32_t *sfa = reinterpret_cast<uint32_t *>(smem + S.sfa);
-        sfa[tid - 64] = 0x7F7F7F7Fu;
+    if (!WUE && warp >= 2 && warp < 6) {  // the weight operand's scale atom: 2^0 everywhere (128 threads x 4 bytes)
+        reinterpret_cast<uint32_t *>(smem + S.wsf)[tid - 64] = 0x7F7F7F7Fu;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     tc_fence_before();
@@ -352,29 +382,27 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(misc_s);
-    // tensor-memory columns: NB groups x SL accumulator buffers of MP columns, then 4 activation-scale
-    // columns (one scale atom) per buffer, then the 4 weight-scale columns
-    const uint32_t t_sfb0 = tmem_base + (uint32_t)(NB * SL * MP);
-    const uint32_t t_sfa = t_sfb0 + (uint32_t)(NB * SL * 4);
+    // tensor-memory columns.  fp32 weight scales: NB groups x SL accumulator buffers of MP columns, 4
+    // activation-scale columns (one scale atom) per buffer, the 4 weight-scale columns.  UE8M0: NB
+    // accumulators of MP columns, then for two stages and SL slabs each 4 activation- and 4 weight-scale columns.
+    const uint32_t t_sf0 = tmem_base + (uint32_t)(NB * (WUE ? 1 : SL) * MP);
+    const uint32_t t_sfa = t_sf0 + (uint32_t)(NB * SL * 4);  // fp32 weight scales only
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer (one thread)
         if (lane == 0) {
             // Weights are static: the first ring's worth streams before the wait on the prep kernel;
-            // the activations and their scales follow once it has finished.
-            const uint32_t slab_tx = (uint32_t)(TR * 128 + MP * 128 + kBsAtomBytes);
+            // the activations follow once it has finished.
+            constexpr uint32_t kXSlab = MP * 128 + kBsAtomBytes;
+            const int whole = p.k >> 7;  // slabs of the 3-D map
             auto issue_w = [&](int s, int tile, int s0, int nsl) {
-                mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * slab_tx);
-                for (int j = 0; j < nsl; ++j)
-                    tma_load_2d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (s0 + j) * 128, tile * TR, full0 + s * 8);
-            };
-            auto issue_x = [&](int s, int s0, int nsl) {
-                for (int j = 0; j < nsl; ++j) {
-                    tma_load_2d(b0 + (s * SL + j) * p.b_pitch, &p.tmap_x[vr], (s0 + j) * 128, 0, full0 + s * 8);
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                 ::"r"(sf0 + (s * SL + j) * kBsAtomBytes), "l"(p.sfb[vr] + (size_t)(s0 + j) * kBsAtomBytes),
-                                   "r"((uint32_t)kBsAtomBytes), "r"(full0 + s * 8) : "memory");
+                mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + kXSlab));
+                const uint32_t dst = a0 + s * SL * p.a_pitch;
+                if (nsl == SL && s0 + nsl <= whole) {
+                    tma_load_3d(dst, &p.tmap_w[vr], 0, tile * TR, s0, full0 + s * 8);
+                } else {
+                    for (int j = 0; j < nsl; ++j) tma_load_2d(dst + j * p.a_pitch, &p.tmap_t[vr], (s0 + j) * 128, tile * TR, full0 + s * 8);
                 }
             };
             int tile, s0, nsl;
@@ -391,7 +419,7 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
                     if (!mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status)) break;
                     issue_w(s, tile, s0, nsl);
                 }
-                issue_x(s, s0, nsl);
+                bulk_load(x0 + s * p.x_pitch, p.img[vr] + (size_t)s0 * kXSlab, (uint32_t)nsl * kXSlab, full0 + s * 8);
             }
         }
     } else if (warp == 1) {
@@ -403,37 +431,87 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
         // one thread; the barrier hand-offs are the same either way, so the cause is not known.
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (lane == 0) {
-            tmem_cp_atom(t_sfa, umma_desc(smem_u32(smem + S.sfa), 128, false));
+            if (!WUE) tmem_cp_atom(t_sfa, umma_desc(wsf0, 128, false));
             // Everything the loop needs per MMA is an add away: descriptor halves per stage slot, the
             // four instruction descriptors (one per K block of a slab), ring positions kept incrementally.
-            const uint32_t id0 = bs_idesc(MP, 0, 0), id1 = bs_idesc(MP, 0, 1), id2 = bs_idesc(MP, 0, 2), id3 = bs_idesc(MP, 0, 3);
-            const uint32_t a_lo0 = umma_desc_lo(a0), b_lo0 = umma_desc_lo(b0);
-            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, b_step = (uint32_t)p.b_pitch >> 4;
-            const uint64_t sf_desc0 = umma_desc(sf0, 128, false);
-            const uint32_t sf_step = (uint32_t)kBsAtomBytes >> 4;
+            uint32_t id[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) id[q] = bs_idesc(MP, WUE ? q : 0, q);
+            const uint32_t a_lo0 = umma_desc_lo(a0), x_lo0 = umma_desc_lo(x0);
+            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, x_stage = (uint32_t)p.x_pitch >> 4;
+            const uint64_t xsf_desc0 = umma_desc(x0, 128, false), wsf_desc0 = umma_desc(wsf0, 128, false);
+            constexpr uint32_t kXStep = (uint32_t)(MP * 128) >> 4, kSfStep = (uint32_t)kBsAtomBytes >> 4;
             BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
-            RingPos st, ag;  // stage ring, accumulator-group ring
+            RingPos st, ag;  // stage ring, accumulator ring
             int tile, s0, nsl;
-            for (int item = 0; w.next(tile, s0, nsl); ++item, st.next(NS), ag.next(NB)) {
+            for (int item = 0; w.next(tile, s0, nsl); ++item, st.next(NS)) {
                 const int s = st.s, g = ag.s;
-                if (!mbar_wait(full0 + s * 8, st.ph, X.status) || !mbar_wait(accempty0 + g * 8, ag.ph ^ 1u, X.status)) break;
+                if (!mbar_wait(full0 + s * 8, st.ph, X.status)) break;
+                if ((!WUE || s0 == k_lo) && !mbar_wait(accempty0 + g * 8, ag.ph ^ 1u, X.status)) break;
                 tc_fence_after();
-                uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = b_lo0 + (uint32_t)(s * SL) * b_step;
-                uint64_t sf_desc = sf_desc0 + (uint64_t)((uint32_t)(s * SL) * sf_step);
-                uint32_t t_acc = tmem_base + (uint32_t)(g * SL * MP), t_sfb = t_sfb0 + (uint32_t)(g * SL * 4);
+                uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = x_lo0 + (uint32_t)s * x_stage;
+                uint64_t xsf = xsf_desc0 + (uint64_t)((uint32_t)s * x_stage + (uint32_t)nsl * kXStep);
+                uint64_t wsf = wsf_desc0 + (uint64_t)((uint32_t)(s * SL) * kSfStep);
+                uint32_t t_acc = tmem_base + (uint32_t)((WUE ? g : g * SL) * MP);
+                uint32_t t_sf = t_sf0 + (WUE ? (uint32_t)((item & 1) * SL * 8) : (uint32_t)(g * SL * 4));
                 for (int j = 0; j < nsl; ++j) {
-                    tmem_cp_atom(t_sfb, sf_desc);
-                    umma_bs_ss<false>(t_acc, a_lo, b_lo, kUmmaDescHiSw128, kUmmaDescHiSw128, id0, t_sfa, t_sfb);
-                    umma_bs_ss<true>(t_acc, a_lo + 2, b_lo + 2, kUmmaDescHiSw128, kUmmaDescHiSw128, id1, t_sfa, t_sfb);
-                    umma_bs_ss<true>(t_acc, a_lo + 4, b_lo + 4, kUmmaDescHiSw128, kUmmaDescHiSw128, id2, t_sfa, t_sfb);
-                    umma_bs_ss<true>(t_acc, a_lo + 6, b_lo + 6, kUmmaDescHiSw128, kUmmaDescHiSw128, id3, t_sfa, t_sfb);
-                    a_lo += a_step; b_lo += b_step; sf_desc += sf_step;
-                    t_acc += MP; t_sfb += 4;
+                    const uint32_t t_w = WUE ? t_sf + 4 : t_sfa;
+                    tmem_cp_atom(t_sf, xsf);
+                    if (WUE) tmem_cp_atom(t_sf + 4, wsf);
+                    if (WUE && s0 + j != k_lo) umma_bs_ss<true>(t_acc, a_lo, b_lo, kUmmaDescHiSw128, kUmmaDescHiSw128, id[0], t_w, t_sf);
+                    else umma_bs_ss<false>(t_acc, a_lo, b_lo, kUmmaDescHiSw128, kUmmaDescHiSw128, id[0], t_w, t_sf);
+                    umma_bs_ss<true>(t_acc, a_lo + 2, b_lo + 2, kUmmaDescHiSw128, kUmmaDescHiSw128, id[1], t_w, t_sf);
+                    umma_bs_ss<true>(t_acc, a_lo + 4, b_lo + 4, kUmmaDescHiSw128, kUmmaDescHiSw128, id[2], t_w, t_sf);
+                    umma_bs_ss<true>(t_acc, a_lo + 6, b_lo + 6, kUmmaDescHiSw128, kUmmaDescHiSw128, id[3], t_w, t_sf);
+                    a_lo += a_step; b_lo += kXStep; xsf += kSfStep; wsf += kSfStep;
+                    t_sf += WUE ? 8 : 4;
+                    if (!WUE) t_acc += MP;
                 }
-                umma_commit(done0 + s * 8);  // the stage may be refilled and its accumulators read
+                umma_commit(done0 + s * 8);  // the stage may be refilled (fp32 weight scales: and its accumulators read)
+                if (!WUE) ag.next(NB);
+                else if (s0 + nsl == k_hi) {
+                    umma_commit(accfull0 + g * 8);
+                    ag.next(NB);
+                }
             }
         }
         __syncwarp();
+    } else if (warp >= 2 + EW) {
+        // ------------------------------------------------------------ auxiliary warps (UE8M0 weight scales)
+        // The scale bytes of the tile's rows (thread = row) become the stage's scale atoms; static, so they
+        // do not wait for the predecessor.
+        if constexpr (WUE) {
+            const int r = tid - 64 - ET;
+            BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
+            RingPos st;
+            int tile, s0, nsl;
+            bool ok = true;
+            for (int item = 0; w.next(tile, s0, nsl); ++item, st.next(NS)) {
+                const int s = st.s, row = tile * TR + r;
+                const bool real = r < TR && row < p.n;
+                const uint8_t *src = static_cast<const uint8_t *>(A.scales) + ((A.row0 + (real ? row : 0)) >> p.bn_shift) * A.scale_ld;
+                uint32_t sc[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    sc[j] = 0u;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int kk = (s0 + j) * 128 + q * 32;
+                        const uint32_t b = real && j < nsl && kk < p.k ? __ldg(src + ((A.k0 + kk) >> p.bk_shift)) : 0x7Fu;
+                        sc[j] |= b << (8 * q);
+                    }
+                }
+                if (item >= NS) ok = mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status);
+                if (!__all_sync(0xffffffffu, ok)) break;
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (j < nsl)
+                        *reinterpret_cast<uint32_t *>(smem + S.wsf + (s * SL + j) * kBsAtomBytes + (r & 31) * 16 + (r >> 5) * 4) = sc[j];
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full0 + s * 8);
+            }
+        }
     } else {
         // ------------------------------------------------------------ epilogue warps
         const int et = tid - 64;                     // 0..ET-1
@@ -443,16 +521,18 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
         const int col0 = (ew >> 2) * CP;             // first token column of this thread
         const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
         const int t_lo = (int)((int64_t)ntiles * part / nparts), t_hi = (int)((int64_t)ntiles * (part + 1) / nparts) - 1;  // this CTA's tiles
-        // weight scales of the rows this CTA touches as fp32: sw_s[slot][column].  They are static, so
-        // they are fetched before the wait on the predecessor.
         const int64_t kcol0 = A.k0 >> p.bk_shift;
-        const int row_lo = t_lo * TR, row_hi = min(p.n, (t_hi + 1) * TR);
-        const int64_t srow_lo = (A.row0 + row_lo) >> p.bn_shift;
-        const int nslot = row_hi > row_lo ? (int)(((A.row0 + row_hi - 1) >> p.bn_shift) - srow_lo + 1) : 0;
-        const int ncols = (int)(((A.k0 + p.k - 1) >> p.bk_shift) - kcol0 + 1);
-        for (int i = et; i < nslot * ncols; i += ET) {
-            const int sl = i / ncols, c = i - sl * ncols;
-            sw_s[sl * p.skb + c] = __ldg(static_cast<const float *>(A.scales) + (srow_lo + sl) * A.scale_ld + kcol0 + c);
+        const int64_t srow_lo = (A.row0 + t_lo * TR) >> p.bn_shift;
+        if constexpr (!WUE) {
+            // weight scales of the rows this CTA touches as fp32: sw_s[slot][column].  They are static, so
+            // they are fetched before the wait on the predecessor.
+            const int row_lo = t_lo * TR, row_hi = min(p.n, (t_hi + 1) * TR);
+            const int nslot = row_hi > row_lo ? (int)(((A.row0 + row_hi - 1) >> p.bn_shift) - srow_lo + 1) : 0;
+            const int ncols = (int)(((A.k0 + p.k - 1) >> p.bk_shift) - kcol0 + 1);
+            for (int i = et; i < nslot * ncols; i += ET) {
+                const int sl = i / ncols, c = i - sl * ncols;
+                sw_s[sl * p.skb + c] = __ldg(static_cast<const float *>(A.scales) + (srow_lo + sl) * A.scale_ld + kcol0 + c);
+            }
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint32_t seq = step_begin(X);
@@ -467,15 +547,21 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
         if (p.mode == kModeLmHead)
             for (int i = lane; i < MP; i += 32) { cv_s[ew * MP + i] = -INFINITY; ci_s[ew * MP + i] = 0xFFFFFFFFu; }
 
-        // A finished tile: its rows go to the output or to the peers; of an lm_head tile the candidates are kept.
+        // A finished tile: its rows go to the output or to the peers; of an lm_head tile the candidates are
+        // kept and, when the caller wants them, the logits stored.
         auto finalize = [&](const float (&v)[CP], int tile) {  // v[i]: token col0 + i
             const int row = tile * TR + rc;
             const bool mine = rc < TR && row < p.n;
+            // element (token, row) of a float matrix with `ld` floats per token
+            auto store = [&](float *base, size_t ld) {
+                float *dst = base + (size_t)col0 * ld + row;
+#pragma unroll
+                for (int i = 0; i < CP; ++i)
+                    if (col0 + i < p.m) dst[(size_t)i * ld] = v[i];
+            };
             if (mine) {
                 if (solo) {
-#pragma unroll
-                    for (int i = 0; i < CP; ++i)
-                        if (col0 + i < p.m) A.out[(size_t)(col0 + i) * p.n + row] = v[i];
+                    store(A.out, (size_t)p.n);
                 } else if (p.mode == kModeAllReduce) {
                     // every rank gets the partial sums, or (many rows, many ranks) only the tile's owner
                     const int pr0 = p.owner_reduce ? tile % p.world : 0, pr1 = p.owner_reduce ? pr0 + 1 : p.world;
@@ -485,85 +571,105 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
                         for (int i = 0; i < CP; ++i)
                             if (col0 + i < p.m) st_word_sys(dst + (size_t)(col0 + i) * p.n + row, seq, v[i]);
                     }
+                } else if (p.gather_logits && p.world == 1) {  // a lone rank's logits are final where they are
+                    store(A.logits + A.vocab_row0, (size_t)p.vocab);
+                } else if (p.gather_logits) {
+                    for (int pr = 0; pr < p.world; ++pr)
+                        store(reinterpret_cast<float *>(X.sym[pr] + p.lay.gather_off) + (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab +
+                                  A.vocab_row0, (size_t)p.lay.max_vocab);
                 }
             }
             if (p.mode == kModeLmHead) {
-                // best (value, lowest index) of this warp's rows per token, merged into the warp's running best
-                const uint32_t idx = (uint32_t)(A.vocab_row0 + row);
+                // Best (value, lowest index) of this warp's 32 rows per token, merged into the warp's running
+                // best: the largest key by one redux, the lowest lane that holds it by one ballot.
+                const uint32_t idx0 = (uint32_t)(A.vocab_row0 + tile * TR + quad * 32);
 #pragma unroll
                 for (int i = 0; i < CP; ++i) {
                     const int t = col0 + i;
                     if (t >= p.m) break;
-                    float bv = (mine && v[i] > -INFINITY) ? v[i] : -INFINITY;
-                    uint32_t bi = (mine && v[i] > -INFINITY) ? idx : 0xFFFFFFFFu;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                        const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                        if (cand_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+                    const uint32_t key = mine ? order_key(v[i]) : 0u;
+                    const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+                    const int who = __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
+                    if (lane == who && top != 0u && cand_better(v[i], idx0 + (uint32_t)who, cv_s[ew * MP + t], ci_s[ew * MP + t])) {
+                        cv_s[ew * MP + t] = v[i];
+                        ci_s[ew * MP + t] = idx0 + (uint32_t)who;
                     }
-                    if (lane == 0 && cand_better(bv, bi, cv_s[ew * MP + t], ci_s[ew * MP + t])) {
-                        cv_s[ew * MP + t] = bv;
-                        ci_s[ew * MP + t] = bi;
-                    }
+                    __syncwarp();
                 }
             }
         };
 
         BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
-        RingPos st, ag;  // stage ring, accumulator-group ring
+        RingPos st, ag;  // stage ring, accumulator ring
         bool ok = true;
         int tile, s0, nsl, ntile_done = 0;
         float acc[CP];
         const float *swrow = sw_s;
         while (w.next(tile, s0, nsl)) {
-            if (s0 == k_lo) {  // a new tile
-#pragma unroll
-                for (int i = 0; i < CP; ++i) acc[i] = 0.0f;
-                const int row = min(tile * TR + min(rc, TR - 1), p.n - 1);
-                swrow = sw_s + (int)(((A.row0 + row) >> p.bn_shift) - srow_lo) * p.skb;
-            }
+            const bool last = s0 + nsl == k_hi;  // this CTA's slabs of the tile end with this item
             const int g = ag.s;
-            if (ok && !mbar_wait(done0 + st.s * 8, st.ph, X.status)) ok = false;
-            ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads below need the whole warp
-            tc_fence_after();
-            if (ok) {
-                for (int j = 0; j < nsl; ++j) {
-                    const float sw = swrow[(kofs + (s0 + j) * 128) >> p.bk_shift];
-                    uint32_t r[CP];
-                    tmem_ld_cols<CP>(tlane + (uint32_t)((g * SL + j) * MP + col0), r);  // returns once the values are in registers
+            if constexpr (WUE) {
+                if (!last) continue;
+                if (ok && !mbar_wait(accfull0 + g * 8, ag.ph, X.status)) ok = false;
+                ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads below need the whole warp
+                tc_fence_after();
+                uint32_t r[CP];
 #pragma unroll
-                    for (int i = 0; i < CP; ++i) acc[i] = fmaf(__uint_as_float(r[i]), sw, acc[i]);
+                for (int i = 0; i < CP; ++i) r[i] = 0u;
+                if (ok) tmem_ld_cols<CP>(tlane + (uint32_t)(g * MP + col0), r);
+#pragma unroll
+                for (int i = 0; i < CP; ++i) acc[i] = __uint_as_float(r[i]);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accempty0 + g * 8);
+                ag.next(NB);
+            } else {
+                if (s0 == k_lo) {  // a new tile
+#pragma unroll
+                    for (int i = 0; i < CP; ++i) acc[i] = 0.0f;
+                    const int row = min(tile * TR + min(rc, TR - 1), p.n - 1);
+                    swrow = sw_s + (int)(((A.row0 + row) >> p.bn_shift) - srow_lo) * p.skb;
                 }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(accempty0 + g * 8);
-            st.next(NS);
-            ag.next(NB);
-            if (s0 + nsl == k_hi) {  // this CTA's slabs of the tile are done
-                if (p.csize == 1) {
-                    finalize(acc, tile);
-                } else if (crank == 1) {
-                    // second CTA of the pair: hand the sums to the first one, into its shared memory
-                    if (ntile_done > 0) mbar_wait_cluster(rxempty, (uint32_t)(ntile_done - 1) & 1u, X.status);  // the previous tile's have been read
-                    const uint32_t dst = mapa_u32(smem_u32(smem + S.rx) + (uint32_t)rc * 4u, 0u);
+                if (ok && !mbar_wait(done0 + st.s * 8, st.ph, X.status)) ok = false;
+                ok = __all_sync(0xffffffffu, ok);
+                tc_fence_after();
+                if (ok) {
+                    for (int j = 0; j < nsl; ++j) {
+                        const float sw = swrow[(kofs + (s0 + j) * 128) >> p.bk_shift];
+                        uint32_t r[CP];
+                        tmem_ld_cols<CP>(tlane + (uint32_t)((g * SL + j) * MP + col0), r);  // returns once the values are in registers
 #pragma unroll
-                    for (int i = 0; i < CP; ++i)
-                        if (col0 + i < p.m) st_cluster_f32(dst + (uint32_t)((col0 + i) * kBsMmaRows * 4), acc[i]);
-                    mbar_arrive_cluster(mapa_u32(rxfull, 0u));
-                } else {
-                    // first CTA: K half 0 (own) + K half 1 (the partner's), in that order
-                    mbar_wait_cluster(rxfull, (uint32_t)ntile_done & 1u, X.status);
-                    const float *rx = reinterpret_cast<const float *>(smem + S.rx) + rc;
-#pragma unroll
-                    for (int i = 0; i < CP; ++i)
-                        if (col0 + i < p.m) acc[i] += rx[(col0 + i) * kBsMmaRows];
-                    mbar_arrive_cluster(mapa_u32(rxempty, 1u));
-                    finalize(acc, tile);
+                        for (int i = 0; i < CP; ++i) acc[i] = fmaf(__uint_as_float(r[i]), sw, acc[i]);
+                    }
                 }
-                ++ntile_done;
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accempty0 + g * 8);
+                st.next(NS);
+                ag.next(NB);
+                if (!last) continue;
             }
+            if (p.csize == 1) {
+                finalize(acc, tile);
+            } else if (crank == 1) {
+                // second CTA of the pair: hand the sums to the first one, into its shared memory
+                if (ntile_done > 0) mbar_wait_cluster(rxempty, (uint32_t)(ntile_done - 1) & 1u, X.status);  // the previous tile's have been read
+                const uint32_t dst = mapa_u32(smem_u32(smem + S.rx) + (uint32_t)rc * 4u, 0u);
+#pragma unroll
+                for (int i = 0; i < CP; ++i)
+                    if (col0 + i < p.m) st_cluster_f32(dst + (uint32_t)((col0 + i) * kBsMmaRows * 4), acc[i]);
+                mbar_arrive_cluster(mapa_u32(rxfull, 0u));
+            } else {
+                // first CTA: K half 0 (own) + K half 1 (the partner's), in that order
+                mbar_wait_cluster(rxfull, (uint32_t)ntile_done & 1u, X.status);
+                const float *rx = reinterpret_cast<const float *>(smem + S.rx) + rc;
+#pragma unroll
+                for (int i = 0; i < CP; ++i)
+                    if (col0 + i < p.m) acc[i] += rx[(col0 + i) * kBsMmaRows];
+                mbar_arrive_cluster(mapa_u32(rxempty, 1u));
+                finalize(acc, tile);
+            }
+            ++ntile_done;
         }
 
         // ---- exchange (the epilogue threads)
@@ -616,7 +722,7 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
                 }
             }
         } else if (p.mode == kModeLmHead) {
-            // Only the argmax is wanted.  The CTAs of a rank leave their candidates in the rank's own
+            // The argmax.  The CTAs of a rank leave their candidates in the rank's own
             // table; the CTA that arrives last merges them into ONE (value, lowest index) per token,
             // sends it to every peer and merges the ranks' candidates: one 64-bit store and one flag
             // per peer and step instead of one per CTA.
@@ -681,6 +787,26 @@ __global__ void __launch_bounds__(bs_threads(MP), 1) fp8_bs_kernel(const __grid_
                         const uint64_t best = merge(t, p.world, [&](int i) { return table + ((size_t)i * kMaxCtas + kRankRow) * p.lay.max_m; });
                         if (lane == 0) A.argmax[t] = ((uint32_t)best == 0xFFFFFFFFu) ? 0u : (uint32_t)best;
                     }
+            }
+            if (p.gather_logits && p.world > 1) {
+                // every CTA's rows are in every rank's gather buffer once its flag is there (the barriers above
+                // order the stores before this release); each CTA then copies a share of the vocabulary out
+                if (et < p.world) {
+                    uint32_t *f = reinterpret_cast<uint32_t *>(X.sym[et] + p.lay.flags_off) + ((size_t)bank * p.world + X.rank) * nflag;
+                    st_release_sys(f + cta, seq);
+                }
+                if (A.logits != nullptr) {
+                    for (int i = et; i < p.world * ncta; i += ET)
+                        wait_flag(myflags + (size_t)(i / ncta) * nflag + (i % ncta), seq, p.timeout_ns, X.status, kStatTimeoutGather);
+                    bs_epi_bar();
+                    const float *gl = reinterpret_cast<const float *>(X.sym[X.rank] + p.lay.gather_off) +
+                                      (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab;
+                    const int64_t per = ((int64_t)p.vocab + ncta - 1) / ncta;
+                    const int64_t v0 = (int64_t)cta * per, v1 = min((int64_t)p.vocab, v0 + per);
+                    for (int tok = 0; tok < p.m; ++tok)
+                        for (int64_t v = v0 + et; v < v1; v += ET)
+                            A.logits[(size_t)tok * p.vocab + v] = __ldcg(gl + (size_t)tok * p.lay.max_vocab + v);
+                }
             }
         }
     }

@@ -192,12 +192,6 @@ __host__ __device__ inline MoeBsSmem moe_bs_smem_layout(int nstages, int slabs_p
     return s;
 }
 
-// 3-D TMA tile load (codes, rows, expert), completion on an mbarrier.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
-}
-
 // Instruction descriptor: E2M1 weights (format code 5) x E4M3 activations, UE8M0 scales, M = 128, N = 16.
 __device__ __forceinline__ uint32_t moe_bs_idesc(int sf_id) {
     return ((uint32_t)sf_id << 4) | (5u << 7) | (0u << 10) | ((uint32_t)(kMoeBsCols >> 3) << 17) | (1u << 23) | (8u << 24) |
