@@ -611,7 +611,7 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     void (*kernel)(BsParams);
     if (u.wue) kernel = u.mp == 16 ? fp8_bs_kernel<16, true> : u.mp == 32 ? fp8_bs_kernel<32, true> : u.mp == 64 ? fp8_bs_kernel<64, true> : fp8_bs_kernel<128, true>;
     else kernel = u.mp == 16 ? fp8_bs_kernel<16, false> : u.mp == 32 ? fp8_bs_kernel<32, false> : u.mp == 64 ? fp8_bs_kernel<64, false> : fp8_bs_kernel<128, false>;
-    const int prep_blocks = (int)(((int64_t)mt * u.ks * 16 + 255) / 256);
+    const int prep_blocks = (int)std::min<int64_t>(std::max(1, t0->sm_count / n), ((int64_t)mt * u.ks * 16 + 255) / 256);
     ws_status_t s = zero_lone_shard(ranks, n, lm, m0, mt, streams);
     for (int i = 0; i < (same_device ? 1 : n) && s == WS_OK; ++i) {
         if (i > 0) {  // one launch per device, each sees itself as virtual rank 0

@@ -36,6 +36,8 @@
 
 #include <math.h>
 
+#include <type_traits>
+
 #include "ws_device.cuh"
 #include "ws_fp8_kernel.cuh"
 
@@ -81,31 +83,41 @@ struct ActPrepParams {
     ActPrepRank r[WS_MAX_WORLD];
 };
 
-// Thread = 8 values of one token; tokens the step does not carry are left out (their MMA columns are
-// never read), the K tail of the last slab is written as zeros.
+// Thread = 8 values of one token at a time; tokens the step does not carry are left out (their MMA columns
+// are never read), the K tail of the last slab is written as zeros.  At most one block per SM: with two
+// there are no registers left for the main kernel's CTA, which then starts late (measured at 40 rows:
+// some CTAs 4.6 us after the predecessor's end instead of 1).
 __global__ void __launch_bounds__(256) act_prep_kernel(const __grid_constant__ ActPrepParams p) {
     // The step that follows may become resident at once (it streams weights until its own wait);
     // the activations come from earlier work on the stream.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const ActPrepRank &A = p.r[blockIdx.y];
-    const int chunks_per_row = p.ks << 4;
-    const int64_t total = (int64_t)p.m * chunks_per_row;
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = c < total;
-    const int tok = in ? (int)(c / chunks_per_row) : 0;
-    const int ch = in ? (int)(c - (int64_t)tok * chunks_per_row) : 0;
-    const bool valid = in && ch * 8 < p.k;
-    float v[8];
-    load_act8(A.x, p.x_dtype, (int64_t)tok * A.ldx + ch * 8, valid, v);
-    int e;
-    uint32_t lo, hi;
-    act_quant8(v, e, lo, hi);  // the four lanes of a 32-block are adjacent threads of one warp
-    if (in) {
-        const BsImage o = bs_image_at(ch >> 4, p.ks, p.csize, p.sl, p.mp);
-        *reinterpret_cast<uint2 *>(A.img + o.tile + tok * 128 + ((((ch >> 1) & 7) ^ (tok & 7)) << 4) + (ch & 1) * 8) = make_uint2(lo, hi);
-        if ((ch & 3) == 0)
-            A.img[o.atom + (tok & 31) * 16 + (tok >> 5) * 4 + ((ch >> 2) & 3)] = (uint8_t)min(max(e + 127, 0), 255);
+    const int chunks_per_row = p.ks << 4, total = p.m * chunks_per_row, step = gridDim.x * blockDim.x;
+    constexpr int U = 4;  // chunks whose loads are in flight together
+    for (int c0 = blockIdx.x * blockDim.x + threadIdx.x; c0 - (int)(threadIdx.x & 31) < total; c0 += U * step) {  // whole warps
+        float v[U][8];
+        int tok[U], ch[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + u * step;
+            tok[u] = c < total ? c / chunks_per_row : 0;
+            ch[u] = c - tok[u] * chunks_per_row;
+            load_act8(A.x, p.x_dtype, (int64_t)tok[u] * A.ldx + ch[u] * 8, c < total && ch[u] * 8 < p.k, v[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            int e;
+            uint32_t lo, hi;
+            act_quant8(v[u], e, lo, hi);  // the four lanes of a 32-block are adjacent threads of one warp
+            if (c0 + u * step < total) {
+                const BsImage o = bs_image_at(ch[u] >> 4, p.ks, p.csize, p.sl, p.mp);
+                const int t = tok[u];
+                *reinterpret_cast<uint2 *>(A.img + o.tile + t * 128 + ((((ch[u] >> 1) & 7) ^ (t & 7)) << 4) + (ch[u] & 1) * 8) = make_uint2(lo, hi);
+                if ((ch[u] & 3) == 0)
+                    A.img[o.atom + (t & 31) * 16 + (t >> 5) * 4 + ((ch[u] >> 2) & 3)] = (uint8_t)min(max(e + 127, 0), 255);
+            }
+        }
     }
 }
 
@@ -184,15 +196,14 @@ __device__ __forceinline__ uint32_t bs_idesc(int n, int sfa, int sfb) {
 // D[tmem] (+)= A[smem] * B[smem] with per-32 scales from tensor memory.  The descriptors arrive as
 // their 32-bit halves: the upper half is the same for every operand tile, the lower one advances by
 // two (32 bytes) per K block, so the single issuing thread spends two adds per MMA on them.
-template <bool ACCUMULATE>
 __device__ __forceinline__ void umma_bs_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t a_hi, uint32_t b_hi,
-                                           uint32_t idesc, uint32_t tsfa, uint32_t tsfb) {
+                                           uint32_t idesc, uint32_t tsfa, uint32_t tsfb, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
         "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %4};\n\t"
         "setp.ne.b32 p, %8, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], da, db, %5, [%6], [%7], p;\n\t}"
-        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(a_hi), "r"(b_hi), "r"(idesc), "r"(tsfa), "r"(tsfb), "n"(ACCUMULATE ? 1 : 0)
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(a_hi), "r"(b_hi), "r"(idesc), "r"(tsfa), "r"(tsfb), "r"(accumulate)
         : "memory");
 }
 // Halves of the 128B-swizzled K-major operand descriptor (see umma_desc): 8-row groups 1024 bytes apart.
@@ -328,7 +339,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
     const int vr = blockIdx.y, cta = blockIdx.x, ncta = gridDim.x;
     const Fp8RankArgs &A = p.r[vr];
     const RankCtx &X = A.ctx;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
 
     const int KS = p.ks;                                    // slabs per tile
     // CTA pairs: which half of K is this CTA's, and which pair of how many it belongs to
@@ -391,7 +402,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer (one thread)
-        if (lane == 0) {
+        if (elect_one()) {
             // Weights are static: the first ring's worth streams before the wait on the prep kernel;
             // the activations follow once it has finished.
             constexpr uint32_t kXSlab = MP * 128 + kBsAtomBytes;
@@ -430,7 +441,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
         // launch failure" in most attempts, in a different CTA and stage item each time, and never with
         // one thread; the barrier hand-offs are the same either way, so the cause is not known.
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (lane == 0) {
+        if (elect_one()) {
             if (!WUE) tmem_cp_atom(t_sfa, umma_desc(wsf0, 128, false));
             // Everything the loop needs per MMA is an add away: descriptor halves per stage slot, the
             // four instruction descriptors (one per K block of a slab), ring positions kept incrementally.
@@ -449,24 +460,31 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
                 if (!mbar_wait(full0 + s * 8, st.ph, X.status)) break;
                 if ((!WUE || s0 == k_lo) && !mbar_wait(accempty0 + g * 8, ag.ph ^ 1u, X.status)) break;
                 tc_fence_after();
-                uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = x_lo0 + (uint32_t)s * x_stage;
-                uint64_t xsf = xsf_desc0 + (uint64_t)((uint32_t)s * x_stage + (uint32_t)nsl * kXStep);
-                uint64_t wsf = wsf_desc0 + (uint64_t)((uint32_t)(s * SL) * kSfStep);
-                uint32_t t_acc = tmem_base + (uint32_t)((WUE ? g : g * SL) * MP);
-                uint32_t t_sf = t_sf0 + (WUE ? (uint32_t)((item & 1) * SL * 8) : (uint32_t)(g * SL * 4));
-                for (int j = 0; j < nsl; ++j) {
-                    const uint32_t t_w = WUE ? t_sf + 4 : t_sfa;
-                    tmem_cp_atom(t_sf, xsf);
-                    if (WUE) tmem_cp_atom(t_sf + 4, wsf);
-                    if (WUE && s0 + j != k_lo) umma_bs_ss<true>(t_acc, a_lo, b_lo, kUmmaDescHiSw128, kUmmaDescHiSw128, id[0], t_w, t_sf);
-                    else umma_bs_ss<false>(t_acc, a_lo, b_lo, kUmmaDescHiSw128, kUmmaDescHiSw128, id[0], t_w, t_sf);
-                    umma_bs_ss<true>(t_acc, a_lo + 2, b_lo + 2, kUmmaDescHiSw128, kUmmaDescHiSw128, id[1], t_w, t_sf);
-                    umma_bs_ss<true>(t_acc, a_lo + 4, b_lo + 4, kUmmaDescHiSw128, kUmmaDescHiSw128, id[2], t_w, t_sf);
-                    umma_bs_ss<true>(t_acc, a_lo + 6, b_lo + 6, kUmmaDescHiSw128, kUmmaDescHiSw128, id[3], t_w, t_sf);
-                    a_lo += a_step; b_lo += kXStep; xsf += kSfStep; wsf += kSfStep;
-                    t_sf += WUE ? 8 : 4;
-                    if (!WUE) t_acc += MP;
-                }
+                const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = x_lo0 + (uint32_t)s * x_stage;
+                const uint64_t xsf = xsf_desc0 + (uint64_t)((uint32_t)s * x_stage + (uint32_t)nsl * kXStep);
+                const uint64_t wsf = wsf_desc0 + (uint64_t)((uint32_t)(s * SL) * kSfStep);
+                const uint32_t t_acc = tmem_base + (uint32_t)((WUE ? g : g * SL) * MP);
+                const uint32_t t_sf = t_sf0 + (WUE ? (uint32_t)((item & 1) * SL * 8) : (uint32_t)(g * SL * 4));
+                const uint32_t carry = WUE && s0 != k_lo ? 1u : 0u;  // the stage's first MMA adds to earlier stages' sums
+                // straight-line code per slab count: a rolled loop costs the issuing thread twice the time
+                auto issue = [&](auto count) {
+#pragma unroll
+                    for (int j = 0; j < decltype(count)::value; ++j) {
+                        const uint32_t a = a_lo + (uint32_t)j * a_step, b = b_lo + (uint32_t)j * kXStep;
+                        const uint32_t d = WUE ? t_acc : t_acc + (uint32_t)(j * MP);
+                        const uint32_t sx = t_sf + (uint32_t)(j * (WUE ? 8 : 4)), sw = WUE ? sx + 4 : t_sfa;
+                        tmem_cp_atom(sx, xsf + (uint64_t)(j * kSfStep));
+                        if (WUE) tmem_cp_atom(sw, wsf + (uint64_t)(j * kSfStep));
+                        umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiSw128, id[0], sw, sx, WUE && j > 0 ? 1u : carry);
+                        umma_bs_ss(d, a + 2, b + 2, kUmmaDescHiSw128, kUmmaDescHiSw128, id[1], sw, sx, 1u);
+                        umma_bs_ss(d, a + 4, b + 4, kUmmaDescHiSw128, kUmmaDescHiSw128, id[2], sw, sx, 1u);
+                        umma_bs_ss(d, a + 6, b + 6, kUmmaDescHiSw128, kUmmaDescHiSw128, id[3], sw, sx, 1u);
+                    }
+                };
+                if (nsl == 4) issue(std::integral_constant<int, 4>{});
+                else if (nsl == 3) issue(std::integral_constant<int, 3>{});
+                else if (nsl == 2) issue(std::integral_constant<int, 2>{});
+                else issue(std::integral_constant<int, 1>{});
                 umma_commit(done0 + s * 8);  // the stage may be refilled (fp32 weight scales: and its accumulators read)
                 if (!WUE) ag.next(NB);
                 else if (s0 + nsl == k_hi) {
@@ -666,7 +684,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
 #pragma unroll
                 for (int i = 0; i < CP; ++i)
                     if (col0 + i < p.m) acc[i] += rx[(col0 + i) * kBsMmaRows];
-                mbar_arrive_cluster(mapa_u32(rxempty, 1u));
+                if (tile < t_hi) mbar_arrive_cluster(mapa_u32(rxempty, 1u));  // nobody waits for the last one
                 finalize(acc, tile);
             }
             ++ntile_done;
@@ -815,7 +833,10 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
     tc_fence_before();
     __syncthreads();
     if (p.csize == 2) {  // neither CTA of a pair leaves while the other may still write to or signal it
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        // The first CTA's remote arrivals were all seen by the second, so it need not wait for its own output
+        // stores to reach memory (a release would: ~1 us).
+        if (crank == 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+        else asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     if (warp == 1) {

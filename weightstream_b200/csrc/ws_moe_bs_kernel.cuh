@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
     const int vr = blockIdx.y, cta = blockIdx.x, ncta = gridDim.x;
     const MoeBsRank &A = p.r[vr];
     const RankCtx &X = A.ctx;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
     uint32_t crank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
     const int part = cta >> 1, TR = p.tile_rows;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer (one thread)
-        if (lane == 0) {
+        if (elect_one()) {
             // the unpacking copy counts the packed bytes it read (64 per row), not the 128 it wrote
             const uint32_t slab_tx = (uint32_t)(TR * 64 + kMoeBsXSlab);
             RingPos st;
@@ -285,12 +285,12 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issue (one thread)
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t id0 = moe_bs_idesc(0), id1 = moe_bs_idesc(1), id2 = moe_bs_idesc(2), id3 = moe_bs_idesc(3);
             const uint32_t a_lo0 = umma_desc_lo(a0), b_lo0 = umma_desc_lo(b0);
             const uint32_t a_step = (uint32_t)p.a_pitch >> 4, b_step = (uint32_t)kMoeBsXTile >> 4;
             const uint64_t sf_desc0 = umma_desc(b0 + (uint32_t)(SL * kMoeBsXTile), 128, false);  // a stage's atoms follow its tiles
-            const uint32_t sf_step = (uint32_t)kBsAtomBytes >> 4;
+            constexpr uint32_t sf_step = (uint32_t)kBsAtomBytes >> 4;
             RingPos st;
             bool ok = true;
             for (int ps = 0; ps < npass && ok; ++ps) {
@@ -300,24 +300,29 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
                 tc_fence_after();
                 const uint32_t t_acc = tmem_base + (uint32_t)(g * kMoeBsCols);
                 uint32_t t_sc = t_sc0 + (uint32_t)(g * NSLAB * 8);
-                bool first = true;
                 for (int i = 0; i < IP; ++i, st.next(NS)) {
                     const int s = st.s, nsl = min(SL, NSLAB - i * SL);
                     if (!mbar_wait(full0 + s * 8, st.ph, X.status)) { ok = false; break; }
                     tc_fence_after();
-                    uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = b_lo0 + (uint32_t)s * (stage_x >> 4);
-                    uint64_t sf_desc = sf_desc0 + (uint64_t)((uint32_t)s * (stage_x >> 4));
-                    for (int j = 0; j < nsl; ++j) {
-                        tmem_cp_atom(t_sc, sf_desc);          // the activations' scales of this slab (the weights' are there already)
-                        if (first) umma_bs_ss<false>(t_acc, a_lo, b_lo, kUmmaDescHiSw128, kUmmaDescHiSw128, id0, t_sc + 4, t_sc);
-                        else umma_bs_ss<true>(t_acc, a_lo, b_lo, kUmmaDescHiSw128, kUmmaDescHiSw128, id0, t_sc + 4, t_sc);
-                        umma_bs_ss<true>(t_acc, a_lo + 2, b_lo + 2, kUmmaDescHiSw128, kUmmaDescHiSw128, id1, t_sc + 4, t_sc);
-                        umma_bs_ss<true>(t_acc, a_lo + 4, b_lo + 4, kUmmaDescHiSw128, kUmmaDescHiSw128, id2, t_sc + 4, t_sc);
-                        umma_bs_ss<true>(t_acc, a_lo + 6, b_lo + 6, kUmmaDescHiSw128, kUmmaDescHiSw128, id3, t_sc + 4, t_sc);
-                        first = false;
-                        a_lo += a_step; b_lo += b_step; sf_desc += sf_step;
-                        t_sc += 8;
-                    }
+                    const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = b_lo0 + (uint32_t)s * (stage_x >> 4);
+                    const uint64_t sf_desc = sf_desc0 + (uint64_t)((uint32_t)s * (stage_x >> 4));
+                    // straight-line code per slab count, as in the FP8 kernel
+                    auto issue = [&](auto count) {
+#pragma unroll
+                        for (int j = 0; j < decltype(count)::value; ++j) {
+                            const uint32_t a = a_lo + (uint32_t)j * a_step, b = b_lo + (uint32_t)j * b_step, sx = t_sc + (uint32_t)(j * 8);
+                            tmem_cp_atom(sx, sf_desc + (uint64_t)(j * sf_step));  // the activations' scales of this slab (the weights' are there already)
+                            umma_bs_ss(t_acc, a, b, kUmmaDescHiSw128, kUmmaDescHiSw128, id0, sx + 4, sx, j > 0 || i > 0 ? 1u : 0u);
+                            umma_bs_ss(t_acc, a + 2, b + 2, kUmmaDescHiSw128, kUmmaDescHiSw128, id1, sx + 4, sx, 1u);
+                            umma_bs_ss(t_acc, a + 4, b + 4, kUmmaDescHiSw128, kUmmaDescHiSw128, id2, sx + 4, sx, 1u);
+                            umma_bs_ss(t_acc, a + 6, b + 6, kUmmaDescHiSw128, kUmmaDescHiSw128, id3, sx + 4, sx, 1u);
+                        }
+                    };
+                    if (nsl == 4) issue(std::integral_constant<int, 4>{});
+                    else if (nsl == 3) issue(std::integral_constant<int, 3>{});
+                    else if (nsl == 2) issue(std::integral_constant<int, 2>{});
+                    else issue(std::integral_constant<int, 1>{});
+                    t_sc += (uint32_t)(nsl * 8);
                     umma_commit(done0 + s * 8);  // the stage may be refilled
                 }
                 if (!ok) break;
@@ -349,11 +354,12 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("bar.sync 3, 128;" ::: "memory");
             if (*reinterpret_cast<volatile uint32_t *>(misc_s + 8) != 0u) break;
-            if (r == 0) {
+            if (warp == 6 && elect_one()) {
                 tc_fence_after();
                 const uint32_t t_sfa = t_sc0 + (uint32_t)(g * NSLAB * 8) + 4u;
-                for (int j = 0; j < NSLAB; ++j)
-                    tmem_cp_atom(t_sfa + (uint32_t)(j * 8), sfa_desc0 + (uint64_t)((uint32_t)(g * NSLAB + j) * ((uint32_t)kBsAtomBytes >> 4)));
+                const uint64_t sfa_desc = sfa_desc0 + (uint64_t)((uint32_t)(g * NSLAB) * ((uint32_t)kBsAtomBytes >> 4));
+#pragma unroll 4
+                for (int j = 0; j < NSLAB; ++j) tmem_cp_atom(t_sfa + (uint32_t)(j * 8), sfa_desc + (uint64_t)((uint32_t)j * ((uint32_t)kBsAtomBytes >> 4)));
                 umma_commit(sfafull0 + g * 8);
             }
         }
