@@ -488,12 +488,12 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     u.ntiles = (a.n + u.tile_rows - 1) / u.tile_rows;
     const int tiles_per_cta = (u.ntiles + nparts - 1) / nparts;
     u.a_pitch = u.tile_rows * 128;
-    const int x_slab = u.mp * 128 + kBsAtomBytes, slab_bytes = u.a_pitch + x_slab + (u.wue ? kBsAtomBytes : 0);
+    const int x_slab = mt * 128 + bs_atom_bytes(mt), slab_bytes = u.a_pitch + x_slab + (u.wue ? kBsAtomBytes : 0);
     // slabs per stage: one MMA commit (a ~160 ns stall of the issuing thread) and two copies (~100 ns each)
     // per stage, so several slabs share it; bounded by the stage size and by tensor memory (fp32 scales: each
     // slab has its own accumulator buffer, groups x slabs x (mp + 4) + 8 columns of 512, at least two groups)
     u.nslot_max = (tiles_per_cta * u.tile_rows) / a.block_n + 2;
-    const int rx_rows = u.csize == 2 ? mt : 0, kcta = (u.ks + u.csize - 1) / u.csize;
+    const int rx_rows = u.csize == 2 ? (mt + 1) / 2 : 0, kcta = (u.ks + u.csize - 1) / u.csize;
     // Half an SM (shared memory and tensor memory) when the tokens are few and the CTA's whole share of
     // the weights fits such a ring (TP-8 shards): the next step's CTA is then resident beside this one
     // (one CTA per SM and step) and loads all of its weights under this step's exchange and exit.
@@ -506,7 +506,7 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         u.slabs_per_stage = std::max(1, std::min({4, stage_target / slab_bytes, kcta, u.wue ? 4 : (tmem - 8) / (2 * (u.mp + 4))}));
         const int groups = (kcta + u.slabs_per_stage - 1) / u.slabs_per_stage;
         u.slabs_per_stage = (kcta + groups - 1) / groups;  // groups of equal size, so that few slabs travel outside whole boxes
-        u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * x_slab, 1024);
+        u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * x_slab, 128);
         u.nacc = u.wue ? std::min(2, std::max(1, (tmem - 8 - 2 * u.slabs_per_stage * 8) / u.mp))
                        : std::min((int)kBsMaxAcc, (tmem - 8) / (u.slabs_per_stage * (u.mp + 4)));
         auto total = [&](int ns) {
@@ -524,7 +524,10 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         if (!u.ok || (half && items > ns)) continue;  // half an SM only when the CTA's whole share of the weights fits the ring
         u.smem = (size_t)total(ns);
         int cols = 32;
-        while (cols < (u.wue ? u.nacc * u.mp + 2 * u.slabs_per_stage * 8 : u.nacc * u.slabs_per_stage * (u.mp + 4) + 4)) cols *= 2;
+        // (fp32 scales: the epilogue reads the accumulators of a group in batches, see fp8_bs_kernel)
+        const int batch = std::max(1, 64 / (u.mp * 4 / bs_epi_warps(u.mp))), read = (u.slabs_per_stage + batch - 1) / batch * batch;
+        while (cols < (u.wue ? u.nacc * u.mp + 2 * u.slabs_per_stage * 8
+                             : std::max(u.nacc * u.slabs_per_stage * (u.mp + 4) + 4, ((u.nacc - 1) * u.slabs_per_stage + read) * u.mp))) cols *= 2;
         u.tmem_cols = half ? std::min(cols, 256) : 512;
         break;
     }
@@ -564,7 +567,7 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     ws_tp *t0 = ranks[0];
     const ws_fp8_gemm_args_t &a0 = lm ? lm[0].g : args[0];
     BsParams p{};
-    p.m = mt; p.mp = u.mp; p.n = a0.n; p.k = a0.k; p.ks = u.ks; p.world = t0->world;
+    p.m = mt; p.cols = (mt + 15) / 16 * 16; p.n = a0.n; p.k = a0.k; p.ks = u.ks; p.world = t0->world;
     for (p.bk_shift = 0; (1 << p.bk_shift) < a0.block_k; ++p.bk_shift) {}
     for (p.bn_shift = 0; (1 << p.bn_shift) < a0.block_n; ++p.bn_shift) {}
     p.mode = lm ? kModeLmHead : kModeAllReduce;
@@ -578,14 +581,14 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
     ActPrepParams q{};
-    q.m = mt; q.mp = u.mp; q.k = a0.k; q.x_dtype = a0.x_dtype; q.ks = u.ks; q.csize = u.csize; q.sl = u.slabs_per_stage;
-    // scratch of one endpoint: the activation image
-    const size_t img_bytes = (size_t)u.ks * (kBsMaxTokens * 128 + kBsAtomBytes);
+    q.m = mt; q.k = a0.k; q.x_dtype = a0.x_dtype; q.ks = u.ks;
+    // scratch of one endpoint: the quantised activations and their scale atoms
+    const size_t xq_bytes = (size_t)u.ks * kBsMaxTokens * 128, xsf_bytes = (size_t)u.ks * kBsAtomBytes;
 
     for (int i = 0; i < n; ++i) {
         ws_tp *t = ranks[i];
         const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
-        ws_status_t s = ensure_bs_scratch(t, img_bytes);
+        ws_status_t s = ensure_bs_scratch(t, xq_bytes + xsf_bytes);
         if (s == WS_OK)  // (with less than one whole slab only the second map is used)
             s = make_tmap_slabs(t, &p.tmap_w[i], a.w, (uint64_t)a.n, (uint64_t)std::max(1, a.k / 128), (uint64_t)a.ldw, (uint32_t)u.tile_rows,
                                 (uint32_t)u.slabs_per_stage);
@@ -602,29 +605,30 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         r.vocab_row0 = lm ? lm[i].vocab_row0 : 0;
         r.ctx = make_ctx(t);
         if (last) r.ctx.host_done = t->host_done_arm;
-        p.img[i] = t->bs_work;
+        p.xq[i] = q.r[i].xq = t->bs_work;
+        p.xsf[i] = q.r[i].xsf = t->bs_work + xq_bytes;
         q.r[i].x = static_cast<const char *>(a.x) + (size_t)m0 * a.ldx * (a.x_dtype == WS_ACT_BF16 ? 2 : 4);
-        q.r[i].img = t->bs_work;
         q.r[i].ldx = a.ldx;
     }
     for (int i = 0; i < n; ++i) ranks[i]->step++;
     void (*kernel)(BsParams);
     if (u.wue) kernel = u.mp == 16 ? fp8_bs_kernel<16, true> : u.mp == 32 ? fp8_bs_kernel<32, true> : u.mp == 64 ? fp8_bs_kernel<64, true> : fp8_bs_kernel<128, true>;
     else kernel = u.mp == 16 ? fp8_bs_kernel<16, false> : u.mp == 32 ? fp8_bs_kernel<32, false> : u.mp == 64 ? fp8_bs_kernel<64, false> : fp8_bs_kernel<128, false>;
-    const int prep_blocks = (int)std::min<int64_t>(std::max(1, t0->sm_count / n), ((int64_t)mt * u.ks * 16 + 255) / 256);
+    const int prep_blocks = (int)std::min<int64_t>(std::max(1, t0->sm_count / n), ((int64_t)mt * u.ks * 8 + kActPrepThreads - 1) / kActPrepThreads);
     ws_status_t s = zero_lone_shard(ranks, n, lm, m0, mt, streams);
     for (int i = 0; i < (same_device ? 1 : n) && s == WS_OK; ++i) {
         if (i > 0) {  // one launch per device, each sees itself as virtual rank 0
             p.r[0] = p.r[i];
             p.tmap_w[0] = p.tmap_w[i];
             p.tmap_t[0] = p.tmap_t[i];
-            p.img[0] = p.img[i];
+            p.xq[0] = p.xq[i];
+            p.xsf[0] = p.xsf[i];
             q.r[0] = q.r[i];
         }
         const int nvr = same_device ? n : 1;
         WS_CUDA(ranks[i], cudaSetDevice(ranks[i]->device));
         cudaStream_t cs = static_cast<cudaStream_t>(streams ? streams[i] : nullptr);
-        s = launch(ranks[i], act_prep_kernel, q, prep_blocks, nvr, 256, 0, cs, t0->pdl != 0, false);
+        s = launch(ranks[i], act_prep_kernel, q, prep_blocks, nvr, kActPrepThreads, 0, cs, t0->pdl != 0, false);
         if (s == WS_OK) s = launch(ranks[i], kernel, p, u.ncta, nvr, bs_threads(u.mp, u.wue), u.smem, cs, t0->pdl != 0, true, u.csize);
         if (s != WS_OK) t0->err = ranks[i]->err;
     }
@@ -958,29 +962,32 @@ static ws_status_t ensure_moe_scratch(ws_tp *tp, size_t work_bytes, size_t acc_b
 // in halves of at most 16 slabs, a pair's rows are one MMA tile, the per-token sums live in shared memory).
 struct MoeBsPlan {
     bool ok;
-    int ncta, tile_rows, a_pitch, slabs_per_stage, nstages, tmem_cols;
+    int ncta, tile_rows, a_pitch, slabs_per_stage, nstages, tmem_cols, x_pitch, alias;
     size_t smem;
 };
 static MoeBsPlan moe_bs_plan(const ws_moe_down_args_t &a, int ncta) {
     MoeBsPlan u{};
     u.ncta = ncta & ~1;
-    const int nparts = u.ncta / 2, kslabs = a.k / 128;
-    if (nparts < 1 || a.k % 256 || kslabs / 2 > kMoeBsMaxSlabs || a.m > 64) return u;  // 64 tokens: their sums fill 64 KB of shared memory
+    const int nparts = u.ncta / 2, nslab = a.k / 256;
+    if (nparts < 1 || a.k % 256 || nslab > kMoeBsMaxSlabs) return u;
     u.tile_rows = (a.n + nparts - 1) / nparts;
     if (u.tile_rows > kBsMmaRows) return u;
     u.a_pitch = (u.tile_rows + 7) / 8 * 8 * 128;
-    const int nslab = kslabs / 2;
-    // a stage = 4 slabs (2 when the half of K is not a multiple of 4): one commit and one activation copy per stage
-    if (nslab % 2) return u;
-    u.slabs_per_stage = nslab % 4 ? 2 : 4;
+    u.slabs_per_stage = std::min(4, nslab);  // one commit and two activation copies per stage
+    if (getenv("X1")) u.slabs_per_stage = std::min(atoi(getenv("X1")), nslab);
+    const int nr = std::min((int)kMoeBsCols, a.m * a.top_k);  // most routes of a pass
+    u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * (nr * 128 + nr * 16), 128);
+    // the partner's sums land behind the ring, or, when there are many, in the ring itself after the last pass
+    u.alias = a.m > 8 ? 1 : 0;
+    auto total = [&](int ns) { return moe_bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, a.m, nslab, u.alias).total + 1024; };
     int ns = kMaxStages;
-    while (ns >= 2 && moe_bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, a.m, nslab).total + 1024 > kSmemBudget) --ns;
+    while (ns >= 2 && total(ns) > kSmemBudget - 8 * 1024) --ns;  // (beside a few blocks of the prep kernel)
     u.nstages = ns;
     int cols = 32;
     while (cols < 2 * kMoeBsCols + 2 * nslab * 8) cols *= 2;
     u.tmem_cols = cols;
-    u.ok = ns >= 2 && cols <= 512;
-    if (u.ok) u.smem = (size_t)moe_bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, a.m, nslab).total + 1024;
+    u.ok = ns >= 2 && cols <= 512 && (!u.alias || (a.m + 1) / 2 * kBsMmaRows * 4 <= ns * u.slabs_per_stage * u.a_pitch);
+    if (u.ok) u.smem = (size_t)total(ns);
     return u;
 }
 
@@ -993,11 +1000,11 @@ static ws_status_t moe_bs_step(ws_tp *const *ranks, int n, const ws_moe_down_arg
     MoeBsParams p{};
     p.m = a0.m; p.n = a0.n; p.k = a0.k; p.world = t0->world;
     p.tile_rows = u.tile_rows; p.a_pitch = u.a_pitch; p.slabs_per_stage = u.slabs_per_stage; p.nstages = u.nstages;
-    p.tmem_cols = u.tmem_cols;
+    p.tmem_cols = u.tmem_cols; p.x_pitch = u.x_pitch; p.alias = u.alias;
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
     MoeBsPrepParams q{};
-    q.m = a0.m; q.k = a0.k; q.top_k = a0.top_k; q.h_dtype = a0.h_dtype; q.sl = u.slabs_per_stage;
+    q.m = a0.m; q.k = a0.k; q.top_k = a0.top_k; q.h_dtype = a0.h_dtype;
     const MoeBsWork W = moe_bs_work_layout(a0.k);
     const int nblk = a0.m * a0.top_k + 1;
     for (int i = 0; i < n; ++i) ranks[i]->step++;

@@ -477,6 +477,22 @@ __device__ __forceinline__ void act_quant8(const float (&v)[8], int &e, uint32_t
     hi = cvt_e4m3x2(v[4] * inv, v[5] * inv) | (cvt_e4m3x2(v[6] * inv, v[7] * inv) << 16);
 }
 
+// Sixteen values held by one lane (half of a 32-block shared by two adjacent lanes): the block exponent
+// and the sixteen E4M3 bytes in k order.
+__device__ __forceinline__ uint4 act_quant16(const float (&v)[16], int &e) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    e = act_scale_exp(amax);
+    const float inv = e > 127 ? 0.0f : pow2_f32(-e);  // an infinite block scale divides everything to zero
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        w[i] = cvt_e4m3x2(v[4 * i] * inv, v[4 * i + 1] * inv) | (cvt_e4m3x2(v[4 * i + 2] * inv, v[4 * i + 3] * inv) << 16);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // Load eight consecutive activations (bf16 or f32) as floats, zero beyond `valid`.
 __device__ __forceinline__ void load_act8(const void *base, int x_dtype, int64_t elem_off, bool valid,
                                           float (&v)[8]) {

@@ -3,15 +3,21 @@
 // exchange (sm_100a).  One pass over the weights for up to 128 activation rows.
 //
 //   act_prep_kernel   quantises the activations once per step exactly as the reference does
-//                     (crates/weightstream-ref/src/actquant.rs:21-57) into an image of what the main
-//                     kernel's stages hold, so that one bulk copy fills a stage's share of it.
+//                     (crates/weightstream-ref/src/actquant.rs:21-57) into the form the MMA reads: 16-byte
+//                     chunks of K, chunk-major ([chunk][token][16 bytes]), and the per-32 exponents as one
+//                     scale atom per 128-wide K slab.
 //   fp8_bs_kernel     persistent, one CTA per SM.  The rows are cut into tiles of at most 128 rows (the
 //                     M of the MMA), dealt out whole; a CTA (or a CTA pair, each CTA one half of K)
 //                     streams the weights of its tiles, so every output is a complete dot product inside
 //                     one CTA pair and nothing is combined through global memory.  A stage of the ring
-//                     holds SL K slabs of 128: their weight rows (ONE 3-D TMA box, 128B swizzle) and their
-//                     activation image (SL tiles of tokens x 128 bytes, swizzled alike, then SL 512-byte
-//                     scale atoms: byte (t & 31) * 16 + (t >> 5) * 4 + j = exponent of token t, K block j).
+//                     holds SL K slabs of 128: their weight rows (ONE 3-D TMA box, 128B swizzle), their
+//                     activations and their scale atoms (one bulk copy each).  The activation operand is
+//                     unswizzled K-major with core matrices 16 * m bytes apart along K, so m tokens take
+//                     m * 128 bytes per slab whatever N is: its columns past m read the neighbouring chunk
+//                     and are never looked at.  (Padded to N rows the activations of 40 tokens were as many
+//                     bytes as the weights, and what L2 can hand the SMs bound the step.)  An atom is
+//                     min(m, 32) rows of 16 bytes: byte (t & 31) * 16 + (t >> 5) * 4 + j = exponent of token
+//                     t, K block j.
 //                     One thread copies the atoms into tensor memory (tcgen05.cp) and issues four MMAs per
 //                     slab (M=128, N=tokens, K=32): the activations' per-32 scales ride the MMA's scale
 //                     operand.
@@ -22,11 +28,10 @@
 //                     bytes out as atoms in the stage, a tile accumulates over all of its K in tensor
 //                     memory and is read back once.
 //
-// Measured on B200 and kept in mind above: every TMA or bulk copy costs its issuing thread ~100 ns, so a
-// stage is two copies (one box, one image) and not three per slab; the tensor pipe needs 30-45 ns per K=32
-// MMA at M=128 however few of the rows are real (M=64 is not available with block scaling); a
-// tcgen05.commit stalls the issuing thread for ~160 ns; handing partial sums from one CTA to another
-// through L2 (a split of K across CTAs) costs 3-5 us, more than it saves on these shapes.
+// Measured on B200 and kept in mind above: a slab's four MMAs, scale copy and share of the commit take the
+// tensor pipe 84 ns with N=16, 105 with 64 and 135 with 128, however few of the 128 rows are real (M=64 is
+// not available with block scaling); handing partial sums from one CTA to another through L2 (a split of K
+// across CTAs) costs 3-5 us, more than it saves on these shapes.
 //
 // MMA rows past a tile's end are computed on whatever follows in shared memory and never read back.
 // Exchange and lm_head mode are those of the decode kernels (ws_fp8_kernel.cuh): tagged 64-bit
@@ -44,78 +49,68 @@
 namespace ws {
 
 // Threads of a CTA.  Warp 0: producer, warp 1: MMA issue (and owner of the tensor memory), then the
-// epilogue warps: four (one per 32-lane quarter of the tensor memory, all token columns) for up to 32
-// tokens, eight (two per quarter, half of the token columns each) for 64, where reading the
-// accumulators back is what a stage waits for (measured on B200, 64 rows: lm_head 324 -> 249 us;
-// with 32 rows eight warps were 3 % slower than four); then, for UE8M0 weight scales, four auxiliary warps.
-__host__ __device__ constexpr int bs_epi_warps(int mp) { return mp >= 64 ? 8 : 4; }
+// epilogue warps: four (one per 32-lane quarter of the tensor memory, all token columns) for up to 16
+// tokens, eight (two per quarter, half of the token columns each) beyond, where reading the
+// accumulators back is what a stage waits for; then, for UE8M0 weight scales, four auxiliary warps.
+__host__ __device__ constexpr int bs_epi_warps(int mp) { return mp >= 32 ? 8 : 4; }
 constexpr int kBsAuxWarps = 4;
 __host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 * (bs_epi_warps(mp) + (wue ? kBsAuxWarps : 0)); }
+// Registers per thread.  Up to 16 tokens two CTAs and a block of the prep kernel fit an SM together.
+__host__ __device__ constexpr int bs_regs(int mp, bool wue) { return mp == 16 ? (wue ? 88 : 144) : wue ? 128 : 168; }
 constexpr int kBsMaxAcc = 8;         // accumulator groups in tensor memory (a group = one stage's slabs)
 constexpr int kBsMaxTokens = 128;    // activation rows one launch takes (16, 32, 64 or 128 MMA columns)
 constexpr int kBsAtomBytes = 512;    // one scale atom: 128 rows x 4 K blocks
 constexpr int kBsMmaRows = 128;      // M of the MMA; a tile of output rows holds at most as many
 
-// The activation image of a step: the slabs in order, grouped as the CTAs' stages take them.  CTA half h
-// of K owns slabs [h * ks / csize, (h + 1) * ks / csize), in groups of at most sl; a group is its tiles
-// [mp tokens x 128 bytes, 16-byte chunk c of token t at c ^ (t & 7)], then its atoms.
-struct BsImage {
-    int32_t tile, atom;  // byte offsets of the slab's tile and atom inside the image
-};
-__host__ __device__ inline BsImage bs_image_at(int slab, int ks, int csize, int sl, int mp) {
-    int lo = 0, hi = ks;
-    if (csize == 2) {
-        if (slab >= ks / 2) lo = ks / 2;
-        else hi = ks / 2;
-    }
-    const int g0 = lo + (slab - lo) / sl * sl, n = sl < hi - g0 ? sl : hi - g0, base = g0 * (mp * 128 + kBsAtomBytes);
-    return BsImage{base + (slab - g0) * mp * 128, base + n * mp * 128 + (slab - g0) * kBsAtomBytes};
-}
+// Rows of a scale atom that exist in memory: the copy into tensor memory takes 32, those past the tokens'
+// come from whatever follows and scale columns that are never read.
+__host__ __device__ constexpr int bs_atom_bytes(int m) { return 16 * (m < 32 ? m : 32); }
 
 // ---------------------------------------------------------------- activation prep
 struct ActPrepRank {
     const void *x;
-    uint8_t *img;  // see BsImage
+    uint8_t *xq;   // [ks * 8 chunks][m][16] E4M3
+    uint8_t *xsf;  // [ks][bs_atom_bytes(m)]
     int64_t ldx;
 };
 struct ActPrepParams {
-    int32_t m, mp, k, x_dtype, ks, csize, sl, pad0;
+    int32_t m, k, x_dtype, ks;
     ActPrepRank r[WS_MAX_WORLD];
 };
 
-// Thread = 8 values of one token at a time; tokens the step does not carry are left out (their MMA columns
-// are never read), the K tail of the last slab is written as zeros.  At most one block per SM: with two
-// there are no registers left for the main kernel's CTA, which then starts late (measured at 40 rows:
-// some CTAs 4.6 us after the predecessor's end instead of 1).
-__global__ void __launch_bounds__(256) act_prep_kernel(const __grid_constant__ ActPrepParams p) {
+// Thread = 16 values of one token at a time (two adjacent lanes share a 32-block); the K tail of the last
+// slab is written as zeros.  Few threads per SM: beside 256 of them the main kernel's CTA found no registers
+// and started late (measured at 40 rows: some CTAs 4.6 us after the predecessor's end instead of 1).
+constexpr int kActPrepThreads = 128;
+__global__ void __launch_bounds__(kActPrepThreads) act_prep_kernel(const __grid_constant__ ActPrepParams p) {
     // The step that follows may become resident at once (it streams weights until its own wait);
     // the activations come from earlier work on the stream.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const ActPrepRank &A = p.r[blockIdx.y];
-    const int chunks_per_row = p.ks << 4, total = p.m * chunks_per_row, step = gridDim.x * blockDim.x;
-    constexpr int U = 4;  // chunks whose loads are in flight together
-    for (int c0 = blockIdx.x * blockDim.x + threadIdx.x; c0 - (int)(threadIdx.x & 31) < total; c0 += U * step) {  // whole warps
-        float v[U][8];
+    const int chunks = p.ks << 3, total = p.m * chunks, step = gridDim.x * kActPrepThreads;
+    constexpr int U = 2;  // chunks whose loads are in flight together
+    for (int c0 = blockIdx.x * kActPrepThreads + threadIdx.x; c0 - (int)(threadIdx.x & 31) < total; c0 += U * step) {  // whole warps
+        float v[U][16];
         int tok[U], ch[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int c = c0 + u * step;
-            tok[u] = c < total ? c / chunks_per_row : 0;
-            ch[u] = c - tok[u] * chunks_per_row;
-            load_act8(A.x, p.x_dtype, (int64_t)tok[u] * A.ldx + ch[u] * 8, c < total && ch[u] * 8 < p.k, v[u]);
+            tok[u] = c < total ? c / chunks : 0;
+            ch[u] = c - tok[u] * chunks;
+            const bool valid = c < total && ch[u] * 16 < p.k;
+            load_act8(A.x, p.x_dtype, (int64_t)tok[u] * A.ldx + ch[u] * 16, valid, *reinterpret_cast<float(*)[8]>(v[u]));
+            load_act8(A.x, p.x_dtype, (int64_t)tok[u] * A.ldx + ch[u] * 16 + 8, valid, *reinterpret_cast<float(*)[8]>(v[u] + 8));
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             int e;
-            uint32_t lo, hi;
-            act_quant8(v[u], e, lo, hi);  // the four lanes of a 32-block are adjacent threads of one warp
+            const uint4 q = act_quant16(v[u], e);
             if (c0 + u * step < total) {
-                const BsImage o = bs_image_at(ch[u] >> 4, p.ks, p.csize, p.sl, p.mp);
-                const int t = tok[u];
-                *reinterpret_cast<uint2 *>(A.img + o.tile + t * 128 + ((((ch[u] >> 1) & 7) ^ (t & 7)) << 4) + (ch[u] & 1) * 8) = make_uint2(lo, hi);
-                if ((ch[u] & 3) == 0)
-                    A.img[o.atom + (t & 31) * 16 + (t >> 5) * 4 + ((ch[u] >> 2) & 3)] = (uint8_t)min(max(e + 127, 0), 255);
+                *reinterpret_cast<uint4 *>(A.xq + ((int64_t)ch[u] * p.m + tok[u]) * 16) = q;
+                if ((ch[u] & 1) == 0)
+                    A.xsf[(int64_t)(ch[u] >> 3) * bs_atom_bytes(p.m) + (tok[u] & 31) * 16 + (tok[u] >> 5) * 4 + ((ch[u] >> 1) & 3)] =
+                        (uint8_t)min(max(e + 127, 0), 255);
             }
         }
     }
@@ -125,18 +120,18 @@ __global__ void __launch_bounds__(256) act_prep_kernel(const __grid_constant__ A
 struct alignas(64) BsParams {
     CUtensorMap tmap_w[WS_MAX_WORLD];  // weight shard as [whole slabs][n][128 bytes]: box SL slabs x tile_rows x 128 bytes, 128B swizzle
     CUtensorMap tmap_t[WS_MAX_WORLD];  // weight shard as [n][k bytes], box tile_rows x 128 bytes: slabs of a group that is not whole
-    int32_t m, mp, n, k, ks, bn_shift, bk_shift;
+    int32_t m, cols, n, k, ks, bn_shift, bk_shift;  // cols: N of the MMA, a multiple of 16 in [m, MP]
     int32_t world, mode, vocab, tmem_cols;  // tmem_cols: tensor-memory columns to allocate (512, or at most 256 when two CTAs share an SM)
     int32_t owner_reduce;              // all-reduce by owners: tile t is folded by rank t % world, which sends the sums back
     int32_t csize;                     // 1, or 2: CTA pairs (a cluster) share a tile, each streams half of K
     int32_t tile_rows, ntiles;         // output rows per tile (a multiple of 8, <= 128) and tiles of the shard
     int32_t slabs_per_stage, nstages;
-    int32_t a_pitch, x_pitch;          // bytes one slab's weights / one stage's activation image occupy (multiples of 1024)
+    int32_t a_pitch, x_pitch;          // bytes one slab's weights (a multiple of 1024) / one stage's activations and atoms (of 128) occupy
     int32_t skb, nslot_max, nacc, gather_logits;
     uint64_t timeout_ns;
     SymLayout lay;
     Fp8RankArgs r[WS_MAX_WORLD];       // x is unused here; scales/out/logits/argmax/row0/k0/ctx as in the decode kernels
-    const uint8_t *img[WS_MAX_WORLD];  // the prep kernel's activation image
+    const uint8_t *xq[WS_MAX_WORLD], *xsf[WS_MAX_WORLD];  // the prep kernel's activations and scale atoms
 };
 
 struct BsSmem {
@@ -149,12 +144,13 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
     int o = 0;
     s.a = o;    o += nsl * a_pitch;
     s.x = o;    o += nstages * x_pitch;
-    // an MMA reads 128 rows of its weight slab however many the tile holds: keep 16 KB readable behind the last one
-    if (nstages * x_pitch < kBsMmaRows * 128) o += kBsMmaRows * 128 - nstages * x_pitch;
+    // an MMA reads 128 rows of its weight slab however many the tile holds, and up to 128 tokens and 32 atom
+    // rows whatever m is: keep 16 KB readable behind the last slab and 2 KB behind the last activations
+    o += nstages * x_pitch + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - nstages * x_pitch : 2048;
     s.wsf = o;  o += wue ? nsl * kBsAtomBytes : kBsAtomBytes;  // the weights' scale atoms (fp32 scales: one atom of 2^0)
     s.sw = o;   o += wue ? 0 : (int)align_up((int64_t)nslot_max * skb * 4, 16);
     s.cand = o; o += bs_epi_warps(mp) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
-    s.rx = o;   o += rx_rows * kBsMmaRows * 4;           // CTA pairs: the partner's partial sums of one tile, [token][row]
+    s.rx = o;   o += rx_rows * kBsMmaRows * 4;           // CTA pairs: the partner's sums of one tile for this CTA's tokens, [token][row]
     s.bars = o; o += (2 * kMaxStages + 2 * kBsMaxAcc + 2) * 8;
     s.misc = o; o += 64;
     s.total = o;
@@ -209,6 +205,9 @@ __device__ __forceinline__ void umma_bs_ss(uint32_t tmem_d, uint32_t a_lo, uint3
 // Halves of the 128B-swizzled K-major operand descriptor (see umma_desc): 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
 constexpr uint32_t kUmmaDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
+// Upper half of the activation operand's descriptor: no swizzle, 8-token groups 128 bytes apart (the lower half
+// carries the stride between 16-byte chunks of K).
+constexpr uint32_t kUmmaDescHiX = (128u >> 4) | (1u << 14);
 // One 512-byte scale atom (32 rows x 16 bytes) -> 4 columns of all 128 TMEM lanes.
 __device__ __forceinline__ void tmem_cp_atom(uint32_t taddr, uint64_t sdesc) {
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
@@ -244,6 +243,31 @@ __device__ __forceinline__ void tmem_ld_cols<64>(uint32_t taddr, uint32_t (&r)[6
         "tcgen05.wait::ld.sync.aligned;"
         : WS_R16(r, 0), WS_R16(r, 16), WS_R16(r, 32), WS_R16(r, 48) : "r"(taddr) : "memory");
 }
+// The same columns of up to 64 / N consecutive accumulators, `pitch` columns apart, under one wait.
+template <int N>
+__device__ __forceinline__ void tmem_ld_batch(uint32_t taddr, uint32_t pitch, uint32_t (&r)[64]);
+template <>
+__device__ __forceinline__ void tmem_ld_batch<16>(uint32_t t, uint32_t pitch, uint32_t (&r)[64]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%65];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47}, [%66];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%67];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : WS_R16(r, 0), WS_R16(r, 16), WS_R16(r, 32), WS_R16(r, 48) : "r"(t), "r"(t + pitch), "r"(t + 2 * pitch), "r"(t + 3 * pitch) : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_ld_batch<32>(uint32_t t, uint32_t pitch, uint32_t (&r)[64]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,"
+        "%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%65];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : WS_R16(r, 0), WS_R16(r, 16), WS_R16(r, 32), WS_R16(r, 48) : "r"(t), "r"(t + pitch) : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_ld_batch<64>(uint32_t t, uint32_t, uint32_t (&r)[64]) { tmem_ld_cols<64>(t, r); }
 #undef WS_R16
 #undef WS_R4
 
@@ -328,7 +352,7 @@ __device__ __forceinline__ uint32_t order_key(float v) {
 }
 
 template <int MP, bool WUE>
-__global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_kernel(const __grid_constant__ BsParams p) {
+__global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, WUE)) fp8_bs_kernel(const __grid_constant__ BsParams p) {
     constexpr int EW = bs_epi_warps(MP), ET = EW * 32;  // epilogue warps / threads
     constexpr int CP = MP * 4 / EW;                      // token columns one epilogue thread holds
     auto bs_epi_bar = [] { bs_epi_bar_n<ET>(); };
@@ -350,7 +374,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
     const int SL = p.slabs_per_stage, NS = p.nstages, NB = p.nacc;
     const int ntiles = p.ntiles, TR = p.tile_rows;
 
-    const BsSmem S = bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? p.m : 0, WUE);
+    const BsSmem S = bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? (p.m + 1) / 2 : 0, WUE);
     float *sw_s = reinterpret_cast<float *>(smem + S.sw);
     uint32_t *misc_s = reinterpret_cast<uint32_t *>(smem + S.misc);
     const uint32_t a0 = smem_u32(smem + S.a), x0 = smem_u32(smem + S.x), wsf0 = smem_u32(smem + S.wsf);
@@ -405,10 +429,10 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
         if (elect_one()) {
             // Weights are static: the first ring's worth streams before the wait on the prep kernel;
             // the activations follow once it has finished.
-            constexpr uint32_t kXSlab = MP * 128 + kBsAtomBytes;
+            const uint32_t x_slab = (uint32_t)p.m * 128u, x_atom = (uint32_t)bs_atom_bytes(p.m);
             const int whole = p.k >> 7;  // slabs of the 3-D map
             auto issue_w = [&](int s, int tile, int s0, int nsl) {
-                mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + kXSlab));
+                mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + x_slab + x_atom));
                 const uint32_t dst = a0 + s * SL * p.a_pitch;
                 if (nsl == SL && s0 + nsl <= whole) {
                     tma_load_3d(dst, &p.tmap_w[vr], 0, tile * TR, s0, full0 + s * 8);
@@ -430,7 +454,9 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
                     if (!mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status)) break;
                     issue_w(s, tile, s0, nsl);
                 }
-                bulk_load(x0 + s * p.x_pitch, p.img[vr] + (size_t)s0 * kXSlab, (uint32_t)nsl * kXSlab, full0 + s * 8);
+                const uint32_t dst = x0 + s * p.x_pitch;
+                bulk_load(dst, p.xq[vr] + (size_t)s0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
+                bulk_load(dst + (uint32_t)SL * x_slab, p.xsf[vr] + (size_t)s0 * x_atom, (uint32_t)nsl * x_atom, full0 + s * 8);
             }
         }
     } else if (warp == 1) {
@@ -447,11 +473,13 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
             // four instruction descriptors (one per K block of a slab), ring positions kept incrementally.
             uint32_t id[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) id[q] = bs_idesc(MP, WUE ? q : 0, q);
-            const uint32_t a_lo0 = umma_desc_lo(a0), x_lo0 = umma_desc_lo(x0);
-            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, x_stage = (uint32_t)p.x_pitch >> 4;
-            const uint64_t xsf_desc0 = umma_desc(x0, 128, false), wsf_desc0 = umma_desc(wsf0, 128, false);
-            constexpr uint32_t kXStep = (uint32_t)(MP * 128) >> 4, kSfStep = (uint32_t)kBsAtomBytes >> 4;
+            for (int q = 0; q < 4; ++q) id[q] = bs_idesc(p.cols, WUE ? q : 0, q);
+            const uint32_t m16 = (uint32_t)p.m;  // 16-byte units: one chunk of all tokens
+            const uint32_t a_lo0 = umma_desc_lo(a0), x_lo0 = ((x0 & 0x3FFFFu) >> 4) | (m16 << 16);
+            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, x_stage = (uint32_t)p.x_pitch >> 4, x_step = 8u * m16, x_kb = 2u * m16;
+            const uint64_t xsf_desc0 = umma_desc(x0, 128, false) + (uint64_t)((uint32_t)SL * x_step), wsf_desc0 = umma_desc(wsf0, 128, false);
+            const uint32_t xsf_step = (uint32_t)bs_atom_bytes(p.m) >> 4;
+            constexpr uint32_t kSfStep = (uint32_t)kBsAtomBytes >> 4;
             BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
             RingPos st, ag;  // stage ring, accumulator ring
             int tile, s0, nsl;
@@ -461,7 +489,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
                 if ((!WUE || s0 == k_lo) && !mbar_wait(accempty0 + g * 8, ag.ph ^ 1u, X.status)) break;
                 tc_fence_after();
                 const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = x_lo0 + (uint32_t)s * x_stage;
-                const uint64_t xsf = xsf_desc0 + (uint64_t)((uint32_t)s * x_stage + (uint32_t)nsl * kXStep);
+                const uint64_t xsf = xsf_desc0 + (uint64_t)((uint32_t)s * x_stage);
                 const uint64_t wsf = wsf_desc0 + (uint64_t)((uint32_t)(s * SL) * kSfStep);
                 const uint32_t t_acc = tmem_base + (uint32_t)((WUE ? g : g * SL) * MP);
                 const uint32_t t_sf = t_sf0 + (WUE ? (uint32_t)((item & 1) * SL * 8) : (uint32_t)(g * SL * 4));
@@ -470,15 +498,15 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
                 auto issue = [&](auto count) {
 #pragma unroll
                     for (int j = 0; j < decltype(count)::value; ++j) {
-                        const uint32_t a = a_lo + (uint32_t)j * a_step, b = b_lo + (uint32_t)j * kXStep;
+                        const uint32_t a = a_lo + (uint32_t)j * a_step, b = b_lo + (uint32_t)j * x_step;
                         const uint32_t d = WUE ? t_acc : t_acc + (uint32_t)(j * MP);
                         const uint32_t sx = t_sf + (uint32_t)(j * (WUE ? 8 : 4)), sw = WUE ? sx + 4 : t_sfa;
-                        tmem_cp_atom(sx, xsf + (uint64_t)(j * kSfStep));
+                        tmem_cp_atom(sx, xsf + (uint64_t)((uint32_t)j * xsf_step));
                         if (WUE) tmem_cp_atom(sw, wsf + (uint64_t)(j * kSfStep));
-                        umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiSw128, id[0], sw, sx, WUE && j > 0 ? 1u : carry);
-                        umma_bs_ss(d, a + 2, b + 2, kUmmaDescHiSw128, kUmmaDescHiSw128, id[1], sw, sx, 1u);
-                        umma_bs_ss(d, a + 4, b + 4, kUmmaDescHiSw128, kUmmaDescHiSw128, id[2], sw, sx, 1u);
-                        umma_bs_ss(d, a + 6, b + 6, kUmmaDescHiSw128, kUmmaDescHiSw128, id[3], sw, sx, 1u);
+                        umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id[0], sw, sx, WUE && j > 0 ? 1u : carry);
+                        umma_bs_ss(d, a + 2, b + x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[1], sw, sx, 1u);
+                        umma_bs_ss(d, a + 4, b + 2 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[2], sw, sx, 1u);
+                        umma_bs_ss(d, a + 6, b + 3 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[3], sw, sx, 1u);
                     }
                 };
                 if (nsl == 4) issue(std::integral_constant<int, 4>{});
@@ -558,6 +586,9 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
         bs_epi_bar();
         const int kofs = (int)(A.k0 - kcol0 * ((int64_t)1 << p.bk_shift));
         const bool solo = p.mode == kModeAllReduce && p.world == 1;
+        // tokens this CTA finishes: of a pair, the first CTA the lower half, the second the upper
+        const int split = p.csize == 2 ? (p.m + 1) / 2 : p.m;
+        const int tok_lo = crank == 0 ? 0 : split, tok_hi = crank == 0 ? split : p.m;
         const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
         const int nflag = kMaxCtas + kMaxShared;
         float *cv_s = reinterpret_cast<float *>(smem + S.cand);        // [EW warps][MP]; a warp fills its own columns
@@ -575,7 +606,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
                 float *dst = base + (size_t)col0 * ld + row;
 #pragma unroll
                 for (int i = 0; i < CP; ++i)
-                    if (col0 + i < p.m) dst[(size_t)i * ld] = v[i];
+                    if (col0 + i >= tok_lo && col0 + i < tok_hi) dst[(size_t)i * ld] = v[i];
             };
             if (mine) {
                 if (solo) {
@@ -587,7 +618,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
                         uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride;
 #pragma unroll
                         for (int i = 0; i < CP; ++i)
-                            if (col0 + i < p.m) st_word_sys(dst + (size_t)(col0 + i) * p.n + row, seq, v[i]);
+                            if (col0 + i >= tok_lo && col0 + i < tok_hi) st_word_sys(dst + (size_t)(col0 + i) * p.n + row, seq, v[i]);
                     }
                 } else if (p.gather_logits && p.world == 1) {  // a lone rank's logits are final where they are
                     store(A.logits + A.vocab_row0, (size_t)p.vocab);
@@ -604,7 +635,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
 #pragma unroll
                 for (int i = 0; i < CP; ++i) {
                     const int t = col0 + i;
-                    if (t >= p.m) break;
+                    if (t < tok_lo || t >= tok_hi) continue;  // warp-uniform
                     const uint32_t key = mine ? order_key(v[i]) : 0u;
                     const uint32_t top = __reduce_max_sync(0xffffffffu, key);
                     const int who = __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
@@ -652,12 +683,19 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
                 ok = __all_sync(0xffffffffu, ok);
                 tc_fence_after();
                 if (ok) {
-                    for (int j = 0; j < nsl; ++j) {
-                        const float sw = swrow[(kofs + (s0 + j) * 128) >> p.bk_shift];
-                        uint32_t r[CP];
-                        tmem_ld_cols<CP>(tlane + (uint32_t)((g * SL + j) * MP + col0), r);  // returns once the values are in registers
+                    // as many slabs per round trip to tensor memory as 64 registers hold (a last round may read
+                    // accumulators of other stages, inside the allocation, and leaves them unused)
+                    constexpr int B = 64 / CP;
+                    for (int j0 = 0; j0 < nsl; j0 += B) {
+                        uint32_t r[64];
+                        tmem_ld_batch<CP>(tlane + (uint32_t)((g * SL + j0) * MP + col0), (uint32_t)MP, r);
 #pragma unroll
-                        for (int i = 0; i < CP; ++i) acc[i] = fmaf(__uint_as_float(r[i]), sw, acc[i]);
+                        for (int j = 0; j < B; ++j)
+                            if (j0 + j < nsl) {
+                                const float sw = swrow[(kofs + (s0 + j0 + j) * 128) >> p.bk_shift];
+#pragma unroll
+                                for (int i = 0; i < CP; ++i) acc[i] = fmaf(__uint_as_float(r[j * CP + i]), sw, acc[i]);
+                            }
                     }
                 }
                 tc_fence_before();
@@ -667,26 +705,27 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
                 ag.next(NB);
                 if (!last) continue;
             }
-            if (p.csize == 1) {
-                finalize(acc, tile);
-            } else if (crank == 1) {
-                // second CTA of the pair: hand the sums to the first one, into its shared memory
-                if (ntile_done > 0) mbar_wait_cluster(rxempty, (uint32_t)(ntile_done - 1) & 1u, X.status);  // the previous tile's have been read
-                const uint32_t dst = mapa_u32(smem_u32(smem + S.rx) + (uint32_t)rc * 4u, 0u);
+            if (p.csize == 2) {
+                // a pair swaps its sums: each CTA gets the partner's for the tokens it finishes, in its shared memory
+                if (ntile_done > 0) mbar_wait_cluster(rxempty, (uint32_t)(ntile_done - 1) & 1u, X.status);  // the partner has read the previous tile's
+                const uint32_t dst = mapa_u32(smem_u32(smem + S.rx) + (uint32_t)rc * 4u, crank ^ 1u);
+                const int base = crank == 0 ? split : 0;  // the partner's first token
 #pragma unroll
-                for (int i = 0; i < CP; ++i)
-                    if (col0 + i < p.m) st_cluster_f32(dst + (uint32_t)((col0 + i) * kBsMmaRows * 4), acc[i]);
-                mbar_arrive_cluster(mapa_u32(rxfull, 0u));
-            } else {
-                // first CTA: K half 0 (own) + K half 1 (the partner's), in that order
+                for (int i = 0; i < CP; ++i) {
+                    const int t = col0 + i;
+                    if (t < p.m && (t < tok_lo || t >= tok_hi)) st_cluster_f32(dst + (uint32_t)((t - base) * kBsMmaRows * 4), acc[i]);
+                }
+                mbar_arrive_cluster(mapa_u32(rxfull, crank ^ 1u));
                 mbar_wait_cluster(rxfull, (uint32_t)ntile_done & 1u, X.status);
                 const float *rx = reinterpret_cast<const float *>(smem + S.rx) + rc;
 #pragma unroll
-                for (int i = 0; i < CP; ++i)
-                    if (col0 + i < p.m) acc[i] += rx[(col0 + i) * kBsMmaRows];
-                if (tile < t_hi) mbar_arrive_cluster(mapa_u32(rxempty, 1u));  // nobody waits for the last one
-                finalize(acc, tile);
+                for (int i = 0; i < CP; ++i) {  // K half 0 + K half 1, in that order (the sum of two does not depend on it)
+                    const int t = col0 + i;
+                    if (t >= tok_lo && t < tok_hi) acc[i] += rx[(t - tok_lo) * kBsMmaRows];
+                }
+                if (tile < t_hi) mbar_arrive_cluster(mapa_u32(rxempty, crank ^ 1u));  // nobody waits for the last one
             }
+            finalize(acc, tile);
             ++ntile_done;
         }
 
@@ -696,18 +735,18 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
         if (!solo && p.mode == kModeAllReduce) {
             // fold the rows of the tiles this CTA finished, in rank order, as the ranks' words arrive
             const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
-            for (int t = t_lo; t <= t_hi && crank == 0; ++t) {  // in a pair the first CTA finished the tiles
+            for (int t = t_lo; t <= t_hi; ++t) {
                 const int row = t * TR + rc;
                 if (rc >= TR || row >= p.n) continue;
                 // 16 tokens at a time: their words of one rank are all requested before the first is
                 // looked at (one memory round trip per batch, not per word); a word that has not
                 // arrived yet is then waited for on its own.  Ranks are added in rank order.
-                const int tend = min(p.m, col0 + CP);  // this thread's token columns
+                const int tbeg = max(tok_lo, col0), tend = min(tok_hi, col0 + CP);  // this thread's token columns
                 // Fold by owners: the sums of tile t are formed on rank t % world only (in rank order, as
                 // everywhere) and travel back in that rank's own slot at every peer, so all ranks end up
                 // with the same bits and each partial sum crosses the links once instead of world - 1 times.
                 const int owner = p.owner_reduce ? t % p.world : X.rank;
-                for (int tok0 = col0; tok0 < tend; tok0 += 16) {
+                for (int tok0 = tbeg; tok0 < tend; tok0 += 16) {
                     float sum[16];
                     const int rr0 = owner == X.rank ? 0 : owner, rr1 = owner == X.rank ? p.world : owner + 1;
                     for (int rr = rr0; rr < rr1; ++rr) {
@@ -833,10 +872,9 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE), MP == 16 ? 2 : 1) fp8_bs_
     tc_fence_before();
     __syncthreads();
     if (p.csize == 2) {  // neither CTA of a pair leaves while the other may still write to or signal it
-        // The first CTA's remote arrivals were all seen by the second, so it need not wait for its own output
-        // stores to reach memory (a release would: ~1 us).
-        if (crank == 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-        else asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        // What each sent was waited for by the other, so neither need wait for its own output stores to reach
+        // memory (a release would: ~1 us).
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     if (warp == 1) {

@@ -137,16 +137,15 @@ __device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
         for (int t = 0; t < GT; ++t)
 #pragma unroll
             for (int i = 0; i < C; ++i) {
-                float amax = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[t][i][j]));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));  // a 32-block is two adjacent lanes
-                const int e = act_scale_exp(amax);
-                const float inv = e > 127 ? 0.0f : pow2_f32(-e);  // an infinite block scale divides everything to zero
+                int e;
+                const uint4 q = act_quant16(v[t][i], e);  // a 32-block is two adjacent lanes
+                const uint32_t qq[4] = {q.x, q.y, q.z, q.w};
                 sa[t][i] = live[i] ? pow2_f32(e) : 0.0f;
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    xh[t][i][j] = live[i] ? e4m3x2_to_f16x2(cvt_e4m3x2(v[t][i][2 * j] * inv, v[t][i][2 * j + 1] * inv)) : 0u;
+                for (int j = 0; j < 4; ++j) {
+                    xh[t][i][2 * j] = live[i] ? e4m3x2_half_to_f16x2<0>(qq[j]) : 0u;
+                    xh[t][i][2 * j + 1] = live[i] ? e4m3x2_half_to_f16x2<1>(qq[j]) : 0u;
+                }
             }
     }
     const bool solo = p.mode == kModeAllReduce && p.world == 1;

@@ -9,24 +9,27 @@
 //                       (a pass = one local expert with up to 16 of its routes as MMA columns, experts
 //                       in ascending id as crates/weightstream-ref/src/moe.rs:75-84 adds them),
 //                       hidden x routing-weight quantised as the reference does (moe.rs:150, then
-//                       actquant.rs:21-57) into E4M3 rows at that position, and the per-32 exponents
-//                       into the pass's 512-byte scale atoms (one per 128-wide K slab: byte
-//                       (t & 31) * 16 + (t >> 5) * 4 + j = exponent of column t, K block j).
+//                       actquant.rs:21-57) into the form the MMA reads: per pass 16-byte chunks of K,
+//                       chunk-major ([chunk][route of the pass][16 bytes]), and the per-32 exponents as the
+//                       pass's scale atoms (one per 128-wide K slab, a row of 16 bytes per route: byte j =
+//                       exponent of K block j).
 //   moe_bs_kernel       persistent CTA pairs (clusters of 2), one pair per tile of ~97 output rows,
 //                       each CTA of a pair streams half of K of every pass: with a lone CTA's ~48
 //                       rows under half of the MMA's 128 rows would be real, and the tensor pipe
 //                       needs the same ~35 ns per K=32 MMA however few are.  Warp 0 lane 0 streams,
-//                       per 128-wide K slab, the expert's rows (TMA, 4-bit codes unpacked by the
-//                       copy into the 16-bytes-per-16-codes form the MMA reads), the pass's
-//                       activation rows (TMA) and their scale atom (bulk copy).  Four warps turn the
+//                       per stage of up to four 128-wide K slabs, the expert's rows (TMA, 4-bit codes
+//                       unpacked by the copy into the 16-bytes-per-16-codes form the MMA reads) and the
+//                       pass's activations and scale atoms (one bulk copy each, only of the routes there
+//                       are: padded to the MMA's 16 columns they were 40 % of the weights' bytes, and what
+//                       L2 can hand the SMs bound the step).  Four warps turn the
 //                       weights' UE8M0 bytes (4 consecutive bytes per row and slab in the reference's
 //                       [expert][row][k/32] layout) into scale atoms in shared memory, one pass ahead.
 //                       Warp 1 lane 0 copies both atoms of a slab into tensor memory and issues its
 //                       four MMAs; one commit per stage frees it, one per pass hands the accumulator
 //                       (16 columns, double-buffered) to the four epilogue warps, which add column t
 //                       to the shared-memory sums of the token that route belongs to.  After the last
-//                       pass the second CTA hands its sums to the first through distributed shared
-//                       memory; that one adds them after its own and stores the rows or exchanges them.
+//                       pass the CTAs of a pair swap their sums through distributed shared memory, each
+//                       adds the halves of K for half of the tokens and stores or exchanges those rows.
 //
 // Exchange: as in the FP8 kernels (partials stored to every peer as tagged words, folded in rank order).
 #pragma once
@@ -44,13 +47,8 @@ constexpr int kMoeBsThreads = 320;    // warp 0 producer, 1 MMA issue, 2-5 epilo
 constexpr int kMoeBsMaxSlabs = 16;    // K slabs one CTA walks per pass (k <= 4096 with pairs)
 
 // Per-endpoint scratch written by moe_bs_prep_kernel and read by moe_bs_kernel.
-// The activations of a pass are stored as the main kernel's shared memory wants them, so that ONE bulk
-// copy fills a stage: per pass and group of `sl` K slabs, sl tiles of 16 rows x 128 bytes (128B-swizzled
-// K-major, the layout a TMA box would produce) followed by their sl scale atoms.
-constexpr int kMoeBsXTile = kMoeBsCols * 128;                 // 2048
-constexpr int kMoeBsXSlab = kMoeBsXTile + kBsAtomBytes;       // 2560 bytes of a stage per slab
 struct MoeBsWork {
-    int64_t hdr, pass, stok, xs, total;  // byte offsets
+    int64_t hdr, pass, stok, xq, xsf, total;  // byte offsets
 };
 __host__ __device__ inline MoeBsWork moe_bs_work_layout(int k) {
     MoeBsWork w{};
@@ -58,14 +56,14 @@ __host__ __device__ inline MoeBsWork moe_bs_work_layout(int k) {
     w.hdr = o;  o += 64;
     w.pass = o; o += (int64_t)kMoeMaxRoutes * sizeof(MoePass);
     w.stok = o; o += align_up((int64_t)(kMoeMaxRoutes + kMoeBsCols) * 2, 256);
-    w.xs = o;   o += (int64_t)kMoeMaxRoutes * (k / 128) * kMoeBsXSlab;  // [pass][slab group][tiles | atoms]
+    w.xq = o;   o += (int64_t)kMoeMaxRoutes * k;               // a pass starts at its first route's row: [k / 16 chunks][nr][16]
+    w.xsf = o;  o += (int64_t)kMoeMaxRoutes * (k / 128) * 16;  // likewise: [k / 128 slabs][nr][16]
     w.total = o;
     return w;
 }
 
 struct MoeBsPrepParams {
     int32_t m, k, top_k, h_dtype;
-    int32_t sl, pad0;  // K slabs per stage of the main kernel (a group of the layout above)
     MoePrepRank r[WS_MAX_WORLD];
 };
 
@@ -83,8 +81,8 @@ __device__ __forceinline__ int block_sum_256(int v, int *red_s) {  // all 256 th
 }
 
 __global__ void __launch_bounds__(256) moe_bs_prep_kernel(const __grid_constant__ MoeBsPrepParams p) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const MoePrepRank &A = p.r[blockIdx.y];
     const int NR = p.m * p.top_k, tid = threadIdx.x;
     const MoeBsWork W = moe_bs_work_layout(p.k);
@@ -133,23 +131,18 @@ __global__ void __launch_bounds__(256) moe_bs_prep_kernel(const __grid_constant_
         reinterpret_cast<uint16_t *>(A.work + W.stok)[pos] = (uint16_t)(route / p.top_k);
     }
     const float w = A.route_w[route];
-    uint8_t *xs = A.work + W.xs + (size_t)pass * (p.k >> 7) * kMoeBsXSlab;
-    const int group_bytes = p.sl * kMoeBsXSlab;
-    for (int c = tid; c < (p.k >> 3); c += blockDim.x) {  // the four chunks of a 32-block are adjacent lanes
-        float v[8];
-        load_act8(A.h, p.h_dtype, (int64_t)route * A.ldh + c * 8, true, v);
+    const int first = pos - t, nr = min(kMoeBsCols, cnt_s[e] - (rnk - t));  // the pass's first route and route count
+    uint8_t *xq = A.work + W.xq + (size_t)first * p.k, *xsf = A.work + W.xsf + (size_t)first * (p.k >> 7) * 16;
+    for (int c = tid; c < (p.k >> 4); c += blockDim.x) {  // the two chunks of a 32-block are adjacent lanes
+        float v[16];
+        load_act8(A.h, p.h_dtype, (int64_t)route * A.ldh + c * 16, true, *reinterpret_cast<float(*)[8]>(v));
+        load_act8(A.h, p.h_dtype, (int64_t)route * A.ldh + c * 16 + 8, true, *reinterpret_cast<float(*)[8]>(v + 8));
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] *= w;
+        for (int i = 0; i < 16; ++i) v[i] *= w;
         int ex;
-        uint32_t lo, hi;
-        act_quant8(v, ex, lo, hi);
-        // 8 values = half of a 16-byte chunk of row t of the slab's tile; chunk cc sits at (cc ^ (t & 7))
-        const int slab = c >> 4, cc = (c >> 1) & 7, half = c & 1;
-        uint8_t *grp = xs + (size_t)(slab / p.sl) * group_bytes;
-        const int j = slab % p.sl;
-        *reinterpret_cast<uint2 *>(grp + j * kMoeBsXTile + t * 128 + ((cc ^ (t & 7)) << 4) + half * 8) = make_uint2(lo, hi);
-        if ((c & 3) == 0)
-            grp[p.sl * kMoeBsXTile + j * kBsAtomBytes + t * 16 + ((c >> 2) & 3)] = (uint8_t)min(max(ex + 127, 0), 255);
+        const uint4 q = act_quant16(v, ex);
+        *reinterpret_cast<uint4 *>(xq + ((size_t)c * nr + t) * 16) = q;
+        if ((c & 1) == 0) xsf[((size_t)(c >> 3) * nr + t) * 16 + ((c >> 1) & 3)] = (uint8_t)min(max(ex + 127, 0), 255);
     }
 }
 
@@ -166,7 +159,7 @@ struct alignas(64) MoeBsParams {
     CUtensorMap tmap_w[WS_MAX_WORLD];  // expert slab as [e_len][n][k] 4-bit codes; boxes of 128 codes x tile_rows x 1, unpacked, 128B swizzle
     int32_t m, n, k, world;
     int32_t tile_rows, a_pitch, slabs_per_stage, nstages;
-    int32_t tmem_cols, pad0;
+    int32_t tmem_cols, x_pitch, alias, pad0;  // alias: the partner's sums land in the ring
     uint64_t timeout_ns;
     SymLayout lay;
     MoeBsRank r[WS_MAX_WORLD];
@@ -175,17 +168,18 @@ struct alignas(64) MoeBsParams {
 struct MoeBsSmem {
     int32_t a, b, sfa, acc, rx, bars, misc, total;
 };
-__host__ __device__ inline MoeBsSmem moe_bs_smem_layout(int nstages, int slabs_per_stage, int a_pitch, int m, int nslab_cta) {
+__host__ __device__ inline MoeBsSmem moe_bs_smem_layout(int nstages, int slabs_per_stage, int a_pitch, int x_pitch, int m, int nslab_cta,
+                                                        int alias) {
     MoeBsSmem s{};
-    const int nsl = nstages * slabs_per_stage;
-    const int b_bytes = nsl * kMoeBsXSlab;  // per stage: its slabs' activation tiles, then their scale atoms (one bulk copy)
     int o = 0;
-    s.a = o;    o += nsl * a_pitch;
-    s.b = o;    o += b_bytes;
-    if (b_bytes < kBsMmaRows * 128) o += kBsMmaRows * 128 - b_bytes;  // an MMA reads 128 rows behind the last weight slab
+    s.a = o;    o += nstages * slabs_per_stage * a_pitch;
+    s.b = o;    o += nstages * x_pitch;  // per stage: its slabs' activations, then their scale atoms
+    // an MMA reads 128 rows behind the last weight slab, 16 routes and 32 atom rows whatever the pass has
+    o += nstages * x_pitch + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - nstages * x_pitch : 2048;
     s.sfa = o;  o += 2 * nslab_cta * kBsAtomBytes;                      // weight-scale atoms of two passes
     s.acc = o;  o += m * kBsMmaRows * 4;                                // sums of (token, row)
-    s.rx = o;   o += m * kBsMmaRows * 4;                                // the partner's, at the end
+    s.rx = alias ? 0 : o;                                               // the partner's, at the end
+    o += alias ? 0 : (m + 1) / 2 * kBsMmaRows * 4;
     s.bars = o; o += (2 * kMaxStages + 8) * 8;
     s.misc = o; o += 64;
     s.total = o;
@@ -217,12 +211,11 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
     const int SL = p.slabs_per_stage, NS = p.nstages;
     const int IP = (NSLAB + SL - 1) / SL;                           // stage items per pass
 
-    const MoeBsSmem S = moe_bs_smem_layout(NS, SL, p.a_pitch, p.m, NSLAB);
+    const MoeBsSmem S = moe_bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.m, NSLAB, p.alias);
     const MoeBsWork W = moe_bs_work_layout(p.k);
     float *acc_s = reinterpret_cast<float *>(smem + S.acc);
     uint32_t *misc_s = reinterpret_cast<uint32_t *>(smem + S.misc);
     const uint32_t a0 = smem_u32(smem + S.a), b0 = smem_u32(smem + S.b), sfa0 = smem_u32(smem + S.sfa);
-    const uint32_t stage_x = (uint32_t)(SL * kMoeBsXSlab);  // a stage's activation tiles and scale atoms
     // full[s]: a stage's bytes landed; done[s]: its MMAs have completed (stage free); accfull[g] /
     // accempty[g]: a pass's accumulator is complete (and its scale columns free again) / has been read;
     // sfafull[g]: the weight scales of a pass are in tensor memory.
@@ -265,21 +258,23 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
     if (warp == 0) {
         // ------------------------------------------------------------ producer (one thread)
         if (elect_one()) {
-            // the unpacking copy counts the packed bytes it read (64 per row), not the 128 it wrote
-            const uint32_t slab_tx = (uint32_t)(TR * 64 + kMoeBsXSlab);
             RingPos st;
             int item = 0;
             for (int ps = 0; ps < npass; ++ps) {
                 const MoePass P = passes[ps];
-                const uint8_t *xs = A.work + W.xs + ((size_t)ps * KS + k_lo) * kMoeBsXSlab;  // this CTA's slab groups of the pass
+                const uint32_t x_slab = (uint32_t)P.nr * 128u, x_atom = (uint32_t)P.nr * 16u;
+                const uint8_t *xq = A.work + W.xq + (size_t)P.first * p.k + (size_t)k_lo * x_slab;
+                const uint8_t *xsf = A.work + W.xsf + ((size_t)P.first * KS + (size_t)k_lo * P.nr) * 16;
                 for (int i = 0; i < IP; ++i, ++item, st.next(NS)) {
                     const int s = st.s, j0 = i * SL, nsl = min(SL, NSLAB - j0);
                     if (item >= NS && !mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status)) { ps = npass; break; }
-                    mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * slab_tx);
+                    // the unpacking copy counts the packed bytes it read (64 per row), not the 128 it wrote
+                    mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 64u + x_slab + x_atom));
                     for (int j = 0; j < nsl; ++j)
                         tma_load_3d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (k_lo + j0 + j) * 128, row0, (int)P.expert, full0 + s * 8);
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                 ::"r"(b0 + s * stage_x), "l"(xs + (size_t)i * stage_x), "r"(stage_x), "r"(full0 + s * 8) : "memory");
+                    const uint32_t dst = b0 + s * p.x_pitch;
+                    bulk_load(dst, xq + (size_t)j0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
+                    bulk_load(dst + (uint32_t)SL * x_slab, xsf + (size_t)j0 * x_atom, (uint32_t)nsl * x_atom, full0 + s * 8);
                 }
             }
         }
@@ -287,10 +282,9 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
         // ------------------------------------------------------------ MMA issue (one thread)
         if (elect_one()) {
             const uint32_t id0 = moe_bs_idesc(0), id1 = moe_bs_idesc(1), id2 = moe_bs_idesc(2), id3 = moe_bs_idesc(3);
-            const uint32_t a_lo0 = umma_desc_lo(a0), b_lo0 = umma_desc_lo(b0);
-            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, b_step = (uint32_t)kMoeBsXTile >> 4;
-            const uint64_t sf_desc0 = umma_desc(b0 + (uint32_t)(SL * kMoeBsXTile), 128, false);  // a stage's atoms follow its tiles
-            constexpr uint32_t sf_step = (uint32_t)kBsAtomBytes >> 4;
+            const uint32_t a_lo0 = umma_desc_lo(a0), b_lo0 = (b0 & 0x3FFFFu) >> 4;
+            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, x_stage = (uint32_t)p.x_pitch >> 4;
+            const uint64_t sf_desc0 = umma_desc(b0, 128, false);
             RingPos st;
             bool ok = true;
             for (int ps = 0; ps < npass && ok; ++ps) {
@@ -300,22 +294,23 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
                 tc_fence_after();
                 const uint32_t t_acc = tmem_base + (uint32_t)(g * kMoeBsCols);
                 uint32_t t_sc = t_sc0 + (uint32_t)(g * NSLAB * 8);
+                const uint32_t nr = passes[ps].nr, b_step = 8u * nr, x_kb = 2u * nr;  // 16-byte units, as in the FP8 kernel
                 for (int i = 0; i < IP; ++i, st.next(NS)) {
                     const int s = st.s, nsl = min(SL, NSLAB - i * SL);
                     if (!mbar_wait(full0 + s * 8, st.ph, X.status)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = b_lo0 + (uint32_t)s * (stage_x >> 4);
-                    const uint64_t sf_desc = sf_desc0 + (uint64_t)((uint32_t)s * (stage_x >> 4));
+                    const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = (b_lo0 + (uint32_t)s * x_stage) | (nr << 16);
+                    const uint64_t sf_desc = sf_desc0 + (uint64_t)((uint32_t)s * x_stage + (uint32_t)SL * b_step);  // a stage's atoms follow its activations
                     // straight-line code per slab count, as in the FP8 kernel
                     auto issue = [&](auto count) {
 #pragma unroll
                         for (int j = 0; j < decltype(count)::value; ++j) {
                             const uint32_t a = a_lo + (uint32_t)j * a_step, b = b_lo + (uint32_t)j * b_step, sx = t_sc + (uint32_t)(j * 8);
-                            tmem_cp_atom(sx, sf_desc + (uint64_t)(j * sf_step));  // the activations' scales of this slab (the weights' are there already)
-                            umma_bs_ss(t_acc, a, b, kUmmaDescHiSw128, kUmmaDescHiSw128, id0, sx + 4, sx, j > 0 || i > 0 ? 1u : 0u);
-                            umma_bs_ss(t_acc, a + 2, b + 2, kUmmaDescHiSw128, kUmmaDescHiSw128, id1, sx + 4, sx, 1u);
-                            umma_bs_ss(t_acc, a + 4, b + 4, kUmmaDescHiSw128, kUmmaDescHiSw128, id2, sx + 4, sx, 1u);
-                            umma_bs_ss(t_acc, a + 6, b + 6, kUmmaDescHiSw128, kUmmaDescHiSw128, id3, sx + 4, sx, 1u);
+                            tmem_cp_atom(sx, sf_desc + (uint64_t)((uint32_t)j * nr));  // the activations' scales of this slab (the weights' are there already)
+                            umma_bs_ss(t_acc, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id0, sx + 4, sx, j > 0 || i > 0 ? 1u : 0u);
+                            umma_bs_ss(t_acc, a + 2, b + x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id1, sx + 4, sx, 1u);
+                            umma_bs_ss(t_acc, a + 4, b + 2 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id2, sx + 4, sx, 1u);
+                            umma_bs_ss(t_acc, a + 6, b + 3 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id3, sx + 4, sx, 1u);
                         }
                     };
                     if (nsl == 4) issue(std::integral_constant<int, 4>{});
@@ -389,51 +384,53 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
         }
     }
 
-    // ---- the pair's halves of K: the second CTA's sums go to the first
+    // ---- the pair's halves of K: each CTA sends the other the sums of the tokens that one finishes
+    tc_fence_before();
     __syncthreads();
     float *rx_s = reinterpret_cast<float *>(smem + S.rx);
-    if (crank == 1) {
-        const uint32_t dst = mapa_u32(smem_u32(rx_s), 0u);
-        for (int i = tid; i < p.m * kBsMmaRows; i += kMoeBsThreads) st_cluster_f32(dst + (uint32_t)i * 4u, acc_s[i]);
+    if (p.alias) {  // the partner's ring is idle: its copies have landed and its MMAs have completed
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    const int split = (p.m + 1) / 2;
+    const int tok_lo = crank == 0 ? 0 : split, ntok = crank == 0 ? split : p.m - split;
+    {
+        const int other = crank == 0 ? split : 0, nother = p.m - ntok;
+        const uint32_t dst = mapa_u32(smem_u32(rx_s), crank ^ 1u);
+        for (int i = tid; i < nother * kBsMmaRows; i += kMoeBsThreads) st_cluster_f32(dst + (uint32_t)i * 4u, acc_s[other * kBsMmaRows + i]);
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // nothing crosses the pair after this
 
     const bool solo = p.world == 1;
-    if (crank == 0) {
-        const uint32_t seq = step_begin(X);
-        const uint32_t bank = seq & 1u;
-        const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
-        // K half 0 (own) + K half 1 (the partner's), in that order; thread -> (token, row)
-        for (int i = tid; i < p.m * kBsMmaRows; i += kMoeBsThreads) {
-            const int tok = i >> 7, rc = i & 127, row = row0 + rc;
-            if (rc >= TR || row >= p.n) continue;
-            const float v = acc_s[i] + rx_s[i];
-            if (solo) {
-                A.out[(size_t)tok * p.n + row] = v;
-            } else {
-                for (int pr = 0; pr < p.world; ++pr) {
-                    uint64_t *dstw = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride;
-                    st_word_sys(dstw + (size_t)tok * p.n + row, seq, v);
-                }
+    const uint32_t seq = step_begin(X);
+    const uint32_t bank = seq & 1u;
+    const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
+    // K half 0 + K half 1; thread -> (token, row)
+    for (int i = tid; i < ntok * kBsMmaRows; i += kMoeBsThreads) {
+        const int tok = tok_lo + (i >> 7), rc = i & 127, row = row0 + rc;
+        if (rc >= TR || row >= p.n) continue;
+        const float v = acc_s[tok_lo * kBsMmaRows + i] + rx_s[i];
+        if (solo) {
+            A.out[(size_t)tok * p.n + row] = v;
+        } else {
+            for (int pr = 0; pr < p.world; ++pr) {
+                uint64_t *dstw = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride;
+                st_word_sys(dstw + (size_t)tok * p.n + row, seq, v);
             }
         }
-        if (!solo) {  // fold the same rows in rank order as the ranks' words arrive
-            const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
-            for (int i = tid; i < p.m * kBsMmaRows; i += kMoeBsThreads) {
-                const int tok = i >> 7, rc = i & 127, row = row0 + rc;
-                if (rc >= TR || row >= p.n) continue;
-                const size_t off = (size_t)tok * p.n + row;
-                A.out[off] = fold_words(slots, astride, off, p.world, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
-            }
+    }
+    if (!solo) {  // fold the same rows in rank order as the ranks' words arrive
+        const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
+        for (int i = tid; i < ntok * kBsMmaRows; i += kMoeBsThreads) {
+            const int tok = tok_lo + (i >> 7), rc = i & 127, row = row0 + rc;
+            if (rc >= TR || row >= p.n) continue;
+            const size_t off = (size_t)tok * p.n + row;
+            A.out[off] = fold_words(slots, astride, off, p.world, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
         }
     }
 
     // ---- teardown
-    tc_fence_before();
-    __syncthreads();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
