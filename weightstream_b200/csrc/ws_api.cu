@@ -128,25 +128,6 @@ ws_status_t make_tmap(ws_tp *tp, CUtensorMap *map, const void *base, uint64_t ro
     return WS_OK;
 }
 
-// The same matrix as [whole 128-byte slabs of K][rows][128 bytes]: one box carries `slabs` slabs of box_rows rows,
-// slab after slab, each in the layout of make_tmap's box (box_rows a multiple of 8 keeps the swizzle's phase).
-ws_status_t make_tmap_slabs(ws_tp *tp, CUtensorMap *map, const void *base, uint64_t rows, uint64_t whole_slabs, uint64_t ld,
-                            uint32_t box_rows, uint32_t slabs) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(tp, WS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld & 15))
-        return fail(tp, WS_ERR_INVALID, "weight base and row stride must be multiples of 16 bytes");
-    cuuint64_t dims[3] = {128, rows, whole_slabs};
-    cuuint64_t strides[2] = {ld, 128};
-    cuuint32_t box[3] = {128, box_rows, slabs};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(tp, WS_ERR_CUDA, "cuTensorMapEncodeTiled (slabs) failed (%d)", (int)r);
-    return WS_OK;
-}
-
 // Expert slab [experts][rows][k] of packed 4-bit codes (row stride k/2 bytes), boxes of 128 codes x
 // box_rows x 1 expert; the copy unpacks 16 codes (8 bytes) into 16 bytes of shared memory, the form
 // tcgen05.mma.kind::mxf8f6f4 reads 4-bit operands in; 128B swizzle.
@@ -481,16 +462,15 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     u.ncta = u.csize == 2 ? ncta & ~1 : ncta;
     const int nparts = u.ncta / u.csize;
     // tiles of equal height that deal out evenly: a CTA's share of the rows, cut into as few pieces of at
-    // most 128 rows as possible; multiples of 8, so that the slabs of one TMA box keep the swizzle's phase
+    // most 128 rows as possible (multiples of 8, which one TMA box of several slabs needs, left 5 of 74 pairs idle)
     const int crmax = (a.n + nparts - 1) / nparts;
     const int pieces = (crmax + kBsMmaRows - 1) / kBsMmaRows;
-    u.tile_rows = std::min((int)kBsMmaRows, ((crmax + pieces - 1) / pieces + 7) / 8 * 8);
+    u.tile_rows = (crmax + pieces - 1) / pieces;
     u.ntiles = (a.n + u.tile_rows - 1) / u.tile_rows;
     const int tiles_per_cta = (u.ntiles + nparts - 1) / nparts;
-    u.a_pitch = u.tile_rows * 128;
+    u.a_pitch = (u.tile_rows + 7) / 8 * 8 * 128;
     const int x_slab = mt * 128 + bs_atom_bytes(mt), slab_bytes = u.a_pitch + x_slab + (u.wue ? kBsAtomBytes : 0);
-    // slabs per stage: one MMA commit (a ~160 ns stall of the issuing thread) and two copies (~100 ns each)
-    // per stage, so several slabs share it; bounded by the stage size and by tensor memory (fp32 scales: each
+    // slabs per stage: barrier round trips, a commit and two copies are per stage, so several slabs share them; bounded by the stage size and by tensor memory (fp32 scales: each
     // slab has its own accumulator buffer, groups x slabs x (mp + 4) + 8 columns of 512, at least two groups)
     u.nslot_max = (tiles_per_cta * u.tile_rows) / a.block_n + 2;
     const int rx_rows = u.csize == 2 ? (mt + 1) / 2 : 0, kcta = (u.ks + u.csize - 1) / u.csize;
@@ -505,7 +485,7 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         const int stage_target = half ? 32 * 1024 : 56 * 1024;
         u.slabs_per_stage = std::max(1, std::min({4, stage_target / slab_bytes, kcta, u.wue ? 4 : (tmem - 8) / (2 * (u.mp + 4))}));
         const int groups = (kcta + u.slabs_per_stage - 1) / u.slabs_per_stage;
-        u.slabs_per_stage = (kcta + groups - 1) / groups;  // groups of equal size, so that few slabs travel outside whole boxes
+        u.slabs_per_stage = (kcta + groups - 1) / groups;
         u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * x_slab, 128);
         u.nacc = u.wue ? std::min(2, std::max(1, (tmem - 8 - 2 * u.slabs_per_stage * 8) / u.mp))
                        : std::min((int)kBsMaxAcc, (tmem - 8) / (u.slabs_per_stage * (u.mp + 4)));
@@ -589,10 +569,7 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         ws_tp *t = ranks[i];
         const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
         ws_status_t s = ensure_bs_scratch(t, xq_bytes + xsf_bytes);
-        if (s == WS_OK)  // (with less than one whole slab only the second map is used)
-            s = make_tmap_slabs(t, &p.tmap_w[i], a.w, (uint64_t)a.n, (uint64_t)std::max(1, a.k / 128), (uint64_t)a.ldw, (uint32_t)u.tile_rows,
-                                (uint32_t)u.slabs_per_stage);
-        if (s == WS_OK) s = make_tmap(t, &p.tmap_t[i], a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, (uint32_t)u.tile_rows);
+        if (s == WS_OK) s = make_tmap(t, &p.tmap_w[i], a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, (uint32_t)u.tile_rows);
         if (s != WS_OK) { t0->err = t->err; return s; }
         Fp8RankArgs &r = p.r[i];
         r.x = nullptr;
@@ -620,7 +597,6 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         if (i > 0) {  // one launch per device, each sees itself as virtual rank 0
             p.r[0] = p.r[i];
             p.tmap_w[0] = p.tmap_w[i];
-            p.tmap_t[0] = p.tmap_t[i];
             p.xq[0] = p.xq[i];
             p.xsf[0] = p.xsf[i];
             q.r[0] = q.r[i];
@@ -962,7 +938,7 @@ static ws_status_t ensure_moe_scratch(ws_tp *tp, size_t work_bytes, size_t acc_b
 // in halves of at most 16 slabs, a pair's rows are one MMA tile, the per-token sums live in shared memory).
 struct MoeBsPlan {
     bool ok;
-    int ncta, tile_rows, a_pitch, slabs_per_stage, nstages, tmem_cols, x_pitch, alias;
+    int ncta, tile_rows, a_pitch, slabs_per_stage, nstages, tmem_cols, x_pitch, alias, inline_x;
     size_t smem;
 };
 static MoeBsPlan moe_bs_plan(const ws_moe_down_args_t &a, int ncta) {
@@ -973,18 +949,18 @@ static MoeBsPlan moe_bs_plan(const ws_moe_down_args_t &a, int ncta) {
     u.tile_rows = (a.n + nparts - 1) / nparts;
     if (u.tile_rows > kBsMmaRows) return u;
     u.a_pitch = (u.tile_rows + 7) / 8 * 8 * 128;
-    u.slabs_per_stage = std::min(4, nslab);  // one commit and two activation copies per stage
-    if (getenv("X1")) u.slabs_per_stage = std::min(atoi(getenv("X1")), nslab);
+    u.slabs_per_stage = std::min(getenv("X2") ? atoi(getenv("X2")) : 2, nslab);
+    u.inline_x = a.m * a.top_k <= (getenv("X1") ? atoi(getenv("X1")) : kMoeBsInlineRoutes) ? 1 : 0;
     const int nr = std::min((int)kMoeBsCols, a.m * a.top_k);  // most routes of a pass
     u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * (nr * 128 + nr * 16), 128);
     // the partner's sums land behind the ring, or, when there are many, in the ring itself after the last pass
     u.alias = a.m > 8 ? 1 : 0;
-    auto total = [&](int ns) { return moe_bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, a.m, nslab, u.alias).total + 1024; };
+    auto total = [&](int ns) { return moe_bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, a.m, nslab, u.alias, a.m * a.top_k, u.inline_x).total + 1024; };
     int ns = kMaxStages;
     while (ns >= 2 && total(ns) > kSmemBudget - 8 * 1024) --ns;  // (beside a few blocks of the prep kernel)
     u.nstages = ns;
     int cols = 32;
-    while (cols < 2 * kMoeBsCols + 2 * nslab * 8) cols *= 2;
+    while (cols < 2 * kMoeBsCols + 2 * nslab * 8 + a.m) cols *= 2;
     u.tmem_cols = cols;
     u.ok = ns >= 2 && cols <= 512 && (!u.alias || (a.m + 1) / 2 * kBsMmaRows * 4 <= ns * u.slabs_per_stage * u.a_pitch);
     if (u.ok) u.smem = (size_t)total(ns);
@@ -1000,7 +976,8 @@ static ws_status_t moe_bs_step(ws_tp *const *ranks, int n, const ws_moe_down_arg
     MoeBsParams p{};
     p.m = a0.m; p.n = a0.n; p.k = a0.k; p.world = t0->world;
     p.tile_rows = u.tile_rows; p.a_pitch = u.a_pitch; p.slabs_per_stage = u.slabs_per_stage; p.nstages = u.nstages;
-    p.tmem_cols = u.tmem_cols; p.x_pitch = u.x_pitch; p.alias = u.alias;
+    p.tmem_cols = u.tmem_cols; p.x_pitch = u.x_pitch; p.alias = u.alias; p.prefetch = getenv("X3") ? atoi(getenv("X3")) : 1;
+    p.inline_x = u.inline_x; p.nroutes = a0.m * a0.top_k; p.top_k = a0.top_k; p.h_dtype = a0.h_dtype;
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
     MoeBsPrepParams q{};
@@ -1011,18 +988,19 @@ static ws_status_t moe_bs_step(ws_tp *const *ranks, int n, const ws_moe_down_arg
     for (int i = 0; i < n; ++i) {
         ws_tp *t = ranks[i];
         const ws_moe_down_args_t &a = args[i];
-        ws_status_t s = ensure_moe_scratch(t, (size_t)W.total, 0);
+        ws_status_t s = u.inline_x ? WS_OK : ensure_moe_scratch(t, (size_t)W.total, 0);
         if (s == WS_OK) s = make_tmap_fp4(t, &p.tmap_w[0], a.w2, (uint64_t)a.e_len, (uint64_t)a.n, (uint64_t)a.k, (uint32_t)u.tile_rows);
         if (s != WS_OK) { t0->err = t->err; return s; }
         MoeBsRank &r = p.r[0];
         r.s2 = a.s2; r.work = t->moe_work; r.out = a.out; r.e_start = a.e_start; r.e_len = a.e_len;
+        r.h = a.h; r.route_ids = a.route_ids; r.route_w = a.route_w; r.ldh = a.ldh;
         r.ctx = make_ctx(t);
         MoePrepRank &pr = q.r[0];
         pr.h = a.h; pr.route_ids = a.route_ids; pr.route_w = a.route_w; pr.work = t->moe_work;
         pr.ldh = a.ldh; pr.e_start = a.e_start; pr.e_len = a.e_len;
         WS_CUDA(t, cudaSetDevice(t->device));
         cudaStream_t cs = static_cast<cudaStream_t>(streams ? streams[i] : nullptr);
-        s = launch(t, moe_bs_prep_kernel, q, nblk, 1, 256, 0, cs, t0->pdl != 0, false);
+        if (!u.inline_x) s = launch(t, moe_bs_prep_kernel, q, nblk, 1, 256, 0, cs, t0->pdl != 0, false);
         if (s == WS_OK) s = launch(t, moe_bs_kernel, p, u.ncta, 1, kMoeBsThreads, u.smem, cs, t0->pdl != 0, true, 2);
         if (s != WS_OK) { t0->err = t->err; return s; }
     }

@@ -10,7 +10,7 @@
 //                     M of the MMA), dealt out whole; a CTA (or a CTA pair, each CTA one half of K)
 //                     streams the weights of its tiles, so every output is a complete dot product inside
 //                     one CTA pair and nothing is combined through global memory.  A stage of the ring
-//                     holds SL K slabs of 128: their weight rows (ONE 3-D TMA box, 128B swizzle), their
+//                     holds SL K slabs of 128: their weight rows (a TMA box each, 128B swizzle), their
 //                     activations and their scale atoms (one bulk copy each).  The activation operand is
 //                     unswizzled K-major with core matrices 16 * m bytes apart along K, so m tokens take
 //                     m * 128 bytes per slab whatever N is: its columns past m read the neighbouring chunk
@@ -55,8 +55,10 @@ namespace ws {
 __host__ __device__ constexpr int bs_epi_warps(int mp) { return mp >= 32 ? 8 : 4; }
 constexpr int kBsAuxWarps = 4;
 __host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 * (bs_epi_warps(mp) + (wue ? kBsAuxWarps : 0)); }
-// Registers per thread.  Up to 16 tokens two CTAs and a block of the prep kernel fit an SM together.
-__host__ __device__ constexpr int bs_regs(int mp, bool wue) { return mp == 16 ? (wue ? 88 : 144) : wue ? 128 : 168; }
+// Registers per thread: what leaves a warp of the prep kernel room in every quarter of the SM's register file
+// (a CTA of ten warps has three in two of them; the next step's CTA otherwise waits for the prep block to
+// leave), and, up to 16 tokens, a second CTA.
+__host__ __device__ constexpr int bs_regs(int mp, bool wue) { return mp == 16 ? (wue ? 88 : 144) : wue ? 112 : 152; }
 constexpr int kBsMaxAcc = 8;         // accumulator groups in tensor memory (a group = one stage's slabs)
 constexpr int kBsMaxTokens = 128;    // activation rows one launch takes (16, 32, 64 or 128 MMA columns)
 constexpr int kBsAtomBytes = 512;    // one scale atom: 128 rows x 4 K blocks
@@ -82,7 +84,7 @@ struct ActPrepParams {
 // slab is written as zeros.  Few threads per SM: beside 256 of them the main kernel's CTA found no registers
 // and started late (measured at 40 rows: some CTAs 4.6 us after the predecessor's end instead of 1).
 constexpr int kActPrepThreads = 128;
-__global__ void __launch_bounds__(kActPrepThreads) act_prep_kernel(const __grid_constant__ ActPrepParams p) {
+__global__ void __launch_bounds__(kActPrepThreads, 12) act_prep_kernel(const __grid_constant__ ActPrepParams p) {
     // The step that follows may become resident at once (it streams weights until its own wait);
     // the activations come from earlier work on the stream.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -118,13 +120,12 @@ __global__ void __launch_bounds__(kActPrepThreads) act_prep_kernel(const __grid_
 
 // ---------------------------------------------------------------- main kernel
 struct alignas(64) BsParams {
-    CUtensorMap tmap_w[WS_MAX_WORLD];  // weight shard as [whole slabs][n][128 bytes]: box SL slabs x tile_rows x 128 bytes, 128B swizzle
-    CUtensorMap tmap_t[WS_MAX_WORLD];  // weight shard as [n][k bytes], box tile_rows x 128 bytes: slabs of a group that is not whole
+    CUtensorMap tmap_w[WS_MAX_WORLD];  // weight shard [n][k bytes], box 128 bytes x tile_rows, 128B swizzle
     int32_t m, cols, n, k, ks, bn_shift, bk_shift;  // cols: N of the MMA, a multiple of 16 in [m, MP]
     int32_t world, mode, vocab, tmem_cols;  // tmem_cols: tensor-memory columns to allocate (512, or at most 256 when two CTAs share an SM)
     int32_t owner_reduce;              // all-reduce by owners: tile t is folded by rank t % world, which sends the sums back
     int32_t csize;                     // 1, or 2: CTA pairs (a cluster) share a tile, each streams half of K
-    int32_t tile_rows, ntiles;         // output rows per tile (a multiple of 8, <= 128) and tiles of the shard
+    int32_t tile_rows, ntiles;         // output rows per tile (<= 128) and tiles of the shard
     int32_t slabs_per_stage, nstages;
     int32_t a_pitch, x_pitch;          // bytes one slab's weights (a multiple of 1024) / one stage's activations and atoms (of 128) occupy
     int32_t skb, nslot_max, nacc, gather_logits;
@@ -430,15 +431,10 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             // Weights are static: the first ring's worth streams before the wait on the prep kernel;
             // the activations follow once it has finished.
             const uint32_t x_slab = (uint32_t)p.m * 128u, x_atom = (uint32_t)bs_atom_bytes(p.m);
-            const int whole = p.k >> 7;  // slabs of the 3-D map
             auto issue_w = [&](int s, int tile, int s0, int nsl) {
                 mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + x_slab + x_atom));
-                const uint32_t dst = a0 + s * SL * p.a_pitch;
-                if (nsl == SL && s0 + nsl <= whole) {
-                    tma_load_3d(dst, &p.tmap_w[vr], 0, tile * TR, s0, full0 + s * 8);
-                } else {
-                    for (int j = 0; j < nsl; ++j) tma_load_2d(dst + j * p.a_pitch, &p.tmap_t[vr], (s0 + j) * 128, tile * TR, full0 + s * 8);
-                }
+                for (int j = 0; j < nsl; ++j)
+                    tma_load_2d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (s0 + j) * 128, tile * TR, full0 + s * 8);
             };
             int tile, s0, nsl;
             {   // first lap of the ring: weights at once

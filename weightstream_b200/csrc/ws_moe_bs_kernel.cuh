@@ -31,6 +31,10 @@
 //                       pass the CTAs of a pair swap their sums through distributed shared memory, each
 //                       adds the halves of K for half of the tokens and stores or exchanges those rows.
 //
+// A step of up to kMoeBsInlineRoutes routes has no prep kernel: every CTA reads the route ids, makes the pass
+// table and quantises its K half of the routes' hidden into shared memory while the weights stream (the prep
+// kernel's launch, run and completion stood in front of the first weight byte: ~3 us of a one-token step).
+//
 // Exchange: as in the FP8 kernels (partials stored to every peer as tagged words, folded in rank order).
 #pragma once
 
@@ -44,6 +48,7 @@ namespace ws {
 
 constexpr int kMoeBsCols = 16;        // routes of one expert per pass = N of the MMA
 constexpr int kMoeBsThreads = 320;    // warp 0 producer, 1 MMA issue, 2-5 epilogue, 6-9 weight-scale atoms
+constexpr int kMoeBsInlineRoutes = 16;  // up to so many routes the main kernel sorts and quantises itself (no prep launch)
 constexpr int kMoeBsMaxSlabs = 16;    // K slabs one CTA walks per pass (k <= 4096 with pairs)
 
 // Per-endpoint scratch written by moe_bs_prep_kernel and read by moe_bs_kernel.
@@ -151,6 +156,10 @@ struct MoeBsRank {
     const uint8_t *s2;    // [e_len][n][k/32] UE8M0
     const uint8_t *work;  // MoeBsWork
     float *out;           // [m][n]
+    const void *h;        // inline form only: hidden, route ids and weights as the prep kernel takes them
+    const int32_t *route_ids;
+    const float *route_w;
+    int64_t ldh;
     int32_t e_start, e_len;
     RankCtx ctx;
 };
@@ -159,29 +168,33 @@ struct alignas(64) MoeBsParams {
     CUtensorMap tmap_w[WS_MAX_WORLD];  // expert slab as [e_len][n][k] 4-bit codes; boxes of 128 codes x tile_rows x 1, unpacked, 128B swizzle
     int32_t m, n, k, world;
     int32_t tile_rows, a_pitch, slabs_per_stage, nstages;
-    int32_t tmem_cols, x_pitch, alias, pad0;  // alias: the partner's sums land in the ring
+    int32_t tmem_cols, x_pitch, alias, nroutes;  // alias: the partner's sums land in the ring; nroutes = m * top_k
+    int32_t inline_x, top_k, h_dtype, prefetch;
     uint64_t timeout_ns;
     SymLayout lay;
     MoeBsRank r[WS_MAX_WORLD];
 };
 
 struct MoeBsSmem {
-    int32_t a, b, sfa, acc, rx, bars, misc, total;
+    int32_t a, b, sfa, rx, pass, tok, bars, misc, total;
 };
 __host__ __device__ inline MoeBsSmem moe_bs_smem_layout(int nstages, int slabs_per_stage, int a_pitch, int x_pitch, int m, int nslab_cta,
-                                                        int alias) {
+                                                        int alias, int nroutes, int inline_x) {
     MoeBsSmem s{};
     int o = 0;
     s.a = o;    o += nstages * slabs_per_stage * a_pitch;
-    s.b = o;    o += nstages * x_pitch;  // per stage: its slabs' activations, then their scale atoms
+    // per stage: its slabs' activations, then their scale atoms; inline: those of all routes, this K half
+    const int b_bytes = inline_x ? nroutes * nslab_cta * 144 : nstages * x_pitch;
+    s.b = o;    o += (b_bytes + 127) / 128 * 128;
     // an MMA reads 128 rows behind the last weight slab, 16 routes and 32 atom rows whatever the pass has
-    o += nstages * x_pitch + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - nstages * x_pitch : 2048;
+    o += b_bytes + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - b_bytes / 128 * 128 : 2048;
     s.sfa = o;  o += 2 * nslab_cta * kBsAtomBytes;                      // weight-scale atoms of two passes
-    s.acc = o;  o += m * kBsMmaRows * 4;                                // sums of (token, row)
     s.rx = alias ? 0 : o;                                               // the partner's, at the end
     o += alias ? 0 : (m + 1) / 2 * kBsMmaRows * 4;
-    s.bars = o; o += (2 * kMaxStages + 8) * 8;
-    s.misc = o; o += 64;
+    s.pass = o; o += (nroutes * (int)sizeof(MoePass) + 15) / 16 * 16;
+    s.tok = o;  o += ((nroutes > kMoeBsInlineRoutes ? nroutes : 2 * kMoeBsInlineRoutes) * 2 + 15) / 16 * 16;
+    s.bars = o; o += (2 * kMaxStages + 10) * 8;
+    s.misc = o; o += 128;
     s.total = o;
     return s;
 }
@@ -190,6 +203,59 @@ __host__ __device__ inline MoeBsSmem moe_bs_smem_layout(int nstages, int slabs_p
 __device__ __forceinline__ uint32_t moe_bs_idesc(int sf_id) {
     return ((uint32_t)sf_id << 4) | (5u << 7) | (0u << 10) | ((uint32_t)(kMoeBsCols >> 3) << 17) | (1u << 23) | (8u << 24) |
            ((uint32_t)sf_id << 29);
+}
+
+// Inline form: the 256 threads of warps 2-9 quantise hidden x routing-weight of this CTA's K half into the
+// resident activation area: per pass [chunk][nr][16 bytes], then, after those of all routes, the scale atoms.
+// The first two rounds' values (all there are in a one-token step) are loaded before the table is there.
+__device__ __forceinline__ void moe_bs_quantise(const MoeBsParams &p, const MoeBsRank &A, uint8_t *xres, const uint16_t *place,
+                                                int nslab, int k_lo, int t256) {
+    const int chunks = nslab * 8, total = p.nroutes * chunks;  // two adjacent lanes share a 32-block
+    uint8_t *atoms = xres + (size_t)p.nroutes * chunks * 16;
+    for (int c0 = t256; c0 - (t256 & 31) < total; c0 += 512) {  // whole warps
+        float v[2][16], w[2];
+        int rt[2], ch[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int c = c0 + u * 256;
+            const bool in = c < total;
+            rt[u] = in ? c / chunks : 0;
+            ch[u] = in ? c - rt[u] * chunks : 0;
+            const int64_t at = (int64_t)rt[u] * A.ldh + (int64_t)k_lo * 128 + ch[u] * 16;
+            load_act8(A.h, p.h_dtype, at, in, *reinterpret_cast<float(*)[8]>(v[u]));
+            load_act8(A.h, p.h_dtype, at + 8, in, *reinterpret_cast<float(*)[8]>(v[u] + 8));
+            w[u] = in ? A.route_w[rt[u]] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[u][i] *= w[u];
+            int ex;
+            const uint4 q = act_quant16(v[u], ex);
+            const int pl = place[rt[u]], first = pl & 31, t = pl >> 5 & 31, nr = pl >> 10;
+            if (c0 + u * 256 < total && nr > 0) {
+                *reinterpret_cast<uint4 *>(xres + ((size_t)first * chunks + (size_t)ch[u] * nr + t) * 16) = q;
+                if ((ch[u] & 1) == 0)
+                    atoms[((size_t)first * nslab + (size_t)(ch[u] >> 3) * nr + t) * 16 + ((ch[u] >> 1) & 3)] = (uint8_t)min(max(ex + 127, 0), 255);
+            }
+        }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// One tensor-memory column of this warp's lanes.
+__device__ __forceinline__ float tmem_ld_one(uint32_t taddr) {
+    uint32_t r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\ttcgen05.wait::ld.sync.aligned;" : "=r"(r) : "r"(taddr) : "memory");
+    return __uint_as_float(r);
+}
+__device__ __forceinline__ void tmem_st_one(uint32_t taddr, float v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(__float_as_uint(v)) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// L2 prefetch of a box of the expert slab.
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int x, int y, int z) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(x), "r"(y), "r"(z) : "memory");
 }
 
 __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_constant__ MoeBsParams p) {
@@ -211,9 +277,8 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
     const int SL = p.slabs_per_stage, NS = p.nstages;
     const int IP = (NSLAB + SL - 1) / SL;                           // stage items per pass
 
-    const MoeBsSmem S = moe_bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.m, NSLAB, p.alias);
+    const MoeBsSmem S = moe_bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.m, NSLAB, p.alias, p.nroutes, p.inline_x);
     const MoeBsWork W = moe_bs_work_layout(p.k);
-    float *acc_s = reinterpret_cast<float *>(smem + S.acc);
     uint32_t *misc_s = reinterpret_cast<uint32_t *>(smem + S.misc);
     const uint32_t a0 = smem_u32(smem + S.a), b0 = smem_u32(smem + S.b), sfa0 = smem_u32(smem + S.sfa);
     // full[s]: a stage's bytes landed; done[s]: its MMAs have completed (stage free); accfull[g] /
@@ -221,6 +286,7 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
     // sfafull[g]: the weight scales of a pass are in tensor memory.
     const uint32_t full0 = smem_u32(smem + S.bars), done0 = full0 + kMaxStages * 8;
     const uint32_t accfull0 = done0 + kMaxStages * 8, accempty0 = accfull0 + 16, sfafull0 = accempty0 + 16;
+    const uint32_t xready = sfafull0 + 16;  // inline: the routes' activations are in shared memory
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
@@ -232,13 +298,13 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
             mbar_init(accempty0 + b * 8, 4);    // one arrival per epilogue warp
             mbar_init(sfafull0 + b * 8, 1);     // the commit that follows the scale warps' copies
         }
+        mbar_init(xready, 256);
         mbar_fence_init();
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(misc_s), (uint32_t)p.tmem_cols);
         tmem_relinquish();
     }
-    for (int i = tid; i < p.m * kBsMmaRows; i += kMoeBsThreads) acc_s[i] = 0.0f;
     if (tid == 0) misc_s[8] = 0u;
     tc_fence_before();
     __syncthreads();
@@ -246,14 +312,53 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(misc_s);
-    // tensor-memory columns: two accumulators of 16, then per pass buffer and slab 4 activation-scale
-    // and 4 weight-scale columns
-    const uint32_t t_sc0 = tmem_base + 2u * kMoeBsCols;
+    // tensor-memory columns: two accumulators of 16, per pass buffer and slab 4 activation-scale and 4
+    // weight-scale columns, then the sums of every token (lane = row): in shared memory those of 64 tokens took
+    // 32 KB from the ring, and the step was bound by the bytes in flight
+    const uint32_t t_sc0 = tmem_base + 2u * kMoeBsCols, t_tok0 = t_sc0 + (uint32_t)(2 * NSLAB * 8);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // everything below depends on the prep kernel's pass table
+    // everything below depends on the routes (or the prep kernel's pass table)
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int npass = *reinterpret_cast<const volatile int32_t *>(A.work + W.hdr);
-    const MoePass *passes = reinterpret_cast<const MoePass *>(A.work + W.pass);
+    MoePass *passes = reinterpret_cast<MoePass *>(smem + S.pass);
+    uint16_t *stok = reinterpret_cast<uint16_t *>(smem + S.tok);  // token of every route, sorted by (expert, route)
+    int npass;
+    if (p.inline_x) {
+        // One pass per expert (at most 16 routes).  Lane = route, every warp for itself: the lanes of the same
+        // expert by one match, a route's place by counting the routes before it in (expert, route) order.
+        const int e = lane < p.nroutes ? A.route_ids[lane] - A.e_start : -1;
+        const bool local = e >= 0 && e < A.e_len;
+        const uint32_t valid = __ballot_sync(0xffffffffu, local);
+        const uint32_t same = __match_any_sync(0xffffffffu, local ? e : -1 - lane);
+        const uint32_t leaders = __ballot_sync(0xffffffffu, local && (same & ((1u << lane) - 1u)) == 0u);
+        npass = __popc(leaders);
+        if (warp == 0) {
+            int below = 0, before = 0;  // routes and passes of smaller experts
+#pragma unroll
+            for (int i = 0; i < kMoeBsInlineRoutes; ++i) {
+                const int ei = __shfl_sync(0xffffffffu, e, i);
+                const bool less = (valid >> i & 1u) && ei < e;
+                below += less ? 1 : 0;
+                before += less && (leaders >> i & 1u) ? 1 : 0;
+            }
+            if (local) {
+                const int t = __popc(same & ((1u << lane) - 1u)), pos = below + t;
+                if (t == 0) passes[before] = MoePass{(uint16_t)e, (uint16_t)below, (uint16_t)__popc(same), (uint16_t)0};
+                stok[pos] = (uint16_t)(lane / p.top_k);
+                // for the quantiser, by route: its pass's first place and count, its own place in the pass (the
+                // token table has room for 16 more entries)
+                stok[kMoeBsInlineRoutes + lane] = (uint16_t)(below | t << 5 | __popc(same) << 10);
+            } else if (lane < p.nroutes) {
+                stok[kMoeBsInlineRoutes + lane] = 0;  // another rank's
+            }
+        }
+    } else {
+        npass = *reinterpret_cast<const volatile int32_t *>(A.work + W.hdr);
+        const MoePass *src = reinterpret_cast<const MoePass *>(A.work + W.pass);
+        for (int i = tid; i < npass; i += kMoeBsThreads) passes[i] = src[i];
+        const uint16_t *st = reinterpret_cast<const uint16_t *>(A.work + W.stok);
+        for (int i = tid; i < p.nroutes; i += kMoeBsThreads) stok[i] = st[i];
+    }
+    __syncthreads();
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer (one thread)
@@ -269,9 +374,10 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
                     const int s = st.s, j0 = i * SL, nsl = min(SL, NSLAB - j0);
                     if (item >= NS && !mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status)) { ps = npass; break; }
                     // the unpacking copy counts the packed bytes it read (64 per row), not the 128 it wrote
-                    mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 64u + x_slab + x_atom));
+                    mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 64u + (p.inline_x ? 0u : x_slab + x_atom)));
                     for (int j = 0; j < nsl; ++j)
                         tma_load_3d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (k_lo + j0 + j) * 128, row0, (int)P.expert, full0 + s * 8);
+                    if (p.inline_x) continue;
                     const uint32_t dst = b0 + s * p.x_pitch;
                     bulk_load(dst, xq + (size_t)j0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
                     bulk_load(dst + (uint32_t)SL * x_slab, xsf + (size_t)j0 * x_atom, (uint32_t)nsl * x_atom, full0 + s * 8);
@@ -286,7 +392,7 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
             const uint32_t a_step = (uint32_t)p.a_pitch >> 4, x_stage = (uint32_t)p.x_pitch >> 4;
             const uint64_t sf_desc0 = umma_desc(b0, 128, false);
             RingPos st;
-            bool ok = true;
+            bool ok = !p.inline_x || mbar_wait(xready, 0, X.status);
             for (int ps = 0; ps < npass && ok; ++ps) {
                 const int g = ps & 1;
                 const uint32_t lap = (uint32_t)(ps >> 1) & 1u;
@@ -294,13 +400,17 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
                 tc_fence_after();
                 const uint32_t t_acc = tmem_base + (uint32_t)(g * kMoeBsCols);
                 uint32_t t_sc = t_sc0 + (uint32_t)(g * NSLAB * 8);
-                const uint32_t nr = passes[ps].nr, b_step = 8u * nr, x_kb = 2u * nr;  // 16-byte units, as in the FP8 kernel
+                const MoePass P = passes[ps];
+                const uint32_t nr = P.nr, b_step = 8u * nr, x_kb = 2u * nr;  // 16-byte units, as in the FP8 kernel
+                // inline: the pass's activations and atoms in the resident area
+                const uint32_t x_res = b_lo0 + (uint32_t)P.first * (uint32_t)NSLAB * 8u, sf_res = (uint32_t)(p.nroutes * NSLAB) * 8u + (uint32_t)P.first * (uint32_t)NSLAB;
                 for (int i = 0; i < IP; ++i, st.next(NS)) {
                     const int s = st.s, nsl = min(SL, NSLAB - i * SL);
                     if (!mbar_wait(full0 + s * 8, st.ph, X.status)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = (b_lo0 + (uint32_t)s * x_stage) | (nr << 16);
-                    const uint64_t sf_desc = sf_desc0 + (uint64_t)((uint32_t)s * x_stage + (uint32_t)SL * b_step);  // a stage's atoms follow its activations
+                    const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = (p.inline_x ? x_res + (uint32_t)(i * SL) * b_step : b_lo0 + (uint32_t)s * x_stage) | (nr << 16);
+                    const uint64_t sf_desc = sf_desc0 + (uint64_t)(p.inline_x ? sf_res + (uint32_t)(i * SL) * nr
+                                                                             : (uint32_t)s * x_stage + (uint32_t)SL * b_step);  // a stage's atoms follow its activations
                     // straight-line code per slab count, as in the FP8 kernel
                     auto issue = [&](auto count) {
 #pragma unroll
@@ -335,17 +445,34 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
         const bool real = r < TR && row < p.n;
         const int kb32 = p.k >> 5;
         const uint64_t sfa_desc0 = umma_desc(sfa0, 128, false);
+        uint32_t sc[kMoeBsMaxSlabs];  // the next pass's bytes, on their way while this one is written
+        auto fetch = [&](int ps) {
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(A.s2 + ((size_t)passes[ps].expert * p.n + (real ? row : 0)) * kb32) + k_lo;
+#pragma unroll
+            for (int j = 0; j < kMoeBsMaxSlabs; ++j)
+                if (j < NSLAB) sc[j] = real ? __ldg(src + j) : 0x7F7F7F7Fu;
+        };
+        if (npass > 0) fetch(0);
+        if (p.inline_x) {
+            moe_bs_quantise(p, A, smem + S.b, stok + kMoeBsInlineRoutes, NSLAB, k_lo, tid - 64);
+            mbar_arrive(xready);
+        }
         for (int ps = 0; ps < npass; ++ps) {
             const int g = ps & 1;
             const uint32_t lap = (uint32_t)(ps >> 1) & 1u;
             // the pass that used these columns and this buffer last (ps - 2) has completed; a wait that
             // gave up is told to all four warps at the barrier below, so that they leave the loop together
             if (ps >= 2 && !mbar_wait(accfull0 + g * 8, lap ^ 1u, X.status)) misc_s[8] = 1u;
-            const int e = passes[ps].expert;
             uint8_t *dst = smem + S.sfa + (size_t)(g * NSLAB) * kBsAtomBytes + (r & 31) * 16 + (r >> 5) * 4;
-            const uint32_t *src = reinterpret_cast<const uint32_t *>(A.s2 + ((size_t)e * p.n + (real ? row : 0)) * kb32) + k_lo;
-            for (int j = 0; j < NSLAB; ++j)
-                *reinterpret_cast<uint32_t *>(dst + (size_t)j * kBsAtomBytes) = real ? __ldg(src + j) : 0x7F7F7F7Fu;
+#pragma unroll
+            for (int j = 0; j < kMoeBsMaxSlabs; ++j)
+                if (j < NSLAB) *reinterpret_cast<uint32_t *>(dst + (size_t)j * kBsAtomBytes) = sc[j];
+            if (ps + 1 < npass) fetch(ps + 1);
+            if (p.prefetch && warp == 9 && ps + p.prefetch < npass && elect_one()) {
+                const int e = passes[ps + p.prefetch].expert;
+                for (int j = 0; j < NSLAB; ++j) tma_prefetch_3d(&p.tmap_w[vr], (k_lo + j) * 128, row0, e);
+            }
+            __syncwarp();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("bar.sync 3, 128;" ::: "memory");
             if (*reinterpret_cast<volatile uint32_t *>(misc_s + 8) != 0u) break;
@@ -362,8 +489,13 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
         // ------------------------------------------------------------ epilogue warps 2-5
         const int quad = warp & 3;
         const int rc = quad * 32 + lane;  // row inside the tile = TMEM lane
-        const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
-        const uint16_t *stok = reinterpret_cast<const uint16_t *>(A.work + W.stok);
+        const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16), t_tok = t_tok0 - tmem_base;
+        if (p.inline_x) {
+            moe_bs_quantise(p, A, smem + S.b, stok + kMoeBsInlineRoutes, NSLAB, k_lo, tid - 64);
+            mbar_arrive(xready);
+        }
+        for (int t = 0; t < p.m; ++t) tmem_st_one(tlane + t_tok + (uint32_t)t, 0.0f);
+        tmem_wait_st();
         bool ok = true;
         for (int ps = 0; ps < npass; ++ps) {
             const int g = ps & 1;
@@ -380,8 +512,13 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
             if (lane == 0) mbar_arrive(accempty0 + g * 8);
 #pragma unroll
             for (int t = 0; t < kMoeBsCols; ++t)
-                if (t < (int)P.nr) acc_s[(int)stok[P.first + t] * kBsMmaRows + rc] += __uint_as_float(v[t]);
+                if (t < (int)P.nr) {  // in route order: two routes of one pass may belong to one token
+                    const uint32_t at = tlane + t_tok + (uint32_t)stok[P.first + t];
+                    tmem_st_one(at, tmem_ld_one(at) + __uint_as_float(v[t]));
+                    tmem_wait_st();
+                }
         }
+        tc_fence_before();
     }
 
     // ---- the pair's halves of K: each CTA sends the other the sums of the tokens that one finishes
@@ -393,44 +530,49 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     const int split = (p.m + 1) / 2;
-    const int tok_lo = crank == 0 ? 0 : split, ntok = crank == 0 ? split : p.m - split;
-    {
-        const int other = crank == 0 ? split : 0, nother = p.m - ntok;
-        const uint32_t dst = mapa_u32(smem_u32(rx_s), crank ^ 1u);
-        for (int i = tid; i < nother * kBsMmaRows; i += kMoeBsThreads) st_cluster_f32(dst + (uint32_t)i * 4u, acc_s[other * kBsMmaRows + i]);
+    const int tok_lo = crank == 0 ? 0 : split, tok_hi = crank == 0 ? split : p.m;
+    const int quad = warp & 3, rc = quad * 32 + lane, row = row0 + rc;  // the epilogue warps: row = TMEM lane
+    const uint32_t tlane = t_tok0 + ((uint32_t)(quad * 32) << 16);
+    const bool epi = warp >= 2 && warp < 6;
+    if (epi) {
+        tc_fence_after();
+        const int lo = crank == 0 ? split : 0, hi = crank == 0 ? p.m : split;  // the partner's tokens
+        const uint32_t dst = mapa_u32(smem_u32(rx_s) + (uint32_t)rc * 4u, crank ^ 1u);
+        for (int t = lo; t < hi; ++t) st_cluster_f32(dst + (uint32_t)((t - lo) * kBsMmaRows * 4), tmem_ld_one(tlane + (uint32_t)t));
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // nothing crosses the pair after this
 
     const bool solo = p.world == 1;
-    const uint32_t seq = step_begin(X);
-    const uint32_t bank = seq & 1u;
-    const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
-    // K half 0 + K half 1; thread -> (token, row)
-    for (int i = tid; i < ntok * kBsMmaRows; i += kMoeBsThreads) {
-        const int tok = tok_lo + (i >> 7), rc = i & 127, row = row0 + rc;
-        if (rc >= TR || row >= p.n) continue;
-        const float v = acc_s[tok_lo * kBsMmaRows + i] + rx_s[i];
-        if (solo) {
-            A.out[(size_t)tok * p.n + row] = v;
-        } else {
-            for (int pr = 0; pr < p.world; ++pr) {
-                uint64_t *dstw = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride;
-                st_word_sys(dstw + (size_t)tok * p.n + row, seq, v);
+    const bool mine = rc < TR && row < p.n;
+    if (epi) {
+        const uint32_t seq = step_begin(X);
+        const uint32_t bank = seq & 1u;
+        const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
+        for (int t = tok_lo; t < tok_hi; ++t) {  // K half 0 + K half 1
+            const float v = tmem_ld_one(tlane + (uint32_t)t) + rx_s[(t - tok_lo) * kBsMmaRows + rc];
+            if (!mine) continue;
+            if (solo) {
+                A.out[(size_t)t * p.n + row] = v;
+            } else {
+                for (int pr = 0; pr < p.world; ++pr) {
+                    uint64_t *dstw = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride;
+                    st_word_sys(dstw + (size_t)t * p.n + row, seq, v);
+                }
             }
         }
-    }
-    if (!solo) {  // fold the same rows in rank order as the ranks' words arrive
-        const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
-        for (int i = tid; i < ntok * kBsMmaRows; i += kMoeBsThreads) {
-            const int tok = tok_lo + (i >> 7), rc = i & 127, row = row0 + rc;
-            if (rc >= TR || row >= p.n) continue;
-            const size_t off = (size_t)tok * p.n + row;
-            A.out[off] = fold_words(slots, astride, off, p.world, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
+        if (!solo && mine) {  // fold the same rows in rank order as the ranks' words arrive
+            const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
+            for (int t = tok_lo; t < tok_hi; ++t) {
+                const size_t off = (size_t)t * p.n + row;
+                A.out[off] = fold_words(slots, astride, off, p.world, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
+            }
         }
     }
 
     // ---- teardown
+    tc_fence_before();
+    __syncthreads();
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
