@@ -128,20 +128,20 @@ ws_status_t make_tmap(ws_tp *tp, CUtensorMap *map, const void *base, uint64_t ro
     return WS_OK;
 }
 
-// Expert slab [experts][rows][k] of packed 4-bit codes (row stride k/2 bytes), boxes of 128 codes x
-// box_rows x 1 expert; the copy unpacks 16 codes (8 bytes) into 16 bytes of shared memory, the form
+// Expert slab [experts][rows][k] of packed 4-bit codes (row stride k/2 bytes) as [experts][k / 128][rows][128
+// codes], boxes of 128 codes x box_rows x `slabs` x 1 expert; the copy unpacks 16 codes (8 bytes) into 16 bytes of shared memory, the form
 // tcgen05.mma.kind::mxf8f6f4 reads 4-bit operands in; 128B swizzle.
 ws_status_t make_tmap_fp4(ws_tp *tp, CUtensorMap *map, const void *base, uint64_t experts, uint64_t rows, uint64_t k,
-                          uint32_t box_rows) {
+                          uint32_t box_rows, uint32_t slabs) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(tp, WS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     if ((reinterpret_cast<uintptr_t>(base) & 31) || (k & 255))
         return fail(tp, WS_ERR_INVALID, "expert slab must be 32-byte aligned with k a multiple of 256");
-    cuuint64_t dims[3] = {k, rows, experts};
-    cuuint64_t strides[2] = {k / 2, rows * (k / 2)};
-    cuuint32_t box[3] = {128, (cuuint32_t)box_rows, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, const_cast<void *>(base), dims, strides, box, estr,
+    cuuint64_t dims[4] = {128, rows, k / 128, experts};
+    cuuint64_t strides[3] = {k / 2, 64, rows * (k / 2)};
+    cuuint32_t box[4] = {128, box_rows, slabs, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 4, const_cast<void *>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(tp, WS_ERR_CUDA, "cuTensorMapEncodeTiled (4-bit) failed (%d)", (int)r);
@@ -462,7 +462,7 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     u.ncta = u.csize == 2 ? ncta & ~1 : ncta;
     const int nparts = u.ncta / u.csize;
     // tiles of equal height that deal out evenly: a CTA's share of the rows, cut into as few pieces of at
-    // most 128 rows as possible (multiples of 8, which one TMA box of several slabs needs, left 5 of 74 pairs idle)
+    // most 128 rows as possible
     const int crmax = (a.n + nparts - 1) / nparts;
     const int pieces = (crmax + kBsMmaRows - 1) / kBsMmaRows;
     u.tile_rows = (crmax + pieces - 1) / pieces;
@@ -561,14 +561,14 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
     ActPrepParams q{};
-    q.m = mt; q.k = a0.k; q.x_dtype = a0.x_dtype; q.ks = u.ks;
+    q.m = mt; q.k = a0.k; q.x_dtype = a0.x_dtype; q.ks = u.ks; q.csize = u.csize; q.sl = u.slabs_per_stage;
     // scratch of one endpoint: the quantised activations and their scale atoms
-    const size_t xq_bytes = (size_t)u.ks * kBsMaxTokens * 128, xsf_bytes = (size_t)u.ks * kBsAtomBytes;
+    const size_t xq_bytes = (size_t)u.ks * (kBsMaxTokens * 128 + kBsAtomBytes);
 
     for (int i = 0; i < n; ++i) {
         ws_tp *t = ranks[i];
         const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
-        ws_status_t s = ensure_bs_scratch(t, xq_bytes + xsf_bytes);
+        ws_status_t s = ensure_bs_scratch(t, xq_bytes);
         if (s == WS_OK) s = make_tmap(t, &p.tmap_w[i], a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, (uint32_t)u.tile_rows);
         if (s != WS_OK) { t0->err = t->err; return s; }
         Fp8RankArgs &r = p.r[i];
@@ -583,7 +583,6 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         r.ctx = make_ctx(t);
         if (last) r.ctx.host_done = t->host_done_arm;
         p.xq[i] = q.r[i].xq = t->bs_work;
-        p.xsf[i] = q.r[i].xsf = t->bs_work + xq_bytes;
         q.r[i].x = static_cast<const char *>(a.x) + (size_t)m0 * a.ldx * (a.x_dtype == WS_ACT_BF16 ? 2 : 4);
         q.r[i].ldx = a.ldx;
     }
@@ -598,7 +597,6 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
             p.r[0] = p.r[i];
             p.tmap_w[0] = p.tmap_w[i];
             p.xq[0] = p.xq[i];
-            p.xsf[0] = p.xsf[i];
             q.r[0] = q.r[i];
         }
         const int nvr = same_device ? n : 1;
@@ -949,7 +947,8 @@ static MoeBsPlan moe_bs_plan(const ws_moe_down_args_t &a, int ncta) {
     u.tile_rows = (a.n + nparts - 1) / nparts;
     if (u.tile_rows > kBsMmaRows) return u;
     u.a_pitch = (u.tile_rows + 7) / 8 * 8 * 128;
-    u.slabs_per_stage = std::min(getenv("X2") ? atoi(getenv("X2")) : 2, nslab);
+    const int groups = getenv("X2") ? atoi(getenv("X2")) : 2;
+    u.slabs_per_stage = (nslab + groups - 1) / groups;
     u.inline_x = a.m * a.top_k <= (getenv("X1") ? atoi(getenv("X1")) : kMoeBsInlineRoutes) ? 1 : 0;
     const int nr = std::min((int)kMoeBsCols, a.m * a.top_k);  // most routes of a pass
     u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * (nr * 128 + nr * 16), 128);
@@ -958,6 +957,7 @@ static MoeBsPlan moe_bs_plan(const ws_moe_down_args_t &a, int ncta) {
     auto total = [&](int ns) { return moe_bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, a.m, nslab, u.alias, a.m * a.top_k, u.inline_x).total + 1024; };
     int ns = kMaxStages;
     while (ns >= 2 && total(ns) > kSmemBudget - 8 * 1024) --ns;  // (beside a few blocks of the prep kernel)
+    ns = std::min(ns, 4 * ((nslab + u.slabs_per_stage - 1) / u.slabs_per_stage));  // four pass barriers: see moe_bs_kernel
     u.nstages = ns;
     int cols = 32;
     while (cols < 2 * kMoeBsCols + 2 * nslab * 8 + a.m) cols *= 2;
@@ -976,12 +976,12 @@ static ws_status_t moe_bs_step(ws_tp *const *ranks, int n, const ws_moe_down_arg
     MoeBsParams p{};
     p.m = a0.m; p.n = a0.n; p.k = a0.k; p.world = t0->world;
     p.tile_rows = u.tile_rows; p.a_pitch = u.a_pitch; p.slabs_per_stage = u.slabs_per_stage; p.nstages = u.nstages;
-    p.tmem_cols = u.tmem_cols; p.x_pitch = u.x_pitch; p.alias = u.alias; p.prefetch = getenv("X3") ? atoi(getenv("X3")) : 1;
+    p.tmem_cols = u.tmem_cols; p.x_pitch = u.x_pitch; p.alias = u.alias;
     p.inline_x = u.inline_x; p.nroutes = a0.m * a0.top_k; p.top_k = a0.top_k; p.h_dtype = a0.h_dtype;
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
     MoeBsPrepParams q{};
-    q.m = a0.m; q.k = a0.k; q.top_k = a0.top_k; q.h_dtype = a0.h_dtype;
+    q.m = a0.m; q.k = a0.k; q.top_k = a0.top_k; q.h_dtype = a0.h_dtype; q.sl = u.slabs_per_stage;
     const MoeBsWork W = moe_bs_work_layout(a0.k);
     const int nblk = a0.m * a0.top_k + 1;
     for (int i = 0; i < n; ++i) ranks[i]->step++;
@@ -989,7 +989,8 @@ static ws_status_t moe_bs_step(ws_tp *const *ranks, int n, const ws_moe_down_arg
         ws_tp *t = ranks[i];
         const ws_moe_down_args_t &a = args[i];
         ws_status_t s = u.inline_x ? WS_OK : ensure_moe_scratch(t, (size_t)W.total, 0);
-        if (s == WS_OK) s = make_tmap_fp4(t, &p.tmap_w[0], a.w2, (uint64_t)a.e_len, (uint64_t)a.n, (uint64_t)a.k, (uint32_t)u.tile_rows);
+        if (s == WS_OK) s = make_tmap_fp4(t, &p.tmap_w[0], a.w2, (uint64_t)a.e_len, (uint64_t)a.n, (uint64_t)a.k, (uint32_t)u.tile_rows, (uint32_t)u.slabs_per_stage);
+        if (s == WS_OK) s = make_tmap_fp4(t, &p.tmap_t[0], a.w2, (uint64_t)a.e_len, (uint64_t)a.n, (uint64_t)a.k, (uint32_t)u.tile_rows, 1);
         if (s != WS_OK) { t0->err = t->err; return s; }
         MoeBsRank &r = p.r[0];
         r.s2 = a.s2; r.work = t->moe_work; r.out = a.out; r.e_start = a.e_start; r.e_len = a.e_len;

@@ -108,7 +108,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // caller unwind instead of spinning forever.  Once any wait of the launch has failed (the status
 // word is set) every later wait that is not satisfied at once returns false immediately, so a
 // kernel with hundreds of stage waits ends in one time-out, not hundreds.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *status) {
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint32_t *status) {
     for (int i = 0; i < 64; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     if (*(volatile uint32_t *)status != 0u) return false;
@@ -121,6 +121,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
     }
     atomicCAS(status, 0u, kStatTimeoutTma | (uint32_t)(-WS_ERR_TIMEOUT));
     return false;
+}
+// Most waits of the issuing threads find their phase complete: that costs one probe and a branch.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *status) {
+    return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, status);
 }
 
 // True on one lane of a converged warp.  TMA and tcgen05 instructions take their operands from uniform

@@ -11,7 +11,7 @@
 //                     streams the weights of its tiles, so every output is a complete dot product inside
 //                     one CTA pair and nothing is combined through global memory.  A stage of the ring
 //                     holds SL K slabs of 128: their weight rows (a TMA box each, 128B swizzle), their
-//                     activations and their scale atoms (one bulk copy each).  The activation operand is
+//                     activations and their scale atoms (one bulk copy).  The activation operand is
 //                     unswizzled K-major with core matrices 16 * m bytes apart along K, so m tokens take
 //                     m * 128 bytes per slab whatever N is: its columns past m read the neighbouring chunk
 //                     and are never looked at.  (Padded to N rows the activations of 40 tokens were as many
@@ -28,7 +28,8 @@
 //                     bytes out as atoms in the stage, a tile accumulates over all of its K in tensor
 //                     memory and is read back once.
 //
-// Measured on B200 and kept in mind above: a slab's four MMAs, scale copy and share of the commit take the
+// Measured on B200 and kept in mind above: every TMA or bulk copy costs its issuing thread 85-100 ns, but
+// one 3-D box for a stage's slabs was slower than a box each (128 rows 32.0 against 29.4 us); a slab's four MMAs, scale copy and share of the commit take the
 // tensor pipe 84 ns with N=16, 105 with 64 and 135 with 128, however few of the 128 rows are real (M=64 is
 // not available with block scaling); handing partial sums from one CTA to another through L2 (a split of K
 // across CTAs) costs 3-5 us, more than it saves on these shapes.
@@ -68,15 +69,23 @@ constexpr int kBsMmaRows = 128;      // M of the MMA; a tile of output rows hold
 // come from whatever follows and scale columns that are never read.
 __host__ __device__ constexpr int bs_atom_bytes(int m) { return 16 * (m < 32 ? m : 32); }
 
+// The activation image of a step: the K slabs in the groups that the CTAs' stages take (half h of K owns slabs
+// [h * ks / csize, (h + 1) * ks / csize), cut into groups of at most sl), a group being its chunks, then its atoms.
+__host__ __device__ inline int bs_group(int slab, int ks, int csize, int sl, int &count) {  // first slab of the group, slabs in it
+    const int half = ks / 2, lo = csize == 2 && slab >= half ? half : 0, hi = csize == 2 && slab < half ? half : ks;
+    const int g0 = lo + (slab - lo) / sl * sl;
+    count = sl < hi - g0 ? sl : hi - g0;
+    return g0;
+}
+
 // ---------------------------------------------------------------- activation prep
 struct ActPrepRank {
     const void *x;
-    uint8_t *xq;   // [ks * 8 chunks][m][16] E4M3
-    uint8_t *xsf;  // [ks][bs_atom_bytes(m)]
+    uint8_t *xq;  // see bs_group
     int64_t ldx;
 };
 struct ActPrepParams {
-    int32_t m, k, x_dtype, ks;
+    int32_t m, k, x_dtype, ks, csize, sl;
     ActPrepRank r[WS_MAX_WORLD];
 };
 
@@ -109,9 +118,13 @@ __global__ void __launch_bounds__(kActPrepThreads, 12) act_prep_kernel(const __g
             int e;
             const uint4 q = act_quant16(v[u], e);
             if (c0 + u * step < total) {
-                *reinterpret_cast<uint4 *>(A.xq + ((int64_t)ch[u] * p.m + tok[u]) * 16) = q;
+                const int slab = ch[u] >> 3, t = tok[u], atom = bs_atom_bytes(p.m);
+                int count;
+                const int g0 = bs_group(slab, p.ks, p.csize, p.sl, count);
+                uint8_t *grp = A.xq + (int64_t)g0 * (p.m * 128 + atom);
+                *reinterpret_cast<uint4 *>(grp + ((int64_t)(ch[u] - g0 * 8) * p.m + t) * 16) = q;
                 if ((ch[u] & 1) == 0)
-                    A.xsf[(int64_t)(ch[u] >> 3) * bs_atom_bytes(p.m) + (tok[u] & 31) * 16 + (tok[u] >> 5) * 4 + ((ch[u] >> 1) & 3)] =
+                    grp[(int64_t)count * p.m * 128 + (slab - g0) * atom + (t & 31) * 16 + (t >> 5) * 4 + ((ch[u] >> 1) & 3)] =
                         (uint8_t)min(max(e + 127, 0), 255);
             }
         }
@@ -132,7 +145,7 @@ struct alignas(64) BsParams {
     uint64_t timeout_ns;
     SymLayout lay;
     Fp8RankArgs r[WS_MAX_WORLD];       // x is unused here; scales/out/logits/argmax/row0/k0/ctx as in the decode kernels
-    const uint8_t *xq[WS_MAX_WORLD], *xsf[WS_MAX_WORLD];  // the prep kernel's activations and scale atoms
+    const uint8_t *xq[WS_MAX_WORLD];   // the prep kernel's activations and scale atoms
 };
 
 struct BsSmem {
@@ -310,12 +323,6 @@ __device__ __forceinline__ void bs_epi_bar_n() {  // the epilogue warps
     asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
 }
 
-// 3-D TMA tile load, completion on an mbarrier.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
-}
-
 // The sequence of stage items of one CTA.  The shard's rows are cut into tiles of tile_rows rows
 // (at most 128, the M of the MMA; chosen so that the tiles deal out evenly) and CTA c takes tiles
 // [c * T / ncta, (c + 1) * T / ncta) whole, so every output row is a complete dot product inside one
@@ -430,9 +437,9 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         if (elect_one()) {
             // Weights are static: the first ring's worth streams before the wait on the prep kernel;
             // the activations follow once it has finished.
-            const uint32_t x_slab = (uint32_t)p.m * 128u, x_atom = (uint32_t)bs_atom_bytes(p.m);
+            const uint32_t x_slab = (uint32_t)(p.m * 128 + bs_atom_bytes(p.m));
             auto issue_w = [&](int s, int tile, int s0, int nsl) {
-                mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + x_slab + x_atom));
+                mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + x_slab));
                 for (int j = 0; j < nsl; ++j)
                     tma_load_2d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (s0 + j) * 128, tile * TR, full0 + s * 8);
             };
@@ -450,9 +457,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                     if (!mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status)) break;
                     issue_w(s, tile, s0, nsl);
                 }
-                const uint32_t dst = x0 + s * p.x_pitch;
-                bulk_load(dst, p.xq[vr] + (size_t)s0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
-                bulk_load(dst + (uint32_t)SL * x_slab, p.xsf[vr] + (size_t)s0 * x_atom, (uint32_t)nsl * x_atom, full0 + s * 8);
+                bulk_load(x0 + s * p.x_pitch, p.xq[vr] + (size_t)s0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
             }
         }
     } else if (warp == 1) {
@@ -465,55 +470,82 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (elect_one()) {
             if (!WUE) tmem_cp_atom(t_sfa, umma_desc(wsf0, 128, false));
-            // Everything the loop needs per MMA is an add away: descriptor halves per stage slot, the
-            // four instruction descriptors (one per K block of a slab), ring positions kept incrementally.
+            // The tensor pipe runs on for ~200 clocks after the last MMA it was given, so what this thread does
+            // between two stages has to stay below that: everything is an add away, the waits are on barriers
+            // whose phase is usually complete.
             uint32_t id[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) id[q] = bs_idesc(p.cols, WUE ? q : 0, q);
+            uint32_t *const status = X.status;
             const uint32_t m16 = (uint32_t)p.m;  // 16-byte units: one chunk of all tokens
-            const uint32_t a_lo0 = umma_desc_lo(a0), x_lo0 = ((x0 & 0x3FFFFu) >> 4) | (m16 << 16);
-            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, x_stage = (uint32_t)p.x_pitch >> 4, x_step = 8u * m16, x_kb = 2u * m16;
-            const uint64_t xsf_desc0 = umma_desc(x0, 128, false) + (uint64_t)((uint32_t)SL * x_step), wsf_desc0 = umma_desc(wsf0, 128, false);
-            const uint32_t xsf_step = (uint32_t)bs_atom_bytes(p.m) >> 4;
+            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, x_step = 8u * m16, x_kb = 2u * m16, xsf_step = (uint32_t)bs_atom_bytes(p.m) >> 4;
             constexpr uint32_t kSfStep = (uint32_t)kBsAtomBytes >> 4;
-            BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
-            RingPos st, ag;  // stage ring, accumulator ring
-            int tile, s0, nsl;
-            for (int item = 0; w.next(tile, s0, nsl); ++item, st.next(NS)) {
-                const int s = st.s, g = ag.s;
-                if (!mbar_wait(full0 + s * 8, st.ph, X.status)) break;
-                if ((!WUE || s0 == k_lo) && !mbar_wait(accempty0 + g * 8, ag.ph ^ 1u, X.status)) break;
-                tc_fence_after();
-                const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = x_lo0 + (uint32_t)s * x_stage;
-                const uint64_t xsf = xsf_desc0 + (uint64_t)((uint32_t)s * x_stage);
-                const uint64_t wsf = wsf_desc0 + (uint64_t)((uint32_t)(s * SL) * kSfStep);
-                const uint32_t t_acc = tmem_base + (uint32_t)((WUE ? g : g * SL) * MP);
-                const uint32_t t_sf = t_sf0 + (WUE ? (uint32_t)((item & 1) * SL * 8) : (uint32_t)(g * SL * 4));
-                const uint32_t carry = WUE && s0 != k_lo ? 1u : 0u;  // the stage's first MMA adds to earlier stages' sums
-                // straight-line code per slab count: a rolled loop costs the issuing thread twice the time
-                auto issue = [&](auto count) {
+            // of the current stage: barrier, operand descriptors (low halves), scale atoms; and of ring start
+            const uint32_t a_stage = (uint32_t)SL * a_step, x_stage = (uint32_t)p.x_pitch >> 4;
+            const uint32_t a_lo0 = umma_desc_lo(a0), x_lo0 = ((x0 & 0x3FFFFu) >> 4) | (m16 << 16);
+            const uint64_t xsf0 = umma_desc(x0, 128, false), wsf_desc0 = umma_desc(wsf0, 128, false);
+            uint32_t full = full0, done = done0, a_lo = a_lo0, x_lo = x_lo0, x_off = 0, w_off = 0, ph = 0;
+            const uint32_t full_end = full0 + NS * 8;
+            // accumulator ring
+            uint32_t accempty = accempty0, t_acc = tmem_base, t_sf = t_sf0, acc_ph = 1;
+            const uint32_t acc_end = accempty0 + NB * 8;
+            // one stage: straight-line code per slab count (a rolled loop costs twice the time); `carry`: the first
+            // MMA adds to earlier stages' sums (UE8M0)
+            auto issue = [&](auto count, uint32_t carry) {
+                constexpr int C = decltype(count)::value;
+                const uint64_t xsf = xsf0 + (uint64_t)(x_off + (uint32_t)C * x_step), wsf = wsf_desc0 + (uint64_t)w_off;
 #pragma unroll
-                    for (int j = 0; j < decltype(count)::value; ++j) {
-                        const uint32_t a = a_lo + (uint32_t)j * a_step, b = b_lo + (uint32_t)j * x_step;
-                        const uint32_t d = WUE ? t_acc : t_acc + (uint32_t)(j * MP);
-                        const uint32_t sx = t_sf + (uint32_t)(j * (WUE ? 8 : 4)), sw = WUE ? sx + 4 : t_sfa;
-                        tmem_cp_atom(sx, xsf + (uint64_t)((uint32_t)j * xsf_step));
-                        if (WUE) tmem_cp_atom(sw, wsf + (uint64_t)(j * kSfStep));
-                        umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id[0], sw, sx, WUE && j > 0 ? 1u : carry);
-                        umma_bs_ss(d, a + 2, b + x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[1], sw, sx, 1u);
-                        umma_bs_ss(d, a + 4, b + 2 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[2], sw, sx, 1u);
-                        umma_bs_ss(d, a + 6, b + 3 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[3], sw, sx, 1u);
+                for (int j = 0; j < C; ++j) {
+                    const uint32_t a = a_lo + (uint32_t)j * a_step, b = x_lo + (uint32_t)j * x_step;
+                    const uint32_t d = WUE ? t_acc : t_acc + (uint32_t)(j * MP);
+                    const uint32_t sx = t_sf + (uint32_t)(j * (WUE ? 8 : 4)), sw = WUE ? sx + 4 : t_sfa;
+                    tmem_cp_atom(sx, xsf + (uint64_t)((uint32_t)j * xsf_step));
+                    if (WUE) tmem_cp_atom(sw, wsf + (uint64_t)(j * kSfStep));
+                    umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id[0], sw, sx, WUE && j > 0 ? 1u : carry);
+                    umma_bs_ss(d, a + 2, b + x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[1], sw, sx, 1u);
+                    umma_bs_ss(d, a + 4, b + 2 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[2], sw, sx, 1u);
+                    umma_bs_ss(d, a + 6, b + 3 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[3], sw, sx, 1u);
+                }
+            };
+            const int my_tiles = (int)((int64_t)ntiles * (part + 1) / nparts) - (int)((int64_t)ntiles * part / nparts), kcta = k_hi - k_lo;
+            bool ok = true;
+            uint32_t odd = 0;  // UE8M0: which of the two sets of scale columns
+            for (int t = kcta > 0 ? my_tiles : 0; t > 0 && ok; --t) {
+                uint32_t carry = 0;
+                for (int left = kcta; left > 0; left -= SL) {
+                    if ((!WUE || carry == 0) && !mbar_wait(accempty, acc_ph, status)) { ok = false; break; }
+                    if (!mbar_wait(full, ph, status)) { ok = false; break; }
+                    tc_fence_after();
+                    if (left >= 4 && SL == 4) issue(std::integral_constant<int, 4>{}, carry);
+                    else if (left >= 3 && SL >= 3) issue(std::integral_constant<int, 3>{}, carry);
+                    else if (left >= 2 && SL >= 2) issue(std::integral_constant<int, 2>{}, carry);
+                    else issue(std::integral_constant<int, 1>{}, carry);
+                    umma_commit(done);  // the stage may be refilled (fp32 weight scales: and its accumulators read)
+                    const bool tile_end = WUE && left <= SL;
+                    if (tile_end) umma_commit(accempty + (accfull0 - accempty0));
+                    if (WUE) {
+                        carry = 1;
+                        odd ^= 1u;
                     }
-                };
-                if (nsl == 4) issue(std::integral_constant<int, 4>{});
-                else if (nsl == 3) issue(std::integral_constant<int, 3>{});
-                else if (nsl == 2) issue(std::integral_constant<int, 2>{});
-                else issue(std::integral_constant<int, 1>{});
-                umma_commit(done0 + s * 8);  // the stage may be refilled (fp32 weight scales: and its accumulators read)
-                if (!WUE) ag.next(NB);
-                else if (s0 + nsl == k_hi) {
-                    umma_commit(accfull0 + g * 8);
-                    ag.next(NB);
+                    // next stage
+                    full += 8; done += 8; a_lo += a_stage; x_lo += x_stage; x_off += x_stage;
+                    if (WUE) w_off += (uint32_t)SL * kSfStep;
+                    if (full == full_end) {
+                        full = full0; done = done0; a_lo = a_lo0; x_lo = x_lo0; x_off = 0; w_off = 0;
+                        ph ^= 1u;
+                    }
+                    // next accumulator (group)
+                    if (!WUE || tile_end) {
+                        accempty += 8;
+                        t_acc += (uint32_t)((WUE ? 1 : SL) * MP);
+                        if (!WUE) t_sf += (uint32_t)(SL * 4);
+                        if (accempty == acc_end) {
+                            accempty = accempty0; t_acc = tmem_base;
+                            if (!WUE) t_sf = t_sf0;
+                            acc_ph ^= 1u;
+                        }
+                    }
+                    if (WUE) t_sf = t_sf0 + odd * (uint32_t)(SL * 8);
                 }
             }
         }

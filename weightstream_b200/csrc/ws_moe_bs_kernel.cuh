@@ -17,7 +17,7 @@
 //                       each CTA of a pair streams half of K of every pass: with a lone CTA's ~48
 //                       rows under half of the MMA's 128 rows would be real, and the tensor pipe
 //                       needs the same ~35 ns per K=32 MMA however few are.  Warp 0 lane 0 streams,
-//                       per stage of up to four 128-wide K slabs, the expert's rows (TMA, 4-bit codes
+//                       per stage of several 128-wide K slabs, the expert's rows (TMA, 4-bit codes
 //                       unpacked by the copy into the 16-bytes-per-16-codes form the MMA reads) and the
 //                       pass's activations and scale atoms (one bulk copy each, only of the routes there
 //                       are: padded to the MMA's 16 columns they were 40 % of the weights' bytes, and what
@@ -53,7 +53,7 @@ constexpr int kMoeBsMaxSlabs = 16;    // K slabs one CTA walks per pass (k <= 40
 
 // Per-endpoint scratch written by moe_bs_prep_kernel and read by moe_bs_kernel.
 struct MoeBsWork {
-    int64_t hdr, pass, stok, xq, xsf, total;  // byte offsets
+    int64_t hdr, pass, stok, xq, total;  // byte offsets
 };
 __host__ __device__ inline MoeBsWork moe_bs_work_layout(int k) {
     MoeBsWork w{};
@@ -61,14 +61,15 @@ __host__ __device__ inline MoeBsWork moe_bs_work_layout(int k) {
     w.hdr = o;  o += 64;
     w.pass = o; o += (int64_t)kMoeMaxRoutes * sizeof(MoePass);
     w.stok = o; o += align_up((int64_t)(kMoeMaxRoutes + kMoeBsCols) * 2, 256);
-    w.xq = o;   o += (int64_t)kMoeMaxRoutes * k;               // a pass starts at its first route's row: [k / 16 chunks][nr][16]
-    w.xsf = o;  o += (int64_t)kMoeMaxRoutes * (k / 128) * 16;  // likewise: [k / 128 slabs][nr][16]
+    // a pass starts at its first route's share; per K half and group of up to SL slabs: [8 * slabs chunks][nr][16],
+    // then the group's atoms [slabs][nr][16]
+    w.xq = o;   o += (int64_t)kMoeMaxRoutes * (k / 128) * 144;
     w.total = o;
     return w;
 }
 
 struct MoeBsPrepParams {
-    int32_t m, k, top_k, h_dtype;
+    int32_t m, k, top_k, h_dtype, sl, pad0;
     MoePrepRank r[WS_MAX_WORLD];
 };
 
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(256) moe_bs_prep_kernel(const __grid_constant_
     }
     const float w = A.route_w[route];
     const int first = pos - t, nr = min(kMoeBsCols, cnt_s[e] - (rnk - t));  // the pass's first route and route count
-    uint8_t *xq = A.work + W.xq + (size_t)first * p.k, *xsf = A.work + W.xsf + (size_t)first * (p.k >> 7) * 16;
+    uint8_t *xq = A.work + W.xq + (size_t)first * (p.k >> 7) * 144;
     for (int c = tid; c < (p.k >> 4); c += blockDim.x) {  // the two chunks of a 32-block are adjacent lanes
         float v[16];
         load_act8(A.h, p.h_dtype, (int64_t)route * A.ldh + c * 16, true, *reinterpret_cast<float(*)[8]>(v));
@@ -146,8 +147,11 @@ __global__ void __launch_bounds__(256) moe_bs_prep_kernel(const __grid_constant_
         for (int i = 0; i < 16; ++i) v[i] *= w;
         int ex;
         const uint4 q = act_quant16(v, ex);
-        *reinterpret_cast<uint4 *>(xq + ((size_t)c * nr + t) * 16) = q;
-        if ((c & 1) == 0) xsf[((size_t)(c >> 3) * nr + t) * 16 + ((c >> 1) & 3)] = (uint8_t)min(max(ex + 127, 0), 255);
+        int count;
+        const int slab = c >> 3, g0 = bs_group(slab, p.k >> 7, 2, p.sl, count);
+        uint8_t *grp = xq + (size_t)g0 * nr * 144;
+        *reinterpret_cast<uint4 *>(grp + ((size_t)(c - g0 * 8) * nr + t) * 16) = q;
+        if ((c & 1) == 0) grp[(size_t)count * nr * 128 + ((size_t)(slab - g0) * nr + t) * 16 + ((c >> 1) & 3)] = (uint8_t)min(max(ex + 127, 0), 255);
     }
 }
 
@@ -165,11 +169,13 @@ struct MoeBsRank {
 };
 
 struct alignas(64) MoeBsParams {
-    CUtensorMap tmap_w[WS_MAX_WORLD];  // expert slab as [e_len][n][k] 4-bit codes; boxes of 128 codes x tile_rows x 1, unpacked, 128B swizzle
+    // expert slab as [e_len][k / 128][n][128] 4-bit codes; boxes of 128 codes x tile_rows x SL slabs ([0]) or one
+    // slab ([t]: those of a group that is not whole), unpacked, 128B swizzle
+    CUtensorMap tmap_w[WS_MAX_WORLD], tmap_t[WS_MAX_WORLD];
     int32_t m, n, k, world;
     int32_t tile_rows, a_pitch, slabs_per_stage, nstages;
     int32_t tmem_cols, x_pitch, alias, nroutes;  // alias: the partner's sums land in the ring; nroutes = m * top_k
-    int32_t inline_x, top_k, h_dtype, prefetch;
+    int32_t inline_x, top_k, h_dtype, pad0;
     uint64_t timeout_ns;
     SymLayout lay;
     MoeBsRank r[WS_MAX_WORLD];
@@ -193,7 +199,7 @@ __host__ __device__ inline MoeBsSmem moe_bs_smem_layout(int nstages, int slabs_p
     o += alias ? 0 : (m + 1) / 2 * kBsMmaRows * 4;
     s.pass = o; o += (nroutes * (int)sizeof(MoePass) + 15) / 16 * 16;
     s.tok = o;  o += ((nroutes > kMoeBsInlineRoutes ? nroutes : 2 * kMoeBsInlineRoutes) * 2 + 15) / 16 * 16;
-    s.bars = o; o += (2 * kMaxStages + 10) * 8;
+    s.bars = o; o += (2 * kMaxStages + 12) * 8;
     s.misc = o; o += 128;
     s.total = o;
     return s;
@@ -253,9 +259,10 @@ __device__ __forceinline__ void tmem_st_one(uint32_t taddr, float v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(__float_as_uint(v)) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// L2 prefetch of a box of the expert slab.
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int x, int y, int z) {
-    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(x), "r"(y), "r"(z) : "memory");
+// 4-D TMA tile load (codes, rows, slab, expert), completion on an mbarrier.
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, int w, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar) : "memory");
 }
 
 __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_constant__ MoeBsParams p) {
@@ -281,11 +288,12 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
     const MoeBsWork W = moe_bs_work_layout(p.k);
     uint32_t *misc_s = reinterpret_cast<uint32_t *>(smem + S.misc);
     const uint32_t a0 = smem_u32(smem + S.a), b0 = smem_u32(smem + S.b), sfa0 = smem_u32(smem + S.sfa);
-    // full[s]: a stage's bytes landed; done[s]: its MMAs have completed (stage free); accfull[g] /
-    // accempty[g]: a pass's accumulator is complete (and its scale columns free again) / has been read;
-    // sfafull[g]: the weight scales of a pass are in tensor memory.
+    // full[s]: a stage's bytes landed; done[s]: its MMAs have completed (stage free), except for the last stage
+    // of a pass, where accfull says so too (a second commit right behind the first waits for the first's MMAs);
+    // accfull[pass mod 4] / accempty[g]: a pass's accumulator is complete (and its scale columns free again) /
+    // has been read; sfafull[g]: the weight scales of a pass are in tensor memory.
     const uint32_t full0 = smem_u32(smem + S.bars), done0 = full0 + kMaxStages * 8;
-    const uint32_t accfull0 = done0 + kMaxStages * 8, accempty0 = accfull0 + 16, sfafull0 = accempty0 + 16;
+    const uint32_t accfull0 = done0 + kMaxStages * 8, accempty0 = accfull0 + 32, sfafull0 = accempty0 + 16;
     const uint32_t xready = sfafull0 + 16;  // inline: the routes' activations are in shared memory
 
     if (tid == 0) {
@@ -293,8 +301,8 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
             mbar_init(full0 + s * 8, 1);
             mbar_init(done0 + s * 8, 1);
         }
+        for (int b = 0; b < 4; ++b) mbar_init(accfull0 + b * 8, 1);
         for (int b = 0; b < 2; ++b) {
-            mbar_init(accfull0 + b * 8, 1);
             mbar_init(accempty0 + b * 8, 4);    // one arrival per epilogue warp
             mbar_init(sfafull0 + b * 8, 1);     // the commit that follows the scale warps' copies
         }
@@ -364,74 +372,95 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
         // ------------------------------------------------------------ producer (one thread)
         if (elect_one()) {
             RingPos st;
-            int item = 0;
+            int item = 0, pp = 0, pi = 0;
+            uint32_t done_ph = 0;  // per stage: parity of the next completion of done[s]
             for (int ps = 0; ps < npass; ++ps) {
                 const MoePass P = passes[ps];
-                const uint32_t x_slab = (uint32_t)P.nr * 128u, x_atom = (uint32_t)P.nr * 16u;
-                const uint8_t *xq = A.work + W.xq + (size_t)P.first * p.k + (size_t)k_lo * x_slab;
-                const uint8_t *xsf = A.work + W.xsf + ((size_t)P.first * KS + (size_t)k_lo * P.nr) * 16;
+                const uint32_t x_slab = (uint32_t)P.nr * 144u;
+                const uint8_t *xq = A.work + W.xq + (size_t)P.first * KS * 144 + (size_t)k_lo * x_slab;
                 for (int i = 0; i < IP; ++i, ++item, st.next(NS)) {
                     const int s = st.s, j0 = i * SL, nsl = min(SL, NSLAB - j0);
-                    if (item >= NS && !mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status)) { ps = npass; break; }
+                    if (item >= NS) {  // the stage's previous item, number pi of pass pp, has been read
+                        const bool freed = pi == IP - 1 ? mbar_wait(accfull0 + (pp & 3) * 8, (uint32_t)(pp >> 2) & 1u, X.status)
+                                                        : mbar_wait(done0 + s * 8, done_ph >> s & 1u, X.status);
+                        if (!freed) { ps = npass; break; }
+                        if (pi == IP - 1) { pi = 0; ++pp; }
+                        else { ++pi; done_ph ^= 1u << s; }
+                    }
                     // the unpacking copy counts the packed bytes it read (64 per row), not the 128 it wrote
-                    mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 64u + (p.inline_x ? 0u : x_slab + x_atom)));
-                    for (int j = 0; j < nsl; ++j)
-                        tma_load_3d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (k_lo + j0 + j) * 128, row0, (int)P.expert, full0 + s * 8);
-                    if (p.inline_x) continue;
-                    const uint32_t dst = b0 + s * p.x_pitch;
-                    bulk_load(dst, xq + (size_t)j0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
-                    bulk_load(dst + (uint32_t)SL * x_slab, xsf + (size_t)j0 * x_atom, (uint32_t)nsl * x_atom, full0 + s * 8);
+                    mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 64u + (p.inline_x ? 0u : x_slab)));
+                    const uint32_t dst = a0 + s * SL * p.a_pitch;
+                    if (nsl == SL) {
+                        tma_load_4d(dst, &p.tmap_w[vr], 0, row0, k_lo + j0, (int)P.expert, full0 + s * 8);
+                    } else {
+                        for (int j = 0; j < nsl; ++j) tma_load_4d(dst + j * p.a_pitch, &p.tmap_t[vr], 0, row0, k_lo + j0 + j, (int)P.expert, full0 + s * 8);
+                    }
+                    if (!p.inline_x) bulk_load(b0 + s * p.x_pitch, xq + (size_t)j0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issue (one thread)
         if (elect_one()) {
+            // As in the FP8 kernel, what stands between two stages' MMAs has to stay short.
             const uint32_t id0 = moe_bs_idesc(0), id1 = moe_bs_idesc(1), id2 = moe_bs_idesc(2), id3 = moe_bs_idesc(3);
+            uint32_t *const status = X.status;
+            const bool inl = p.inline_x != 0;
             const uint32_t a_lo0 = umma_desc_lo(a0), b_lo0 = (b0 & 0x3FFFFu) >> 4;
-            const uint32_t a_step = (uint32_t)p.a_pitch >> 4, x_stage = (uint32_t)p.x_pitch >> 4;
+            const uint32_t a_stage = (uint32_t)(SL * p.a_pitch) >> 4, x_stage = (uint32_t)p.x_pitch >> 4;
+            const uint32_t whole_step = (uint32_t)TR * 8u, part_step = (uint32_t)p.a_pitch >> 4;  // slabs of one box follow row by row
             const uint64_t sf_desc0 = umma_desc(b0, 128, false);
-            RingPos st;
-            bool ok = !p.inline_x || mbar_wait(xready, 0, X.status);
+            const uint32_t sf_inl = (uint32_t)(p.nroutes * NSLAB) * 8u;
+            uint32_t full = full0, done = done0, a_lo = a_lo0, x_off = 0, ph = 0;
+            const uint32_t full_end = full0 + NS * 8;
+            bool ok = !inl || mbar_wait(xready, 0, status);
+            MoePass P = npass > 0 ? passes[0] : MoePass{};
             for (int ps = 0; ps < npass && ok; ++ps) {
-                const int g = ps & 1;
-                const uint32_t lap = (uint32_t)(ps >> 1) & 1u;
-                if (!mbar_wait(sfafull0 + g * 8, lap, X.status) || !mbar_wait(accempty0 + g * 8, lap ^ 1u, X.status)) break;
-                tc_fence_after();
-                const uint32_t t_acc = tmem_base + (uint32_t)(g * kMoeBsCols);
-                uint32_t t_sc = t_sc0 + (uint32_t)(g * NSLAB * 8);
-                const MoePass P = passes[ps];
-                const uint32_t nr = P.nr, b_step = 8u * nr, x_kb = 2u * nr;  // 16-byte units, as in the FP8 kernel
-                // inline: the pass's activations and atoms in the resident area
-                const uint32_t x_res = b_lo0 + (uint32_t)P.first * (uint32_t)NSLAB * 8u, sf_res = (uint32_t)(p.nroutes * NSLAB) * 8u + (uint32_t)P.first * (uint32_t)NSLAB;
-                for (int i = 0; i < IP; ++i, st.next(NS)) {
-                    const int s = st.s, nsl = min(SL, NSLAB - i * SL);
-                    if (!mbar_wait(full0 + s * 8, st.ph, X.status)) { ok = false; break; }
+                const uint32_t g = (uint32_t)ps & 1u, lap = (uint32_t)(ps >> 1) & 1u;
+                const uint32_t t_acc = tmem_base + g * kMoeBsCols;
+                uint32_t t_sc = t_sc0 + g * (uint32_t)(NSLAB * 8);
+                const uint32_t nr = P.nr, b_step = 8u * nr, x_kb = 2u * nr;  // 16-byte units
+                // inline: the pass's activations and atoms in the resident area, else a stage's, atoms after activations
+                uint32_t x_in = (uint32_t)P.first * (uint32_t)NSLAB * 8u, sf_in = sf_inl + (uint32_t)P.first * (uint32_t)NSLAB;
+                uint32_t acc = 0;
+                if (!mbar_wait(accempty0 + g * 8, lap ^ 1u, status) || !mbar_wait(sfafull0 + g * 8, lap, status)) break;
+                for (int left = NSLAB; left > 0; left -= SL) {
+                    if (!mbar_wait(full, ph, status)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t a_lo = a_lo0 + (uint32_t)(s * SL) * a_step, b_lo = (p.inline_x ? x_res + (uint32_t)(i * SL) * b_step : b_lo0 + (uint32_t)s * x_stage) | (nr << 16);
-                    const uint64_t sf_desc = sf_desc0 + (uint64_t)(p.inline_x ? sf_res + (uint32_t)(i * SL) * nr
-                                                                             : (uint32_t)s * x_stage + (uint32_t)SL * b_step);  // a stage's atoms follow its activations
-                    // straight-line code per slab count, as in the FP8 kernel
+                    const int nsl = min(left, SL);
+                    const uint32_t a_step = nsl == SL ? whole_step : part_step;
+                    uint32_t a = a_lo, b = (b_lo0 + (inl ? x_in : x_off)) | (nr << 16);
+                    uint64_t sf = sf_desc0 + (uint64_t)(inl ? sf_in : x_off + (uint32_t)nsl * b_step);
+                    // straight-line code, four slabs at a time
                     auto issue = [&](auto count) {
+                        constexpr int C = decltype(count)::value;
 #pragma unroll
-                        for (int j = 0; j < decltype(count)::value; ++j) {
-                            const uint32_t a = a_lo + (uint32_t)j * a_step, b = b_lo + (uint32_t)j * b_step, sx = t_sc + (uint32_t)(j * 8);
-                            tmem_cp_atom(sx, sf_desc + (uint64_t)((uint32_t)j * nr));  // the activations' scales of this slab (the weights' are there already)
-                            umma_bs_ss(t_acc, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id0, sx + 4, sx, j > 0 || i > 0 ? 1u : 0u);
-                            umma_bs_ss(t_acc, a + 2, b + x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id1, sx + 4, sx, 1u);
-                            umma_bs_ss(t_acc, a + 4, b + 2 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id2, sx + 4, sx, 1u);
-                            umma_bs_ss(t_acc, a + 6, b + 3 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id3, sx + 4, sx, 1u);
+                        for (int j = 0; j < C; ++j) {
+                            const uint32_t aj = a + (uint32_t)j * a_step, bj = b + (uint32_t)j * b_step, sx = t_sc + (uint32_t)(j * 8);
+                            tmem_cp_atom(sx, sf + (uint64_t)((uint32_t)j * nr));  // the activations' scales of this slab (the weights' are there already)
+                            umma_bs_ss(t_acc, aj, bj, kUmmaDescHiSw128, kUmmaDescHiX, id0, sx + 4, sx, j > 0 ? 1u : acc);
+                            umma_bs_ss(t_acc, aj + 2, bj + x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id1, sx + 4, sx, 1u);
+                            umma_bs_ss(t_acc, aj + 4, bj + 2 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id2, sx + 4, sx, 1u);
+                            umma_bs_ss(t_acc, aj + 6, bj + 3 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id3, sx + 4, sx, 1u);
                         }
+                        acc = 1;
+                        a += (uint32_t)C * a_step; b += (uint32_t)C * b_step; sf += (uint64_t)((uint32_t)C * nr); t_sc += C * 8;
                     };
-                    if (nsl == 4) issue(std::integral_constant<int, 4>{});
-                    else if (nsl == 3) issue(std::integral_constant<int, 3>{});
-                    else if (nsl == 2) issue(std::integral_constant<int, 2>{});
-                    else issue(std::integral_constant<int, 1>{});
-                    t_sc += (uint32_t)(nsl * 8);
-                    umma_commit(done0 + s * 8);  // the stage may be refilled
+                    int n4 = nsl;
+                    for (; n4 >= 4; n4 -= 4) issue(std::integral_constant<int, 4>{});
+                    if (n4 == 3) issue(std::integral_constant<int, 3>{});
+                    else if (n4 == 2) issue(std::integral_constant<int, 2>{});
+                    else if (n4 == 1) issue(std::integral_constant<int, 1>{});
+                    // the stage may be refilled (and, at the end of the pass, its sums are complete and its scale columns free)
+                    umma_commit(left <= SL ? accfull0 + ((uint32_t)ps & 3u) * 8u : done);
+                    x_in += (uint32_t)SL * b_step; sf_in += (uint32_t)SL * nr;
+                    full += 8; done += 8; a_lo += a_stage; x_off += x_stage;
+                    if (full == full_end) {
+                        full = full0; done = done0; a_lo = a_lo0; x_off = 0;
+                        ph ^= 1u;
+                    }
                 }
-                if (!ok) break;
-                umma_commit(accfull0 + g * 8);   // the pass's sums are complete; its scale columns may be rewritten
+                if (ps + 1 < npass) P = passes[ps + 1];
             }
         }
         __syncwarp();
@@ -462,17 +491,12 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
             const uint32_t lap = (uint32_t)(ps >> 1) & 1u;
             // the pass that used these columns and this buffer last (ps - 2) has completed; a wait that
             // gave up is told to all four warps at the barrier below, so that they leave the loop together
-            if (ps >= 2 && !mbar_wait(accfull0 + g * 8, lap ^ 1u, X.status)) misc_s[8] = 1u;
+            if (ps >= 2 && !mbar_wait(accfull0 + ((ps - 2) & 3) * 8, (uint32_t)((ps - 2) >> 2) & 1u, X.status)) misc_s[8] = 1u;
             uint8_t *dst = smem + S.sfa + (size_t)(g * NSLAB) * kBsAtomBytes + (r & 31) * 16 + (r >> 5) * 4;
 #pragma unroll
             for (int j = 0; j < kMoeBsMaxSlabs; ++j)
                 if (j < NSLAB) *reinterpret_cast<uint32_t *>(dst + (size_t)j * kBsAtomBytes) = sc[j];
             if (ps + 1 < npass) fetch(ps + 1);
-            if (p.prefetch && warp == 9 && ps + p.prefetch < npass && elect_one()) {
-                const int e = passes[ps + p.prefetch].expert;
-                for (int j = 0; j < NSLAB; ++j) tma_prefetch_3d(&p.tmap_w[vr], (k_lo + j) * 128, row0, e);
-            }
-            __syncwarp();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("bar.sync 3, 128;" ::: "memory");
             if (*reinterpret_cast<volatile uint32_t *>(misc_s + 8) != 0u) break;
@@ -501,7 +525,7 @@ __global__ void __launch_bounds__(kMoeBsThreads, 1) moe_bs_kernel(const __grid_c
             const int g = ps & 1;
             const uint32_t lap = (uint32_t)(ps >> 1) & 1u;
             const MoePass P = passes[ps];
-            if (ok && !mbar_wait(accfull0 + g * 8, lap, X.status)) ok = false;
+            if (ok && !mbar_wait(accfull0 + (ps & 3) * 8, (uint32_t)(ps >> 2) & 1u, X.status)) ok = false;
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
