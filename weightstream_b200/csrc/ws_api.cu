@@ -505,7 +505,7 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         u.smem = (size_t)total(ns);
         int cols = 32;
         // (fp32 scales: the epilogue reads the accumulators of a group in batches, see fp8_bs_kernel)
-        const int batch = std::max(1, 64 / (u.mp * 4 / bs_epi_warps(u.mp))), read = (u.slabs_per_stage + batch - 1) / batch * batch;
+        const int batch = bs_read_batch(u.mp), read = (u.slabs_per_stage + batch - 1) / batch * batch;
         while (cols < (u.wue ? u.nacc * u.mp + 2 * u.slabs_per_stage * 8
                              : std::max(u.nacc * u.slabs_per_stage * (u.mp + 4) + 4, ((u.nacc - 1) * u.slabs_per_stage + read) * u.mp))) cols *= 2;
         u.tmem_cols = half ? std::min(cols, 256) : 512;

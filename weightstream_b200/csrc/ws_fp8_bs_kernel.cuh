@@ -52,14 +52,18 @@ namespace ws {
 // Threads of a CTA.  Warp 0: producer, warp 1: MMA issue (and owner of the tensor memory), then the
 // epilogue warps: four (one per 32-lane quarter of the tensor memory, all token columns) for up to 16
 // tokens, eight (two per quarter, half of the token columns each) beyond, where reading the
-// accumulators back is what a stage waits for; then, for UE8M0 weight scales, four auxiliary warps.
-__host__ __device__ constexpr int bs_epi_warps(int mp) { return mp >= 32 ? 8 : 4; }
+// accumulators back is what a stage waits for (sixteen for 128 tokens: 38 against 31 us; UE8M0
+// sums are read once per tile: eight from 64 tokens); then, for UE8M0
+// weight scales, four auxiliary warps.
+__host__ __device__ constexpr int bs_epi_warps(int mp, bool wue) { return mp >= (wue ? 64 : 32) ? 8 : 4; }
 constexpr int kBsAuxWarps = 4;
-__host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 * (bs_epi_warps(mp) + (wue ? kBsAuxWarps : 0)); }
+__host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 * (bs_epi_warps(mp, wue) + (wue ? kBsAuxWarps : 0)); }
 // Registers per thread: what leaves a warp of the prep kernel room in every quarter of the SM's register file
 // (a CTA of ten warps has three in two of them; the next step's CTA otherwise waits for the prep block to
 // leave), and, up to 16 tokens, a second CTA.
-__host__ __device__ constexpr int bs_regs(int mp, bool wue) { return mp == 16 ? (wue ? 88 : 144) : wue ? 112 : 152; }
+__host__ __device__ constexpr int bs_regs(int mp, bool wue) { return mp == 16 ? (wue ? 120 : 144) : wue && mp > 32 ? 128 : 152; }
+// Slabs whose accumulators an epilogue thread reads at once (fp32 weight scales): 64 registers' worth.
+__host__ __device__ constexpr int bs_read_batch(int mp) { return 64 / (mp * 4 / bs_epi_warps(mp, false)); }
 constexpr int kBsMaxAcc = 8;         // accumulator groups in tensor memory (a group = one stage's slabs)
 constexpr int kBsMaxTokens = 128;    // activation rows one launch takes (16, 32, 64 or 128 MMA columns)
 constexpr int kBsAtomBytes = 512;    // one scale atom: 128 rows x 4 K blocks
@@ -163,7 +167,7 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
     o += nstages * x_pitch + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - nstages * x_pitch : 2048;
     s.wsf = o;  o += wue ? nsl * kBsAtomBytes : kBsAtomBytes;  // the weights' scale atoms (fp32 scales: one atom of 2^0)
     s.sw = o;   o += wue ? 0 : (int)align_up((int64_t)nslot_max * skb * 4, 16);
-    s.cand = o; o += bs_epi_warps(mp) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
+    s.cand = o; o += bs_epi_warps(mp, wue) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
     s.rx = o;   o += rx_rows * kBsMmaRows * 4;           // CTA pairs: the partner's sums of one tile for this CTA's tokens, [token][row]
     s.bars = o; o += (2 * kMaxStages + 2 * kBsMaxAcc + 2) * 8;
     s.misc = o; o += 64;
@@ -257,11 +261,11 @@ __device__ __forceinline__ void tmem_ld_cols<64>(uint32_t taddr, uint32_t (&r)[6
         "tcgen05.wait::ld.sync.aligned;"
         : WS_R16(r, 0), WS_R16(r, 16), WS_R16(r, 32), WS_R16(r, 48) : "r"(taddr) : "memory");
 }
-// The same columns of up to 64 / N consecutive accumulators, `pitch` columns apart, under one wait.
-template <int N>
-__device__ __forceinline__ void tmem_ld_batch(uint32_t taddr, uint32_t pitch, uint32_t (&r)[64]);
+// The same N columns of B consecutive accumulators, `pitch` columns apart, under one wait.
+template <int N, int B>
+__device__ __forceinline__ void tmem_ld_batch(uint32_t taddr, uint32_t pitch, uint32_t (&r)[N * B]);
 template <>
-__device__ __forceinline__ void tmem_ld_batch<16>(uint32_t t, uint32_t pitch, uint32_t (&r)[64]) {
+__device__ __forceinline__ void tmem_ld_batch<16, 4>(uint32_t t, uint32_t pitch, uint32_t (&r)[64]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%64];\n\t"
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%65];\n\t"
@@ -271,7 +275,7 @@ __device__ __forceinline__ void tmem_ld_batch<16>(uint32_t t, uint32_t pitch, ui
         : WS_R16(r, 0), WS_R16(r, 16), WS_R16(r, 32), WS_R16(r, 48) : "r"(t), "r"(t + pitch), "r"(t + 2 * pitch), "r"(t + 3 * pitch) : "memory");
 }
 template <>
-__device__ __forceinline__ void tmem_ld_batch<32>(uint32_t t, uint32_t pitch, uint32_t (&r)[64]) {
+__device__ __forceinline__ void tmem_ld_batch<32, 2>(uint32_t t, uint32_t pitch, uint32_t (&r)[64]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
         "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%64];\n\t"
@@ -281,7 +285,7 @@ __device__ __forceinline__ void tmem_ld_batch<32>(uint32_t t, uint32_t pitch, ui
         : WS_R16(r, 0), WS_R16(r, 16), WS_R16(r, 32), WS_R16(r, 48) : "r"(t), "r"(t + pitch) : "memory");
 }
 template <>
-__device__ __forceinline__ void tmem_ld_batch<64>(uint32_t t, uint32_t, uint32_t (&r)[64]) { tmem_ld_cols<64>(t, r); }
+__device__ __forceinline__ void tmem_ld_batch<64, 1>(uint32_t t, uint32_t, uint32_t (&r)[64]) { tmem_ld_cols<64>(t, r); }
 #undef WS_R16
 #undef WS_R4
 
@@ -361,7 +365,7 @@ __device__ __forceinline__ uint32_t order_key(float v) {
 
 template <int MP, bool WUE>
 __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, WUE)) fp8_bs_kernel(const __grid_constant__ BsParams p) {
-    constexpr int EW = bs_epi_warps(MP), ET = EW * 32;  // epilogue warps / threads
+    constexpr int EW = bs_epi_warps(MP, WUE), ET = EW * 32;  // epilogue warps / threads
     constexpr int CP = MP * 4 / EW;                      // token columns one epilogue thread holds
     auto bs_epi_bar = [] { bs_epi_bar_n<ET>(); };
     extern __shared__ uint8_t smem_raw[];
@@ -396,18 +400,33 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
     const uint32_t accempty0 = done0 + kMaxStages * 8, accfull0 = accempty0 + kBsMaxAcc * 8;
     const uint32_t rxfull = accfull0 + kBsMaxAcc * 8, rxempty = rxfull + 8;  // CTA pairs: the partner's sums of a tile have arrived / been read
 
-    if (tid == 0) {
-        for (int s = 0; s < NS; ++s) {
-            mbar_init(full0 + s * 8, WUE ? 1 + kBsAuxWarps : 1);
-            mbar_init(done0 + s * 8, 1);
+    // Weights are static: the first ring's worth is on its way before the CTA has set itself up (barriers,
+    // tensor memory and the pair's meeting take ~1.3 us, in which HBM would idle), let alone before the wait on
+    // the prep kernel.
+    const uint32_t x_slab = (uint32_t)(p.m * 128 + bs_atom_bytes(p.m));
+    auto issue_w = [&](int s, int tile, int s0, int nsl) {
+        mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + x_slab));
+        for (int j = 0; j < nsl; ++j)
+            tma_load_2d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (s0 + j) * 128, tile * TR, full0 + s * 8);
+    };
+    if (warp == 0) {
+        if (elect_one()) {
+            for (int s = 0; s < NS; ++s) {
+                mbar_init(full0 + s * 8, WUE ? 1 + kBsAuxWarps : 1);
+                mbar_init(done0 + s * 8, 1);
+            }
+            for (int b = 0; b < kBsMaxAcc; ++b) {
+                mbar_init(accempty0 + b * 8, EW);  // one arrival per epilogue warp
+                mbar_init(accfull0 + b * 8, 1);
+            }
+            mbar_init(rxfull, EW);   // every epilogue warp of the partner arrives after its stores
+            mbar_init(rxempty, EW);
+            mbar_fence_init();
+            int tile, s0, nsl;
+            BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
+            for (int item = 0; item < NS && w.next(tile, s0, nsl); ++item) issue_w(item, tile, s0, nsl);
         }
-        for (int b = 0; b < kBsMaxAcc; ++b) {
-            mbar_init(accempty0 + b * 8, EW);  // one arrival per epilogue warp
-            mbar_init(accfull0 + b * 8, 1);
-        }
-        mbar_init(rxfull, ET);   // every epilogue thread of the partner arrives after its stores
-        mbar_init(rxempty, ET);
-        mbar_fence_init();
+        __syncwarp();
     }
     if (warp == 1) {  // tensor memory: allocated and freed by the same warp
         tmem_alloc(smem_u32(misc_s), (uint32_t)p.tmem_cols);
@@ -435,19 +454,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
     if (warp == 0) {
         // ------------------------------------------------------------ producer (one thread)
         if (elect_one()) {
-            // Weights are static: the first ring's worth streams before the wait on the prep kernel;
-            // the activations follow once it has finished.
-            const uint32_t x_slab = (uint32_t)(p.m * 128 + bs_atom_bytes(p.m));
-            auto issue_w = [&](int s, int tile, int s0, int nsl) {
-                mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + x_slab));
-                for (int j = 0; j < nsl; ++j)
-                    tma_load_2d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (s0 + j) * 128, tile * TR, full0 + s * 8);
-            };
             int tile, s0, nsl;
-            {   // first lap of the ring: weights at once
-                BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
-                for (int item = 0; item < NS && w.next(tile, s0, nsl); ++item) issue_w(item, tile, s0, nsl);
-            }
             asm volatile("griddepcontrol.wait;" ::: "memory");
             BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
             RingPos st;
@@ -626,34 +633,43 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
 
         // A finished tile: its rows go to the output or to the peers; of an lm_head tile the candidates are
         // kept and, when the caller wants them, the logits stored.
-        auto finalize = [&](const float (&v)[CP], int tile) {  // v[i]: token col0 + i
+        auto finalize = [&](const float (&v)[CP], int tile, const int tok_lo, const int tok_hi) {  // v[i]: token col0 + i
             const int row = tile * TR + rc;
             const bool mine = rc < TR && row < p.n;
             // element (token, row) of a float matrix with `ld` floats per token
-            auto store = [&](float *base, size_t ld) {
-                float *dst = base + (size_t)col0 * ld + row;
+            // (its stride is hidden from the optimiser, which would keep every column's offset in registers through
+            // the main loop: 60 more of them, and spills in the other roles' loops)
+            auto store = [&](float *base, int64_t ld) {
+                asm volatile("" : "+l"(ld));
+                float *dst = base + col0 * ld + row;
 #pragma unroll
-                for (int i = 0; i < CP; ++i)
-                    if (col0 + i >= tok_lo && col0 + i < tok_hi) dst[(size_t)i * ld] = v[i];
+                for (int i = 0; i < CP; ++i) {
+                    if (col0 + i >= tok_lo && col0 + i < tok_hi) *dst = v[i];
+                    dst += ld;
+                }
             };
             if (mine) {
                 if (solo) {
-                    store(A.out, (size_t)p.n);
+                    store(A.out, p.n);
                 } else if (p.mode == kModeAllReduce) {
                     // every rank gets the partial sums, or (many rows, many ranks) only the tile's owner
                     const int pr0 = p.owner_reduce ? tile % p.world : 0, pr1 = p.owner_reduce ? pr0 + 1 : p.world;
                     for (int pr = pr0; pr < pr1; ++pr) {
-                        uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride;
+                        int64_t ld = p.n;
+                        asm volatile("" : "+l"(ld));
+                        uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride + col0 * ld + row;
 #pragma unroll
-                        for (int i = 0; i < CP; ++i)
-                            if (col0 + i >= tok_lo && col0 + i < tok_hi) st_word_sys(dst + (size_t)(col0 + i) * p.n + row, seq, v[i]);
+                        for (int i = 0; i < CP; ++i) {
+                            if (col0 + i >= tok_lo && col0 + i < tok_hi) st_word_sys(dst, seq, v[i]);
+                            dst += ld;
+                        }
                     }
                 } else if (p.gather_logits && p.world == 1) {  // a lone rank's logits are final where they are
-                    store(A.logits + A.vocab_row0, (size_t)p.vocab);
+                    store(A.logits + A.vocab_row0, p.vocab);
                 } else if (p.gather_logits) {
                     for (int pr = 0; pr < p.world; ++pr)
                         store(reinterpret_cast<float *>(X.sym[pr] + p.lay.gather_off) + (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab +
-                                  A.vocab_row0, (size_t)p.lay.max_vocab);
+                                  A.vocab_row0, p.lay.max_vocab);
                 }
             }
             if (p.mode == kModeLmHead) {
@@ -676,84 +692,92 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             }
         };
 
-        BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
-        RingPos st, ag;  // stage ring, accumulator ring
         bool ok = true;
-        int tile, s0, nsl, ntile_done = 0;
+        int ntile_done = 0;
         float acc[CP];
-        const float *swrow = sw_s;
-        while (w.next(tile, s0, nsl)) {
-            const bool last = s0 + nsl == k_hi;  // this CTA's slabs of the tile end with this item
-            const int g = ag.s;
+        // positions in the stage and accumulator rings, advanced incrementally
+        uint32_t done = done0, ph = 0, accempty = accempty0, acc_ph = 0, t_col = tlane + (uint32_t)col0;
+        const uint32_t done_end = done0 + NS * 8, acc_end = accempty0 + NB * 8;
+        const int kcta = k_hi - k_lo;
+        for (int tile = t_lo; tile <= t_hi && kcta > 0; ++tile) {
             if constexpr (WUE) {
-                if (!last) continue;
-                if (ok && !mbar_wait(accfull0 + g * 8, ag.ph, X.status)) ok = false;
+                if (ok && !mbar_wait(accempty + (accfull0 - accempty0), acc_ph, X.status)) ok = false;
                 ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads below need the whole warp
                 tc_fence_after();
                 uint32_t r[CP];
 #pragma unroll
                 for (int i = 0; i < CP; ++i) r[i] = 0u;
-                if (ok) tmem_ld_cols<CP>(tlane + (uint32_t)(g * MP + col0), r);
+                if (ok) tmem_ld_cols<CP>(t_col, r);
 #pragma unroll
                 for (int i = 0; i < CP; ++i) acc[i] = __uint_as_float(r[i]);
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(accempty0 + g * 8);
-                ag.next(NB);
+                if (lane == 0) mbar_arrive(accempty);
+                accempty += 8; t_col += MP;
+                if (accempty == acc_end) { accempty = accempty0; t_col = tlane + (uint32_t)col0; acc_ph ^= 1u; }
             } else {
-                if (s0 == k_lo) {  // a new tile
 #pragma unroll
-                    for (int i = 0; i < CP; ++i) acc[i] = 0.0f;
-                    const int row = min(tile * TR + min(rc, TR - 1), p.n - 1);
-                    swrow = sw_s + (int)(((A.row0 + row) >> p.bn_shift) - srow_lo) * p.skb;
-                }
-                if (ok && !mbar_wait(done0 + st.s * 8, st.ph, X.status)) ok = false;
-                ok = __all_sync(0xffffffffu, ok);
-                tc_fence_after();
-                if (ok) {
-                    // as many slabs per round trip to tensor memory as 64 registers hold (a last round may read
-                    // accumulators of other stages, inside the allocation, and leaves them unused)
-                    constexpr int B = 64 / CP;
-                    for (int j0 = 0; j0 < nsl; j0 += B) {
-                        uint32_t r[64];
-                        tmem_ld_batch<CP>(tlane + (uint32_t)((g * SL + j0) * MP + col0), (uint32_t)MP, r);
+                for (int i = 0; i < CP; ++i) acc[i] = 0.0f;
+                const int row = min(tile * TR + min(rc, TR - 1), p.n - 1);
+                const float *swrow = sw_s + (int)(((A.row0 + row) >> p.bn_shift) - srow_lo) * p.skb;
+                int kk = kofs + k_lo * 128;  // K offset of the stage's first slab inside the scale matrix
+                for (int left = kcta; left > 0; left -= SL) {
+                    const int nsl = min(left, SL);
+                    if (ok && !mbar_wait(done, ph, X.status)) ok = false;
+                    ok = __all_sync(0xffffffffu, ok);
+                    tc_fence_after();
+                    if (ok) {
+                        // as many slabs per round trip to tensor memory as the registers hold (a last round may read
+                        // accumulators of other stages, inside the allocation, and leaves them unused)
+                        constexpr int B = bs_read_batch(MP);
+                        for (int j0 = 0; j0 < nsl; j0 += B) {
+                            uint32_t r[B * CP];
+                            tmem_ld_batch<CP, B>(t_col + (uint32_t)(j0 * MP), (uint32_t)MP, r);
 #pragma unroll
-                        for (int j = 0; j < B; ++j)
-                            if (j0 + j < nsl) {
-                                const float sw = swrow[(kofs + (s0 + j0 + j) * 128) >> p.bk_shift];
+                            for (int j = 0; j < B; ++j)
+                                if (j == 0 || j0 + j < nsl) {
+                                    const float sw = swrow[(kk + (j0 + j) * 128) >> p.bk_shift];
 #pragma unroll
-                                for (int i = 0; i < CP; ++i) acc[i] = fmaf(__uint_as_float(r[j * CP + i]), sw, acc[i]);
-                            }
+                                    for (int i = 0; i < CP; ++i) acc[i] = fmaf(__uint_as_float(r[j * CP + i]), sw, acc[i]);
+                                }
+                        }
                     }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(accempty);
+                    kk += SL * 128;
+                    done += 8;
+                    if (done == done_end) { done = done0; ph ^= 1u; }
+                    accempty += 8; t_col += (uint32_t)(SL * MP);
+                    if (accempty == acc_end) { accempty = accempty0; t_col = tlane + (uint32_t)col0; }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(accempty0 + g * 8);
-                st.next(NS);
-                ag.next(NB);
-                if (!last) continue;
             }
+            // what depends on the tile's end only is not worth registers in the main loop: hidden from the optimiser
+            int lo = tok_lo, hi = tok_hi, m = p.m;
+            asm volatile("" : "+r"(lo), "+r"(hi), "+r"(m));
             if (p.csize == 2) {
                 // a pair swaps its sums: each CTA gets the partner's for the tokens it finishes, in its shared memory
                 if (ntile_done > 0) mbar_wait_cluster(rxempty, (uint32_t)(ntile_done - 1) & 1u, X.status);  // the partner has read the previous tile's
                 const uint32_t dst = mapa_u32(smem_u32(smem + S.rx) + (uint32_t)rc * 4u, crank ^ 1u);
-                const int base = crank == 0 ? split : 0;  // the partner's first token
+                const int base = crank == 0 ? hi : 0;  // the partner's first token
 #pragma unroll
                 for (int i = 0; i < CP; ++i) {
                     const int t = col0 + i;
-                    if (t < p.m && (t < tok_lo || t >= tok_hi)) st_cluster_f32(dst + (uint32_t)((t - base) * kBsMmaRows * 4), acc[i]);
+                    if (t < m && (t < lo || t >= hi)) st_cluster_f32(dst + (uint32_t)((t - base) * kBsMmaRows * 4), acc[i]);
                 }
-                mbar_arrive_cluster(mapa_u32(rxfull, crank ^ 1u));
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(mapa_u32(rxfull, crank ^ 1u));
                 mbar_wait_cluster(rxfull, (uint32_t)ntile_done & 1u, X.status);
                 const float *rx = reinterpret_cast<const float *>(smem + S.rx) + rc;
 #pragma unroll
                 for (int i = 0; i < CP; ++i) {  // K half 0 + K half 1, in that order (the sum of two does not depend on it)
                     const int t = col0 + i;
-                    if (t >= tok_lo && t < tok_hi) acc[i] += rx[(t - tok_lo) * kBsMmaRows];
+                    if (t >= lo && t < hi) acc[i] += rx[(t - lo) * kBsMmaRows];
                 }
-                if (tile < t_hi) mbar_arrive_cluster(mapa_u32(rxempty, crank ^ 1u));  // nobody waits for the last one
+                __syncwarp();
+                if (lane == 0 && tile < t_hi) mbar_arrive_cluster(mapa_u32(rxempty, crank ^ 1u));  // nobody waits for the last one
             }
-            finalize(acc, tile);
+            finalize(acc, tile, lo, hi);
             ++ntile_done;
         }
 
