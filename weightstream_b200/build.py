@@ -12,7 +12,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libws_tp.so")
 TORCH_EXT = os.path.join(HERE, "_ws_torch.so")
 SOURCES = ["ws_api.cu", "ws_bootstrap.cu"]
-HEADERS = ["ws_device.cuh", "ws_fp8_kernel.cuh", "ws_fp8_gemv_kernel.cuh", "ws_fp8_bs_kernel.cuh", "ws_moe_kernel.cuh", "ws_moe_gemv_kernel.cuh", "ws_moe_bs_kernel.cuh", "ws_misc_kernels.cuh",
+HEADERS = ["ws_device.cuh", "ws_fp8_kernel.cuh", "ws_fp8_gemv_kernel.cuh", "ws_fp8_bs_kernel.cuh", "ws_fp8_tile_kernel.cuh", "ws_moe_kernel.cuh", "ws_moe_gemv_kernel.cuh", "ws_moe_bs_kernel.cuh", "ws_misc_kernels.cuh",
            os.path.join("..", "..", "include", "ws_tp.h")]
 
 

@@ -17,6 +17,7 @@
 #include "ws_fp8_kernel.cuh"
 #include "ws_fp8_gemv_kernel.cuh"
 #include "ws_fp8_bs_kernel.cuh"
+#include "ws_fp8_tile_kernel.cuh"
 #include "ws_misc_kernels.cuh"
 #include "ws_moe_kernel.cuh"
 #include "ws_moe_gemv_kernel.cuh"
@@ -302,7 +303,8 @@ ws_status_t ws_tp_create(int32_t world, int32_t rank, int32_t device, const ws_t
         set_smem(tp, fp8_gemv_kernel<2, 1>) != WS_OK || set_smem(tp, fp8_gemv_kernel<2, 2>) != WS_OK ||
         set_smem(tp, fp8_gemv_kernel<2, 4>) != WS_OK || set_smem(tp, moe_down_kernel) != WS_OK ||
         set_smem(tp, fp8_bs_kernel<16, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<64, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, false>) != WS_OK ||
-        set_smem(tp, fp8_bs_kernel<16, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<64, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, true>) != WS_OK || set_smem(tp, moe_bs_kernel) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<16, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<64, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, true>) != WS_OK || set_smem(tp, fp8_tile_kernel<false>) != WS_OK || set_smem(tp, fp8_tile_kernel<true>) != WS_OK ||
+        set_smem(tp, moe_bs_kernel) != WS_OK ||
         cudaFuncSetAttribute(moe_bs_prep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         // The prep kernel uses no shared memory, but a main-kernel CTA (which needs almost all of an SM's)
         // cannot move onto an SM whose L1/shared split must first change, and that has to wait for the prep
@@ -561,7 +563,7 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
     ActPrepParams q{};
-    q.m = mt; q.k = a0.k; q.x_dtype = a0.x_dtype; q.ks = u.ks; q.csize = u.csize; q.sl = u.slabs_per_stage;
+    q.m = mt; q.k = a0.k; q.x_dtype = a0.x_dtype; q.ks = u.ks; q.csize = u.csize; q.sl = u.slabs_per_stage; q.tokens = mt;
     // scratch of one endpoint: the quantised activations and their scale atoms
     const size_t xq_bytes = (size_t)u.ks * (kBsMaxTokens * 128 + kBsAtomBytes);
 
@@ -606,6 +608,58 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         if (s == WS_OK) s = launch(ranks[i], kernel, p, u.ncta, nvr, bs_threads(u.mp, u.wue), u.smem, cs, t0->pdl != 0, true, u.csize);
         if (s != WS_OK) t0->err = ranks[i]->err;
     }
+    return s;
+}
+
+// Plan of the tile kernel: one launch over all activation rows of a lone rank's step.
+struct TilePlan {
+    bool ok, wue;
+    int ks, tokens, ntok, nrow, nstages, x_pitch;
+    size_t smem;
+};
+static TilePlan tile_plan(const ws_fp8_gemm_args_t &a, int ncta) {
+    TilePlan u{};
+    u.wue = a.scale_kind == WS_SCALE_UE8M0;
+    if (!u.wue && (a.block_k % 128 || a.k % 128 || a.k0 % 128)) return u;
+    u.ks = (a.k + 127) / 128;
+    u.nrow = (a.n + 127) / 128;
+    // Tokens per tile: the fewest waves of CTAs, each as long as a slab's bytes (128 rows, N tokens) take to come
+    // out of L2.
+    int64_t best = -1;
+    for (int n = 64; n <= kTileTokens; n += 16) {
+        const int nt = (a.m + n - 1) / n;
+        const int64_t waves = ((int64_t)u.nrow * nt + ncta - 1) / ncta, cost = waves * (n + 128);
+        if (best < 0 || cost < best) { best = cost; u.tokens = n; u.ntok = nt; }
+    }
+    u.x_pitch = (int)align_up((int64_t)u.tokens * 128 + bs_atom_bytes(u.tokens), 128);
+    u.nstages = kTileMaxStages;
+    while (u.nstages > 2 && tile_smem_layout(u.nstages, u.x_pitch, u.wue).total + 1024 > kSmemBudget) --u.nstages;
+    u.ok = u.nstages >= 3;
+    u.smem = (size_t)tile_smem_layout(u.nstages, u.x_pitch, u.wue).total + 1024;
+    return u;
+}
+
+static ws_status_t tile_step(ws_tp *tp, const ws_fp8_gemm_args_t &a, cudaStream_t cs, int ncta, const TilePlan &u) {
+    TileParams p{};
+    p.m = a.m; p.n = a.n; p.k = a.k; p.ks = u.ks; p.tokens = u.tokens; p.ntok = u.ntok; p.nrow = u.nrow; p.nstages = u.nstages; p.x_pitch = u.x_pitch;
+    for (p.bk_shift = 0; (1 << p.bk_shift) < a.block_k; ++p.bk_shift) {}
+    for (p.bn_shift = 0; (1 << p.bn_shift) < a.block_n; ++p.bn_shift) {}
+    p.scales = a.scales; p.scale_ld = a.scale_ld; p.row0 = a.row0; p.k0 = a.k0; p.out = a.out;
+    ws_status_t s = ensure_bs_scratch(tp, (size_t)u.ntok * u.ks * (u.tokens * 128 + bs_atom_bytes(u.tokens)));
+    if (s == WS_OK) s = make_tmap(tp, &p.tmap_w, a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, 128);
+    if (s != WS_OK) return s;
+    p.xq = tp->bs_work;
+    p.ctx = make_ctx(tp);
+    p.ctx.host_done = tp->host_done_arm;
+    ActPrepParams q{};
+    q.m = a.m; q.k = a.k; q.x_dtype = a.x_dtype; q.ks = u.ks; q.csize = 1; q.sl = 1; q.tokens = u.tokens;
+    q.r[0].x = a.x; q.r[0].xq = tp->bs_work; q.r[0].ldx = a.ldx;
+    tp->step++;
+    const int prep_blocks = (int)std::min<int64_t>(4 * tp->sm_count, ((int64_t)a.m * u.ks * 8 + kActPrepThreads - 1) / kActPrepThreads);
+    WS_CUDA(tp, cudaSetDevice(tp->device));
+    s = launch(tp, act_prep_kernel, q, prep_blocks, 1, kActPrepThreads, 0, cs, tp->pdl != 0, false);
+    const int grid = std::min(ncta, u.nrow * u.ntok);
+    if (s == WS_OK) s = launch(tp, u.wue ? fp8_tile_kernel<true> : fp8_tile_kernel<false>, p, grid, 1, kTileThreads, u.smem, cs, tp->pdl != 0);
     return s;
 }
 
@@ -857,6 +911,10 @@ ws_status_t ws_fp8_rowpar_gemm_allreduce_group(ws_tp_t *const *ranks, int32_t n,
     if (args[0].m > t0->cfg.max_m || args[0].n > t0->cfg.max_n)
         return fail(t0, WS_ERR_CAPACITY, "m=%d n=%d exceed the endpoint's max_m=%d max_n=%d", args[0].m, args[0].n,
                     t0->cfg.max_m, t0->cfg.max_n);
+    if (n == 1 && t0->world == 1 && args[0].m > kBsMaxTokens && bs_wanted(t0, kBsMaxTokens, args[0])) {  // prefill on a lone rank
+        const TilePlan u = tile_plan(args[0], ncta);
+        if (u.ok) return tile_step(t0, args[0], static_cast<cudaStream_t>(streams ? streams[0] : nullptr), ncta, u);
+    }
     for (int m0 = 0; m0 < args[0].m;) {
         const int mt = fp8_rows_per_launch(t0, args[0], ncta, args[0].m - m0);
         s = fp8_step(ranks, n, args, nullptr, m0, mt, streams, ncta, same, m0 + mt >= args[0].m);

@@ -108,7 +108,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // caller unwind instead of spinning forever.  Once any wait of the launch has failed (the status
 // word is set) every later wait that is not satisfied at once returns false immediately, so a
 // kernel with hundreds of stage waits ends in one time-out, not hundreds.
-static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint32_t *status) {
+__device__ __forceinline__ bool mbar_wait_inline(uint32_t bar, uint32_t parity, uint32_t *status) {
     for (int i = 0; i < 64; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     if (*(volatile uint32_t *)status != 0u) return false;
@@ -122,6 +122,8 @@ static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity
     atomicCAS(status, 0u, kStatTimeoutTma | (uint32_t)(-WS_ERR_TIMEOUT));
     return false;
 }
+// Out of line: inlined into every role's loops it cost them 10 % (MoE step of 64 tokens 364 against 331 us).
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint32_t *status) { return mbar_wait_inline(bar, parity, status); }
 // Most waits of the issuing threads find their phase complete: that costs one probe and a branch.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *status) {
     return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, status);

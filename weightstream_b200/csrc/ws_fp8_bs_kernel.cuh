@@ -70,8 +70,8 @@ constexpr int kBsAtomBytes = 512;    // one scale atom: 128 rows x 4 K blocks
 constexpr int kBsMmaRows = 128;      // M of the MMA; a tile of output rows holds at most as many
 
 // Rows of a scale atom that exist in memory: the copy into tensor memory takes 32, those past the tokens'
-// come from whatever follows and scale columns that are never read.
-__host__ __device__ constexpr int bs_atom_bytes(int m) { return 16 * (m < 32 ? m : 32); }
+// come from whatever follows and scale columns that are never read.  More than 128 tokens have two atoms.
+__host__ __device__ constexpr int bs_atom_bytes(int m) { return m < 32 ? 16 * m : m <= 128 ? kBsAtomBytes : 2 * kBsAtomBytes; }
 
 // The activation image of a step: the K slabs in the groups that the CTAs' stages take (half h of K owns slabs
 // [h * ks / csize, (h + 1) * ks / csize), cut into groups of at most sl), a group being its chunks, then its atoms.
@@ -90,6 +90,7 @@ struct ActPrepRank {
 };
 struct ActPrepParams {
     int32_t m, k, x_dtype, ks, csize, sl;
+    int32_t tokens, pad0;  // tokens per image: m, or (tile kernel) those of a tile, the tiles' images one after another
     ActPrepRank r[WS_MAX_WORLD];
 };
 
@@ -122,14 +123,15 @@ __global__ void __launch_bounds__(kActPrepThreads, 12) act_prep_kernel(const __g
             int e;
             const uint4 q = act_quant16(v[u], e);
             if (c0 + u * step < total) {
-                const int slab = ch[u] >> 3, t = tok[u], atom = bs_atom_bytes(p.m);
+                const int tile = tok[u] < p.tokens ? 0 : tok[u] / p.tokens, t = tok[u] - tile * p.tokens;
+                const int m = min(p.tokens, p.m - tile * p.tokens), slab = ch[u] >> 3, atom = bs_atom_bytes(m);
                 int count;
                 const int g0 = bs_group(slab, p.ks, p.csize, p.sl, count);
-                uint8_t *grp = A.xq + (int64_t)g0 * (p.m * 128 + atom);
-                *reinterpret_cast<uint4 *>(grp + ((int64_t)(ch[u] - g0 * 8) * p.m + t) * 16) = q;
+                uint8_t *grp = A.xq + (int64_t)tile * p.ks * (p.tokens * 128 + bs_atom_bytes(p.tokens)) + (int64_t)g0 * (m * 128 + atom);
+                *reinterpret_cast<uint4 *>(grp + ((int64_t)(ch[u] - g0 * 8) * m + t) * 16) = q;
                 if ((ch[u] & 1) == 0)
-                    grp[(int64_t)count * p.m * 128 + (slab - g0) * atom + (t & 31) * 16 + (t >> 5) * 4 + ((ch[u] >> 1) & 3)] =
-                        (uint8_t)min(max(e + 127, 0), 255);
+                    grp[(int64_t)count * m * 128 + (slab - g0) * atom + (t >> 7) * kBsAtomBytes + (t & 31) * 16 + ((t >> 5) & 3) * 4 +
+                        ((ch[u] >> 1) & 3)] = (uint8_t)min(max(e + 127, 0), 255);
             }
         }
     }
