@@ -302,8 +302,13 @@ ws_status_t ws_tp_create(int32_t world, int32_t rank, int32_t device, const ws_t
         set_smem(tp, fp8_gemv_kernel<1, 4>) != WS_OK || set_smem(tp, fp8_gemv_kernel<1, 8>) != WS_OK ||
         set_smem(tp, fp8_gemv_kernel<2, 1>) != WS_OK || set_smem(tp, fp8_gemv_kernel<2, 2>) != WS_OK ||
         set_smem(tp, fp8_gemv_kernel<2, 4>) != WS_OK || set_smem(tp, moe_down_kernel) != WS_OK ||
-        set_smem(tp, fp8_bs_kernel<16, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<64, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, false>) != WS_OK ||
-        set_smem(tp, fp8_bs_kernel<16, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<64, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, true>) != WS_OK || set_smem(tp, fp8_tile_kernel<false>) != WS_OK || set_smem(tp, fp8_tile_kernel<true>) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<16, false, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, false, false>) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<64, false, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, false, false>) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<16, true, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, true, false>) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<64, true, false>) != WS_OK || set_smem(tp, fp8_bs_kernel<128, true, false>) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<16, false, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, false, true>) != WS_OK ||
+        set_smem(tp, fp8_bs_kernel<16, true, true>) != WS_OK || set_smem(tp, fp8_bs_kernel<32, true, true>) != WS_OK ||
+        set_smem(tp, fp8_tile_kernel<false>) != WS_OK || set_smem(tp, fp8_tile_kernel<true>) != WS_OK ||
         set_smem(tp, moe_bs_kernel) != WS_OK ||
         cudaFuncSetAttribute(moe_bs_prep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         // The prep kernel uses no shared memory, but a main-kernel CTA (which needs almost all of an SM's)
@@ -446,7 +451,7 @@ static ws_status_t validate_fp8(ws_tp *tp, const ws_fp8_gemm_args_t &a, bool lm_
 // neither: a 32-wide scale block is the MMA's own).
 struct BsPlan {
     bool ok, wue;
-    int mp, ks, tile_rows, ntiles, a_pitch, x_pitch, slabs_per_stage, nstages, nslot_max, nacc;
+    int mp, ks, tile_rows, ntiles, a_pitch, x_pitch, slabs_per_stage, nstages, nslot_max, nacc, inline_x;
     int csize;  // 2: CTA pairs share a tile, each CTA streams half of K (tiles of a lone CTA would fill under half of the MMA's rows)
     int ncta;   // CTAs the plan is for (even with pairs)
     int tmem_cols;  // tensor-memory columns the CTA allocates (a power of two)
@@ -471,6 +476,10 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     u.ntiles = (a.n + u.tile_rows - 1) / u.tile_rows;
     const int tiles_per_cta = (u.ntiles + nparts - 1) / nparts;
     u.a_pitch = (u.tile_rows + 7) / 8 * 8 * 128;
+    // Up to 8192 values per CTA it quantises them itself, without the prep kernel's launch and the wait for it
+    // (K/rank 1024: 4 rows 6.1 against 7.5 us per step, 16 rows 7.4 against 8.2; with 16 K values, 2048 x 16 rows,
+    // 12.3 against 9.7).
+    u.inline_x = u.mp <= 32 && mt * ((u.ks + u.csize - 1) / u.csize) * 128 <= 8192 ? 1 : 0;
     const int x_slab = mt * 128 + bs_atom_bytes(mt), slab_bytes = u.a_pitch + x_slab + (u.wue ? kBsAtomBytes : 0);
     // slabs per stage: barrier round trips, a commit and two copies are per stage, so several slabs share them; bounded by the stage size and by tensor memory (fp32 scales: each
     // slab has its own accumulator buffer, groups x slabs x (mp + 4) + 8 columns of 512, at least two groups)
@@ -492,7 +501,8 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         u.nacc = u.wue ? std::min(2, std::max(1, (tmem - 8 - 2 * u.slabs_per_stage * 8) / u.mp))
                        : std::min((int)kBsMaxAcc, (tmem - 8) / (u.slabs_per_stage * (u.mp + 4)));
         auto total = [&](int ns) {
-            return bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, u.nslot_max, skb, u.mp, rx_rows, u.wue).total + 1024;
+            return bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, u.nslot_max, skb, u.mp, rx_rows, u.wue,
+                                  u.inline_x ? kcta * x_slab : 0).total + 1024;
         };
         int ns = kMaxStages;  // the most stages whose layout fits
         while (ns >= 2 && total(ns) > budget) --ns;
@@ -558,6 +568,7 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     p.slabs_per_stage = u.slabs_per_stage; p.nstages = u.nstages; p.nslot_max = u.nslot_max; p.skb = skb; p.nacc = u.nacc;
     p.csize = u.csize;
     p.tmem_cols = u.tmem_cols;
+    p.x_dtype = a0.x_dtype;
     // 32 rows and more on four ranks and more: all-to-all of every partial sum costs more link time than the second hop
     p.owner_reduce = (t0->world >= 4 && u.mp >= 32) ? 1 : 0;
     p.timeout_ns = t0->timeout_ns;
@@ -570,11 +581,11 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     for (int i = 0; i < n; ++i) {
         ws_tp *t = ranks[i];
         const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
-        ws_status_t s = ensure_bs_scratch(t, xq_bytes);
+        ws_status_t s = u.inline_x ? WS_OK : ensure_bs_scratch(t, xq_bytes);
         if (s == WS_OK) s = make_tmap(t, &p.tmap_w[i], a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, (uint32_t)u.tile_rows);
         if (s != WS_OK) { t0->err = t->err; return s; }
         Fp8RankArgs &r = p.r[i];
-        r.x = nullptr;
+        r.x = static_cast<const char *>(a.x) + (size_t)m0 * a.ldx * (a.x_dtype == WS_ACT_BF16 ? 2 : 4);
         r.scales = a.scales;
         r.out = lm ? nullptr : a.out + (size_t)m0 * a.n;
         r.logits = lm && lm[i].logits ? lm[i].logits + (size_t)m0 * lm[i].vocab : nullptr;
@@ -585,13 +596,21 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         r.ctx = make_ctx(t);
         if (last) r.ctx.host_done = t->host_done_arm;
         p.xq[i] = q.r[i].xq = t->bs_work;
-        q.r[i].x = static_cast<const char *>(a.x) + (size_t)m0 * a.ldx * (a.x_dtype == WS_ACT_BF16 ? 2 : 4);
+        q.r[i].x = r.x;
         q.r[i].ldx = a.ldx;
     }
     for (int i = 0; i < n; ++i) ranks[i]->step++;
     void (*kernel)(BsParams);
-    if (u.wue) kernel = u.mp == 16 ? fp8_bs_kernel<16, true> : u.mp == 32 ? fp8_bs_kernel<32, true> : u.mp == 64 ? fp8_bs_kernel<64, true> : fp8_bs_kernel<128, true>;
-    else kernel = u.mp == 16 ? fp8_bs_kernel<16, false> : u.mp == 32 ? fp8_bs_kernel<32, false> : u.mp == 64 ? fp8_bs_kernel<64, false> : fp8_bs_kernel<128, false>;
+    if (u.inline_x) kernel = u.wue ? (u.mp == 16 ? fp8_bs_kernel<16, true, true> : fp8_bs_kernel<32, true, true>)
+                                   : (u.mp == 16 ? fp8_bs_kernel<16, false, true> : fp8_bs_kernel<32, false, true>);
+    else if (u.wue) kernel = u.mp == 16   ? fp8_bs_kernel<16, true, false>
+                             : u.mp == 32 ? fp8_bs_kernel<32, true, false>
+                             : u.mp == 64 ? fp8_bs_kernel<64, true, false>
+                                          : fp8_bs_kernel<128, true, false>;
+    else kernel = u.mp == 16   ? fp8_bs_kernel<16, false, false>
+                  : u.mp == 32 ? fp8_bs_kernel<32, false, false>
+                  : u.mp == 64 ? fp8_bs_kernel<64, false, false>
+                               : fp8_bs_kernel<128, false, false>;
     const int prep_blocks = (int)std::min<int64_t>(std::max(1, t0->sm_count / n), ((int64_t)mt * u.ks * 8 + kActPrepThreads - 1) / kActPrepThreads);
     ws_status_t s = zero_lone_shard(ranks, n, lm, m0, mt, streams);
     for (int i = 0; i < (same_device ? 1 : n) && s == WS_OK; ++i) {
@@ -604,7 +623,8 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         const int nvr = same_device ? n : 1;
         WS_CUDA(ranks[i], cudaSetDevice(ranks[i]->device));
         cudaStream_t cs = static_cast<cudaStream_t>(streams ? streams[i] : nullptr);
-        s = launch(ranks[i], act_prep_kernel, q, prep_blocks, nvr, kActPrepThreads, 0, cs, t0->pdl != 0, false);
+        if (!u.inline_x)
+            s = launch(ranks[i], act_prep_kernel, q, prep_blocks, nvr, kActPrepThreads, 0, cs, t0->pdl != 0, false);
         if (s == WS_OK) s = launch(ranks[i], kernel, p, u.ncta, nvr, bs_threads(u.mp, u.wue), u.smem, cs, t0->pdl != 0, true, u.csize);
         if (s != WS_OK) t0->err = ranks[i]->err;
     }
@@ -1005,17 +1025,20 @@ static MoeBsPlan moe_bs_plan(const ws_moe_down_args_t &a, int ncta) {
     u.tile_rows = (a.n + nparts - 1) / nparts;
     if (u.tile_rows > kBsMmaRows) return u;
     u.a_pitch = (u.tile_rows + 7) / 8 * 8 * 128;
-    const int groups = getenv("X2") ? atoi(getenv("X2")) : 2;
-    u.slabs_per_stage = (nslab + groups - 1) / groups;
-    u.inline_x = a.m * a.top_k <= (getenv("X1") ? atoi(getenv("X1")) : kMoeBsInlineRoutes) ? 1 : 0;
+    u.inline_x = a.m * a.top_k <= kMoeBsInlineRoutes ? 1 : 0;
     const int nr = std::min((int)kMoeBsCols, a.m * a.top_k);  // most routes of a pass
-    u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * (nr * 128 + nr * 16), 128);
     // the partner's sums land behind the ring, or, when there are many, in the ring itself after the last pass
     u.alias = a.m > 8 ? 1 : 0;
     auto total = [&](int ns) { return moe_bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, a.m, nslab, u.alias, a.m * a.top_k, u.inline_x).total + 1024; };
-    int ns = kMaxStages;
-    while (ns >= 2 && total(ns) > kSmemBudget - 8 * 1024) --ns;  // (beside a few blocks of the prep kernel)
-    ns = std::min(ns, 4 * ((nslab + u.slabs_per_stage - 1) / u.slabs_per_stage));  // four pass barriers: see moe_bs_kernel
+    // A stage is a whole pass when two of them fit (5120 x 2304: 44 against 46 us with two stages per pass), else
+    // half of one: every stage costs the issuing thread two barriers, a box and a commit.
+    int ns = 0;
+    for (int groups = 1; groups <= 2 && ns < 2; ++groups) {
+        u.slabs_per_stage = (nslab + groups - 1) / groups;
+        u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * (nr * 128 + nr * 16), 128);
+        ns = std::min(kMaxStages, 4 * groups);  // four pass barriers: see moe_bs_kernel
+        while (ns >= 2 && total(ns) > kSmemBudget - 8 * 1024) --ns;  // (beside a few blocks of the prep kernel)
+    }
     u.nstages = ns;
     int cols = 32;
     while (cols < 2 * kMoeBsCols + 2 * nslab * 8 + a.m) cols *= 2;
@@ -1440,7 +1463,8 @@ ws_status_t ws_fp8_rowpar_gemm_allreduce_host(ws_tp_t *tp, const ws_fp8_gemm_arg
             const int skb = (int)((dw->k0 + dw->k - 1) / dw->block_k - dw->k0 / dw->block_k + 1);
             const int mt = fp8_rows_per_launch(tp, a, ncta, a.m);
             direct = true;
-            stage = !(bs_wanted(tp, mt, a) && bs_plan(a, mt, skb, ncta, true).ok);
+            const BsPlan u = bs_plan(a, mt, skb, ncta, true);
+            stage = !(bs_wanted(tp, mt, a) && u.ok && !u.inline_x);  // only the prep kernel reads every value just once
             if (!stage) a.x = pin;
         }
     }

@@ -147,10 +147,10 @@ struct alignas(64) BsParams {
     int32_t tile_rows, ntiles;         // output rows per tile (<= 128) and tiles of the shard
     int32_t slabs_per_stage, nstages;
     int32_t a_pitch, x_pitch;          // bytes one slab's weights (a multiple of 1024) / one stage's activations and atoms (of 128) occupy
-    int32_t skb, nslot_max, nacc, gather_logits;
+    int32_t skb, nslot_max, nacc, gather_logits, x_dtype;
     uint64_t timeout_ns;
     SymLayout lay;
-    Fp8RankArgs r[WS_MAX_WORLD];       // x is unused here; scales/out/logits/argmax/row0/k0/ctx as in the decode kernels
+    Fp8RankArgs r[WS_MAX_WORLD];       // x is used when the kernel quantises itself (INL); the rest as in the decode kernels
     const uint8_t *xq[WS_MAX_WORLD];   // the prep kernel's activations and scale atoms
 };
 
@@ -158,20 +158,21 @@ struct BsSmem {
     int32_t a, x, wsf, sw, cand, rx, bars, misc, total;
 };
 __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stage, int a_pitch, int x_pitch, int nslot_max,
-                                                 int skb, int mp, int rx_rows, bool wue) {
+                                                 int skb, int mp, int rx_rows, bool wue, int x_resident) {
     BsSmem s{};
     const int nsl = nstages * slabs_per_stage;
+    const int x_bytes = x_resident > 0 ? (x_resident + 127) / 128 * 128 : nstages * x_pitch;  // inline: all of this K half
     int o = 0;
     s.a = o;    o += nsl * a_pitch;
-    s.x = o;    o += nstages * x_pitch;
+    s.x = o;    o += x_bytes;
     // an MMA reads 128 rows of its weight slab however many the tile holds, and up to 128 tokens and 32 atom
     // rows whatever m is: keep 16 KB readable behind the last slab and 2 KB behind the last activations
-    o += nstages * x_pitch + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - nstages * x_pitch : 2048;
+    o += x_bytes + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - x_bytes : 2048;
     s.wsf = o;  o += wue ? nsl * kBsAtomBytes : kBsAtomBytes;  // the weights' scale atoms (fp32 scales: one atom of 2^0)
     s.sw = o;   o += wue ? 0 : (int)align_up((int64_t)nslot_max * skb * 4, 16);
     s.cand = o; o += bs_epi_warps(mp, wue) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
     s.rx = o;   o += rx_rows * kBsMmaRows * 4;           // CTA pairs: the partner's sums of one tile for this CTA's tokens, [token][row]
-    s.bars = o; o += (2 * kMaxStages + 2 * kBsMaxAcc + 2) * 8;
+    s.bars = o; o += (2 * kMaxStages + 2 * kBsMaxAcc + 4) * 8;
     s.misc = o; o += 64;
     s.total = o;
     return s;
@@ -365,7 +366,109 @@ __device__ __forceinline__ uint32_t order_key(float v) {
     return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);
 }
 
-template <int MP, bool WUE>
+// The exchange behind a CTA's finished tiles [t_lo, t_hi]: fold row rc of each for the tokens [tbeg, tend), in rank
+// order, as the ranks' words arrive.  A function of its own: what it holds in registers is not taken from the
+// loops of the kernel.
+static __device__ __noinline__ void bs_fold(const BsParams &p, int vr, uint32_t seq, int t_lo, int t_hi, int rc, int tbeg, int tend) {
+    const Fp8RankArgs &A = p.r[vr];
+    const RankCtx &X = A.ctx;
+    const uint32_t bank = seq & 1u;
+    const int TR = p.tile_rows;
+    const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
+    // fold the rows of the tiles this CTA finished, in rank order, as the ranks' words arrive
+    const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
+    for (int t = t_lo; t <= t_hi; ++t) {
+        const int row = t * TR + rc;
+        if (rc >= TR || row >= p.n) continue;
+        // Fold by owners: the sums of tile t are formed on rank t % world only (in rank order, as
+        // everywhere) and travel back in that rank's own slot at every peer, so all ranks end up
+        // with the same bits and each partial sum crosses the links once instead of world - 1 times.
+        const int owner = p.owner_reduce ? t % p.world : X.rank;
+        if (!p.owner_reduce) {
+            // Two tokens at a time, the words of all their ranks requested before the first is looked at: one
+            // memory round trip instead of one per rank (three rows on eight ranks: 29 of a 50 us step); if one
+            // has not arrived yet they are waited for one by one.  Ranks are added in rank order.
+#pragma unroll 1
+            for (int tok0 = tbeg; tok0 < tend; tok0 += 2) {
+                const uint64_t *src = slots + (size_t)tok0 * p.n + row;
+                const int64_t second = tok0 + 1 < tend ? p.n : 0;
+                uint64_t w0[WS_MAX_WORLD], w1[WS_MAX_WORLD];
+                const uint64_t *at = src;
+#pragma unroll
+                for (int rr = 0; rr < WS_MAX_WORLD; ++rr) {
+                    if (rr < p.world) {
+                        w0[rr] = ld_word_sys(at);
+                        w1[rr] = ld_word_sys(at + second);
+                    }
+                    at += astride;
+                }
+                bool here = true;
+                float sum0 = 0.0f, sum1 = 0.0f;
+#pragma unroll
+                for (int rr = 0; rr < WS_MAX_WORLD; ++rr)
+                    if (rr < p.world) {
+                        here = here && (uint32_t)(w0[rr] >> 32) == seq && (uint32_t)(w1[rr] >> 32) == seq;
+                        const float v0 = __uint_as_float((uint32_t)w0[rr]), v1 = __uint_as_float((uint32_t)w1[rr]);
+                        sum0 = rr == 0 ? v0 : sum0 + v0;
+                        sum1 = rr == 0 ? v1 : sum1 + v1;
+                    }
+                if (!here) {
+#pragma unroll 1
+                    for (int i = 0; i < 2; ++i) {
+                        float sum = 0.0f;
+#pragma unroll 1
+                        for (int rr = 0; rr < p.world; ++rr) {
+                            const float v = wait_word(src + rr * astride + i * second, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
+                            sum = rr == 0 ? v : sum + v;
+                        }
+                        if (i == 0) sum0 = sum;
+                        else sum1 = sum;
+                    }
+                }
+                float *out = A.out + (size_t)tok0 * p.n + row;
+                out[0] = sum0;
+                if (second) out[second] = sum1;
+            }
+            continue;
+        }
+        // 16 tokens at a time: their words of one rank are all requested before the first is
+        // looked at (one memory round trip per batch, not per word); a word that has not
+        // arrived yet is then waited for on its own.  Ranks are added in rank order.
+        for (int tok0 = tbeg; tok0 < tend; tok0 += 16) {
+            float sum[16];
+            const int rr0 = owner == X.rank ? 0 : owner, rr1 = owner == X.rank ? p.world : owner + 1;
+            for (int rr = rr0; rr < rr1; ++rr) {
+                const uint64_t *src = slots + rr * astride + (size_t)tok0 * p.n + row;
+                uint64_t w[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (tok0 + i < tend) w[i] = ld_word_sys(src + (size_t)i * p.n);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (tok0 + i < tend) {
+                        const float v = (uint32_t)(w[i] >> 32) == seq
+                                            ? __uint_as_float((uint32_t)w[i])
+                                            : wait_word(src + (size_t)i * p.n, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
+                        sum[i] = rr == rr0 ? v : sum[i] + v;
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (tok0 + i < tend) A.out[(size_t)(tok0 + i) * p.n + row] = sum[i];
+            if (p.owner_reduce && owner == X.rank)
+                for (int pr = 0; pr < p.world; ++pr) {
+                    if (pr == X.rank) continue;
+                    uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) +
+                                    ((size_t)bank * p.world + X.rank) * astride + (size_t)tok0 * p.n + row;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (tok0 + i < tend) st_word_sys(dst + (size_t)i * p.n, seq, sum[i]);
+                }
+        }
+    }
+}
+
+template <int MP, bool WUE, bool INL>
 __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, WUE)) fp8_bs_kernel(const __grid_constant__ BsParams p) {
     constexpr int EW = bs_epi_warps(MP, WUE), ET = EW * 32;  // epilogue warps / threads
     constexpr int CP = MP * 4 / EW;                      // token columns one epilogue thread holds
@@ -388,7 +491,8 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
     const int SL = p.slabs_per_stage, NS = p.nstages, NB = p.nacc;
     const int ntiles = p.ntiles, TR = p.tile_rows;
 
-    const BsSmem S = bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? (p.m + 1) / 2 : 0, WUE);
+    const BsSmem S = bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? (p.m + 1) / 2 : 0, WUE,
+                                    INL ? (KS + p.csize - 1) / p.csize * (p.m * 128 + bs_atom_bytes(p.m)) : 0);
     float *sw_s = reinterpret_cast<float *>(smem + S.sw);
     uint32_t *misc_s = reinterpret_cast<uint32_t *>(smem + S.misc);
     const uint32_t a0 = smem_u32(smem + S.a), x0 = smem_u32(smem + S.x), wsf0 = smem_u32(smem + S.wsf);
@@ -400,14 +504,14 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
     // buffer (tile mod NB), accfull / accempty hand it over.
     const uint32_t full0 = smem_u32(smem + S.bars), done0 = full0 + kMaxStages * 8;
     const uint32_t accempty0 = done0 + kMaxStages * 8, accfull0 = accempty0 + kBsMaxAcc * 8;
-    const uint32_t rxfull = accfull0 + kBsMaxAcc * 8, rxempty = rxfull + 8;  // CTA pairs: the partner's sums of a tile have arrived / been read
+    const uint32_t rxfull = accfull0 + kBsMaxAcc * 8, rxempty = rxfull + 8, xready = rxempty + 8;  // CTA pairs: the partner's sums of a tile have arrived / been read
 
     // Weights are static: the first ring's worth is on its way before the CTA has set itself up (barriers,
     // tensor memory and the pair's meeting take ~1.3 us, in which HBM would idle), let alone before the wait on
     // the prep kernel.
     const uint32_t x_slab = (uint32_t)(p.m * 128 + bs_atom_bytes(p.m));
     auto issue_w = [&](int s, int tile, int s0, int nsl) {
-        mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + x_slab));
+        mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)nsl * ((uint32_t)TR * 128u + (INL ? 0u : x_slab)));
         for (int j = 0; j < nsl; ++j)
             tma_load_2d(a0 + (s * SL + j) * p.a_pitch, &p.tmap_w[vr], (s0 + j) * 128, tile * TR, full0 + s * 8);
     };
@@ -423,6 +527,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             }
             mbar_init(rxfull, EW);   // every epilogue warp of the partner arrives after its stores
             mbar_init(rxempty, EW);
+            mbar_init(xready, EW);   // inline: the activations are in shared memory
             mbar_fence_init();
             int tile, s0, nsl;
             BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
@@ -466,7 +571,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                     if (!mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status)) break;
                     issue_w(s, tile, s0, nsl);
                 }
-                bulk_load(x0 + s * p.x_pitch, p.xq[vr] + (size_t)s0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
+                if (!INL) bulk_load(x0 + s * p.x_pitch, p.xq[vr] + (size_t)s0 * x_slab, (uint32_t)nsl * x_slab, full0 + s * 8);
             }
         }
     } else if (warp == 1) {
@@ -498,11 +603,13 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             // accumulator ring
             uint32_t accempty = accempty0, t_acc = tmem_base, t_sf = t_sf0, acc_ph = 1;
             const uint32_t acc_end = accempty0 + NB * 8;
+            constexpr bool inl = INL;
+            uint32_t sf_off = 0;
             // one stage: straight-line code per slab count (a rolled loop costs twice the time); `carry`: the first
             // MMA adds to earlier stages' sums (UE8M0)
             auto issue = [&](auto count, uint32_t carry) {
                 constexpr int C = decltype(count)::value;
-                const uint64_t xsf = xsf0 + (uint64_t)(x_off + (uint32_t)C * x_step), wsf = wsf_desc0 + (uint64_t)w_off;
+                const uint64_t xsf = xsf0 + (uint64_t)(inl ? sf_off : x_off + (uint32_t)C * x_step), wsf = wsf_desc0 + (uint64_t)w_off;
 #pragma unroll
                 for (int j = 0; j < C; ++j) {
                     const uint32_t a = a_lo + (uint32_t)j * a_step, b = x_lo + (uint32_t)j * x_step;
@@ -517,10 +624,12 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                 }
             };
             const int my_tiles = (int)((int64_t)ntiles * (part + 1) / nparts) - (int)((int64_t)ntiles * part / nparts), kcta = k_hi - k_lo;
-            bool ok = true;
+            const uint32_t sf_off0 = (uint32_t)kcta * x_step;  // inline: the atoms follow all of the K half's activations
+            bool ok = !INL || mbar_wait(xready, 0, status);
             uint32_t odd = 0;  // UE8M0: which of the two sets of scale columns
             for (int t = kcta > 0 ? my_tiles : 0; t > 0 && ok; --t) {
                 uint32_t carry = 0;
+                if (inl) { x_lo = x_lo0; sf_off = sf_off0; }
                 for (int left = kcta; left > 0; left -= SL) {
                     if ((!WUE || carry == 0) && !mbar_wait(accempty, acc_ph, status)) { ok = false; break; }
                     if (!mbar_wait(full, ph, status)) { ok = false; break; }
@@ -537,10 +646,13 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                         odd ^= 1u;
                     }
                     // next stage
-                    full += 8; done += 8; a_lo += a_stage; x_lo += x_stage; x_off += x_stage;
+                    full += 8; done += 8; a_lo += a_stage; x_off += x_stage;
+                    x_lo += inl ? (uint32_t)SL * x_step : x_stage;
+                    sf_off += (uint32_t)SL * xsf_step;
                     if (WUE) w_off += (uint32_t)SL * kSfStep;
                     if (full == full_end) {
-                        full = full0; done = done0; a_lo = a_lo0; x_lo = x_lo0; x_off = 0; w_off = 0;
+                        full = full0; done = done0; a_lo = a_lo0; x_off = 0; w_off = 0;
+                        if (!inl) x_lo = x_lo0;
                         ph ^= 1u;
                     }
                     // next accumulator (group)
@@ -618,6 +730,39 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             }
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        if constexpr (INL) {  // few enough values: this CTA's K half of the activations, straight into shared memory
+            const int chunks = (k_hi - k_lo) * 8, total = p.m * chunks, atom = bs_atom_bytes(p.m);
+            uint8_t *xs = smem + S.x, *atoms = xs + (size_t)total * 16;
+            constexpr int U = 2;  // chunks whose loads are in flight together
+            for (int c0 = et; c0 - lane < total; c0 += U * ET) {  // whole warps
+                float v[U][16];
+                int tok[U], ch[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int c = c0 + u * ET;
+                    tok[u] = c < total ? c / chunks : 0;
+                    ch[u] = c - tok[u] * chunks;
+                    const int kk = k_lo * 128 + ch[u] * 16;
+                    const bool valid = c < total && kk < p.k;
+                    load_act8(A.x, p.x_dtype, (int64_t)tok[u] * A.ldx + kk, valid, *reinterpret_cast<float(*)[8]>(v[u]));
+                    load_act8(A.x, p.x_dtype, (int64_t)tok[u] * A.ldx + kk + 8, valid, *reinterpret_cast<float(*)[8]>(v[u] + 8));
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    int e;
+                    const uint4 q = act_quant16(v[u], e);
+                    if (c0 + u * ET < total) {
+                        *reinterpret_cast<uint4 *>(xs + ((size_t)ch[u] * p.m + tok[u]) * 16) = q;
+                        if ((ch[u] & 1) == 0)
+                            atoms[(size_t)(ch[u] >> 3) * atom + (tok[u] & 31) * 16 + (tok[u] >> 5) * 4 + ((ch[u] >> 1) & 3)] =
+                                (uint8_t)min(max(e + 127, 0), 255);
+                    }
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(xready);
+        }
         const uint32_t seq = step_begin(X);
         const uint32_t bank = seq & 1u;
         bs_epi_bar();
@@ -787,51 +932,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         const uint32_t *myflags = solo ? nullptr
                                        : reinterpret_cast<const uint32_t *>(X.sym[X.rank] + p.lay.flags_off) + (size_t)bank * p.world * nflag;
         if (!solo && p.mode == kModeAllReduce) {
-            // fold the rows of the tiles this CTA finished, in rank order, as the ranks' words arrive
-            const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
-            for (int t = t_lo; t <= t_hi; ++t) {
-                const int row = t * TR + rc;
-                if (rc >= TR || row >= p.n) continue;
-                // 16 tokens at a time: their words of one rank are all requested before the first is
-                // looked at (one memory round trip per batch, not per word); a word that has not
-                // arrived yet is then waited for on its own.  Ranks are added in rank order.
-                const int tbeg = max(tok_lo, col0), tend = min(tok_hi, col0 + CP);  // this thread's token columns
-                // Fold by owners: the sums of tile t are formed on rank t % world only (in rank order, as
-                // everywhere) and travel back in that rank's own slot at every peer, so all ranks end up
-                // with the same bits and each partial sum crosses the links once instead of world - 1 times.
-                const int owner = p.owner_reduce ? t % p.world : X.rank;
-                for (int tok0 = tbeg; tok0 < tend; tok0 += 16) {
-                    float sum[16];
-                    const int rr0 = owner == X.rank ? 0 : owner, rr1 = owner == X.rank ? p.world : owner + 1;
-                    for (int rr = rr0; rr < rr1; ++rr) {
-                        const uint64_t *src = slots + rr * astride + (size_t)tok0 * p.n + row;
-                        uint64_t w[16];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (tok0 + i < tend) w[i] = ld_word_sys(src + (size_t)i * p.n);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (tok0 + i < tend) {
-                                const float v = (uint32_t)(w[i] >> 32) == seq
-                                                    ? __uint_as_float((uint32_t)w[i])
-                                                    : wait_word(src + (size_t)i * p.n, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
-                                sum[i] = rr == rr0 ? v : sum[i] + v;
-                            }
-                    }
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (tok0 + i < tend) A.out[(size_t)(tok0 + i) * p.n + row] = sum[i];
-                    if (p.owner_reduce && owner == X.rank)
-                        for (int pr = 0; pr < p.world; ++pr) {
-                            if (pr == X.rank) continue;
-                            uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) +
-                                            ((size_t)bank * p.world + X.rank) * astride + (size_t)tok0 * p.n + row;
-#pragma unroll
-                            for (int i = 0; i < 16; ++i)
-                                if (tok0 + i < tend) st_word_sys(dst + (size_t)i * p.n, seq, sum[i]);
-                        }
-                }
-            }
+            bs_fold(p, vr, seq, t_lo, t_hi, rc, max(tok_lo, col0), min(tok_hi, col0 + CP));
         } else if (p.mode == kModeLmHead) {
             // The argmax.  The CTAs of a rank leave their candidates in the rank's own
             // table; the CTA that arrives last merges them into ONE (value, lowest index) per token,
