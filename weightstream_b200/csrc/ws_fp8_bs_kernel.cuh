@@ -366,14 +366,21 @@ __device__ __forceinline__ uint32_t order_key(float v) {
     return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);
 }
 
-// The exchange behind a CTA's finished tiles [t_lo, t_hi]: fold row rc of each for the tokens [tbeg, tend), in rank
-// order, as the ranks' words arrive.  A function of its own: what it holds in registers is not taken from the
-// loops of the kernel.
-static __device__ __noinline__ void bs_fold(const BsParams &p, int vr, uint32_t seq, int t_lo, int t_hi, int rc, int tbeg, int tend) {
+// The exchange behind a CTA's finished tiles: fold its rows, in rank order, as the ranks' words arrive.  Thread
+// `et` of the epilogue (32 * ew of them) takes row et % 128 of each tile and the tokens whose columns it held.  A
+// function of its own, called when nothing else is left to do: inside the epilogue what it holds in registers was
+// taken from the main loops (three rows of K 8192 on one rank 16.0 us instead of 15.0).
+static __device__ __noinline__ void bs_fold(const BsParams &p, int ew, int cp) {
+    const int vr = blockIdx.y, pair = p.csize == 2 ? 1 : 0;
     const Fp8RankArgs &A = p.r[vr];
     const RankCtx &X = A.ctx;
-    const uint32_t bank = seq & 1u;
-    const int TR = p.tile_rows;
+    const uint32_t seq = step_begin(X), bank = seq & 1u;
+    const int TR = p.tile_rows, part = blockIdx.x >> pair, nparts = gridDim.x >> pair, half = (p.m + 1) / 2;
+    const int t_lo = (int)((int64_t)p.ntiles * part / nparts), t_hi = (int)((int64_t)p.ntiles * (part + 1) / nparts) - 1;
+    const int warp = (int)(threadIdx.x >> 5), rc = (warp & 3) * 32 + (int)(threadIdx.x & 31), col0 = ((warp - 2) >> 2) * cp;
+    const bool upper = pair && (blockIdx.x & 1);
+    const int tbeg = max(upper ? half : 0, col0), tend = min(pair && !upper ? half : p.m, col0 + cp);
+    if (warp < 2 || warp >= 2 + ew) return;
     const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
     // fold the rows of the tiles this CTA finished, in rank order, as the ranks' words arrive
     const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
@@ -931,9 +938,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         // ---- exchange (the epilogue threads)
         const uint32_t *myflags = solo ? nullptr
                                        : reinterpret_cast<const uint32_t *>(X.sym[X.rank] + p.lay.flags_off) + (size_t)bank * p.world * nflag;
-        if (!solo && p.mode == kModeAllReduce) {
-            bs_fold(p, vr, seq, t_lo, t_hi, rc, max(tok_lo, col0), min(tok_hi, col0 + CP));
-        } else if (p.mode == kModeLmHead) {
+        if (p.mode == kModeLmHead) {
             // The argmax.  The CTAs of a rank leave their candidates in the rank's own
             // table; the CTA that arrives last merges them into ONE (value, lowest index) per token,
             // sends it to every peer and merges the ranks' candidates: one 64-bit store and one flag
@@ -1036,6 +1041,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         tc_fence_after();
         tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
     }
+    if (p.world > 1 && p.mode == kModeAllReduce) bs_fold(p, EW, CP);
     if (p.world > 1 || p.mode == kModeLmHead) step_end(X, step_begin(X), gridDim.x);
     host_done_signal(X, gridDim.x);
 }
