@@ -481,19 +481,22 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     // 12.3 against 9.7).
     u.inline_x = u.mp <= 32 && mt * ((u.ks + u.csize - 1) / u.csize) * 128 <= 8192 ? 1 : 0;
     const int x_slab = mt * 128 + bs_atom_bytes(mt), slab_bytes = u.a_pitch + x_slab + (u.wue ? kBsAtomBytes : 0);
-    // slabs per stage: barrier round trips, a commit and two copies are per stage, so several slabs share them; bounded by the stage size and by tensor memory (fp32 scales: each
-    // slab has its own accumulator buffer, groups x slabs x (mp + 4) + 8 columns of 512, at least two groups)
+    // slabs per stage: barrier round trips and a commit are per stage, and the scale atoms of UE8M0, so several slabs
+    // share them; bounded by the stage size (128 rows of K 8192: 40 KB 29.4, 56 KB 29.3 us; UE8M0 56 KB 37.1, 72 KB
+    // 33.4) and by tensor memory (fp32 scales: each slab has its own accumulator buffer, groups x slabs x (mp + 4) + 8
+    // columns of 512, at least two groups)
     u.nslot_max = (tiles_per_cta * u.tile_rows) / a.block_n + 2;
     const int rx_rows = u.csize == 2 ? (mt + 1) / 2 : 0, kcta = (u.ks + u.csize - 1) / u.csize;
     // Half an SM (shared memory and tensor memory) when the tokens are few and the CTA's whole share of
     // the weights fits such a ring (TP-8 shards): the next step's CTA is then resident beside this one
     // (one CTA per SM and step) and loads all of its weights under this step's exchange and exit.
     // Measured on B200, K/rank 1024, 8 rows: 7.7 us per step against 10.6.  Larger shares lose more to
-    // the shallower ring than they gain (K/rank 8192: 19.3 against 17.8 us).
-    const bool small = u.mp == 16 && (int64_t)a.n * a.k / u.ncta * u.csize <= ((int64_t)2 << 20);
+    // the shallower ring than they gain (K/rank 8192: 19.3 against 17.8 us).  UE8M0 CTAs are larger: two and prep
+    // blocks do not fit the registers together (5120 x 2304: 4 rows, no prep, 9.5 -> 7.9 us; 12 rows 9.6 -> 11.0).
+    const bool small = u.mp == 16 && (!u.wue || u.inline_x) && (int64_t)a.n * a.k / u.ncta * u.csize <= ((int64_t)2 << 20);
     for (int half = small ? 1 : 0; half >= 0; --half) {
         const int budget = half ? kHalfSmemBudget : kSmemBudget, tmem = half ? 256 : 512;
-        const int stage_target = half ? 32 * 1024 : 56 * 1024;
+        const int stage_target = half ? 32 * 1024 : u.wue ? 72 * 1024 : 56 * 1024;
         u.slabs_per_stage = std::max(1, std::min({4, stage_target / slab_bytes, kcta, u.wue ? 4 : (tmem - 8) / (2 * (u.mp + 4))}));
         const int groups = (kcta + u.slabs_per_stage - 1) / u.slabs_per_stage;
         u.slabs_per_stage = (kcta + groups - 1) / groups;
@@ -683,16 +686,15 @@ static ws_status_t tile_step(ws_tp *tp, const ws_fp8_gemm_args_t &a, cudaStream_
     return s;
 }
 
-// Whether rows [.., +mt) of this step go to the block-scaled tcgen05 path: always when the caller
-// selected it; by default from three rows up, and for one or two rows when the shard is large enough
-// for its streaming rate to outweigh the second launch (measured on B200, M=1: 927 MB 153 against
-// 208 us on CUDA cores; 58.7 MB 17.7 against 17.2 us, 14.7 MB 8.8 against 6.8 us, 7.3 MB 12.8 against 5.9 us).
+// Whether rows [.., +mt) of this step go to the block-scaled tcgen05 path: always when the caller selected it; by
+// default from three rows up.  One row: the CUDA-core kernel is ahead until the stream alone counts (7.3 MB 4.0
+// against 5.6 us, 58.7 MB 12.9 / 13.4, 117 MB 23.2 / 23.4); an lm_head step also saves the exchange of one candidate
+// per CTA (this kernel sends one per rank).  Two rows cost the CUDA cores twice the arithmetic (14.7 MB 8.4 against
+// 8.2 us, 16.8 MB 8.9 / 9.6, 29 MB 12.5 / 10.3), UE8M0 scales more still (11.8 MB 9.8 / 7.1).
 static bool bs_wanted(const ws_tp *t0, int mt, const ws_fp8_gemm_args_t &a, bool lm_head = false) {
     if (t0->kernel_sel == 2) return true;
     if (t0->kernel_sel != 0) return false;
-    // an lm_head step also saves the exchange of one candidate per CTA (this kernel sends one per rank)
-    // two rows: the CUDA-core kernel needs 23 us for a 58.7 MB shard, this one 17.8 (it is the same for 2 to 8 rows)
-    if (mt == 2 && (int64_t)a.n * a.k >= ((int64_t)32 << 20)) return true;
+    if (mt == 2 && (int64_t)a.n * a.k >= (int64_t)(a.scale_kind == WS_SCALE_UE8M0 ? 8 : 24) << 20) return true;
     return mt >= 3 || (int64_t)a.n * a.k >= ((int64_t)(lm_head ? 32 : 128) << 20);
 }
 

@@ -52,18 +52,18 @@ namespace ws {
 // Threads of a CTA.  Warp 0: producer, warp 1: MMA issue (and owner of the tensor memory), then the
 // epilogue warps: four (one per 32-lane quarter of the tensor memory, all token columns) for up to 16
 // tokens, eight (two per quarter, half of the token columns each) beyond, where reading the
-// accumulators back is what a stage waits for (sixteen for 128 tokens: 38 against 31 us; UE8M0
-// sums are read once per tile: eight from 64 tokens); then, for UE8M0
-// weight scales, four auxiliary warps.
-__host__ __device__ constexpr int bs_epi_warps(int mp, bool wue) { return mp >= (wue ? 64 : 32) ? 8 : 4; }
+// accumulators back is what a stage (UE8M0: the end of a tile) waits for (sixteen for 128 tokens: 38 against
+// 31 us); then, for UE8M0 weight scales, four auxiliary warps.
+__host__ __device__ constexpr int bs_epi_warps(int mp) { return mp >= 32 ? 8 : 4; }
 constexpr int kBsAuxWarps = 4;
-__host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 * (bs_epi_warps(mp, wue) + (wue ? kBsAuxWarps : 0)); }
+__host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 * (bs_epi_warps(mp) + (wue ? kBsAuxWarps : 0)); }
 // Registers per thread: what leaves a warp of the prep kernel room in every quarter of the SM's register file
-// (a CTA of ten warps has three in two of them; the next step's CTA otherwise waits for the prep block to
-// leave), and, up to 16 tokens, a second CTA.
-__host__ __device__ constexpr int bs_regs(int mp, bool wue) { return mp == 16 ? (wue ? 120 : 144) : wue && mp > 32 ? 128 : 152; }
+// (a CTA of ten warps has three in two of them, one of fourteen has four; the next step's prep blocks otherwise wait
+// for the CTA to leave: UE8M0, K 2304, 40 rows 13.3 against 10.4 us), and a second CTA, up to 16 tokens with fp32
+// scales and when a UE8M0 step has no prep blocks.
+__host__ __device__ constexpr int bs_regs(int mp, bool wue, bool inl) { return wue ? (mp == 16 && inl ? 96 : 112) : mp == 16 ? 144 : 152; }
 // Slabs whose accumulators an epilogue thread reads at once (fp32 weight scales): 64 registers' worth.
-__host__ __device__ constexpr int bs_read_batch(int mp) { return 64 / (mp * 4 / bs_epi_warps(mp, false)); }
+__host__ __device__ constexpr int bs_read_batch(int mp) { return 64 / (mp * 4 / bs_epi_warps(mp)); }
 constexpr int kBsMaxAcc = 8;         // accumulator groups in tensor memory (a group = one stage's slabs)
 constexpr int kBsMaxTokens = 128;    // activation rows one launch takes (16, 32, 64 or 128 MMA columns)
 constexpr int kBsAtomBytes = 512;    // one scale atom: 128 rows x 4 K blocks
@@ -170,7 +170,7 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
     o += x_bytes + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - x_bytes : 2048;
     s.wsf = o;  o += wue ? nsl * kBsAtomBytes : kBsAtomBytes;  // the weights' scale atoms (fp32 scales: one atom of 2^0)
     s.sw = o;   o += wue ? 0 : (int)align_up((int64_t)nslot_max * skb * 4, 16);
-    s.cand = o; o += bs_epi_warps(mp, wue) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
+    s.cand = o; o += bs_epi_warps(mp) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
     s.rx = o;   o += rx_rows * kBsMmaRows * 4;           // CTA pairs: the partner's sums of one tile for this CTA's tokens, [token][row]
     s.bars = o; o += (2 * kMaxStages + 2 * kBsMaxAcc + 4) * 8;
     s.misc = o; o += 64;
@@ -359,6 +359,35 @@ struct BsWalk {
     }
 };
 
+// UE8M0 weight scales of a shard as scale-operand words: the four exponents of a row's 128-wide K slab (2^0 past the
+// end of K).  32-wide blocks on word boundaries are one load; collected byte by byte with an address each, a warp's
+// instructions took longer than the slab's MMAs.
+struct Ue8m0Scales {
+    const uint8_t *base;
+    int64_t ld, k0;
+    int k, bk_shift;
+    bool words;
+    __device__ __forceinline__ Ue8m0Scales(const void *scales, int64_t ld_, int64_t k0_, int k_, int bk_shift_)
+        : base(static_cast<const uint8_t *>(scales)), ld(ld_), k0(k0_), k(k_), bk_shift(bk_shift_) {
+        words = bk_shift == 5 && (k0 & 127) == 0 && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(base) & 3) == 0;
+        if (words) base += k0 >> 5;
+    }
+    __device__ __forceinline__ const uint8_t *row(int64_t scale_row) const { return base + scale_row * ld; }
+    __device__ __forceinline__ uint32_t slab(const uint8_t *row, int s) const {
+        const int left = k - s * 128;  // a multiple of 32
+        uint32_t v = 0x7F7F7F7Fu;
+        if (words) {
+            v = __ldg(reinterpret_cast<const uint32_t *>(row) + s);
+            if (left < 128) v = (v & ((1u << (left >> 2)) - 1u)) | (0x7F7F7F7Fu << (left >> 2));
+        } else {
+#pragma unroll 1
+            for (int q = 0; q < 4 && q * 32 < left; ++q)
+                v = (v & ~(0xFFu << (8 * q))) | (uint32_t)__ldg(row + ((k0 + s * 128 + q * 32) >> bk_shift)) << (8 * q);
+        }
+        return v;
+    }
+};
+
 // Floats in an order that unsigned comparison keeps; everything that is not above -inf is 0.
 __device__ __forceinline__ uint32_t order_key(float v) {
     if (!(v > -INFINITY)) return 0u;
@@ -476,8 +505,8 @@ static __device__ __noinline__ void bs_fold(const BsParams &p, int ew, int cp) {
 }
 
 template <int MP, bool WUE, bool INL>
-__global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, WUE)) fp8_bs_kernel(const __grid_constant__ BsParams p) {
-    constexpr int EW = bs_epi_warps(MP, WUE), ET = EW * 32;  // epilogue warps / threads
+__global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, WUE, INL)) fp8_bs_kernel(const __grid_constant__ BsParams p) {
+    constexpr int EW = bs_epi_warps(MP), ET = EW * 32;  // epilogue warps / threads
     constexpr int CP = MP * 4 / EW;                      // token columns one epilogue thread holds
     auto bs_epi_bar = [] { bs_epi_bar_n<ET>(); };
     extern __shared__ uint8_t smem_raw[];
@@ -680,38 +709,49 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         __syncwarp();
     } else if (warp >= 2 + EW) {
         // ------------------------------------------------------------ auxiliary warps (UE8M0 weight scales)
-        // The scale bytes of the tile's rows (thread = row) become the stage's scale atoms; static, so they
-        // do not wait for the predecessor.
+        // The scale bytes of the tile's rows (thread = row) become the stage's scale atoms; static, so they do not
+        // wait for the predecessor.  Three items' words are in flight.
         if constexpr (WUE) {
             const int r = tid - 64 - ET;
+            const Ue8m0Scales sc(A.scales, A.scale_ld, A.k0, p.k, p.bk_shift);
             BsWalk w(ntiles, part, nparts, k_lo, k_hi, SL);
             RingPos st;
-            int tile, s0, nsl;
-            bool ok = true;
-            for (int item = 0; w.next(tile, s0, nsl); ++item, st.next(NS)) {
-                const int s = st.s, row = tile * TR + r;
-                const bool real = r < TR && row < p.n;
-                const uint8_t *src = static_cast<const uint8_t *>(A.scales) + ((A.row0 + (real ? row : 0)) >> p.bn_shift) * A.scale_ld;
-                uint32_t sc[4];
+            int item = 0;
+            uint32_t at = smem_u32(smem + S.wsf) + (uint32_t)((r & 31) * 16 + (r >> 5) * 4);
+            const uint32_t at_step = (uint32_t)(SL * kBsAtomBytes), at_end = at + NS * at_step;
+            auto load = [&](uint32_t (&b)[4]) {  // the next item's words; returns its slab count, 0 behind the last
+                int tile, s0, nsl;
+                if (!w.next(tile, s0, nsl)) return 0;
+                const uint8_t *row = sc.row((A.row0 + min(tile * TR + r, p.n - 1)) >> p.bn_shift);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sc[j] = 0u;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int kk = (s0 + j) * 128 + q * 32;
-                        const uint32_t b = real && j < nsl && kk < p.k ? __ldg(src + ((A.k0 + kk) >> p.bk_shift)) : 0x7Fu;
-                        sc[j] |= b << (8 * q);
-                    }
-                }
-                if (item >= NS) ok = mbar_wait(done0 + s * 8, st.ph ^ 1u, X.status);
-                if (!__all_sync(0xffffffffu, ok)) break;
+                for (int j = 0; j < 4; ++j) b[j] = sc.slab(row, min(s0 + j, k_hi - 1));
+                return nsl;
+            };
+            auto put = [&](const uint32_t (&b)[4], int nsl) {
+                bool ok = nsl > 0;
+                if (ok && item >= NS) ok = mbar_wait(done0 + st.s * 8, st.ph ^ 1u, X.status);
+                if (!__all_sync(0xffffffffu, ok)) return false;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (j < nsl)
-                        *reinterpret_cast<uint32_t *>(smem + S.wsf + (s * SL + j) * kBsAtomBytes + (r & 31) * 16 + (r >> 5) * 4) = sc[j];
+                    if (j < nsl) asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + j * kBsAtomBytes), "r"(b[j]) : "memory");
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(full0 + s * 8);
+                if (lane == 0) mbar_arrive(full0 + st.s * 8);
+                ++item;
+                st.next(NS);
+                at += at_step;
+                if (at == at_end) at -= NS * at_step;
+                return true;
+            };
+            uint32_t b0[4], b1[4], b2[4];
+            int n0 = load(b0), n1 = load(b1), n2 = load(b2);
+            for (;;) {
+                if (!put(b0, n0)) break;
+                n0 = load(b0);
+                if (!put(b1, n1)) break;
+                n1 = load(b1);
+                if (!put(b2, n2)) break;
+                n2 = load(b2);
             }
         }
     } else {

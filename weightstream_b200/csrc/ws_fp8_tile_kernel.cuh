@@ -263,28 +263,36 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
         // ------------------------------------------------------------ scale atoms (UE8M0)
         if constexpr (WUE) {
             const int r = tid - 256;
-            int s = 0, lap = 0;
+            const Ue8m0Scales sc(p.scales, p.scale_ld, p.k0, p.k, p.bk_shift);
+            int s = 0, lap = 0, lq = blockIdx.x, lk = 0;  // stage to fill; tile and slab to load
             uint32_t ph = 1;
-            bool ok = true;
-            for (int q = blockIdx.x; q < ntiles && ok; q += gridDim.x) {
-                const int row = q / p.ntok * 128 + r;
-                const bool real = row < p.n;
-                const uint8_t *src = static_cast<const uint8_t *>(p.scales) + ((p.row0 + (real ? row : 0)) >> p.bn_shift) * p.scale_ld;
-                for (int k = 0; k < KS; ++k) {
-                    uint32_t sc = 0;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int kk = k * 128 + j * 32;
-                        sc |= (real && kk < p.k ? (uint32_t)__ldg(src + ((p.k0 + kk) >> p.bk_shift)) : 0x7Fu) << (8 * j);
-                    }
-                    if (lap > 0) ok = mbar_wait(done0 + s * 8, ph, status);
-                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-                    *reinterpret_cast<uint32_t *>(smem + S.wsf + s * kBsAtomBytes + (r & 31) * 16 + (r >> 5) * 4) = sc;
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(full0 + s * 8);
-                    if (++s == NS) { s = 0; ++lap; ph ^= 1u; }
-                }
+            const uint8_t *row = nullptr;
+            auto load = [&](uint32_t &w) {
+                if (lq >= ntiles) return false;
+                if (lk == 0) row = sc.row((p.row0 + min(lq / p.ntok * 128 + r, p.n - 1)) >> p.bn_shift);
+                w = sc.slab(row, lk);
+                if (++lk == KS) { lk = 0; lq += gridDim.x; }
+                return true;
+            };
+            auto put = [&](uint32_t w, bool ok) {
+                if (ok && lap > 0) ok = mbar_wait(done0 + s * 8, ph, status);
+                if (!__all_sync(0xffffffffu, ok)) return false;
+                *reinterpret_cast<uint32_t *>(smem + S.wsf + s * kBsAtomBytes + (r & 31) * 16 + (r >> 5) * 4) = w;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full0 + s * 8);
+                if (++s == NS) { s = 0; ++lap; ph ^= 1u; }
+                return true;
+            };
+            uint32_t w0 = 0, w1 = 0, w2 = 0;  // three slabs' words in flight
+            bool h0 = load(w0), h1 = load(w1), h2 = load(w2);
+            for (;;) {
+                if (!put(w0, h0)) break;
+                h0 = load(w0);
+                if (!put(w1, h1)) break;
+                h1 = load(w1);
+                if (!put(w2, h2)) break;
+                h2 = load(w2);
             }
         }
     }
