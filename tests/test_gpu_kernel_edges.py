@@ -1,0 +1,136 @@
+"""GPU tests of the kernels at the sizes where they can go wrong: edges of tiles, remainders of K, the lines
+between two kernels, the smallest and largest of a kernel's range.  Against the CPU oracle on the same seeded bytes.
+
+Tolerance: every product of an E4M3 (FP4) weight, an E4M3 activation and their scales is exact, so what differs is
+the order of K additions in fp32.  Each is off by at most 2^-24 of a running sum of random signs that is no larger
+than the result's scale: relative L2 <= K * 2^-24, and never above the 5e-5 of the other parity tests.
+"""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    torch.cuda.set_device(0)
+    return torch.device("cuda:0")
+
+
+def check(got, want, k):
+    got, want = got.cpu().numpy().astype(np.float64), want.astype(np.float64)
+    err = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert err <= min(5e-5, k * 2.0 ** -24), err
+
+
+FP8 = [
+    # n, k, k0, K of the whole matrix, scale, rows
+    (1040, 640, 0, 640, "f32", (1, 2)),              # CUDA cores: K not a multiple of 512, rows not of 4
+    (1040, 512, 128, 1024, "f32", (1, 2)),           # a column window of a wider matrix, its rows not contiguous
+    (2064, 544, 32, 1280, "ue8m0", (1, 2)),          # K not a multiple of 128, 32-row scale blocks inside a group of rows
+    (4096, 6400, 0, 6400, "f32", (2,)),              # two rows, above the line to the tensor cores
+    (1040, 1024, 0, 1024, "f32", (3, 16, 17, 32, 33)),    # 8192 values per CTA: quantised there up to 16 rows
+    (1040, 1056, 0, 1056, "ue8m0", (3, 12, 13, 64, 65)),  # 33 scale columns: exponents collected byte by byte
+    (1040, 1056, 128, 1280, "ue8m0", (4, 40)),       # word loads with a K tail
+    (5120, 2304, 0, 2304, "ue8m0", (6, 19, 128)),    # two CTAs per SM, word loads, K halves of nine slabs
+    (1040, 768, 0, 768, "f32", (129, 225, 449)),     # prefill tiles: last row tile of 16, token tiles of 1 and up
+    (1040, 1056, 0, 1056, "ue8m0", (129, 449)),
+    (1040, 1056, 128, 1280, "ue8m0", (200,)),
+]
+
+
+@pytest.mark.parametrize("n,k,k0,kfull,scale,ms", FP8)
+def test_fp8_edges(dev, oracle, n, k, k0, kfull, scale, ms):
+    from weightstream_b200 import formats as F, synth, tp
+    b = 128 if scale == "f32" else 32
+    rng = np.random.default_rng(synth.config_seed(f"fp8-edges-{n}-{k}-{k0}", 0, 1))
+    w, sc = synth.fp8_weight(rng, n, kfull, scale=scale, bn=b, bk=b)
+    wd, sd = torch.from_numpy(w).to(dev), torch.from_numpy(np.ascontiguousarray(sc)).to(dev)
+    ep = tp.Endpoint(max_m=max(16, max(ms)), max_n=n)
+    try:
+        for m in ms:
+            x = F.bf16_bits_to_f32(synth.activations_bf16(rng, m, k))
+            want = oracle.fp8_gemv(w[:, k0:k0 + k], sc, x, bn=b, bk=b, k0=k0, threads=oracle.max_threads())
+            for act in (torch.bfloat16, torch.float32):  # (the values are bf16's: the same result)
+                out = ep.fp8_rowpar_gemm_allreduce(torch.from_numpy(x).to(dev).to(act), wd[:, k0:k0 + k], sd, block=(b, b), k0=k0)
+                ep.check()
+                check(out, want, k)
+    finally:
+        ep.close()
+
+
+@pytest.mark.parametrize("world", [2, 8])
+@pytest.mark.parametrize("m", [1, 3, 40])  # tokens in pairs, one left over; sums by owners from 32 rows on four ranks
+def test_fold_of_virtual_ranks(dev, oracle, world, m):
+    from weightstream_b200 import formats as F, synth, tp
+    n, k = 1040, 256  # K per rank; the last tile of rows is short
+    rng = np.random.default_rng(synth.config_seed("fold-edges", m, world))
+    w, sc = synth.fp8_weight(rng, n, world * k)
+    x = F.bf16_bits_to_f32(synth.activations_bf16(rng, m, world * k))
+    wd, sd, xd = torch.from_numpy(w).to(dev), torch.from_numpy(sc).to(dev), torch.from_numpy(x).to(dev)
+    cut = [slice(r * k, (r + 1) * k) for r in range(world)]
+    parts = [oracle.fp8_gemv(w[:, c], sc, np.ascontiguousarray(x[:, c]), bn=128, bk=128, k0=c.start) for c in cut]
+    grp = tp.LocalGroup(world, max_m=64, max_n=n)
+    try:
+        for _ in range(3):  # both banks of the exchange, and the first again
+            outs = grp.fp8_rowpar_gemm_allreduce([xd[:, c].contiguous() for c in cut], [wd[:, c] for c in cut], [sd] * world,
+                                                 k0s=[c.start for c in cut])
+            grp.check()
+            for o in outs:
+                assert torch.equal(o.view(torch.int32), outs[0].view(torch.int32))
+            check(outs[0], oracle.allreduce_fold(np.stack(parts)), world * k)
+    finally:
+        grp.close()
+
+
+MOE = [
+    # tokens, experts, top_k, n, k, first local expert, local experts
+    (8, 16, 2, 1040, 512, 0, 16),      # 16 routes: sorted and quantised in the main kernel; a whole pass per stage
+    (17, 16, 1, 1040, 512, 0, 16),     # 17: by the prep kernel
+    (2, 32, 6, 2048, 1280, 8, 8),      # few routes, most of them other ranks'
+    (21, 16, 6, 5120, 2304, 4, 8),     # K halves of nine slabs
+    (9, 8, 8, 1040, 2560, 0, 8),       # ten slabs; every expert takes every token
+    (85, 12, 6, 2048, 768, 0, 12),     # the most tokens the form takes; several passes an expert, the last not full
+]
+
+
+@pytest.mark.parametrize("m,experts,top_k,n,k,e0,local", MOE)
+def test_moe_edges(dev, oracle, m, experts, top_k, n, k, e0, local):
+    from weightstream_b200 import synth, tp
+    rng = np.random.default_rng(synth.config_seed(f"moe-edges-{m}-{n}-{k}", 0, 1))
+    w2, s2 = synth.fp4_experts(rng, experts, n, k)
+    ids, rw = synth.routes(rng, m, experts, top_k)
+    h = rng.standard_normal((m * top_k, k)).astype(np.float32)
+    w2, s2 = np.ascontiguousarray(w2[e0:e0 + local]), np.ascontiguousarray(s2[e0:e0 + local])
+    want = oracle.moe_down_combine(w2, s2, e0, h, ids, rw, threads=oracle.max_threads())
+    ep = tp.Endpoint(max_m=85, max_n=n)
+    try:
+        to = lambda a: torch.from_numpy(a).to(dev)
+        out = ep.moe_down_combine_allreduce(to(h), to(ids), to(rw), to(w2), to(s2), e0)
+        ep.check()
+        check(out, want, k * top_k)
+    finally:
+        ep.close()
+
+
+@pytest.mark.parametrize("vocab,k,m", [(16160, 2176, 12), (16160, 2176, 65)])
+def test_lm_head_logits_of_a_lone_rank(dev, oracle, vocab, k, m):
+    """Logits written by the tensor-core kernel itself, rows past the last whole tile, and their argmax."""
+    from weightstream_b200 import formats as F, synth, tp
+    rng = np.random.default_rng(synth.config_seed("head-edges", m, 1))
+    w, sc = synth.fp8_weight(rng, vocab, k)
+    x = F.bf16_bits_to_f32(synth.activations_bf16(rng, m, k))
+    want = oracle.fp8_gemv(w, sc, x, bn=128, bk=128, threads=oracle.max_threads())
+    grp = tp.LocalGroup(1, max_m=128, max_n=16, max_vocab=vocab)
+    try:
+        logits, amax = grp.lm_head_allgather_argmax([torch.from_numpy(x).to(dev)], [torch.from_numpy(w).to(dev)],
+                                                    [torch.from_numpy(sc).to(dev)], vocab=vocab, vocab_row0s=[0], row0s=[0])
+        grp.check()
+        check(logits[0], want, k)
+        assert torch.equal(amax[0].cpu().long(), logits[0].argmax(dim=1).cpu())
+    finally:
+        grp.close()
