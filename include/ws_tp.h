@@ -197,9 +197,10 @@ ws_status_t ws_act_quant_fp8(const void *x, int64_t ldx, int32_t x_dtype, int32_
  * the same number of bytes; 0 hands each leftover tile to one CTA whole. */
 ws_status_t ws_tp_set_split(ws_tp_t *tp, int32_t on);
 /* Kernel choice, also without counterpart in the reference.  0 (default) automatic: FP8 steps run
- * one or two activation rows on CUDA cores and three or more (and shards from 128 MB) on the
- * block-scaled tcgen05 kernel; the MoE step runs on its tcgen05 kernel when the shape fits it
- * (k <= 4096, one rank per launch), else on its CUDA-core decode form.  1: the mma.sync
+ * one or two activation rows on CUDA cores and three or more (two rows of shards from 24 MB, with
+ * UE8M0 scales from 8 MB; one row from 128 MB, lm_head from 32 MB) on the block-scaled tcgen05 kernel;
+ * the MoE step runs on its tcgen05 kernel when the shape fits it (k a multiple of 256 and at most 4096,
+ * one rank per launch), else on its CUDA-core decode form.  1: the mma.sync
  * formulations.  2: the tcgen05 kernels wherever the shape fits.  3: the CUDA-core kernels (MoE: the
  * decode form).  All choices give results within the same tolerance of the reference arithmetic;
  * ranks of one group must make the same choice. */

@@ -18,6 +18,8 @@
 //                     bytes as the weights, and what L2 can hand the SMs bound the step.)  An atom is
 //                     min(m, 32) rows of 16 bytes: byte (t & 31) * 16 + (t >> 5) * 4 + j = exponent of token
 //                     t, K block j.
+//                     INL: up to 8192 values per CTA its epilogue warps quantise them straight into shared memory
+//                     and there is no prep launch.
 //                     One thread copies the atoms into tensor memory (tcgen05.cp) and issues four MMAs per
 //                     slab (M=128, N=tokens, K=32): the activations' per-32 scales ride the MMA's scale
 //                     operand.
@@ -29,10 +31,10 @@
 //                     memory and is read back once.
 //
 // Measured on B200 and kept in mind above: every TMA or bulk copy costs its issuing thread 85-100 ns, but
-// one 3-D box for a stage's slabs was slower than a box each (128 rows 32.0 against 29.4 us); a slab's four MMAs, scale copy and share of the commit take the
-// tensor pipe 84 ns with N=16, 105 with 64 and 135 with 128, however few of the 128 rows are real (M=64 is
-// not available with block scaling); handing partial sums from one CTA to another through L2 (a split of K
-// across CTAs) costs 3-5 us, more than it saves on these shapes.
+// one 3-D box for a stage's slabs was slower than a box each (128 rows 32.0 against 29.4 us); a slab's four
+// MMAs, scale copy and share of the commit take the tensor pipe 84 ns with N=16, 105 with 64 and 135 with 128,
+// however few of the 128 rows are real (M=64 is not available with block scaling); handing partial sums from one
+// CTA to another through L2 (a split of K across CTAs) costs 3-5 us, more than it saves on these shapes.
 //
 // MMA rows past a tile's end are computed on whatever follows in shared memory and never read back.
 // Exchange and lm_head mode are those of the decode kernels (ws_fp8_kernel.cuh): tagged 64-bit
