@@ -397,6 +397,55 @@ __device__ __forceinline__ uint32_t order_key(float v) {
     return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);
 }
 
+// Sums, in rank order, of `count` (<= T) tokens' words of one output row: those of all ranks (R = WS_MAX_WORLD; src is
+// rank 0's) or one rank's (R = 1).  All of them are requested before the first is looked at, one memory round trip
+// instead of one per rank (three rows on eight ranks: 29 of a 50 us step), and requested again while one is missing:
+// waiting for each missing word in turn took a round trip per word (40 rows on eight ranks 198 us a step, 72 now; two
+// tokens at a time 87).  A rank that stays away is left to wait_word, which
+// gives up and records it.
+constexpr int kFoldTokens = 4, kFoldTries = 256;
+template <int T, int R>
+__device__ __forceinline__ void fold_words(const BsParams &p, const RankCtx &X, const uint64_t *src, size_t astride, uint32_t seq, int count, float (&sum)[T]) {
+    const int ranks = R == 1 ? 1 : p.world;
+    bool here = false;
+#pragma unroll 1
+    for (int tries = 0; tries < kFoldTries && !here; ++tries) {
+        if ((tries & 15) == 15 && *(volatile uint32_t *)X.status != 0u) break;  // the step has failed already
+        uint64_t w[R][T];
+        const uint64_t *at = src;
+#pragma unroll
+        for (int rr = 0; rr < R; ++rr) {
+            if (R == 1 || rr < ranks) {
+#pragma unroll
+                for (int i = 0; i < T; ++i) w[rr][i] = ld_word_sys(at + (int64_t)min(i, count - 1) * p.n);
+            }
+            at += astride;
+        }
+        here = true;
+#pragma unroll
+        for (int rr = 0; rr < R; ++rr)
+            if (R == 1 || rr < ranks) {
+#pragma unroll
+                for (int i = 0; i < T; ++i) {
+                    here = here && (uint32_t)(w[rr][i] >> 32) == seq;
+                    const float v = __uint_as_float((uint32_t)w[rr][i]);
+                    sum[i] = rr == 0 ? v : sum[i] + v;
+                }
+            }
+    }
+    if (here) return;
+#pragma unroll
+    for (int i = 0; i < T; ++i) {
+        sum[i] = 0.0f;
+        if (i < count)
+#pragma unroll 1
+            for (int rr = 0; rr < ranks; ++rr) {
+                const float v = wait_word(src + rr * astride + (int64_t)i * p.n, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
+                sum[i] = rr == 0 ? v : sum[i] + v;
+            }
+    }
+}
+
 // The exchange behind a CTA's finished tiles: fold its rows, in rank order, as the ranks' words arrive.  Thread
 // `et` of the epilogue (32 * ew of them) takes row et % 128 of each tile and the tokens whose columns it held.  A
 // function of its own, called when nothing else is left to do: inside the epilogue what it holds in registers was
@@ -413,97 +462,46 @@ static __device__ __noinline__ void bs_fold(const BsParams &p, int ew, int cp) {
     const int tbeg = max(upper ? half : 0, col0), tend = min(pair && !upper ? half : p.m, col0 + cp);
     if (warp < 2 || warp >= 2 + ew) return;
     const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
-    // fold the rows of the tiles this CTA finished, in rank order, as the ranks' words arrive
     const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
-    for (int t = t_lo; t <= t_hi; ++t) {
-        const int row = t * TR + rc;
-        if (rc >= TR || row >= p.n) continue;
-        // Fold by owners: the sums of tile t are formed on rank t % world only (in rank order, as
-        // everywhere) and travel back in that rank's own slot at every peer, so all ranks end up
-        // with the same bits and each partial sum crosses the links once instead of world - 1 times.
-        const int owner = p.owner_reduce ? t % p.world : X.rank;
-        if (!p.owner_reduce) {
-            // Two tokens at a time, the words of all their ranks requested before the first is looked at: one
-            // memory round trip instead of one per rank (three rows on eight ranks: 29 of a 50 us step); if one
-            // has not arrived yet they are waited for one by one.  Ranks are added in rank order.
-#pragma unroll 1
-            for (int tok0 = tbeg; tok0 < tend; tok0 += 2) {
-                const uint64_t *src = slots + (size_t)tok0 * p.n + row;
-                const int64_t second = tok0 + 1 < tend ? p.n : 0;
-                uint64_t w0[WS_MAX_WORLD], w1[WS_MAX_WORLD];
-                const uint64_t *at = src;
+    // Fold by owners (owner_reduce): the sums of tile t are formed on rank t % world only (in rank order, as
+    // everywhere) and travel back in that rank's own slot at every peer, so all ranks end up with the same bits and
+    // each partial sum crosses the links once instead of world - 1 times.  A rank folds its own tiles before it
+    // collects the others': the owners do not wait for one another.
+    for (int pass = p.owner_reduce ? 0 : 1; pass < 2; ++pass)
+        for (int t = t_lo; t <= t_hi; ++t) {
+            const int row = t * TR + rc;
+            if (rc >= TR || row >= p.n) continue;
+            const int owner = p.owner_reduce ? t % p.world : X.rank;
+            if (p.owner_reduce && (owner == X.rank) != (pass == 0)) continue;
+            const uint64_t *src = slots + (size_t)tbeg * p.n + row;
+            float *out = A.out + (size_t)tbeg * p.n + row;
+            if (owner != X.rank) {
+                for (int tok = tbeg; tok < tend; tok += 8, src += 8 * (int64_t)p.n, out += 8 * (int64_t)p.n) {
+                    float sum[8];
+                    fold_words<8, 1>(p, X, src + owner * astride, astride, seq, min(8, tend - tok), sum);
 #pragma unroll
-                for (int rr = 0; rr < WS_MAX_WORLD; ++rr) {
-                    if (rr < p.world) {
-                        w0[rr] = ld_word_sys(at);
-                        w1[rr] = ld_word_sys(at + second);
-                    }
-                    at += astride;
+                    for (int i = 0; i < 8; ++i)
+                        if (tok + i < tend) out[(int64_t)i * p.n] = sum[i];
                 }
-                bool here = true;
-                float sum0 = 0.0f, sum1 = 0.0f;
-#pragma unroll
-                for (int rr = 0; rr < WS_MAX_WORLD; ++rr)
-                    if (rr < p.world) {
-                        here = here && (uint32_t)(w0[rr] >> 32) == seq && (uint32_t)(w1[rr] >> 32) == seq;
-                        const float v0 = __uint_as_float((uint32_t)w0[rr]), v1 = __uint_as_float((uint32_t)w1[rr]);
-                        sum0 = rr == 0 ? v0 : sum0 + v0;
-                        sum1 = rr == 0 ? v1 : sum1 + v1;
-                    }
-                if (!here) {
-#pragma unroll 1
-                    for (int i = 0; i < 2; ++i) {
-                        float sum = 0.0f;
-#pragma unroll 1
-                        for (int rr = 0; rr < p.world; ++rr) {
-                            const float v = wait_word(src + rr * astride + i * second, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
-                            sum = rr == 0 ? v : sum + v;
-                        }
-                        if (i == 0) sum0 = sum;
-                        else sum1 = sum;
-                    }
-                }
-                float *out = A.out + (size_t)tok0 * p.n + row;
-                out[0] = sum0;
-                if (second) out[second] = sum1;
+                continue;
             }
-            continue;
-        }
-        // 16 tokens at a time: their words of one rank are all requested before the first is
-        // looked at (one memory round trip per batch, not per word); a word that has not
-        // arrived yet is then waited for on its own.  Ranks are added in rank order.
-        for (int tok0 = tbeg; tok0 < tend; tok0 += 16) {
-            float sum[16];
-            const int rr0 = owner == X.rank ? 0 : owner, rr1 = owner == X.rank ? p.world : owner + 1;
-            for (int rr = rr0; rr < rr1; ++rr) {
-                const uint64_t *src = slots + rr * astride + (size_t)tok0 * p.n + row;
-                uint64_t w[16];
+            for (int tok = tbeg; tok < tend; tok += kFoldTokens, src += kFoldTokens * (int64_t)p.n, out += kFoldTokens * (int64_t)p.n) {
+                float sum[kFoldTokens];
+                fold_words<kFoldTokens, WS_MAX_WORLD>(p, X, src, astride, seq, min(kFoldTokens, tend - tok), sum);
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (tok0 + i < tend) w[i] = ld_word_sys(src + (size_t)i * p.n);
+                for (int i = 0; i < kFoldTokens; ++i)
+                    if (tok + i < tend) out[(int64_t)i * p.n] = sum[i];
+                if (p.owner_reduce)
+                    for (int pr = 0; pr < p.world; ++pr) {
+                        if (pr == X.rank) continue;
+                        uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) +
+                                        ((size_t)bank * p.world + X.rank) * astride + (size_t)tok * p.n + row;
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (tok0 + i < tend) {
-                        const float v = (uint32_t)(w[i] >> 32) == seq
-                                            ? __uint_as_float((uint32_t)w[i])
-                                            : wait_word(src + (size_t)i * p.n, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
-                        sum[i] = rr == rr0 ? v : sum[i] + v;
+                        for (int i = 0; i < kFoldTokens; ++i)
+                            if (tok + i < tend) st_word_sys(dst + (int64_t)i * p.n, seq, sum[i]);
                     }
             }
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (tok0 + i < tend) A.out[(size_t)(tok0 + i) * p.n + row] = sum[i];
-            if (p.owner_reduce && owner == X.rank)
-                for (int pr = 0; pr < p.world; ++pr) {
-                    if (pr == X.rank) continue;
-                    uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) +
-                                    ((size_t)bank * p.world + X.rank) * astride + (size_t)tok0 * p.n + row;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (tok0 + i < tend) st_word_sys(dst + (size_t)i * p.n, seq, sum[i]);
-                }
         }
-    }
 }
 
 template <int MP, bool WUE, bool INL>
