@@ -678,7 +678,9 @@ static ws_status_t tile_step(ws_tp *tp, const ws_fp8_gemm_args_t &a, cudaStream_
     q.m = a.m; q.k = a.k; q.x_dtype = a.x_dtype; q.ks = u.ks; q.csize = 1; q.sl = 1; q.tokens = u.tokens;
     q.r[0].x = a.x; q.r[0].xq = tp->bs_work; q.r[0].ldx = a.ldx;
     tp->step++;
-    const int prep_blocks = (int)std::min<int64_t>(4 * tp->sm_count, ((int64_t)a.m * u.ks * 8 + kActPrepThreads - 1) / kActPrepThreads);
+    // as many prep blocks as fit the SMs: nothing of this step runs beside them (2000 rows of K 8192, four per SM 176 us
+    // a step, twelve 150)
+    const int prep_blocks = (int)std::min<int64_t>(12 * tp->sm_count, ((int64_t)a.m * u.ks * 8 + kActPrepThreads - 1) / kActPrepThreads);
     WS_CUDA(tp, cudaSetDevice(tp->device));
     s = launch(tp, act_prep_kernel, q, prep_blocks, 1, kActPrepThreads, 0, cs, tp->pdl != 0, false);
     const int grid = std::min(ncta, u.nrow * u.ntok);
