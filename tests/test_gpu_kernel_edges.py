@@ -63,6 +63,41 @@ def test_fp8_edges(dev, oracle, n, k, k0, kfull, scale, ms):
         ep.close()
 
 
+@pytest.mark.parametrize("k,ms", [
+    (512, (1, 2, 3, 40, 65, 128, 200)),  # all of a 64-row launch fits; two launches, three, four
+    (8192, (24, 70)),                    # only eight rows' copies fit
+])
+def test_scale_columns_that_slabs_straddle(dev, oracle, k, ms):
+    """fp32 scales on a K slice that starts inside a scale block: a 128-wide slab has two scale columns, which the
+    tensor-memory kernels cannot take, at any row count.  The device call, the host call and two virtual ranks."""
+    from weightstream_b200 import formats as F, synth, tp
+    n, k0 = 1040, 64
+    rng = np.random.default_rng(synth.config_seed("straddle", k, 1))
+    w, sc = synth.fp8_weight(rng, n, k0 + 2 * k + 64)  # whole blocks; the slice behind this one starts the same way
+    wd, sd = torch.from_numpy(w).to(dev), torch.from_numpy(sc).to(dev)
+    ep, grp = tp.Endpoint(max_m=max(ms), max_n=n), tp.LocalGroup(2, max_m=max(ms), max_n=n)
+    cuts = [slice(k0, k0 + k), slice(k0 + k, k0 + 2 * k)]
+    try:
+        for m in ms:
+            bits = synth.activations_bf16(rng, m, 2 * k)
+            x = F.bf16_bits_to_f32(bits)
+            xd = torch.from_numpy(x).to(dev).to(torch.bfloat16)
+            parts = [oracle.fp8_gemv(w[:, c], sc, np.ascontiguousarray(x[:, i * k:(i + 1) * k]), bn=128, bk=128, k0=c.start,
+                                     threads=oracle.max_threads()) for i, c in enumerate(cuts)]
+            out = ep.fp8_rowpar_gemm_allreduce(xd[:, :k], wd[:, cuts[0]], sd, k0=k0)
+            ep.check()
+            check(out, parts[0], k)
+            host = ep.fp8_rowpar_gemm_allreduce_host(bits[:, :k], wd[:, cuts[0]], sd, k0=k0)
+            assert np.array_equal(host.view(np.uint32), out.cpu().numpy().view(np.uint32))
+            outs = grp.fp8_rowpar_gemm_allreduce([xd[:, :k], xd[:, k:]], [wd[:, c] for c in cuts], [sd, sd], k0s=[c.start for c in cuts])
+            grp.check()
+            assert torch.equal(outs[0].view(torch.int32), outs[1].view(torch.int32))
+            check(outs[0], oracle.allreduce_fold(np.stack(parts)), 2 * k)
+    finally:
+        ep.close()
+        grp.close()
+
+
 @pytest.mark.parametrize("world", [2, 8])
 @pytest.mark.parametrize("m", [1, 3, 40])  # tokens in pairs, one left over; sums by owners from 32 rows on four ranks
 def test_fold_of_virtual_ranks(dev, oracle, world, m):

@@ -700,20 +700,41 @@ static bool bs_wanted(const ws_tp *t0, int mt, const ws_fp8_gemm_args_t &a, bool
     return mt >= 3 || (int64_t)a.n * a.k >= ((int64_t)(lm_head ? 32 : 128) << 20);
 }
 
-// Activation rows the next launch takes: up to 64 when their quantised copies fit in shared
-// memory beside at least three weight stages (the weights are then streamed once for all of
-// them), else 8.
-static int fp8_rows_per_launch(const ws_tp *t0, const ws_fp8_gemm_args_t &a, int ncta, int rem, bool lm_head = false) {
-    {   // the tensor-memory path streams the weights once for up to kBsMaxTokens rows
-        const int mt = std::min(rem, (int)kBsMaxTokens);
-        const int skb = (int)((a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
-        if (bs_wanted(t0, mt, a, lm_head) && bs_plan(a, mt, skb, ncta, false).ok) return mt;
+static const ws_fp8_gemm_args_t &rank_args(const ws_fp8_gemm_args_t *args, const ws_lm_head_args_t *lm, int i) { return lm ? lm[i].g : args[i]; }
+
+// Weight-scale columns that a rank's K slice touches, the most over the ranks.
+static int scale_columns(int n, const ws_fp8_gemm_args_t *args, const ws_lm_head_args_t *lm) {
+    int64_t skb = 1;
+    for (int i = 0; i < n; ++i) {
+        const ws_fp8_gemm_args_t &a = rank_args(args, lm, i);
+        skb = std::max<int64_t>(skb, (a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
     }
+    return (int)skb;
+}
+
+// The plan of the block-scaled tcgen05 path for mt rows of this step on all ranks; ok = false: they run on another
+// kernel.  How many rows a launch takes, the launch itself and the host-buffer call all ask here, so that no row count
+// chosen for one kernel reaches another.
+static BsPlan bs_choice(const ws_tp *t0, int n, const ws_fp8_gemm_args_t *args, const ws_lm_head_args_t *lm, int mt, int ncta) {
+    const ws_fp8_gemm_args_t &a0 = rank_args(args, lm, 0);
+    if (!bs_wanted(t0, mt, a0, lm != nullptr)) return BsPlan{};
+    for (int i = 0; i < n; ++i)  // fp32 scales: a slab of K reads one scale column
+        if (a0.scale_kind != WS_SCALE_UE8M0 && rank_args(args, lm, i).k0 % 128) return BsPlan{};
+    return bs_plan(a0, mt, scale_columns(n, args, lm), ncta, n == 1);  // CTA pairs need a cluster launch, virtual ranks a cooperative one
+}
+
+// Activation rows the next launch takes: up to kBsMaxTokens on the tcgen05 path, which streams the weights once for all
+// of them; else up to kFp8MaxRows when their quantised copies fit in shared memory beside at least three weight stages,
+// else 8.
+static int fp8_rows_per_launch(const ws_tp *t0, int n, const ws_fp8_gemm_args_t *args, const ws_lm_head_args_t *lm, int ncta, int rem) {
+    const int mt = std::min(rem, (int)kBsMaxTokens);
+    if (bs_choice(t0, n, args, lm, mt, ncta).ok) return mt;
     if (rem <= 8) return rem;
+    const ws_fp8_gemm_args_t &a = rank_args(args, lm, 0);
     const int kbox = (a.k + 127) / 128;
     const int Gm = a.n / kGroupRows / ncta;
-    const int skb = (int)((a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
-    for (int mp = std::min(64, (rem + 7) / 8 * 8); mp > 8; mp -= 8) {
+    const int skb = scale_columns(n, args, lm);
+    for (int mp = std::min((int)kFp8MaxRows, (rem + 7) / 8 * 8); mp > 8; mp -= 8) {
         const int m = std::min(rem, mp);
         const Fp8Smem fixed = fp8_smem_layout(0, kbox, mp, (Gm * kGroupRows) / a.block_n + 4, skb, m, (Gm + 2) * kGroupRows);
         if ((kSmemBudget - fixed.total) / (fp8_stage_boxes(kbox) * kBoxBytes) >= 3) return m;
@@ -822,26 +843,16 @@ static ws_status_t fp8_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t
                             int m0, int mt, void *const *streams, int ncta, bool same_device, bool last) {
     ws_tp *t0 = ranks[0];
     const ws_fp8_gemm_args_t &a0 = lm ? lm[0].g : args[0];
-    if (bs_wanted(t0, mt, a0, lm != nullptr)) {  // tensor-memory path whenever the shape fits it
-        int64_t skb_u = 1;
-        bool slabs_fit = true;
-        for (int i = 0; i < n; ++i) {
-            const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
-            skb_u = std::max<int64_t>(skb_u, (a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
-            slabs_fit &= a.scale_kind == WS_SCALE_UE8M0 || a.k0 % 128 == 0;  // a slab reads one scale column
-        }
-        const BsPlan u = bs_plan(a0, mt, (int)skb_u, ncta, n == 1);  // CTA pairs need a cluster launch, virtual ranks a cooperative one
-        if (u.ok && slabs_fit) return bs_step(ranks, n, args, lm, m0, mt, streams, same_device, u, (int)skb_u, last);
+    const int skb = scale_columns(n, args, lm);
+    {   // tensor-memory path whenever the shape fits it
+        const BsPlan u = bs_choice(t0, n, args, lm, mt, ncta);
+        if (u.ok) return bs_step(ranks, n, args, lm, m0, mt, streams, same_device, u, skb, last);
     }
     if (t0->kernel_sel != 1 && mt <= 2) {  // one or two activation rows: CUDA-core dot products
-        int64_t skb_u = 1;
-        for (int i = 0; i < n; ++i) {
-            const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
-            skb_u = std::max<int64_t>(skb_u, (a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
-        }
-        const GemvPlan u = gemv_plan(a0, mt, (int)skb_u, ncta);
-        if (u.ok) return gemv_step(ranks, n, args, lm, m0, mt, streams, ncta, same_device, u, (int)skb_u, last);
+        const GemvPlan u = gemv_plan(a0, mt, skb, ncta);
+        if (u.ok) return gemv_step(ranks, n, args, lm, m0, mt, streams, ncta, same_device, u, skb, last);
     }
+    if (mt > kFp8MaxRows) return fail(t0, WS_ERR_CAPACITY, "%d rows in one launch of a kernel for %d", mt, (int)kFp8MaxRows);
     Fp8Params p{};
     p.m = mt; p.n = a0.n; p.k = a0.k; p.x_dtype = a0.x_dtype; p.scale_kind = a0.scale_kind;
     p.bn = a0.block_n; p.bk = a0.block_k; p.world = t0->world;
@@ -855,13 +866,9 @@ static ws_status_t fp8_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t
     p.lay = t0->lay;
     const int kbox = (p.k + 127) / 128;
     const int Gm = p.n / kGroupRows / ncta;
-    int64_t skb = 1;
-    for (int i = 0; i < n; ++i) {
-        const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
-        skb = std::max<int64_t>(skb, (a.k0 + a.k - 1) / a.block_k - a.k0 / a.block_k + 1);
+    for (int i = 0; i < n; ++i)
         if (lm && lm[i].logits) p.gather_logits = 1;
-    }
-    p.skb = (int)skb;
+    p.skb = skb;
     // Ragged leftover rows pay off when a CTA holds only a few tiles (7168 rows: 3 tiles + 1 row instead
     // of 4 tiles on four CTAs); with many tiles per CTA one whole extra tile is within 2 % of balance.
     p.ragged = (t0->split && Gm < 8) ? 1 : 0;
@@ -896,7 +903,7 @@ static ws_status_t fp8_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t
         r.ctx = make_ctx(t);
         if (last) r.ctx.host_done = t->host_done_arm;
     }
-    zero_lone_shard(ranks, n, lm, m0, mt, streams);
+    if (ws_status_t s = zero_lone_shard(ranks, n, lm, m0, mt, streams); s != WS_OK) return s;
     // every endpoint advances by one step
     for (int i = 0; i < n; ++i) ranks[i]->step++;
     if (same_device) {
@@ -940,7 +947,7 @@ ws_status_t ws_fp8_rowpar_gemm_allreduce_group(ws_tp_t *const *ranks, int32_t n,
         if (u.ok) return tile_step(t0, args[0], static_cast<cudaStream_t>(streams ? streams[0] : nullptr), ncta, u);
     }
     for (int m0 = 0; m0 < args[0].m;) {
-        const int mt = fp8_rows_per_launch(t0, args[0], ncta, args[0].m - m0);
+        const int mt = fp8_rows_per_launch(t0, n, args, nullptr, ncta, args[0].m - m0);
         s = fp8_step(ranks, n, args, nullptr, m0, mt, streams, ncta, same, m0 + mt >= args[0].m);
         if (s != WS_OK) return s;
         m0 += mt;
@@ -979,7 +986,7 @@ ws_status_t ws_lm_head_allgather_argmax_group(ws_tp_t *const *ranks, int32_t n, 
     if (any_logits && args[0].vocab > t0->cfg.max_vocab)
         return fail(t0, WS_ERR_CAPACITY, "vocab=%d exceeds the endpoint's max_vocab=%d", args[0].vocab, t0->cfg.max_vocab);
     for (int m0 = 0; m0 < args[0].g.m;) {
-        const int mt = fp8_rows_per_launch(t0, args[0].g, ncta, args[0].g.m - m0, true);
+        const int mt = fp8_rows_per_launch(t0, n, nullptr, args, ncta, args[0].g.m - m0);
         s = fp8_step(ranks, n, nullptr, args, m0, mt, streams, ncta, same, m0 + mt >= args[0].g.m);
         if (s != WS_OK) return s;
         m0 += mt;
@@ -1464,11 +1471,9 @@ ws_status_t ws_fp8_rowpar_gemm_allreduce_host(ws_tp_t *tp, const ws_fp8_gemm_arg
         bool same = true;
         ws_tp *self[1] = {tp};
         if (validate_fp8(tp, a, false) == WS_OK && group_prelude(self, 1, &ncta, &same) == WS_OK) {
-            const int skb = (int)((dw->k0 + dw->k - 1) / dw->block_k - dw->k0 / dw->block_k + 1);
-            const int mt = fp8_rows_per_launch(tp, a, ncta, a.m);
+            const BsPlan u = bs_choice(tp, 1, &a, nullptr, fp8_rows_per_launch(tp, 1, &a, nullptr, ncta, a.m), ncta);
             direct = true;
-            const BsPlan u = bs_plan(a, mt, skb, ncta, true);
-            stage = !(bs_wanted(tp, mt, a) && u.ok && !u.inline_x);  // only the prep kernel reads every value just once
+            stage = !(u.ok && !u.inline_x);  // only the prep kernel reads every value just once
             if (!stage) a.x = pin;
         }
     }

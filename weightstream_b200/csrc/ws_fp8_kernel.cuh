@@ -27,6 +27,7 @@
 namespace ws {
 
 enum { kModeAllReduce = 0, kModeLmHead = 1 };
+constexpr int kFp8MaxRows = 8 * kConsumerWarps;  // activation rows of one launch of this kernel: eight per consumer warp
 
 struct Fp8RankArgs {
     const void *x;
