@@ -122,6 +122,30 @@ def test_fold_of_virtual_ranks(dev, oracle, world, m):
         grp.close()
 
 
+def test_step_behind_one_that_waits_longer_than_two_seconds(dev):
+    """A step that starts early (programmatic dependent launch) behind one whose peer stays away: the time its
+    predecessor spends waiting (wait_ms) is not its own.  Both take half an SM and the second has more stages to
+    fill than its ring holds, so its producer is at a stage that only the end of the first step can free."""
+    from weightstream_b200 import synth, tp
+    n, k = 7168, 4096
+    w, sc = synth.torch_fp8_weight(n, k, seed=3, device=dev)
+    x = torch.randn((1, k), device=dev)
+    ep, grp = tp.Endpoint(max_m=1, max_n=n), tp.LocalGroup(2, max_m=1, max_n=n, wait_ms=3000)
+    try:
+        want = ep.fp8_rowpar_gemm_allreduce(x, w, sc)
+        ep.check()
+        grp.eps[0].fp8_rowpar_gemm_allreduce(x, w, sc)  # rank 1 takes no step
+        got = ep.fp8_rowpar_gemm_allreduce(x, w, sc)
+        ep.check()
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+        with pytest.raises(tp.WsError) as ei:
+            grp.eps[0].check()
+        assert ei.value.status == tp._lib.WS_ERR_TIMEOUT
+    finally:
+        ep.close()
+        grp.close()
+
+
 MOE = [
     # tokens, experts, top_k, n, k, first local expert, local experts
     (8, 16, 2, 1040, 512, 0, 16),      # 16 routes: sorted and quantised in the main kernel; a whole pass per stage

@@ -158,6 +158,11 @@ struct RingPos {
     }
 };
 
+// Before the first wait on a stage that has to be refilled, by a warp that streams ahead of its kernel's predecessor.
+// Whoever frees the stage waits for the predecessor, which may wait for a late peer as long as the caller's wait_ms
+// says: that is not the two seconds that mbar_wait allows this step's own work.
+__device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // 2-D TMA tile load global -> shared, completion on an mbarrier (no multicast).
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int32_t x,
                                             int32_t y, uint32_t bar) {

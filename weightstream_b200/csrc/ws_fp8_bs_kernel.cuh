@@ -729,6 +729,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             };
             auto put = [&](const uint32_t (&b)[4], int nsl) {
                 bool ok = nsl > 0;
+                if (item == NS) wait_predecessor();
                 if (ok && item >= NS) ok = mbar_wait(done0 + st.s * 8, st.ph ^ 1u, X.status);
                 if (!__all_sync(0xffffffffu, ok)) return false;
 #pragma unroll

@@ -83,6 +83,7 @@ __device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
         RingPos rp;
         for (int it = 0; it < items; ++it, rp.next(NS)) {
             const int s = rp.s, r0 = it * R, nr = min(R, rows - r0);
+            if (it == NS) wait_predecessor();
             if (!mbar_wait(empty0 + s * 8, rp.ph ^ 1u, X.status)) return;  // a wait gave up: stop streaming
             if (lane == 0) mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)(nr * p.k));
             __syncwarp();

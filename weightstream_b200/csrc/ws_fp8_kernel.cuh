@@ -278,12 +278,14 @@ __device__ __forceinline__ void fp8_rowpar_kernel_body(const Fp8Params &p) {
     if (warp == CW) {
         // ------------------------------------------------------------ TMA producer warp
         RingPos rp;
+        int item = 0;
         for (int t = 0; t < ntile; ++t) {
             const int r0 = trow(t), cnt = tcnt(t);
             const int pad = tpad(cnt), cols = p.stage_bytes / (pad * 128);  // box columns one stage holds
             for (int b0 = 0; b0 < kbox; b0 += cols) {
                 const int nb = min(cols, kbox - b0);
                 const int s = rp.s;
+                if (item++ == NS) wait_predecessor();
                 if (!mbar_wait(empty0 + s * 8, rp.ph ^ 1u, X.status)) return;  // a wait gave up: stop streaming
                 if (lane == 0) mbar_arrive_expect_tx(full0 + s * 8, (uint32_t)(nb * cnt * 128));
                 __syncwarp();

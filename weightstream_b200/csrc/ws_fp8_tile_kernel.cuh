@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
                 return true;
             };
             auto put = [&](uint32_t w, bool ok) {
+                if (lap == 1 && s == 0) wait_predecessor();
                 if (ok && lap > 0) ok = mbar_wait(done0 + s * 8, ph, status);
                 if (!__all_sync(0xffffffffu, ok)) return false;
                 *reinterpret_cast<uint32_t *>(smem + S.wsf + s * kBsAtomBytes + (r & 31) * 16 + (r >> 5) * 4) = w;
