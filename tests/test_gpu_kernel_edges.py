@@ -146,6 +146,27 @@ def test_step_behind_one_that_waits_longer_than_two_seconds(dev):
         grp.close()
 
 
+def test_first_steps_on_a_side_stream_behind_a_busy_default_stream(dev):
+    """What an endpoint allocates on its first step is not touched later by work on another stream than the step's."""
+    from weightstream_b200 import synth, tp
+    n, k, m = 1040, 8192, 40
+    w, sc = synth.torch_fp8_weight(n, k, seed=5, device=dev)
+    x = torch.randn((m, k), device=dev).to(torch.bfloat16)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(8):
+        ep = tp.Endpoint(max_m=m, max_n=n)
+        try:
+            torch.cuda._sleep(3_000_000)  # ~1.5 ms on the default stream
+            with torch.cuda.stream(side):
+                outs = [ep.fp8_rowpar_gemm_allreduce(x, w, sc) for _ in range(200)]
+            torch.cuda.synchronize()
+            ep.check()
+            assert all(torch.equal(o.view(torch.int32), outs[-1].view(torch.int32)) for o in outs)
+        finally:
+            ep.close()
+
+
 MOE = [
     # tokens, experts, top_k, n, k, first local expert, local experts
     (8, 16, 2, 1040, 512, 0, 16),      # 16 routes: sorted and quantised in the main kernel; a whole pass per stage

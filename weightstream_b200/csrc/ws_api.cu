@@ -539,8 +539,9 @@ static ws_status_t ensure_bs_scratch(ws_tp *tp, size_t bytes) {
         if (tp->bs_work) cudaFree(tp->bs_work);
         tp->bs_work = nullptr;
         tp->bs_work_bytes = 0;
+        // not cleared: a step's prep kernel writes every byte whose result is used, and a clear on another stream than
+        // the step's could come after it
         WS_CUDA(tp, cudaMalloc(&tp->bs_work, bytes));
-        WS_CUDA(tp, cudaMemset(tp->bs_work, 0, bytes));
         tp->bs_work_bytes = bytes;
     }
     return WS_OK;
