@@ -40,6 +40,7 @@ FP8 = [
     (1040, 768, 0, 768, "f32", (129, 225, 449)),     # prefill tiles: last row tile of 16, token tiles of 1 and up
     (1040, 1056, 0, 1056, "ue8m0", (129, 449)),
     (1040, 1056, 128, 1280, "ue8m0", (200,)),
+    (272, 512, 0, 512, "f32", (4096, 4097)),         # prefill in one launch, and in two
 ]
 
 
@@ -165,6 +166,50 @@ def test_first_steps_on_a_side_stream_behind_a_busy_default_stream(dev):
             assert all(torch.equal(o.view(torch.int32), outs[-1].view(torch.int32)) for o in outs)
         finally:
             ep.close()
+
+
+@pytest.mark.parametrize("scale", ["f32", "ue8m0"])
+def test_captured_steps_outlive_the_growth_of_the_scratch(dev, scale):
+    """A caller's graphs of a decode step, a prefill and a MoE step, captured on an endpoint that has run nothing yet,
+    replay the same bits after a longer prefill and a larger K have made the endpoint's scratch grow."""
+    from weightstream_b200 import synth, tp
+    n, k, kw, top_k = 1040, 1024, 4096, 4
+    b = 128 if scale == "f32" else 32
+    rng = np.random.default_rng(11)
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+    w, sc = map(to, synth.fp8_weight(rng, n, k, scale=scale, bn=b, bk=b))
+    wide, wsc = map(to, synth.fp8_weight(rng, n, kw, scale=scale, bn=b, bk=b))
+    w2, s2 = map(to, synth.fp4_experts(rng, 16, n, k))
+    ids, rw = map(to, synth.routes(rng, 20, 16, top_k))
+    h = torch.randn((20 * top_k, k), device=dev)
+    x = torch.randn((3000, kw), device=dev)
+    steps = [lambda ep: ep.fp8_rowpar_gemm_allreduce(x[:40, :k], w, sc, block=(b, b)),
+             lambda ep: ep.fp8_rowpar_gemm_allreduce(x[:300, :k], w, sc, block=(b, b)),
+             lambda ep: ep.moe_down_combine_allreduce(h, ids, rw, w2, s2, 0)]
+    ep, other = (tp.Endpoint(max_m=3000, max_n=n) for _ in range(2))
+    graphs = []
+    try:
+        want = [f(other) for f in steps]
+        other.check()
+        for f in steps:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                out = f(ep)
+            graphs.append((g, out))
+        ep.fp8_rowpar_gemm_allreduce(x[:, :k], w, sc, block=(b, b))
+        ep.fp8_rowpar_gemm_allreduce(x[:100], wide, wsc, block=(b, b))
+        ep.check()
+        fill = torch.full((64 << 20,), 0x55, dtype=torch.uint8, device=dev)  # what was given back is written by others
+        for _ in range(2):
+            for (g, out), ref in zip(graphs, want):
+                out.zero_()
+                g.replay()
+                ep.check()
+                assert torch.equal(out.view(torch.int32), ref.view(torch.int32))
+        assert bool((fill == 0x55).all())
+    finally:
+        ep.close()
+        other.close()
 
 
 MOE = [

@@ -59,15 +59,17 @@ struct ws_tp {
     uint64_t *pin_done = nullptr;       // pinned: {1, device status} once a host-buffer call's last kernel has finished
     uint64_t *host_done_arm = nullptr;  // set while a host-buffer call enqueues: its last kernel reports to this word
     uint64_t hgraph_clock = 0;
-    // MoE decode step: routes quantised once per step, pass table, large-m accumulators
-    uint8_t *moe_work = nullptr;
-    size_t moe_work_bytes = 0;
-    float *moe_acc = nullptr;
-    size_t moe_acc_bytes = 0;
-    // block-scaled tcgen05 step: the step's quantised activations [64][k] and their scale atoms
+    // Device scratch.  A buffer that a step outgrows stays allocated until the endpoint goes (`outgrown`): a CUDA
+    // graph of the caller's, or one of the host-buffer calls', may hold its address.
+    struct Scratch {
+        uint8_t *p = nullptr;
+        size_t bytes = 0;
+    };
+    Scratch moe_work;  // MoE step: pass table, the routes' quantised activations
+    Scratch moe_acc;   // CUDA-core MoE step: accumulators that do not fit shared memory
+    Scratch bs_work;   // tcgen05 FP8 step: quantised activations and their scale atoms
+    std::vector<void *> outgrown;
     int moe_bs = 1;  // 0: the MoE step stays on the CUDA-core decode form
-    uint8_t *bs_work = nullptr;
-    size_t bs_work_bytes = 0;
     std::string err;
 };
 
@@ -332,9 +334,9 @@ ws_status_t ws_tp_destroy(ws_tp_t *tp) {
     for (auto &g : tp->hgraphs)
         if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
     if (tp->pin_done) cudaFreeHost(tp->pin_done);
-    if (tp->moe_work) cudaFree(tp->moe_work);
-    if (tp->moe_acc) cudaFree(tp->moe_acc);
-    if (tp->bs_work) cudaFree(tp->bs_work);
+    for (const ws_tp::Scratch *s : {&tp->moe_work, &tp->moe_acc, &tp->bs_work})
+        if (s->p) cudaFree(s->p);
+    for (void *old : tp->outgrown) cudaFree(old);
     if (tp->sym) cudaFree(tp->sym);
     if (tp->counters) cudaFree(tp->counters);
     delete tp;
@@ -529,21 +531,25 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     return u;
 }
 
-static ws_status_t ensure_bs_scratch(ws_tp *tp, size_t bytes) {
+// At least `bytes` of scratch: just that at first (below 2 MB the driver serves it from memory it has mapped already,
+// ~10 us; a block of 2 MB of its own cost the first step 1 to 30 ms), then at least twice what is outgrown, so that all
+// that a scratch has outgrown is together no more than what it holds.  A first step may be inside a stream capture (the caller's, or the host-buffer call's own): allocating
+// is no part of what is captured.  Not cleared: what a step reads of it that step's prep kernel has written, and a clear
+// on another stream than the step's could come after it.
+static ws_status_t ensure_scratch(ws_tp *tp, ws_tp::Scratch &s, size_t bytes) {
     WS_CUDA(tp, cudaSetDevice(tp->device));
-    if (bytes > tp->bs_work_bytes) {
-        // graphs of earlier host-buffer calls hold the old buffer's address: they go with it
-        for (auto &g : tp->hgraphs)
-            if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
-        tp->hgraphs.clear();
-        if (tp->bs_work) cudaFree(tp->bs_work);
-        tp->bs_work = nullptr;
-        tp->bs_work_bytes = 0;
-        // not cleared: a step's prep kernel writes every byte whose result is used, and a clear on another stream than
-        // the step's could come after it
-        WS_CUDA(tp, cudaMalloc(&tp->bs_work, bytes));
-        tp->bs_work_bytes = bytes;
-    }
+    if (bytes <= s.bytes) return WS_OK;
+    const size_t cap = std::max(bytes, 2 * s.bytes);
+    void *p = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    WS_CUDA(tp, cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaMalloc(&p, cap);
+    WS_CUDA(tp, cudaThreadExchangeStreamCaptureMode(&mode));
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    WS_CUDA(tp, e);
+    if (s.p) tp->outgrown.push_back(s.p);
+    s.p = static_cast<uint8_t *>(p);
+    s.bytes = cap;
     return WS_OK;
 }
 
@@ -585,7 +591,7 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     for (int i = 0; i < n; ++i) {
         ws_tp *t = ranks[i];
         const ws_fp8_gemm_args_t &a = lm ? lm[i].g : args[i];
-        ws_status_t s = u.inline_x ? WS_OK : ensure_bs_scratch(t, xq_bytes);
+        ws_status_t s = u.inline_x ? WS_OK : ensure_scratch(t, t->bs_work, xq_bytes);
         if (s == WS_OK) s = make_tmap(t, &p.tmap_w[i], a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, (uint32_t)u.tile_rows);
         if (s != WS_OK) { t0->err = t->err; return s; }
         Fp8RankArgs &r = p.r[i];
@@ -599,7 +605,7 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         r.vocab_row0 = lm ? lm[i].vocab_row0 : 0;
         r.ctx = make_ctx(t);
         if (last) r.ctx.host_done = t->host_done_arm;
-        p.xq[i] = q.r[i].xq = t->bs_work;
+        p.xq[i] = q.r[i].xq = t->bs_work.p;
         q.r[i].x = r.x;
         q.r[i].ldx = a.ldx;
     }
@@ -635,7 +641,10 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     return s;
 }
 
-// Plan of the tile kernel: one launch over all activation rows of a lone rank's step.
+// Activation rows one launch of the tile kernel takes: what bounds the scratch of a step (133 * k bytes per 128 rows),
+// at seven waves and more of CTAs a launch at 7168 outputs.
+constexpr int kTileMaxRows = 4096;
+// Plan of the tile kernel: one launch over up to kTileMaxRows activation rows of a lone rank's step.
 struct TilePlan {
     bool ok, wue;
     int ks, tokens, ntok, nrow, nstages, x_pitch;
@@ -663,21 +672,21 @@ static TilePlan tile_plan(const ws_fp8_gemm_args_t &a, int ncta) {
     return u;
 }
 
-static ws_status_t tile_step(ws_tp *tp, const ws_fp8_gemm_args_t &a, cudaStream_t cs, int ncta, const TilePlan &u) {
+static ws_status_t tile_step(ws_tp *tp, const ws_fp8_gemm_args_t &a, cudaStream_t cs, int ncta, const TilePlan &u, bool last) {
     TileParams p{};
     p.m = a.m; p.n = a.n; p.k = a.k; p.ks = u.ks; p.tokens = u.tokens; p.ntok = u.ntok; p.nrow = u.nrow; p.nstages = u.nstages; p.x_pitch = u.x_pitch;
     for (p.bk_shift = 0; (1 << p.bk_shift) < a.block_k; ++p.bk_shift) {}
     for (p.bn_shift = 0; (1 << p.bn_shift) < a.block_n; ++p.bn_shift) {}
     p.scales = a.scales; p.scale_ld = a.scale_ld; p.row0 = a.row0; p.k0 = a.k0; p.out = a.out;
-    ws_status_t s = ensure_bs_scratch(tp, (size_t)u.ntok * u.ks * (u.tokens * 128 + bs_atom_bytes(u.tokens)));
+    ws_status_t s = ensure_scratch(tp, tp->bs_work, (size_t)u.ntok * u.ks * (u.tokens * 128 + bs_atom_bytes(u.tokens)));
     if (s == WS_OK) s = make_tmap(tp, &p.tmap_w, a.w, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldw, 128);
     if (s != WS_OK) return s;
-    p.xq = tp->bs_work;
+    p.xq = tp->bs_work.p;
     p.ctx = make_ctx(tp);
-    p.ctx.host_done = tp->host_done_arm;
+    if (last) p.ctx.host_done = tp->host_done_arm;
     ActPrepParams q{};
     q.m = a.m; q.k = a.k; q.x_dtype = a.x_dtype; q.ks = u.ks; q.csize = 1; q.sl = 1; q.tokens = u.tokens;
-    q.r[0].x = a.x; q.r[0].xq = tp->bs_work; q.r[0].ldx = a.ldx;
+    q.r[0].x = a.x; q.r[0].xq = tp->bs_work.p; q.r[0].ldx = a.ldx;
     tp->step++;
     // as many prep blocks as fit the SMs: nothing of this step runs beside them (2000 rows of K 8192, four per SM 176 us
     // a step, twelve 150)
@@ -944,8 +953,21 @@ ws_status_t ws_fp8_rowpar_gemm_allreduce_group(ws_tp_t *const *ranks, int32_t n,
         return fail(t0, WS_ERR_CAPACITY, "m=%d n=%d exceed the endpoint's max_m=%d max_n=%d", args[0].m, args[0].n,
                     t0->cfg.max_m, t0->cfg.max_n);
     if (n == 1 && t0->world == 1 && args[0].m > kBsMaxTokens && bs_wanted(t0, kBsMaxTokens, args[0])) {  // prefill on a lone rank
-        const TilePlan u = tile_plan(args[0], ncta);
-        if (u.ok) return tile_step(t0, args[0], static_cast<cudaStream_t>(streams ? streams[0] : nullptr), ncta, u);
+        const int rows = (args[0].m + (args[0].m - 1) / kTileMaxRows) / ((args[0].m - 1) / kTileMaxRows + 1);  // equal launches
+        ws_fp8_gemm_args_t a = args[0];
+        a.m = std::min(a.m, rows);
+        TilePlan u = tile_plan(a, ncta);
+        if (u.ok) {
+            for (int m0 = 0; m0 < args[0].m && s == WS_OK; m0 += a.m) {
+                a = args[0];
+                a.x = static_cast<const char *>(a.x) + (size_t)m0 * a.ldx * (a.x_dtype == WS_ACT_BF16 ? 2 : 4);
+                a.out += (size_t)m0 * a.n;
+                a.m = std::min(rows, args[0].m - m0);
+                if (m0 > 0) u = tile_plan(a, ncta);
+                s = tile_step(t0, a, static_cast<cudaStream_t>(streams ? streams[0] : nullptr), ncta, u, m0 + a.m >= args[0].m);
+            }
+            return s;
+        }
     }
     for (int m0 = 0; m0 < args[0].m;) {
         const int mt = fp8_rows_per_launch(t0, n, args, nullptr, ncta, args[0].m - m0);
@@ -1003,25 +1025,6 @@ ws_status_t ws_lm_head_allgather_argmax(ws_tp_t *tp, const ws_lm_head_args_t *ar
 
 
 // ------------------------------------------------------------------------------ MoE down
-static ws_status_t ensure_moe_scratch(ws_tp *tp, size_t work_bytes, size_t acc_bytes) {
-    WS_CUDA(tp, cudaSetDevice(tp->device));
-    if (work_bytes > tp->moe_work_bytes) {
-        if (tp->moe_work) cudaFree(tp->moe_work);
-        tp->moe_work = nullptr;
-        tp->moe_work_bytes = 0;
-        WS_CUDA(tp, cudaMalloc(&tp->moe_work, work_bytes));
-        tp->moe_work_bytes = work_bytes;
-    }
-    if (acc_bytes > tp->moe_acc_bytes) {
-        if (tp->moe_acc) cudaFree(tp->moe_acc);
-        tp->moe_acc = nullptr;
-        tp->moe_acc_bytes = 0;
-        WS_CUDA(tp, cudaMalloc(&tp->moe_acc, acc_bytes));
-        tp->moe_acc_bytes = acc_bytes;
-    }
-    return WS_OK;
-}
-
 // Plan of the MoE step on the tcgen05 path; ok = false when the shape does not fit it (CTA pairs split K
 // in halves of at most 16 slabs, a pair's rows are one MMA tile, the per-token sums live in shared memory).
 struct MoeBsPlan {
@@ -1081,16 +1084,16 @@ static ws_status_t moe_bs_step(ws_tp *const *ranks, int n, const ws_moe_down_arg
     for (int i = 0; i < n; ++i) {
         ws_tp *t = ranks[i];
         const ws_moe_down_args_t &a = args[i];
-        ws_status_t s = u.inline_x ? WS_OK : ensure_moe_scratch(t, (size_t)W.total, 0);
+        ws_status_t s = u.inline_x ? WS_OK : ensure_scratch(t, t->moe_work, (size_t)W.total);
         if (s == WS_OK) s = make_tmap_fp4(t, &p.tmap_w[0], a.w2, (uint64_t)a.e_len, (uint64_t)a.n, (uint64_t)a.k, (uint32_t)u.tile_rows, (uint32_t)u.slabs_per_stage);
         if (s == WS_OK) s = make_tmap_fp4(t, &p.tmap_t[0], a.w2, (uint64_t)a.e_len, (uint64_t)a.n, (uint64_t)a.k, (uint32_t)u.tile_rows, 1);
         if (s != WS_OK) { t0->err = t->err; return s; }
         MoeBsRank &r = p.r[0];
-        r.s2 = a.s2; r.work = t->moe_work; r.out = a.out; r.e_start = a.e_start; r.e_len = a.e_len;
+        r.s2 = a.s2; r.work = t->moe_work.p; r.out = a.out; r.e_start = a.e_start; r.e_len = a.e_len;
         r.h = a.h; r.route_ids = a.route_ids; r.route_w = a.route_w; r.ldh = a.ldh;
         r.ctx = make_ctx(t);
         MoePrepRank &pr = q.r[0];
-        pr.h = a.h; pr.route_ids = a.route_ids; pr.route_w = a.route_w; pr.work = t->moe_work;
+        pr.h = a.h; pr.route_ids = a.route_ids; pr.route_w = a.route_w; pr.work = t->moe_work.p;
         pr.ldh = a.ldh; pr.e_start = a.e_start; pr.e_len = a.e_len;
         WS_CUDA(t, cudaSetDevice(t->device));
         cudaStream_t cs = static_cast<cudaStream_t>(streams ? streams[i] : nullptr);
@@ -1149,7 +1152,8 @@ static ws_status_t moe_gemv_step(ws_tp *const *ranks, int n, const ws_moe_down_a
     const size_t acc_bytes = p.acc_global ? (size_t)nslice * p.m * p.n * 4 : 0;
     for (int i = 0; i < n; ++i) {
         const ws_moe_down_args_t &a = args[i];
-        ws_status_t s = ensure_moe_scratch(ranks[i], work_bytes, acc_bytes);
+        ws_status_t s = ensure_scratch(ranks[i], ranks[i]->moe_work, work_bytes);
+        if (s == WS_OK && acc_bytes) s = ensure_scratch(ranks[i], ranks[i]->moe_acc, acc_bytes);
         if (s != WS_OK) { t0->err = ranks[i]->err; return s; }
         for (int b = 0; b < 2; ++b) {
             s = make_tmap(ranks[i], &p.tmap[i][b], a.w2, (uint64_t)a.e_len * a.n, (uint64_t)kbytes, (uint64_t)kbytes,
@@ -1157,11 +1161,11 @@ static ws_status_t moe_gemv_step(ws_tp *const *ranks, int n, const ws_moe_down_a
             if (s != WS_OK) { t0->err = ranks[i]->err; return s; }
         }
         MoeGemvRank &r = p.r[i];
-        r.s2 = a.s2; r.work = ranks[i]->moe_work; r.out = a.out; r.acc_g = ranks[i]->moe_acc;
+        r.s2 = a.s2; r.work = ranks[i]->moe_work.p; r.out = a.out; r.acc_g = reinterpret_cast<float *>(ranks[i]->moe_acc.p);
         r.e_start = a.e_start; r.e_len = a.e_len;
         r.ctx = make_ctx(ranks[i]);
         MoePrepRank &pr = q.r[i];
-        pr.h = a.h; pr.route_ids = a.route_ids; pr.route_w = a.route_w; pr.work = ranks[i]->moe_work;
+        pr.h = a.h; pr.route_ids = a.route_ids; pr.route_w = a.route_w; pr.work = ranks[i]->moe_work.p;
         pr.ldh = a.ldh; pr.e_start = a.e_start; pr.e_len = a.e_len;
     }
     for (int i = 0; i < n; ++i) ranks[i]->step++;
