@@ -212,6 +212,29 @@ def test_captured_steps_outlive_the_growth_of_the_scratch(dev, scale):
         other.close()
 
 
+@pytest.mark.parametrize("m", [1, 2, 3])
+def test_infinite_weight_scale(dev, oracle, m):
+    """Rows whose first scale is infinite are infinite, the others untouched; K leaves lanes without a chunk."""
+    from weightstream_b200 import tp
+    n, k = 1040, 544
+    rng = np.random.default_rng(9)
+    w = rng.integers(0x30, 0x48, (n, k), dtype=np.uint8)  # positive, 0.5 to 3.75
+    sc = rng.uniform(0.5, 1.0, (9, 5)).astype(np.float32)
+    sc[2, 0] = np.inf
+    x = rng.uniform(1.0, 2.0, (m, k)).astype(np.float32)
+    want = oracle.fp8_gemv(w, sc, x, bn=128, bk=128)
+    ep = tp.Endpoint(max_m=m, max_n=n)
+    try:
+        out = ep.fp8_rowpar_gemm_allreduce(*(torch.from_numpy(a).to(dev) for a in (x, w, sc)))
+        ep.check()
+        hit = np.zeros(n, bool)
+        hit[256:384] = True
+        assert (want[:, hit] == np.inf).all() and (out.cpu().numpy()[:, hit] == np.inf).all()
+        check(out[:, torch.from_numpy(~hit).to(dev)], want[:, ~hit], k)
+    finally:
+        ep.close()
+
+
 MOE = [
     # tokens, experts, top_k, n, k, first local expert, local experts
     (8, 16, 2, 1040, 512, 0, 16),      # 16 routes: sorted and quantised in the main kernel; a whole pass per stage

@@ -153,7 +153,8 @@ __device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
     const uint32_t seq = solo ? 0u : step_begin(X);
 
     // byte offset of each chunk inside a row; lanes past the end of K read the row's first chunk and multiply
-    // it by zero (a NaN there is in the row's sum anyway)
+    // it by zero activations and a zero factor (a NaN weight there is in the row's sum anyway; an infinite scale
+    // must not become one)
     uint32_t off[C];
 #pragma unroll
     for (int i = 0; i < C; ++i) off[i] = live[i] ? (uint32_t)(((slice * C + i) * 32 + lane) * 16) : 0u;
@@ -180,7 +181,7 @@ __device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
                     for (int i = 0; i < C; ++i) {
                         const float sw = sw_s[b * p.skb + swc[i]];
 #pragma unroll
-                        for (int t = 0; t < GT; ++t) f[t][i] = sa[t][i] * sw;
+                        for (int t = 0; t < GT; ++t) f[t][i] = live[i] ? sa[t][i] * sw : 0.0f;
                     }
                 }
                 float acc[GT][4];
