@@ -99,6 +99,32 @@ def test_scale_columns_that_slabs_straddle(dev, oracle, k, ms):
         grp.close()
 
 
+@pytest.mark.parametrize("m", [3, 40, 100, 200])
+def test_ue8m0_sums_against_64_bits(dev, m):
+    """UE8M0 scales spread over 2^24, so that a few blocks carry a sum and every later addition is truncated where the
+    tensor cores make it.  Bound: they make eight of an accumulator's additions (two slabs), each off by less than
+    2^-23 of it; the rest (at most 32 of K 8192) are rounded, errors of random sign: 8 * 2^-23 + sqrt(32) * 2^-24."""
+    from weightstream_b200 import synth, tp
+    n, k = 1040, 8192
+    rng = np.random.default_rng(m)
+    w, sc = synth.fp8_weight(rng, n, k, scale="ue8m0", bn=32, bk=32)
+    sc = rng.integers(103, 128, sc.shape, dtype=np.uint8)
+    wd, sd = torch.from_numpy(w).to(dev), torch.from_numpy(sc).to(dev)
+    x = torch.randn((m, k), device=dev)
+    q, e = tp.act_quant_fp8(x)
+    xq = q.view(torch.float8_e4m3fn).double().view(m, -1, 32) * torch.exp2(e.double() - 127).unsqueeze(2)
+    ws = torch.exp2(sd.double() - 127).repeat_interleave(32, 0)[:n].repeat_interleave(32, 1)
+    want = xq.view(m, k) @ (wd.view(torch.float8_e4m3fn).double() * ws).T
+    ep = tp.Endpoint(max_m=m, max_n=n)
+    try:
+        out = ep.fp8_rowpar_gemm_allreduce(x, wd, sd, block=(32, 32))
+        ep.check()
+        err = float((out.double() - want).norm() / want.norm())
+        assert err <= 8 * 2.0 ** -23 + 32 ** 0.5 * 2.0 ** -24, err
+    finally:
+        ep.close()
+
+
 @pytest.mark.parametrize("world", [2, 8])
 @pytest.mark.parametrize("m", [1, 3, 40])  # tokens in pairs, one left over; sums by owners from 32 rows on four ranks
 def test_fold_of_virtual_ranks(dev, oracle, world, m):

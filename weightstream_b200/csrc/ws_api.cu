@@ -486,7 +486,7 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     // slabs per stage: barrier round trips and a commit are per stage, and the scale atoms of UE8M0, so several slabs
     // share them; bounded by the stage size (128 rows of K 8192: 40 KB 29.4, 56 KB 29.3 us; UE8M0 56 KB 37.1, 72 KB
     // 33.4) and by tensor memory (fp32 scales: each slab has its own accumulator buffer, groups x slabs x (mp + 4) + 8
-    // columns of 512, at least two groups)
+    // columns of 512, at least two groups; UE8M0: one buffer for two slabs, 16 scale columns a slab)
     u.nslot_max = (tiles_per_cta * u.tile_rows) / a.block_n + 2;
     const int rx_rows = u.csize == 2 ? (mt + 1) / 2 : 0, kcta = (u.ks + u.csize - 1) / u.csize;
     // Half an SM (shared memory and tensor memory) when the tokens are few and the CTA's whole share of
@@ -499,12 +499,13 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     for (int half = small ? 1 : 0; half >= 0; --half) {
         const int budget = half ? kHalfSmemBudget : kSmemBudget, tmem = half ? 256 : 512;
         const int stage_target = half ? 32 * 1024 : u.wue ? 72 * 1024 : 56 * 1024;
-        u.slabs_per_stage = std::max(1, std::min({4, stage_target / slab_bytes, kcta, u.wue ? 4 : (tmem - 8) / (2 * (u.mp + 4))}));
+        const int chain = bs_chain(u.wue);
+        u.slabs_per_stage = std::max(1, std::min({4, stage_target / slab_bytes, kcta, u.wue ? chain * ((tmem - 64) / (2 * u.mp)) : (tmem - 8) / (2 * (u.mp + 4))}));
         const int groups = (kcta + u.slabs_per_stage - 1) / u.slabs_per_stage;
         u.slabs_per_stage = (kcta + groups - 1) / groups;
         u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * x_slab, 128);
-        u.nacc = u.wue ? std::min(2, std::max(1, (tmem - 8 - 2 * u.slabs_per_stage * 8) / u.mp))
-                       : std::min((int)kBsMaxAcc, (tmem - 8) / (u.slabs_per_stage * (u.mp + 4)));
+        const int accs = (u.slabs_per_stage + chain - 1) / chain;  // accumulators of a stage
+        u.nacc = std::min((int)kBsMaxAcc, u.wue ? (tmem - 16 * u.slabs_per_stage) / (accs * u.mp) : (tmem - 8) / (accs * (u.mp + 4)));
         auto total = [&](int ns) {
             return bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, u.nslot_max, skb, u.mp, rx_rows, u.wue,
                                   u.inline_x ? kcta * x_slab : 0).total + 1024;
@@ -514,17 +515,16 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         const int items = tiles_per_cta * groups;
         ns = std::min(ns, std::max(2, items));
         u.nstages = ns;
-        // fp32 scales: the epilogue and the producer wait on the same per-stage barrier: the MMA thread must not
-        // get a whole lap of the stage ring ahead of the epilogue, which holds when groups <= stages
-        if (!u.wue) u.nacc = std::max(1, std::min(u.nacc, ns));
+        // the epilogue and the producer wait on the same per-stage barrier: the MMA thread must not get a whole lap
+        // of the stage ring ahead of the epilogue, which holds when groups <= stages
+        u.nacc = std::max(1, std::min(u.nacc, ns));
         u.ok = ns >= 2;
         if (!u.ok || (half && items > ns)) continue;  // half an SM only when the CTA's whole share of the weights fits the ring
         u.smem = (size_t)total(ns);
         int cols = 32;
-        // (fp32 scales: the epilogue reads the accumulators of a group in batches, see fp8_bs_kernel)
-        const int batch = bs_read_batch(u.mp), read = (u.slabs_per_stage + batch - 1) / batch * batch;
-        while (cols < (u.wue ? u.nacc * u.mp + 2 * u.slabs_per_stage * 8
-                             : std::max(u.nacc * u.slabs_per_stage * (u.mp + 4) + 4, ((u.nacc - 1) * u.slabs_per_stage + read) * u.mp))) cols *= 2;
+        // (the epilogue reads the accumulators of a group in batches, see fp8_bs_kernel)
+        const int batch = bs_read_batch(u.mp, u.wue), read = (accs + batch - 1) / batch * batch;
+        while (cols < std::max(u.nacc * accs * u.mp + (u.wue ? 16 * u.slabs_per_stage : u.nacc * accs * 4 + 4), ((u.nacc - 1) * accs + read) * u.mp)) cols *= 2;
         u.tmem_cols = half ? std::min(cols, 256) : 512;
         break;
     }

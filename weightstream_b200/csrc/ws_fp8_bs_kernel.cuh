@@ -27,8 +27,7 @@
 //                     2^0, every slab has its own accumulator buffer, and the epilogue warps read a stage's
 //                     buffers back (tcgen05.ld) and add them x the fp32 scale while later MMAs run.
 //                     UE8M0 (WUE): they ARE an MMA scale operand.  Four auxiliary warps lay the tile's scale
-//                     bytes out as atoms in the stage, a tile accumulates over all of its K in tensor
-//                     memory and is read back once.
+//                     bytes out as atoms in the stage; an accumulator takes two slabs (see bs_chain).
 //
 // Measured on B200 and kept in mind above: every TMA or bulk copy costs its issuing thread 85-100 ns, but
 // one 3-D box for a stage's slabs was slower than a box each (128 rows 32.0 against 29.4 us); a slab's four
@@ -54,8 +53,8 @@ namespace ws {
 // Threads of a CTA.  Warp 0: producer, warp 1: MMA issue (and owner of the tensor memory), then the
 // epilogue warps: four (one per 32-lane quarter of the tensor memory, all token columns) for up to 16
 // tokens, eight (two per quarter, half of the token columns each) beyond, where reading the
-// accumulators back is what a stage (UE8M0: the end of a tile) waits for (sixteen for 128 tokens: 38 against
-// 31 us); then, for UE8M0 weight scales, four auxiliary warps.
+// accumulators back is what a stage waits for (sixteen for 128 tokens: 38 against 31 us); then, for UE8M0
+// weight scales, four auxiliary warps.
 __host__ __device__ constexpr int bs_epi_warps(int mp) { return mp >= 32 ? 8 : 4; }
 constexpr int kBsAuxWarps = 4;
 __host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 * (bs_epi_warps(mp) + (wue ? kBsAuxWarps : 0)); }
@@ -64,8 +63,16 @@ __host__ __device__ constexpr int bs_threads(int mp, bool wue) { return 64 + 32 
 // for the CTA to leave: UE8M0, K 2304, 40 rows 13.3 against 10.4 us), and a second CTA, up to 16 tokens with fp32
 // scales and when a UE8M0 step has no prep blocks.
 __host__ __device__ constexpr int bs_regs(int mp, bool wue, bool inl) { return wue ? (mp == 16 && inl ? 96 : 112) : mp == 16 ? 144 : 152; }
-// Slabs whose accumulators an epilogue thread reads at once (fp32 weight scales): 64 registers' worth.
-__host__ __device__ constexpr int bs_read_batch(int mp) { return 64 / (mp * 4 / bs_epi_warps(mp)); }
+// Slabs an accumulator in tensor memory sums before the epilogue adds it up in fp32 registers.  The tensor cores
+// truncate every addition, so a chain's error has a sign and grows with its length.  UE8M0, 2000 rows of 7168 x 8192,
+// relative to 64-bit sums: all of K in one chain 4.9e-7 (scales spread over 2^24: 3.4e-6), four slabs 8.1e-8 (2.7e-7),
+// two 9.2e-8 (1.8e-7), one 1.0e-7 (1.7e-7), at 124, 126, 131 and 160 us a step; up to 128 rows 2.2e-7 (1.7e-6), 6.8e-8
+// (2.7e-7), 7.1e-8 (1.7e-7) and 7.6e-8 (1.4e-7).
+__host__ __device__ constexpr int bs_chain(bool wue) { return wue ? 2 : 1; }
+// Accumulators an epilogue thread reads at once: 64 registers' worth, UE8M0 (fewer registers a thread) 32.
+__host__ __device__ constexpr int bs_read_batch(int mp, bool wue) {
+    return (wue ? 32 : 64) / (mp * 4 / bs_epi_warps(mp)) > 0 ? (wue ? 32 : 64) / (mp * 4 / bs_epi_warps(mp)) : 1;
+}
 constexpr int kBsMaxAcc = 8;         // accumulator groups in tensor memory (a group = one stage's slabs)
 constexpr int kBsMaxTokens = 128;    // activation rows one launch takes (16, 32, 64 or 128 MMA columns)
 constexpr int kBsAtomBytes = 512;    // one scale atom: 128 rows x 4 K blocks
@@ -174,7 +181,7 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
     s.sw = o;   o += wue ? 0 : (int)align_up((int64_t)nslot_max * skb * 4, 16);
     s.cand = o; o += bs_epi_warps(mp) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
     s.rx = o;   o += rx_rows * kBsMmaRows * 4;           // CTA pairs: the partner's sums of one tile for this CTA's tokens, [token][row]
-    s.bars = o; o += (2 * kMaxStages + 2 * kBsMaxAcc + 4) * 8;
+    s.bars = o; o += (2 * kMaxStages + kBsMaxAcc + 4) * 8;
     s.misc = o; o += 64;
     s.total = o;
     return s;
@@ -291,6 +298,16 @@ __device__ __forceinline__ void tmem_ld_batch<32, 2>(uint32_t t, uint32_t pitch,
 }
 template <>
 __device__ __forceinline__ void tmem_ld_batch<64, 1>(uint32_t t, uint32_t, uint32_t (&r)[64]) { tmem_ld_cols<64>(t, r); }
+template <>
+__device__ __forceinline__ void tmem_ld_batch<32, 1>(uint32_t t, uint32_t, uint32_t (&r)[32]) { tmem_ld_cols<32>(t, r); }
+template <>
+__device__ __forceinline__ void tmem_ld_batch<16, 2>(uint32_t t, uint32_t pitch, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : WS_R16(r, 0), WS_R16(r, 16) : "r"(t), "r"(t + pitch) : "memory");
+}
 #undef WS_R16
 #undef WS_R4
 
@@ -524,7 +541,8 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
     if (p.csize == 2) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
     const int part = p.csize == 2 ? cta >> 1 : cta, nparts = p.csize == 2 ? ncta >> 1 : ncta;
     const int k_lo = (int)crank * KS / p.csize, k_hi = ((int)crank + 1) * KS / p.csize;
-    const int SL = p.slabs_per_stage, NS = p.nstages, NB = p.nacc;
+    constexpr int CH = bs_chain(WUE);
+    const int SL = p.slabs_per_stage, NS = p.nstages, NB = p.nacc, AS = (SL + CH - 1) / CH;  // AS accumulators per stage
     const int ntiles = p.ntiles, TR = p.tile_rows;
 
     const BsSmem S = bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? (p.m + 1) / 2 : 0, WUE,
@@ -534,13 +552,12 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
     const uint32_t a0 = smem_u32(smem + S.a), x0 = smem_u32(smem + S.x), wsf0 = smem_u32(smem + S.wsf);
     // full[s]: the stage's bytes landed (UE8M0: and the auxiliary warps have written its weight scales).
     // done[s]: every MMA that reads the stage has completed (ONE tcgen05.commit per stage: a commit stalls
-    // the issuing thread for ~160 ns, so it is not spent per slab).  fp32 weight scales: a stage's slabs
-    // accumulate into the SL buffers of accumulator group g = item mod NB, done[s] also tells the epilogue
-    // that they are ready, accempty[g] that the group has been read back.  UE8M0: a tile accumulates into
-    // buffer (tile mod NB), accfull / accempty hand it over.
+    // the issuing thread for ~160 ns, so it is not spent per slab).  A stage's slabs accumulate into the AS
+    // buffers of accumulator group g = item mod NB, done[s] also tells the epilogue that they are ready,
+    // accempty[g] that the group has been read back.
     const uint32_t full0 = smem_u32(smem + S.bars), done0 = full0 + kMaxStages * 8;
-    const uint32_t accempty0 = done0 + kMaxStages * 8, accfull0 = accempty0 + kBsMaxAcc * 8;
-    const uint32_t rxfull = accfull0 + kBsMaxAcc * 8, rxempty = rxfull + 8, xready = rxempty + 8;  // CTA pairs: the partner's sums of a tile have arrived / been read
+    const uint32_t accempty0 = done0 + kMaxStages * 8;
+    const uint32_t rxfull = accempty0 + kBsMaxAcc * 8, rxempty = rxfull + 8, xready = rxempty + 8;  // CTA pairs: the partner's sums of a tile have arrived / been read
 
     // Weights are static: the first ring's worth is on its way before the CTA has set itself up (barriers,
     // tensor memory and the pair's meeting take ~1.3 us, in which HBM would idle), let alone before the wait on
@@ -557,10 +574,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                 mbar_init(full0 + s * 8, WUE ? 1 + kBsAuxWarps : 1);
                 mbar_init(done0 + s * 8, 1);
             }
-            for (int b = 0; b < kBsMaxAcc; ++b) {
-                mbar_init(accempty0 + b * 8, EW);  // one arrival per epilogue warp
-                mbar_init(accfull0 + b * 8, 1);
-            }
+            for (int b = 0; b < kBsMaxAcc; ++b) mbar_init(accempty0 + b * 8, EW);  // one arrival per epilogue warp
             mbar_init(rxfull, EW);   // every epilogue warp of the partner arrives after its stores
             mbar_init(rxempty, EW);
             mbar_init(xready, EW);   // inline: the activations are in shared memory
@@ -587,10 +601,10 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(misc_s);
-    // tensor-memory columns.  fp32 weight scales: NB groups x SL accumulator buffers of MP columns, 4
-    // activation-scale columns (one scale atom) per buffer, the 4 weight-scale columns.  UE8M0: NB
-    // accumulators of MP columns, then for two stages and SL slabs each 4 activation- and 4 weight-scale columns.
-    const uint32_t t_sf0 = tmem_base + (uint32_t)(NB * (WUE ? 1 : SL) * MP);
+    // tensor-memory columns: NB groups x AS accumulator buffers of MP columns.  Then, fp32 weight scales: 4
+    // activation-scale columns (one scale atom) per buffer, the 4 weight-scale columns.  UE8M0: for two stages
+    // and SL slabs each 4 activation- and 4 weight-scale columns.
+    const uint32_t t_sf0 = tmem_base + (uint32_t)(NB * AS * MP);
     const uint32_t t_sfa = t_sf0 + (uint32_t)(NB * SL * 4);  // fp32 weight scales only
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -641,19 +655,18 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             const uint32_t acc_end = accempty0 + NB * 8;
             constexpr bool inl = INL;
             uint32_t sf_off = 0;
-            // one stage: straight-line code per slab count (a rolled loop costs twice the time); `carry`: the first
-            // MMA adds to earlier stages' sums (UE8M0)
-            auto issue = [&](auto count, uint32_t carry) {
+            // one stage: straight-line code per slab count (a rolled loop costs twice the time)
+            auto issue = [&](auto count) {
                 constexpr int C = decltype(count)::value;
                 const uint64_t xsf = xsf0 + (uint64_t)(inl ? sf_off : x_off + (uint32_t)C * x_step), wsf = wsf_desc0 + (uint64_t)w_off;
 #pragma unroll
                 for (int j = 0; j < C; ++j) {
                     const uint32_t a = a_lo + (uint32_t)j * a_step, b = x_lo + (uint32_t)j * x_step;
-                    const uint32_t d = WUE ? t_acc : t_acc + (uint32_t)(j * MP);
+                    const uint32_t d = t_acc + (uint32_t)(j / CH * MP);
                     const uint32_t sx = t_sf + (uint32_t)(j * (WUE ? 8 : 4)), sw = WUE ? sx + 4 : t_sfa;
                     tmem_cp_atom(sx, xsf + (uint64_t)((uint32_t)j * xsf_step));
                     if (WUE) tmem_cp_atom(sw, wsf + (uint64_t)(j * kSfStep));
-                    umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id[0], sw, sx, WUE && j > 0 ? 1u : carry);
+                    umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id[0], sw, sx, j % CH ? 1u : 0u);
                     umma_bs_ss(d, a + 2, b + x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[1], sw, sx, 1u);
                     umma_bs_ss(d, a + 4, b + 2 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[2], sw, sx, 1u);
                     umma_bs_ss(d, a + 6, b + 3 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[3], sw, sx, 1u);
@@ -664,23 +677,16 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             bool ok = !INL || mbar_wait(xready, 0, status);
             uint32_t odd = 0;  // UE8M0: which of the two sets of scale columns
             for (int t = kcta > 0 ? my_tiles : 0; t > 0 && ok; --t) {
-                uint32_t carry = 0;
                 if (inl) { x_lo = x_lo0; sf_off = sf_off0; }
                 for (int left = kcta; left > 0; left -= SL) {
-                    if ((!WUE || carry == 0) && !mbar_wait(accempty, acc_ph, status)) { ok = false; break; }
+                    if (!mbar_wait(accempty, acc_ph, status)) { ok = false; break; }
                     if (!mbar_wait(full, ph, status)) { ok = false; break; }
                     tc_fence_after();
-                    if (left >= 4 && SL == 4) issue(std::integral_constant<int, 4>{}, carry);
-                    else if (left >= 3 && SL >= 3) issue(std::integral_constant<int, 3>{}, carry);
-                    else if (left >= 2 && SL >= 2) issue(std::integral_constant<int, 2>{}, carry);
-                    else issue(std::integral_constant<int, 1>{}, carry);
-                    umma_commit(done);  // the stage may be refilled (fp32 weight scales: and its accumulators read)
-                    const bool tile_end = WUE && left <= SL;
-                    if (tile_end) umma_commit(accempty + (accfull0 - accempty0));
-                    if (WUE) {
-                        carry = 1;
-                        odd ^= 1u;
-                    }
+                    if (left >= 4 && SL == 4) issue(std::integral_constant<int, 4>{});
+                    else if (left >= 3 && SL >= 3) issue(std::integral_constant<int, 3>{});
+                    else if (left >= 2 && SL >= 2) issue(std::integral_constant<int, 2>{});
+                    else issue(std::integral_constant<int, 1>{});
+                    umma_commit(done);  // the stage may be refilled and its accumulators read
                     // next stage
                     full += 8; done += 8; a_lo += a_stage; x_off += x_stage;
                     x_lo += inl ? (uint32_t)SL * x_step : x_stage;
@@ -691,18 +697,19 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                         if (!inl) x_lo = x_lo0;
                         ph ^= 1u;
                     }
-                    // next accumulator (group)
-                    if (!WUE || tile_end) {
-                        accempty += 8;
-                        t_acc += (uint32_t)((WUE ? 1 : SL) * MP);
-                        if (!WUE) t_sf += (uint32_t)(SL * 4);
-                        if (accempty == acc_end) {
-                            accempty = accempty0; t_acc = tmem_base;
-                            if (!WUE) t_sf = t_sf0;
-                            acc_ph ^= 1u;
-                        }
+                    // next accumulator group
+                    accempty += 8;
+                    t_acc += (uint32_t)(AS * MP);
+                    if (!WUE) t_sf += (uint32_t)(SL * 4);
+                    if (accempty == acc_end) {
+                        accempty = accempty0; t_acc = tmem_base;
+                        if (!WUE) t_sf = t_sf0;
+                        acc_ph ^= 1u;
                     }
-                    if (WUE) t_sf = t_sf0 + odd * (uint32_t)(SL * 8);
+                    if (WUE) {
+                        odd ^= 1u;
+                        t_sf = t_sf0 + odd * (uint32_t)(SL * 8);
+                    }
                 }
             }
         }
@@ -891,61 +898,51 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         int ntile_done = 0;
         float acc[CP];
         // positions in the stage and accumulator rings, advanced incrementally
-        uint32_t done = done0, ph = 0, accempty = accempty0, acc_ph = 0, t_col = tlane + (uint32_t)col0;
+        uint32_t done = done0, ph = 0, accempty = accempty0, t_col = tlane + (uint32_t)col0;
         const uint32_t done_end = done0 + NS * 8, acc_end = accempty0 + NB * 8;
         const int kcta = k_hi - k_lo;
         for (int tile = t_lo; tile <= t_hi && kcta > 0; ++tile) {
-            if constexpr (WUE) {
-                if (ok && !mbar_wait(accempty + (accfull0 - accempty0), acc_ph, X.status)) ok = false;
+#pragma unroll
+            for (int i = 0; i < CP; ++i) acc[i] = 0.0f;
+            const int row = min(tile * TR + min(rc, TR - 1), p.n - 1);
+            const float *swrow = WUE ? nullptr : sw_s + (int)(((A.row0 + row) >> p.bn_shift) - srow_lo) * p.skb;
+            int kk = kofs + k_lo * 128;  // K offset of the stage's first slab inside the scale matrix
+            for (int left = kcta; left > 0; left -= SL) {
+                const int na = (min(left, SL) + CH - 1) / CH;
+                if (ok && !mbar_wait(done, ph, X.status)) ok = false;
                 ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads below need the whole warp
                 tc_fence_after();
-                uint32_t r[CP];
+                if (ok) {
+                    // as many accumulators per round trip to tensor memory as the registers hold (a last round may
+                    // read accumulators of other stages, inside the allocation, and leaves them unused)
+                    constexpr int B = bs_read_batch(MP, WUE), C = WUE && CP > 32 ? 32 : CP;  // columns of each
+#pragma unroll 1
+                    for (int j0 = 0; j0 < na; j0 += B) {
 #pragma unroll
-                for (int i = 0; i < CP; ++i) r[i] = 0u;
-                if (ok) tmem_ld_cols<CP>(t_col, r);
-#pragma unroll
-                for (int i = 0; i < CP; ++i) acc[i] = __uint_as_float(r[i]);
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(accempty);
-                accempty += 8; t_col += MP;
-                if (accempty == acc_end) { accempty = accempty0; t_col = tlane + (uint32_t)col0; acc_ph ^= 1u; }
-            } else {
-#pragma unroll
-                for (int i = 0; i < CP; ++i) acc[i] = 0.0f;
-                const int row = min(tile * TR + min(rc, TR - 1), p.n - 1);
-                const float *swrow = sw_s + (int)(((A.row0 + row) >> p.bn_shift) - srow_lo) * p.skb;
-                int kk = kofs + k_lo * 128;  // K offset of the stage's first slab inside the scale matrix
-                for (int left = kcta; left > 0; left -= SL) {
-                    const int nsl = min(left, SL);
-                    if (ok && !mbar_wait(done, ph, X.status)) ok = false;
-                    ok = __all_sync(0xffffffffu, ok);
-                    tc_fence_after();
-                    if (ok) {
-                        // as many slabs per round trip to tensor memory as the registers hold (a last round may read
-                        // accumulators of other stages, inside the allocation, and leaves them unused)
-                        constexpr int B = bs_read_batch(MP);
-                        for (int j0 = 0; j0 < nsl; j0 += B) {
-                            uint32_t r[B * CP];
-                            tmem_ld_batch<CP, B>(t_col + (uint32_t)(j0 * MP), (uint32_t)MP, r);
+                        for (int c = 0; c < CP; c += C) {
+                            uint32_t r[B * C];
+                            tmem_ld_batch<C, B>(t_col + (uint32_t)(j0 * MP + c), (uint32_t)MP, r);
 #pragma unroll
                             for (int j = 0; j < B; ++j)
-                                if (j == 0 || j0 + j < nsl) {
-                                    const float sw = swrow[(kk + (j0 + j) * 128) >> p.bk_shift];
+                                if (j == 0 || j0 + j < na) {
+                                    const float sw = WUE ? 1.0f : swrow[(kk + (j0 + j) * 128) >> p.bk_shift];
 #pragma unroll
-                                    for (int i = 0; i < CP; ++i) acc[i] = fmaf(__uint_as_float(r[j * CP + i]), sw, acc[i]);
+                                    for (int i = 0; i < C; ++i) {
+                                        const float v = __uint_as_float(r[j * C + i]);
+                                        acc[c + i] = WUE ? acc[c + i] + v : fmaf(v, sw, acc[c + i]);
+                                    }
                                 }
                         }
                     }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(accempty);
-                    kk += SL * 128;
-                    done += 8;
-                    if (done == done_end) { done = done0; ph ^= 1u; }
-                    accempty += 8; t_col += (uint32_t)(SL * MP);
-                    if (accempty == acc_end) { accempty = accempty0; t_col = tlane + (uint32_t)col0; }
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accempty);
+                kk += SL * 128;
+                done += 8;
+                if (done == done_end) { done = done0; ph ^= 1u; }
+                accempty += 8; t_col += (uint32_t)(AS * MP);
+                if (accempty == acc_end) { accempty = accempty0; t_col = tlane + (uint32_t)col0; }
             }
             // what depends on the tile's end only is not worth registers in the main loop: hidden from the optimiser
             int lo = tok_lo, hi = tok_hi, m = p.m;

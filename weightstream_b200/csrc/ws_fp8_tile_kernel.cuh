@@ -9,9 +9,8 @@
 // ring, warp 1 issues four MMAs per slab (M = 128, N = tokens).  fp32 weight scales: every slab goes to one of
 // two accumulators, and the two epilogue warpgroups (one half of the tokens each) read it back and add it x
 // the scale to registers while the next slab's MMAs fill the other; the register file is split by
-// setmaxnreg, 112 sums per thread do not fit an even share.  UE8M0 weight scales (WUE) are an MMA operand: a
-// tile accumulates over all of K in tensor memory, one warpgroup lays the scale atoms out, one reads the tile
-// back at its end.
+// setmaxnreg, 112 sums per thread do not fit an even share.  UE8M0 weight scales (WUE) are an MMA operand,
+// whose atoms warps 2 and 3 lay out; an accumulator takes two slabs (see bs_chain).
 //
 // Bound: tokens x (128 + tokens) per slab decide between the tensor pipe (N / 2 clocks per MMA) and what L2
 // hands an SM (16 KB + 128 bytes per token a slab); wide token tiles favour both.
@@ -22,7 +21,7 @@
 namespace ws {
 
 constexpr int kTileTokens = 224;   // most tokens of a tile: two accumulators and the scale columns fill tensor memory
-constexpr int kTileThreads = 384;  // warpgroup 0: producer, MMA issue; 1 and 2: epilogue (UE8M0: epilogue, scale atoms)
+constexpr int kTileThreads = 384;  // warpgroup 0: producer, MMA issue, scale atoms (UE8M0); 1 and 2: epilogue
 constexpr int kTileMaxStages = 8;
 
 struct alignas(64) TileParams {
@@ -52,6 +51,29 @@ __host__ __device__ inline TileSmem tile_smem_layout(int nstages, int x_pitch, b
     return s;
 }
 
+// The first `nc` columns of an accumulator, times the weight scale (SCALED), added to a thread's sums; C columns per
+// round trip to tensor memory.
+template <int C, bool SCALED>
+__device__ __forceinline__ void read_back(float (&acc)[kTileTokens / 2], uint32_t t, int nc, float sw) {
+    constexpr int CP = kTileTokens / 2;
+#pragma unroll
+    for (int c = 0; c < CP; c += C) {
+        if (c < nc) {  // warp-uniform
+            if (c + C <= CP) {
+                uint32_t r[C];
+                tmem_ld_cols<C>(t + (uint32_t)c, r);
+#pragma unroll
+                for (int i = 0; i < C; ++i) acc[c + i] = SCALED ? fmaf(__uint_as_float(r[i]), sw, acc[c + i]) : acc[c + i] + __uint_as_float(r[i]);
+            } else {
+                uint32_t r[16];
+                tmem_ld_cols<16>(t + (uint32_t)c, r);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[c + i] = SCALED ? fmaf(__uint_as_float(r[i]), sw, acc[c + i]) : acc[c + i] + __uint_as_float(r[i]);
+            }
+        }
+    }
+}
+
 template <bool WUE>
 __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_constant__ TileParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -61,22 +83,21 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
     const int NS = p.nstages, KS = p.ks, ntiles = p.nrow * p.ntok;
     const TileSmem S = tile_smem_layout(NS, p.x_pitch, WUE);
     const uint32_t a0 = smem_u32(smem + S.a), x0 = smem_u32(smem + S.x), wsf0 = smem_u32(smem + S.wsf);
-    // full[s]: the stage's bytes landed; done[s]: its MMAs have completed (stage free, fp32 scales: accumulator
-    // ready); accempty[g]: accumulator g has been read; accfull[g] (UE8M0): a tile's sums are complete
+    // full[s]: the stage's bytes landed (and its scale atom is laid out); done[s]: its MMAs have completed (stage
+    // free; the last of an accumulator's: accumulator ready); accempty[g]: accumulator g has been read
     const uint32_t full0 = smem_u32(smem + S.bars), done0 = full0 + kTileMaxStages * 8;
-    const uint32_t accempty0 = done0 + kTileMaxStages * 8, accfull0 = accempty0 + 16;
-    constexpr int EW = WUE ? 4 : 8;
+    const uint32_t accempty0 = done0 + kTileMaxStages * 8;
+    constexpr int EW = 8, CH = bs_chain(WUE);
     uint32_t *const status = p.ctx.status;
     if (warp == 0) {
         if (elect_one()) {
             for (int s = 0; s < NS; ++s) {
-                mbar_init(full0 + s * 8, WUE ? 5 : 1);
+                mbar_init(full0 + s * 8, WUE ? 3 : 1);
                 mbar_init(done0 + s * 8, 1);
             }
-            for (int g = 0; g < 2; ++g) {
-                mbar_init(accempty0 + g * 8, EW);
-                mbar_init(accfull0 + g * 8, 1);
-            }
+            // (two are used; with two initialised, fp32 scales took 155 us for 2000 rows of K 8192 instead of 150, in
+            // every form of the loops below that was tried: how the CTAs of a wave meet in L2 depends on their start)
+            for (int g = 0; g < 4; ++g) mbar_init(accempty0 + g * 8, g < 2 ? EW : 1);
             mbar_fence_init();
         }
         __syncwarp();
@@ -99,7 +120,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
     const int64_t tile_bytes = (int64_t)KS * (p.tokens * 128 + atom);
 
     if (warp < 4) {
-        if constexpr (!WUE) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");  // 128 x 56 + 256 x 216 <= 384 x 168
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");  // 128 x 56 + 256 x 216 <= 384 x 168
         if (warp == 0) {
             // -------------------------------------------------------- producer (one thread)
             if (elect_one()) {
@@ -138,7 +159,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
 #pragma unroll
                     for (int j = 0; j < 4; ++j) id[j] = bs_idesc(cols, WUE ? j : 0, j);
                     for (int k = 0; k < KS; ++k) {
-                        if ((!WUE || k == 0) && !mbar_wait(accempty0 + g * 8, acc_ph, status)) { ok = false; break; }
+                        if (k % CH == 0 && !mbar_wait(accempty0 + g * 8, acc_ph, status)) { ok = false; break; }
                         if (!mbar_wait(full0 + s * 8, ph, status)) { ok = false; break; }
                         tc_fence_after();
                         const uint32_t a = a_lo0 + (uint32_t)s * 1024u, x_off = (uint32_t)s * x_stage, b = (x_lo0 + x_off) | (m16 << 16);
@@ -147,145 +168,53 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
                         tmem_cp_atom(sx, sf);
                         if (mt > 128) tmem_cp_atom(sx + 4, sf + 32);
                         if (WUE) tmem_cp_atom(sw, wsf_d0 + (uint64_t)((uint32_t)s * (kBsAtomBytes >> 4)));
-                        umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id[0], sw, sx, WUE && k > 0 ? 1u : 0u);
+                        umma_bs_ss(d, a, b, kUmmaDescHiSw128, kUmmaDescHiX, id[0], sw, sx, k % CH ? 1u : 0u);
                         umma_bs_ss(d, a + 2, b + x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[1], sw, sx, 1u);
                         umma_bs_ss(d, a + 4, b + 2 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[2], sw, sx, 1u);
                         umma_bs_ss(d, a + 6, b + 3 * x_kb, kUmmaDescHiSw128, kUmmaDescHiX, id[3], sw, sx, 1u);
                         umma_commit(done0 + s * 8);
-                        if (WUE && k == KS - 1) umma_commit(accfull0 + g * 8);
                         odd ^= 1u;
                         if (++s == NS) { s = 0; ph ^= 1u; }
-                        if (!WUE || k == KS - 1) {
+                        if (k % CH == CH - 1 || k == KS - 1) {
                             g ^= 1u;
                             if (g == 0) acc_ph ^= 1u;
                         }
                     }
                 }
             }
-        }
-        __syncwarp();
-    } else if (!WUE || warp < 8) {
-        // ------------------------------------------------------------ epilogue warps
-        if constexpr (!WUE) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
-        const int quad = warp & 3, rc = quad * 32 + lane, half = (warp >> 2) - 1;  // TMEM lane quarter; which half of the tokens
-        const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        if constexpr (WUE) {
-            uint32_t g = 0, ph = 0;
-            bool ok = true;
-            for (int q = blockIdx.x; q < ntiles; q += gridDim.x) {
-                const int rt = q / p.ntok, tt = q - rt * p.ntok, mt = min(p.tokens, p.m - tt * p.tokens);
-                if (ok && !mbar_wait(accfull0 + g * 8, ph, status)) ok = false;
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc_fence_after();
-                const int row = rt * 128 + rc;
-                int64_t ld = p.n;
-                asm volatile("" : "+l"(ld));
-                float *dst = p.out + (int64_t)tt * p.tokens * ld + row;
-#pragma unroll 1
-                for (int c = 0; c < mt; c += 32) {
-                    uint32_t r[32];
-                    tmem_ld_cols<32>(tl + g * kTileTokens + (uint32_t)c, r);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        if (row < p.n && c + i < mt) *dst = __uint_as_float(r[i]);
-                        dst += ld;
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(accempty0 + g * 8);
-                g ^= 1u;
-                if (g == 0) ph ^= 1u;
-            }
-        } else {
-            constexpr int CP = kTileTokens / 2;
-            const int hcols = (p.tokens / 2 + 15) / 16 * 16;  // columns of the first half: whole groups of 16
-            const int64_t kcol0 = p.k0 >> p.bk_shift;
-            const int kofs = (int)(p.k0 - (kcol0 << p.bk_shift));
-            int s = 0;
-            uint32_t ph = 0, g = 0;
-            bool ok = true;
-            for (int q = blockIdx.x; q < ntiles; q += gridDim.x) {
-                const int rt = q / p.ntok, tt = q - rt * p.ntok, mt = min(p.tokens, p.m - tt * p.tokens);
-                const int c0 = half * hcols, nc = min(mt - c0, half == 0 ? hcols : CP);  // this half's columns (may be none)
-                const int row = rt * 128 + rc;
-                const float *sw_row = static_cast<const float *>(p.scales) + ((p.row0 + min(row, p.n - 1)) >> p.bn_shift) * p.scale_ld + kcol0;
-                float acc[CP];
-#pragma unroll
-                for (int i = 0; i < CP; ++i) acc[i] = 0.0f;
-                float sw = __ldg(sw_row + (kofs >> p.bk_shift));
-                for (int k = 0; k < KS; ++k) {
-                    const float next = k + 1 < KS ? __ldg(sw_row + ((kofs + (k + 1) * 128) >> p.bk_shift)) : 0.0f;
-                    if (ok && !mbar_wait_inline(done0 + s * 8, ph, status)) ok = false;  // (no call: it would not leave the sums their registers)
-                    ok = __all_sync(0xffffffffu, ok);
-                    tc_fence_after();
-                    if (ok) {
-                        const uint32_t t = tl + g * kTileTokens + (uint32_t)c0;
-#pragma unroll
-                        for (int c = 0; c < CP; c += 32) {
-                            if (c < nc) {  // warp-uniform
-                                if (c + 16 < CP) {
-                                    uint32_t r[32];
-                                    tmem_ld_cols<32>(t + (uint32_t)c, r);
-#pragma unroll
-                                    for (int i = 0; i < 32; ++i) acc[c + i] = fmaf(__uint_as_float(r[i]), sw, acc[c + i]);
-                                } else {
-                                    uint32_t r[16];
-                                    tmem_ld_cols<16>(t + (uint32_t)c, r);
-#pragma unroll
-                                    for (int i = 0; i < 16; ++i) acc[c + i] = fmaf(__uint_as_float(r[i]), sw, acc[c + i]);
-                                }
-                            }
-                        }
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(accempty0 + g * 8);
-                    g ^= 1u;
-                    if (++s == NS) { s = 0; ph ^= 1u; }
-                    sw = next;
-                }
-                if (row < p.n) {
-                    int64_t ld = p.n;
-                    asm volatile("" : "+l"(ld));  // offsets computed here, not kept in registers through the loop
-                    float *dst = p.out + ((int64_t)tt * p.tokens + c0) * ld + row;
-#pragma unroll
-                    for (int i = 0; i < CP; ++i) {
-                        if (i < nc) *dst = acc[i];
-                        dst += ld;
-                    }
-                }
-            }
-        }
-    } else {
-        // ------------------------------------------------------------ scale atoms (UE8M0)
-        if constexpr (WUE) {
-            const int r = tid - 256;
+        } else if constexpr (WUE) {
+            // -------------------------------------------------------- scale atoms (thread = rows r and r + 64)
+            const int r = tid - 64;
             const Ue8m0Scales sc(p.scales, p.scale_ld, p.k0, p.k, p.bk_shift);
             int s = 0, lap = 0, lq = blockIdx.x, lk = 0;  // stage to fill; tile and slab to load
             uint32_t ph = 1;
-            const uint8_t *row = nullptr;
-            auto load = [&](uint32_t &w) {
+            const uint8_t *row_lo = nullptr, *row_hi = nullptr;
+            auto load = [&](uint32_t (&w)[2]) {
                 if (lq >= ntiles) return false;
-                if (lk == 0) row = sc.row((p.row0 + min(lq / p.ntok * 128 + r, p.n - 1)) >> p.bn_shift);
-                w = sc.slab(row, lk);
+                if (lk == 0) {
+                    const int row = lq / p.ntok * 128 + r;
+                    row_lo = sc.row((p.row0 + min(row, p.n - 1)) >> p.bn_shift);
+                    row_hi = sc.row((p.row0 + min(row + 64, p.n - 1)) >> p.bn_shift);
+                }
+                w[0] = sc.slab(row_lo, lk);
+                w[1] = sc.slab(row_hi, lk);
                 if (++lk == KS) { lk = 0; lq += gridDim.x; }
                 return true;
             };
-            auto put = [&](uint32_t w, bool ok) {
+            const uint32_t at = wsf0 + (uint32_t)((r & 31) * 16 + (r >> 5) * 4);
+            auto put = [&](const uint32_t (&w)[2], bool ok) {
                 if (lap == 1 && s == 0) wait_predecessor();
                 if (ok && lap > 0) ok = mbar_wait(done0 + s * 8, ph, status);
                 if (!__all_sync(0xffffffffu, ok)) return false;
-                *reinterpret_cast<uint32_t *>(smem + S.wsf + s * kBsAtomBytes + (r & 31) * 16 + (r >> 5) * 4) = w;
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + s * kBsAtomBytes), "r"(w[0]) : "memory");
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + s * kBsAtomBytes + 8), "r"(w[1]) : "memory");
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full0 + s * 8);
                 if (++s == NS) { s = 0; ++lap; ph ^= 1u; }
                 return true;
             };
-            uint32_t w0 = 0, w1 = 0, w2 = 0;  // three slabs' words in flight
+            uint32_t w0[2], w1[2], w2[2];  // three slabs' words in flight
             bool h0 = load(w0), h1 = load(w1), h2 = load(w2);
             for (;;) {
                 if (!put(w0, h0)) break;
@@ -294,6 +223,69 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
                 h1 = load(w1);
                 if (!put(w2, h2)) break;
                 h2 = load(w2);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------ epilogue warps
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        const int quad = warp & 3, rc = quad * 32 + lane, half = (warp >> 2) - 1;  // TMEM lane quarter; which half of the tokens
+        const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        constexpr int CP = kTileTokens / 2;
+        const int hcols = (p.tokens / 2 + 15) / 16 * 16;  // columns of the first half: whole groups of 16
+        const int64_t kcol0 = p.k0 >> p.bk_shift;
+        const int kofs = (int)(p.k0 - (kcol0 << p.bk_shift));
+        int s = 0;
+        uint32_t ph = 0, g = 0;
+        bool ok = true;
+        for (int q = blockIdx.x; q < ntiles; q += gridDim.x) {
+            const int rt = q / p.ntok, tt = q - rt * p.ntok, mt = min(p.tokens, p.m - tt * p.tokens);
+            const int c0 = half * hcols, nc = min(mt - c0, half == 0 ? hcols : CP);  // this half's columns (may be none)
+            const int row = rt * 128 + rc;
+            float acc[CP];
+#pragma unroll
+            for (int i = 0; i < CP; ++i) acc[i] = 0.0f;
+            if constexpr (WUE) {
+                for (int k = 0; k < KS; k += CH) {
+                    s += min(CH, KS - k) - 1;  // the accumulator's last slab
+                    if (s >= NS) { s -= NS; ph ^= 1u; }
+                    if (ok && !mbar_wait_inline(done0 + s * 8, ph, status)) ok = false;
+                    ok = __all_sync(0xffffffffu, ok);
+                    tc_fence_after();
+                    if (ok) read_back<16, false>(acc, tl + g * kTileTokens + (uint32_t)c0, nc, 1.0f);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(accempty0 + g * 8);
+                    g ^= 1u;
+                    if (++s == NS) { s = 0; ph ^= 1u; }
+                }
+            } else {
+                const float *sw_row = static_cast<const float *>(p.scales) + ((p.row0 + min(row, p.n - 1)) >> p.bn_shift) * p.scale_ld + kcol0;
+                float sw = __ldg(sw_row + (kofs >> p.bk_shift));
+                for (int k = 0; k < KS; ++k) {
+                    const float next = k + 1 < KS ? __ldg(sw_row + ((kofs + (k + 1) * 128) >> p.bk_shift)) : 0.0f;
+                    if (ok && !mbar_wait_inline(done0 + s * 8, ph, status)) ok = false;  // (no call: it would not leave the sums their registers)
+                    ok = __all_sync(0xffffffffu, ok);
+                    tc_fence_after();
+                    if (ok) read_back<32, true>(acc, tl + g * kTileTokens + (uint32_t)c0, nc, sw);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(accempty0 + g * 8);
+                    g ^= 1u;
+                    if (++s == NS) { s = 0; ph ^= 1u; }
+                    sw = next;
+                }
+            }
+            if (row < p.n) {
+                int64_t ld = p.n;
+                asm volatile("" : "+l"(ld));  // offsets computed here, not kept in registers through the loop
+                float *dst = p.out + ((int64_t)tt * p.tokens + c0) * ld + row;
+#pragma unroll
+                for (int i = 0; i < CP; ++i) {
+                    if (i < nc) *dst = acc[i];
+                    dst += ld;
+                }
             }
         }
     }
