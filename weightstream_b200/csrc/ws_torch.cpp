@@ -32,6 +32,15 @@ bool act_dtype(const at::Tensor &t, int32_t *out) {
     return true;
 }
 
+// What a kernel reads or writes has to be there: all rows of scale blocks, a result of m x n floats.  (Block shapes and
+// offsets that make no sense are the C ABI's to refuse.)
+bool covers(const at::Tensor &scales, int64_t row0, int64_t n, int64_t bn) {
+    return bn <= 0 || row0 < 0 || n < 1 || (row0 + n - 1) / bn < scales.size(0);
+}
+bool holds(const at::Tensor &out, int64_t m, int64_t n) {
+    return out.scalar_type() == at::kFloat && out.is_contiguous() && out.numel() >= m * n;
+}
+
 // Everything of a step but its result; false: not the plain form.
 bool fill_fp8(ws_fp8_gemm_args_t &a, PyObject *ox, PyObject *ow, PyObject *os, int32_t bn, int32_t bk, int64_t row0, int64_t k0) {
     const at::Tensor *x = tensor(ox), *w = tensor(ow), *s = tensor(os);
@@ -42,7 +51,7 @@ bool fill_fp8(ws_fp8_gemm_args_t &a, PyObject *ox, PyObject *ow, PyObject *os, i
     else return false;
     if (!act_dtype(*x, &a.x_dtype) || x->stride(1) != 1 || w->stride(1) != 1 || !s->is_contiguous() || w->size(1) != x->size(1)) return false;
     const int64_t m = x->size(0), n = w->size(0), k = x->size(1);
-    if (m > INT32_MAX || n > INT32_MAX || k > INT32_MAX) return false;
+    if (m > INT32_MAX || n > INT32_MAX || k > INT32_MAX || !covers(*s, row0, n, bn)) return false;
     a.m = (int32_t)m; a.n = (int32_t)n; a.k = (int32_t)k;
     a.x = x->data_ptr(); a.ldx = m > 1 ? x->stride(0) : k;
     a.w = static_cast<const uint8_t *>(w->data_ptr()); a.ldw = w->stride(0);
@@ -56,7 +65,9 @@ bool fill_moe(ws_moe_down_args_t &a, PyObject *oh, PyObject *oids, PyObject *orw
     if (!h || !ids || !rw || !w || !s || w->dim() != 3 || s->dim() != 3 || ids->dim() != 2 || h->dim() != 2) return false;
     if (!w->is_contiguous() || !s->is_contiguous() || !ids->is_contiguous() || !rw->is_contiguous()) return false;
     if (ids->scalar_type() != at::kInt || rw->scalar_type() != at::kFloat || !act_dtype(*h, &a.h_dtype)) return false;
-    const int64_t k = w->size(2) * 2;
+    const int64_t k = w->size(2) * 2, routes = ids->numel();
+    if (w->element_size() != 1 || s->element_size() != 1 || s->numel() * 16 < w->numel()) return false;
+    if (h->size(0) < routes || h->size(1) < k || h->stride(1) != 1 || rw->numel() < routes) return false;
     a.h = h->data_ptr(); a.ldh = h->size(0) > 1 ? h->stride(0) : k;
     a.m = (int32_t)ids->size(0); a.top_k = (int32_t)ids->size(1); a.n = (int32_t)w->size(1); a.k = (int32_t)k;
     a.route_ids = ids->data_ptr<int32_t>(); a.route_w = rw->data_ptr<float>();
@@ -107,7 +118,7 @@ PyObject *py_fp8(PyObject *, PyObject *const *v, Py_ssize_t nargs) {
         res = THPVariable_Wrap(std::move(out));
     } else {
         const at::Tensor *out = tensor(v[8]);
-        if (!out) Py_RETURN_NONE;
+        if (!out || !holds(*out, a.m, a.n)) Py_RETURN_NONE;
         a.out = static_cast<float *>(out->data_ptr());
         Py_INCREF(v[8]);
         res = v[8];
@@ -118,7 +129,7 @@ PyObject *py_fp8(PyObject *, PyObject *const *v, Py_ssize_t nargs) {
 }
 
 // fp8_host(handle, x_host, w, scales, block_n, block_k, row0, k0, x_dtype, out_host) -> status: x_host and out_host are
-// C-contiguous buffers (numpy arrays) that the caller has checked the lengths of.
+// C-contiguous buffers (numpy arrays) of at least m * k activations and m * n floats.
 PyObject *py_fp8_host(PyObject *, PyObject *const *v, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     if (nargs != 10) { PyErr_SetString(PyExc_TypeError, "fp8_host takes 10 arguments"); return nullptr; }
@@ -128,7 +139,8 @@ PyObject *py_fp8_host(PyObject *, PyObject *const *v, Py_ssize_t nargs) {
     a.block_n = (int32_t)PyLong_AsLong(v[4]); a.block_k = (int32_t)PyLong_AsLong(v[5]);
     a.row0 = PyLong_AsLongLong(v[6]); a.k0 = PyLong_AsLongLong(v[7]); a.x_dtype = (int32_t)PyLong_AsLong(v[8]);
     if (PyErr_Occurred()) return nullptr;
-    if (!w || !s || w->dim() != 2 || s->dim() != 2) Py_RETURN_NONE;
+    if (!w || !s || w->dim() != 2 || s->dim() != 2 || w->stride(1) != 1 || w->element_size() != 1) Py_RETURN_NONE;
+    if (!s->is_contiguous() || !covers(*s, a.row0, w->size(0), a.block_n)) Py_RETURN_NONE;
     if (s->scalar_type() == at::kFloat) a.scale_kind = WS_SCALE_F32;
     else if (s->scalar_type() == at::kByte) a.scale_kind = WS_SCALE_UE8M0;
     else Py_RETURN_NONE;
@@ -139,9 +151,17 @@ PyObject *py_fp8_host(PyObject *, PyObject *const *v, Py_ssize_t nargs) {
     a.m = x.ndim > 0 ? (int32_t)x.shape[0] : 0;
     a.ldx = a.k; a.w = static_cast<const uint8_t *>(w->data_ptr()); a.ldw = w->stride(0);
     a.scales = s->data_ptr(); a.scale_ld = s->size(1);
-    WS_CALL(st, ws_fp8_rowpar_gemm_allreduce_host(tp, &a, x.buf, static_cast<float *>(out.buf)))
+    const int64_t es = a.x_dtype == WS_ACT_BF16 ? 2 : 4;
+    const bool fits = x.len >= es * a.m * a.k && out.len >= (int64_t)4 * a.m * a.n;
+    ws_status_t st = WS_OK;
+    if (fits) {
+        Py_BEGIN_ALLOW_THREADS
+        st = ws_fp8_rowpar_gemm_allreduce_host(tp, &a, x.buf, static_cast<float *>(out.buf));
+        Py_END_ALLOW_THREADS
+    }
     PyBuffer_Release(&x);
     PyBuffer_Release(&out);
+    if (!fits) Py_RETURN_NONE;
     return PyLong_FromLong(st);
     END_HANDLE_TH_ERRORS
 }
@@ -163,7 +183,7 @@ PyObject *py_moe(PyObject *, PyObject *const *v, Py_ssize_t nargs) {
         res = THPVariable_Wrap(std::move(out));
     } else {
         const at::Tensor *out = tensor(v[7]);
-        if (!out) Py_RETURN_NONE;
+        if (!out || !holds(*out, a.m, a.n)) Py_RETURN_NONE;
         a.out = static_cast<float *>(out->data_ptr());
         Py_INCREF(v[7]);
         res = v[7];

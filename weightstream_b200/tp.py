@@ -121,6 +121,21 @@ def _scale_kind(t: torch.Tensor) -> int:
     raise TypeError(f"scales must be uint8 (UE8M0) or fp32, got {t.dtype}")
 
 
+def _check_weight(w, scales, block, row0) -> None:
+    """What the kernels read of a weight shard is there.  (The C ABI knows neither sizes nor inner strides.)"""
+    if w.stride(1) != 1 or w.element_size() != 1 or not scales.is_contiguous():
+        raise ValueError("w needs one-byte elements with unit inner stride; scales must be contiguous")
+    n, bn = w.shape[0], block[0]
+    if bn > 0 and row0 >= 0 and n > 0 and (row0 + n - 1) // bn >= scales.shape[0]:
+        raise ValueError(f"scales hold {scales.shape[0]} rows of {bn}-row blocks, but rows [{row0}, {row0 + n}) need "
+                         f"{(row0 + n - 1) // bn + 1}")
+
+
+def _check_out(out, m, n) -> None:
+    if out is not None and (out.dtype != torch.float32 or not out.is_contiguous() or out.numel() < m * n):
+        raise ValueError(f"out must be contiguous fp32 with room for [{m}, {n}]")
+
+
 def _fp8_args(x, w, scales, block, row0, k0, out) -> Fp8GemmArgs:
     if x.dim() != 2 or w.dim() != 2 or scales.dim() != 2:
         raise ValueError("x, w and scales must be 2-D")
@@ -132,6 +147,8 @@ def _fp8_args(x, w, scales, block, row0, k0, out) -> Fp8GemmArgs:
     n = w.shape[0]
     if w.shape[1] != k:
         raise ValueError(f"x has k={k} but w has {w.shape[1]} columns")
+    _check_weight(w, scales, block, row0)
+    _check_out(out, m, n)
     a = Fp8GemmArgs()
     a.x, a.ldx, a.x_dtype = x.data_ptr(), (x.stride(0) if m > 1 else k), _act_dtype(x)
     a.m, a.n, a.k = m, n, k
@@ -315,7 +332,10 @@ class Endpoint:
         if st is not None:
             self._result(st)
             return out
-        a = Fp8GemmArgs()  # read-only or otherwise unexported buffers
+        if xh.nbytes < m * k * (2 if x_dtype == WS_ACT_BF16 else 4):
+            raise ValueError(f"x_host holds {xh.nbytes} bytes: too few for [{m}, {k}] activations of this type")
+        _check_weight(w, scales, block, row0)
+        a = Fp8GemmArgs()  # otherwise unexported buffers
         a.x, a.ldx, a.x_dtype = None, k, x_dtype
         a.m, a.n, a.k = m, n, k
         a.w, a.ldw = w.data_ptr(), w.stride(0)
@@ -335,6 +355,11 @@ def _moe_args(h, route_ids, route_w, w2, s2, e_start, out) -> MoeDownArgs:
         raise TypeError("route_ids must be int32 and route_w float32")
     e_len, n, half = w2.shape
     m, top_k = route_ids.shape
+    if w2.element_size() != 1 or s2.element_size() != 1 or s2.numel() * 16 < w2.numel():
+        raise ValueError("w2 needs one-byte elements and s2 one byte for each 32 values of w2")
+    if h.dim() != 2 or h.stride(1) != 1 or h.shape[0] < m * top_k or h.shape[1] < half * 2 or route_w.numel() < m * top_k:
+        raise ValueError(f"h must be [{m * top_k}, {half * 2}] with unit inner stride, route_w one weight per route")
+    _check_out(out, m, n)
     a = MoeDownArgs()
     a.h, a.ldh, a.h_dtype = h.data_ptr(), (h.stride(0) if h.shape[0] > 1 else half * 2), _act_dtype(h)
     a.m, a.n, a.k, a.top_k = m, n, half * 2, top_k
