@@ -36,6 +36,20 @@ def test_no_device_is_an_error_not_a_fallback():
     assert L.ws_tp_create(2, 2, 0, C.byref(cfg), C.byref(h)) == _lib.WS_ERR_INVALID
 
 
+def test_front_end_built_for_another_torch_is_stale(tmp_path, monkeypatch):
+    from weightstream_b200 import build as b
+    ext = tmp_path / "_ws_torch.so"
+    monkeypatch.setattr(b, "TORCH_EXT", str(ext))
+    assert b._torch_ext_is_stale()
+    ext.write_bytes(b"")
+    os.utime(ext, (2 ** 31, 2 ** 31))  # newer than every source
+    assert b._torch_ext_is_stale()  # nothing says what it was built for
+    (tmp_path / "_ws_torch.so.abi").write_text(b._abi())
+    assert not b._torch_ext_is_stale()
+    monkeypatch.setattr(b, "_abi", lambda: "python 3.12 torch another")
+    assert b._torch_ext_is_stale()
+
+
 def test_product_code_never_touches_the_oracle():
     """The oracle is a checker: nothing in the package may import, load or link it."""
     pkg = os.path.join(ROOT, "weightstream_b200")

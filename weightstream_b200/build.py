@@ -34,8 +34,20 @@ def is_stale() -> bool:
     return _older(LIB, [os.path.join(CSRC, f) for f in SOURCES + HEADERS]) or _torch_ext_is_stale()
 
 
+def _abi() -> str:
+    """What the front end's binary interface depends on, kept beside it: it loads with no other Python or torch."""
+    from importlib.metadata import version
+    return f"python {sys.version_info[0]}.{sys.version_info[1]} torch {version('torch')}"
+
+
 def _torch_ext_is_stale() -> bool:
-    return _older(TORCH_EXT, [os.path.join(CSRC, "ws_torch.cpp"), os.path.join(CSRC, HEADERS[-1])])
+    if _older(TORCH_EXT, [os.path.join(CSRC, "ws_torch.cpp"), os.path.join(CSRC, HEADERS[-1])]):
+        return True
+    try:
+        with open(TORCH_EXT + ".abi") as f:
+            return f.read() != _abi()
+    except OSError:
+        return True
 
 
 def _run(cmd, verbose: bool) -> None:
@@ -63,6 +75,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
               "-I" + cuda, "-I" + sysconfig.get_paths()["include"], os.path.join(CSRC, "ws_torch.cpp"), "-o", TORCH_EXT,
               "-L" + HERE, "-lws_tp", "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
               "-Wl,-rpath,$ORIGIN"], verbose)
+        with open(TORCH_EXT + ".abi", "w") as f:
+            f.write(_abi())
     return LIB
 
 
