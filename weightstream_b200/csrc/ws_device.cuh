@@ -238,18 +238,6 @@ __device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t v) {
     asm("{.reg .b16 t; cvt.u16.u32 t, %1; cvt.rn.f16x2.e4m3x2 %0, t;}" : "=r"(r) : "r"(v));
     return r;
 }
-// Two E2M1 codes (the low byte of v; low nibble -> low half) -> f16x2, exact.
-__device__ __forceinline__ uint32_t e2m1x2_to_f16x2(uint32_t v) {
-    uint32_t r;
-    asm("{.reg .b8 b; .reg .b16 t; cvt.u16.u32 t, %1; cvt.u8.u16 b, t; cvt.rn.f16x2.e2m1x2 %0, b;}" : "=r"(r) : "r"(v));
-    return r;
-}
-// f16x2 -> two f32 (exact).
-__device__ __forceinline__ float2 f16x2_to_f32x2(uint32_t v) {
-    float2 r;
-    asm("{.reg .f16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h;}" : "=f"(r.x), "=f"(r.y) : "r"(v));
-    return r;
-}
 // Two E4M3 bytes, the low (H = 0) or high (H = 1) half of v, -> f16x2 (exact).  The half is
 // named by a register unpack so that the conversion can take it as an operand modifier.
 template <int H>
