@@ -70,6 +70,7 @@ struct ws_tp {
     Scratch bs_work;   // tcgen05 FP8 step: quantised activations and their scale atoms
     std::vector<void *> outgrown;
     int moe_bs = 1;  // 0: the MoE step stays on the CUDA-core decode form
+    bool tile = false;  // the prefill kernel may run: its warpgroups' register split fits what a block is launched with
     std::string err;
 };
 
@@ -319,6 +320,10 @@ ws_status_t ws_tp_create(int32_t world, int32_t rank, int32_t device, const ws_t
         cudaFuncSetAttribute(act_prep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         cudaFuncSetAttribute(stage_in_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
         return bail(WS_ERR_CUDA);
+    cudaFuncAttributes f{}, g{};
+    if (cudaFuncGetAttributes(&f, fp8_tile_kernel<false>) != cudaSuccess || cudaFuncGetAttributes(&g, fp8_tile_kernel<true>) != cudaSuccess)
+        return bail(WS_ERR_CUDA);
+    tp->tile = std::min(f.numRegs, g.numRegs) * kTileThreads >= 128 * kTileRegsFeed + 256 * kTileRegsSum;  // (built otherwise it would wait forever)
     *out = tp;
     return WS_OK;
 }
@@ -952,7 +957,7 @@ ws_status_t ws_fp8_rowpar_gemm_allreduce_group(ws_tp_t *const *ranks, int32_t n,
     if (args[0].m > t0->cfg.max_m || args[0].n > t0->cfg.max_n)
         return fail(t0, WS_ERR_CAPACITY, "m=%d n=%d exceed the endpoint's max_m=%d max_n=%d", args[0].m, args[0].n,
                     t0->cfg.max_m, t0->cfg.max_n);
-    if (n == 1 && t0->world == 1 && args[0].m > kBsMaxTokens && bs_wanted(t0, kBsMaxTokens, args[0])) {  // prefill on a lone rank
+    if (t0->tile && n == 1 && t0->world == 1 && args[0].m > kBsMaxTokens && bs_wanted(t0, kBsMaxTokens, args[0])) {  // prefill on a lone rank
         const int rows = (args[0].m + (args[0].m - 1) / kTileMaxRows) / ((args[0].m - 1) / kTileMaxRows + 1);  // equal launches
         ws_fp8_gemm_args_t a = args[0];
         a.m = std::min(a.m, rows);

@@ -23,6 +23,7 @@ namespace ws {
 constexpr int kTileTokens = 224;   // most tokens of a tile: two accumulators and the scale columns fill tensor memory
 constexpr int kTileThreads = 384;  // warpgroup 0: producer, MMA issue, scale atoms (UE8M0); 1 and 2: epilogue
 constexpr int kTileMaxStages = 8;
+constexpr int kTileRegsFeed = 56, kTileRegsSum = 216;  // registers a thread of warpgroup 0 / of 1 and 2: 128 x 56 + 256 x 216 <= 384 x 168
 
 struct alignas(64) TileParams {
     CUtensorMap tmap_w;                // weight shard [n][k bytes], box 128 bytes x 128 rows, 128B swizzle
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
     const int64_t tile_bytes = (int64_t)KS * (p.tokens * 128 + atom);
 
     if (warp < 4) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");  // 128 x 56 + 256 x 216 <= 384 x 168
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTileRegsFeed));
         if (warp == 0) {
             // -------------------------------------------------------- producer (one thread)
             if (elect_one()) {
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) fp8_tile_kernel(const __grid_
         __syncwarp();
     } else {
         // ------------------------------------------------------------ epilogue warps
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTileRegsSum));
         const int quad = warp & 3, rc = quad * 32 + lane, half = (warp >> 2) - 1;  // TMEM lane quarter; which half of the tokens
         const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
         asm volatile("griddepcontrol.wait;" ::: "memory");
