@@ -126,7 +126,7 @@ def test_ue8m0_sums_against_64_bits(dev, m):
 
 
 @pytest.mark.parametrize("world", [2, 8])
-@pytest.mark.parametrize("m", [1, 3, 40])  # tokens in pairs, one left over; sums by owners from 32 rows on four ranks
+@pytest.mark.parametrize("m", [1, 3, 40])  # tokens in pairs, one left over; sums by owners from 17 rows on four ranks
 def test_fold_of_virtual_ranks(dev, oracle, world, m):
     from weightstream_b200 import formats as F, synth, tp
     n, k = 1040, 256  # K per rank; the last tile of rows is short

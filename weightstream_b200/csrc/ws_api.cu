@@ -584,7 +584,8 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     p.csize = u.csize;
     p.tmem_cols = u.tmem_cols;
     p.x_dtype = a0.x_dtype;
-    // 32 rows and more on four ranks and more: all-to-all of every partial sum costs more link time than the second hop
+    // 17 rows and more (32 MMA columns) on four ranks and more: all-to-all of every partial sum costs more link time than
+    // the second hop (o_proj 64 rows on four GPUs 48.8 against 44.5 us)
     p.owner_reduce = (t0->world >= 4 && u.mp >= 32) ? 1 : 0;
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
@@ -1031,7 +1032,7 @@ ws_status_t ws_lm_head_allgather_argmax(ws_tp_t *tp, const ws_lm_head_args_t *ar
 
 // ------------------------------------------------------------------------------ MoE down
 // Plan of the MoE step on the tcgen05 path; ok = false when the shape does not fit it (CTA pairs split K
-// in halves of at most 16 slabs, a pair's rows are one MMA tile, the per-token sums live in shared memory).
+// in halves of at most 16 slabs, a pair's rows are one MMA tile, the per-token sums live in tensor memory).
 struct MoeBsPlan {
     bool ok;
     int ncta, tile_rows, a_pitch, slabs_per_stage, nstages, tmem_cols, x_pitch, alias, inline_x;
@@ -1230,8 +1231,8 @@ ws_status_t ws_moe_down_combine_allreduce_group(ws_tp_t *const *ranks, int32_t n
         if (args[i].e_len != e_len_all) return fail(t0, WS_ERR_INVALID, "ranks must hold equally many experts");
     if (t0->kernel_sel != 1 && (n == 1 || !same) && (reinterpret_cast<uintptr_t>(a0.w2) & 31) == 0) {  // tcgen05 form
         const MoeBsPlan u = moe_bs_plan(a0, ncta);
-        // measured on B200 (384 experts of 7168x2048, top-6), tcgen05 against the CUDA-core decode form:
-        // 1 token 19.5 against 23.6 us, 8 tokens 95 against 130, 64 tokens 495 against 841
+        // measured on B200 (384 experts of 7168x2048, top-6, chained steps), tcgen05 against the CUDA-core decode form:
+        // 1 token 14.7 against 23.5 us, 8 tokens 69 against 128, 64 tokens 329 against 836
         if (u.ok && t0->moe_bs) return moe_bs_step(ranks, n, args, streams, u);
     }
     if (t0->kernel_sel != 1 && a0.k <= 32 * 32 * kMoeGemvWarps)  // decode form: CUDA-core matrix-vector products

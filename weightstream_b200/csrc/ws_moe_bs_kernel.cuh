@@ -27,7 +27,7 @@
 //                       Warp 1 lane 0 copies both atoms of a slab into tensor memory and issues its
 //                       four MMAs; one commit per stage frees it, one per pass hands the accumulator
 //                       (16 columns, double-buffered) to the four epilogue warps, which add column t
-//                       to the shared-memory sums of the token that route belongs to.  After the last
+//                       to the tensor-memory sums of the token that route belongs to.  After the last
 //                       pass the CTAs of a pair swap their sums through distributed shared memory, each
 //                       adds the halves of K for half of the tokens and stores or exchanges those rows.
 //
