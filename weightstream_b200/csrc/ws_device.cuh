@@ -35,7 +35,7 @@ enum : uint32_t {
 // Every rank allocates one region with this layout; peers map it and store into it.
 struct SymLayout {
     int64_t flags_off;   // u32  [2 banks][R src][kMaxCtas + kMaxShared]
-    int64_t pairs_off;   // u64  [2][R][kMaxCtas][max_m]      (argmax candidates)
+    int64_t pairs_off;   // u64  [2][R][kMaxCtas][max_m]      (argmax candidates; tcgen05 kernel [2][R][max_m][kMaxCtas])
     int64_t slotf_off;   // f32  [2][R][max_m*max_n]  plain-float slots (flag-synchronised exchanges: gather, MMA-form MoE, tcgen05 kernel)
     int64_t slota_off;   // u64  [2][R][max_m*max_n]  {step sequence, fp32 bits} words of the all-reduce
     int64_t gather_off;  // f32  [2][max_m*max_vocab]

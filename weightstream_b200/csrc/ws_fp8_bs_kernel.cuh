@@ -187,6 +187,12 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
     return s;
 }
 
+template <int MP, bool WUE, bool INL>
+__device__ __forceinline__ BsSmem bs_layout(const BsParams &p) {
+    return bs_smem_layout(p.nstages, p.slabs_per_stage, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? (p.m + 1) / 2 : 0, WUE,
+                          INL ? (p.ks + p.csize - 1) / p.csize * (p.m * 128 + bs_atom_bytes(p.m)) : 0);
+}
+
 // ---- tcgen05 wrappers
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
@@ -522,6 +528,127 @@ static __device__ __noinline__ void bs_fold(const BsParams &p, int ew, int cp) {
         }
 }
 
+// What follows a CTA's finished tiles in an lm_head step, by its epilogue warps.  The argmax: the CTAs of a rank leave
+// their candidates in the rank's own table; the CTA that arrives last merges them into ONE (value, lowest index) per
+// token, sends it to every peer and merges the ranks' candidates: one 64-bit store and one flag per peer and step instead
+// of one per CTA.  Then the gathered logits.  A function of its own, which finds its shared memory itself, for the same
+// reason as bs_fold: inside the epilogue it cost the main loops of 64 rows their registers (an all-reduce step of 40 rows
+// 21.3 us instead of 19.8; 64 rows of logits over 62944 x 4352 77.7 instead of 64.2).
+template <int MP, bool WUE, bool INL>
+static __device__ __noinline__ void bs_lm_head(const BsParams &p) {
+    constexpr int EW = bs_epi_warps(MP), ET = EW * 32, CP = MP * 4 / EW;
+    if (threadIdx.x < 64 || threadIdx.x >= 64 + ET) return;
+    extern __shared__ uint8_t smem_raw[];
+    const BsSmem S = bs_layout<MP, WUE, INL>(p);
+    uint8_t *smem = smem_raw + (((smem_u32(smem_raw) + 1023u) & ~1023u) - smem_u32(smem_raw));
+    const float *cv_s = reinterpret_cast<const float *>(smem + S.cand);
+    const uint32_t *ci_s = reinterpret_cast<const uint32_t *>(smem + S.cand) + EW * MP;
+    volatile uint32_t *last_s = reinterpret_cast<uint32_t *>(smem + S.misc) + 4;
+    auto bs_epi_bar = [] { bs_epi_bar_n<ET>(); };
+    const Fp8RankArgs &A = p.r[blockIdx.y];
+    const RankCtx &X = A.ctx;
+    const int et = (int)threadIdx.x - 64, ew = et >> 5, lane = et & 31, cta = blockIdx.x, ncta = gridDim.x;
+    const uint32_t seq = step_begin(X), bank = seq & 1u;
+    const int nflag = kMaxCtas + kMaxShared;
+    const uint32_t *myflags = reinterpret_cast<const uint32_t *>(X.sym[X.rank] + p.lay.flags_off) + (size_t)bank * p.world * nflag;
+    bs_epi_bar();
+    auto pairs_of = [&](int r) { return reinterpret_cast<uint64_t *>(X.sym[r] + p.lay.pairs_off) + (size_t)bank * p.world * kMaxCtas * p.lay.max_m; };
+    uint64_t *table = pairs_of(X.rank) + (size_t)X.rank * p.lay.max_m * kMaxCtas;  // [token][CTA]
+    if (et < p.m) {  // token et: the four warps (one per lane quarter) that hold its column
+        const int w0 = (et / CP) * 4;
+        float bv = cv_s[w0 * MP + et];
+        uint32_t bi = ci_s[w0 * MP + et];
+        for (int w = w0 + 1; w < w0 + 4; ++w)
+            if (cand_better(cv_s[w * MP + et], ci_s[w * MP + et], bv, bi)) { bv = cv_s[w * MP + et]; bi = ci_s[w * MP + et]; }
+        table[(size_t)et * kMaxCtas + cta] = ((uint64_t)__float_as_uint(bv) << 32) | bi;
+    }
+    bs_epi_bar();
+    if (et == 0) {
+        __threadfence();
+        const bool last = atomicAdd(X.counters, 1u) + 1u == (uint32_t)ncta;
+        if (last) {
+            X.counters[0] = 0u;  // ready for the next step
+            __threadfence();
+        }
+        *last_s = last ? 1u : 0u;
+    }
+    bs_epi_bar();
+    if (*last_s) {
+        constexpr int kRankSlot = kMaxCtas - 1;  // a token's slot for the rank's merged candidate (a rank runs fewer CTAs than that)
+        // Best of `count` (at most kMaxCtas) entries of the tokens t, t + EW, ...: a warp requests all entries of four
+        // tokens before it looks at the first (one by one, the merge of 15 tokens was 10 us of a 30 us step).
+        auto merge = [&](int count, auto entry, auto done) {
+            constexpr int U = 4, J = kMaxCtas / 32;
+            for (int t0 = ew; t0 < p.m; t0 += U * EW) {
+                uint64_t pr[U][J];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int j = 0; j < J; ++j)
+                        if (t0 + u * EW < p.m && j * 32 + lane < count) pr[u][j] = ld_volatile_u64(entry(t0 + u * EW, j * 32 + lane));
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (t0 + u * EW >= p.m) break;
+                    float bv = -INFINITY;
+                    uint32_t bi = 0xFFFFFFFFu;
+#pragma unroll
+                    for (int j = 0; j < J; ++j) {
+                        const float v = __uint_as_float((uint32_t)(pr[u][j] >> 32));
+                        if (j * 32 + lane < count && cand_better(v, (uint32_t)pr[u][j], bv, bi)) { bv = v; bi = (uint32_t)pr[u][j]; }
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+                        const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                        if (cand_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+                    }
+                    done(t0 + u * EW, bv, bi);
+                }
+            }
+        };
+        auto answer = [&](int t, float, uint32_t bi) {
+            if (lane == 0 && A.argmax != nullptr) A.argmax[t] = bi == 0xFFFFFFFFu ? 0u : bi;
+        };
+        auto own = [&](int t, int i) { return table + (size_t)t * kMaxCtas + i; };
+        if (p.world == 1) {
+            merge(ncta, own, answer);
+        } else {
+            merge(ncta, own, [&](int t, float bv, uint32_t bi) {
+                if (lane < p.world)
+                    pairs_of(lane)[((size_t)X.rank * p.lay.max_m + t) * kMaxCtas + kRankSlot] = ((uint64_t)__float_as_uint(bv) << 32) | bi;
+            });
+            bs_epi_bar();  // the st.release.sys below is cumulative over the stores this barrier ordered
+            if (et < p.world) {
+                uint32_t *f = reinterpret_cast<uint32_t *>(X.sym[et] + p.lay.flags_off) + ((size_t)bank * p.world + X.rank) * nflag;
+                st_release_sys(f + kMaxCtas + 1, seq);
+                wait_flag(myflags + (size_t)et * nflag + kMaxCtas + 1, seq, p.timeout_ns, X.status, kStatTimeoutGather);
+            }
+            bs_epi_bar();
+            merge(p.world, [&](int t, int r) { return pairs_of(X.rank) + ((size_t)r * p.lay.max_m + t) * kMaxCtas + kRankSlot; }, answer);
+        }
+    }
+    if (p.gather_logits && p.world > 1) {
+        // every CTA's rows are in every rank's gather buffer once its flag is there (the barriers above
+        // order the stores before this release); each CTA then copies a share of the vocabulary out
+        if (et < p.world) {
+            uint32_t *f = reinterpret_cast<uint32_t *>(X.sym[et] + p.lay.flags_off) + ((size_t)bank * p.world + X.rank) * nflag;
+            st_release_sys(f + cta, seq);
+        }
+        if (A.logits != nullptr) {
+            for (int i = et; i < p.world * ncta; i += ET)
+                wait_flag(myflags + (size_t)(i / ncta) * nflag + (i % ncta), seq, p.timeout_ns, X.status, kStatTimeoutGather);
+            bs_epi_bar();
+            const float *gl = reinterpret_cast<const float *>(X.sym[X.rank] + p.lay.gather_off) +
+                              (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab;
+            const int64_t per = ((int64_t)p.vocab + ncta - 1) / ncta;
+            const int64_t v0 = (int64_t)cta * per, v1 = min((int64_t)p.vocab, v0 + per);
+            for (int tok = 0; tok < p.m; ++tok)
+                for (int64_t v = v0 + et; v < v1; v += ET)
+                    A.logits[(size_t)tok * p.vocab + v] = __ldcg(gl + (size_t)tok * p.lay.max_vocab + v);
+        }
+    }
+}
+
 template <int MP, bool WUE, bool INL>
 __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, WUE, INL)) fp8_bs_kernel(const __grid_constant__ BsParams p) {
     constexpr int EW = bs_epi_warps(MP), ET = EW * 32;  // epilogue warps / threads
@@ -546,8 +673,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
     const int SL = p.slabs_per_stage, NS = p.nstages, NB = p.nacc, AS = (SL + CH - 1) / CH;  // AS accumulators per stage
     const int ntiles = p.ntiles, TR = p.tile_rows;
 
-    const BsSmem S = bs_smem_layout(NS, SL, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? (p.m + 1) / 2 : 0, WUE,
-                                    INL ? (KS + p.csize - 1) / p.csize * (p.m * 128 + bs_atom_bytes(p.m)) : 0);
+    const BsSmem S = bs_layout<MP, WUE, INL>(p);
     float *sw_s = reinterpret_cast<float *>(smem + S.sw);
     uint32_t *misc_s = reinterpret_cast<uint32_t *>(smem + S.misc);
     const uint32_t a0 = smem_u32(smem + S.a), x0 = smem_u32(smem + S.x), wsf0 = smem_u32(smem + S.wsf);
@@ -990,98 +1116,6 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
             finalize(acc, tile, lo, hi);
             ++ntile_done;
         }
-
-        // ---- exchange (the epilogue threads)
-        const uint32_t *myflags = solo ? nullptr
-                                       : reinterpret_cast<const uint32_t *>(X.sym[X.rank] + p.lay.flags_off) + (size_t)bank * p.world * nflag;
-        if (p.mode == kModeLmHead) {
-            // The argmax.  The CTAs of a rank leave their candidates in the rank's own
-            // table; the CTA that arrives last merges them into ONE (value, lowest index) per token,
-            // sends it to every peer and merges the ranks' candidates: one 64-bit store and one flag
-            // per peer and step instead of one per CTA.
-            bs_epi_bar();
-            uint64_t *table = reinterpret_cast<uint64_t *>(X.sym[X.rank] + p.lay.pairs_off) + (size_t)bank * p.world * kMaxCtas * p.lay.max_m;
-            if (et < p.m) {  // token et: the four warps (one per lane quarter) that hold its column
-                const int w0 = (et / CP) * 4;
-                float bv = cv_s[w0 * MP + et];
-                uint32_t bi = ci_s[w0 * MP + et];
-                for (int w = w0 + 1; w < w0 + 4; ++w)
-                    if (cand_better(cv_s[w * MP + et], ci_s[w * MP + et], bv, bi)) { bv = cv_s[w * MP + et]; bi = ci_s[w * MP + et]; }
-                table[((size_t)X.rank * kMaxCtas + cta) * p.lay.max_m + et] = ((uint64_t)__float_as_uint(bv) << 32) | bi;
-            }
-            volatile uint32_t *last_s = misc_s + 4;
-            bs_epi_bar();
-            if (et == 0) {
-                __threadfence();
-                const bool last = atomicAdd(X.counters, 1u) + 1u == (uint32_t)ncta;
-                if (last) {
-                    X.counters[0] = 0u;  // ready for the next step
-                    __threadfence();
-                }
-                *last_s = last ? 1u : 0u;
-            }
-            bs_epi_bar();
-            if (*last_s) {
-                constexpr int kRankRow = kMaxCtas - 1;  // table row of a rank's merged candidate (a rank runs fewer CTAs than that)
-                auto merge = [&](int t, int count, auto entry) {  // warp-wide: best of `count` table entries of token t
-                    float bv = -INFINITY;
-                    uint32_t bi = 0xFFFFFFFFu;
-                    for (int i = lane; i < count; i += 32) {
-                        const uint64_t pr = ld_volatile_u64(entry(i) + t);
-                        const float v = __uint_as_float((uint32_t)(pr >> 32));
-                        const uint32_t idx = (uint32_t)pr;
-                        if (cand_better(v, idx, bv, bi)) { bv = v; bi = idx; }
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                        const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                        if (cand_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-                    }
-                    return ((uint64_t)__float_as_uint(bv) << 32) | bi;
-                };
-                for (int t = ew; t < p.m; t += EW) {
-                    const uint64_t best = merge(t, ncta, [&](int i) { return table + ((size_t)X.rank * kMaxCtas + i) * p.lay.max_m; });
-                    if (lane < p.world) {
-                        uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[lane] + p.lay.pairs_off) +
-                                        (((size_t)bank * p.world + X.rank) * kMaxCtas + kRankRow) * p.lay.max_m + t;
-                        *dst = best;
-                    }
-                }
-                bs_epi_bar();  // the st.release.sys below is cumulative over the stores this barrier ordered
-                if (et < p.world) {
-                    uint32_t *f = reinterpret_cast<uint32_t *>(X.sym[et] + p.lay.flags_off) + ((size_t)bank * p.world + X.rank) * nflag;
-                    st_release_sys(f + kMaxCtas + 1, seq);
-                    wait_flag(myflags + (size_t)et * nflag + kMaxCtas + 1, seq, p.timeout_ns, X.status, kStatTimeoutGather);
-                }
-                bs_epi_bar();
-                if (A.argmax != nullptr)
-                    for (int t = ew; t < p.m; t += EW) {
-                        const uint64_t best = merge(t, p.world, [&](int i) { return table + ((size_t)i * kMaxCtas + kRankRow) * p.lay.max_m; });
-                        if (lane == 0) A.argmax[t] = ((uint32_t)best == 0xFFFFFFFFu) ? 0u : (uint32_t)best;
-                    }
-            }
-            if (p.gather_logits && p.world > 1) {
-                // every CTA's rows are in every rank's gather buffer once its flag is there (the barriers above
-                // order the stores before this release); each CTA then copies a share of the vocabulary out
-                if (et < p.world) {
-                    uint32_t *f = reinterpret_cast<uint32_t *>(X.sym[et] + p.lay.flags_off) + ((size_t)bank * p.world + X.rank) * nflag;
-                    st_release_sys(f + cta, seq);
-                }
-                if (A.logits != nullptr) {
-                    for (int i = et; i < p.world * ncta; i += ET)
-                        wait_flag(myflags + (size_t)(i / ncta) * nflag + (i % ncta), seq, p.timeout_ns, X.status, kStatTimeoutGather);
-                    bs_epi_bar();
-                    const float *gl = reinterpret_cast<const float *>(X.sym[X.rank] + p.lay.gather_off) +
-                                      (size_t)bank * p.lay.max_m * (size_t)p.lay.max_vocab;
-                    const int64_t per = ((int64_t)p.vocab + ncta - 1) / ncta;
-                    const int64_t v0 = (int64_t)cta * per, v1 = min((int64_t)p.vocab, v0 + per);
-                    for (int tok = 0; tok < p.m; ++tok)
-                        for (int64_t v = v0 + et; v < v1; v += ET)
-                            A.logits[(size_t)tok * p.vocab + v] = __ldcg(gl + (size_t)tok * p.lay.max_vocab + v);
-                }
-            }
-        }
     }
 
     // ---- teardown: every TMEM read and MMA has completed once all threads are here
@@ -1098,6 +1132,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
     }
     if (p.world > 1 && p.mode == kModeAllReduce) bs_fold(p, EW, CP);
+    if (p.mode == kModeLmHead) bs_lm_head<MP, WUE, INL>(p);
     if (p.world > 1 || p.mode == kModeLmHead) step_end(X, step_begin(X), gridDim.x);
     host_done_signal(X, gridDim.x);
 }
