@@ -317,7 +317,8 @@ ws_status_t ws_tp_create(int32_t world, int32_t rank, int32_t device, const ws_t
         // The prep kernel uses no shared memory, but a main-kernel CTA (which needs almost all of an SM's)
         // cannot move onto an SM whose L1/shared split must first change, and that has to wait for the prep
         // blocks there to leave: measured 2.5-4.5 us of late CTAs.  With the same preference nothing changes.
-        cudaFuncSetAttribute(act_prep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+        cudaFuncSetAttribute(act_prep_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+        cudaFuncSetAttribute(act_prep_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         cudaFuncSetAttribute(stage_in_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
         return bail(WS_ERR_CUDA);
     cudaFuncAttributes f{}, g{};
@@ -640,7 +641,8 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
         WS_CUDA(ranks[i], cudaSetDevice(ranks[i]->device));
         cudaStream_t cs = static_cast<cudaStream_t>(streams ? streams[i] : nullptr);
         if (!u.inline_x)
-            s = launch(ranks[i], act_prep_kernel, q, prep_blocks, nvr, kActPrepThreads, 0, cs, t0->pdl != 0, false);
+            s = launch(ranks[i], t0->host_done_arm ? act_prep_kernel<false> : act_prep_kernel<true>, q, prep_blocks, nvr, kActPrepThreads, 0, cs,
+                       t0->pdl != 0, false);
         if (s == WS_OK) s = launch(ranks[i], kernel, p, u.ncta, nvr, bs_threads(u.mp, u.wue), u.smem, cs, t0->pdl != 0, true, u.csize);
         if (s != WS_OK) t0->err = ranks[i]->err;
     }
@@ -698,7 +700,7 @@ static ws_status_t tile_step(ws_tp *tp, const ws_fp8_gemm_args_t &a, cudaStream_
     // a step, twelve 150)
     const int prep_blocks = (int)std::min<int64_t>(12 * tp->sm_count, ((int64_t)a.m * u.ks * 8 + kActPrepThreads - 1) / kActPrepThreads);
     WS_CUDA(tp, cudaSetDevice(tp->device));
-    s = launch(tp, act_prep_kernel, q, prep_blocks, 1, kActPrepThreads, 0, cs, tp->pdl != 0, false);
+    s = launch(tp, act_prep_kernel<false>, q, prep_blocks, 1, kActPrepThreads, 0, cs, tp->pdl != 0, false);
     const int grid = std::min(ncta, u.nrow * u.ntok);
     if (s == WS_OK) s = launch(tp, u.wue ? fp8_tile_kernel<true> : fp8_tile_kernel<false>, p, grid, 1, kTileThreads, u.smem, cs, tp->pdl != 0);
     return s;

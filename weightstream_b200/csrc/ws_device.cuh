@@ -163,6 +163,14 @@ struct RingPos {
 // says: that is not the two seconds that mbar_wait allows this step's own work.
 __device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Asks for the line of a step's input ahead of the wait on the predecessor, which may still be writing it: L2 is where
+// all SMs meet, so nothing stale is read later.  Inputs that have to come from HBM otherwise queue behind the 20 MB of
+// weights that the CTAs request at their start.
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_act(const void *base, int x_dtype, int64_t elem_off) {
+    prefetch_l2(static_cast<const char *>(base) + elem_off * (x_dtype == WS_ACT_BF16 ? 2 : 4));
+}
+
 // 2-D TMA tile load global -> shared, completion on an mbarrier (no multicast).
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int32_t x,
                                             int32_t y, uint32_t bar) {

@@ -110,6 +110,13 @@ __device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
             sw_s[sl * p.skb + c] = v;
         }
     }
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int k = ((slice * C + i) * 32 + lane) * 16;
+        if (k < p.k && grp < G)
+#pragma unroll
+            for (int t = 0; t < GT; ++t) prefetch_act(A.x, p.x_dtype, (int64_t)t * A.ldx + k);
+    }
     consumer_bar();
     // Everything below may read what the previous kernel on the stream wrote (activations, the step
     // sequence, exchange slots).

@@ -88,9 +88,11 @@ __device__ __forceinline__ int block_sum_256(int v, int *red_s) {  // all 256 th
 
 __global__ void __launch_bounds__(256) moe_bs_prep_kernel(const __grid_constant__ MoeBsPrepParams p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const MoePrepRank &A = p.r[blockIdx.y];
     const int NR = p.m * p.top_k, tid = threadIdx.x;
+    if ((int)blockIdx.x < NR)
+        for (int c = tid; c < (p.k >> 4); c += blockDim.x) prefetch_act(A.h, p.h_dtype, (int64_t)blockIdx.x * A.ldh + c * 16);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const MoeBsWork W = moe_bs_work_layout(p.k);
     __shared__ int32_t cnt_s[kMoeMaxExperts];
     __shared__ int red_s[8];
