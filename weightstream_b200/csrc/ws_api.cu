@@ -494,7 +494,7 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
     // 33.4) and by tensor memory (fp32 scales: each slab has its own accumulator buffer, groups x slabs x (mp + 4) + 8
     // columns of 512, at least two groups; UE8M0: one buffer for two slabs, 16 scale columns a slab)
     u.nslot_max = (tiles_per_cta * u.tile_rows) / a.block_n + 2;
-    const int rx_rows = u.csize == 2 ? (mt + 1) / 2 : 0, kcta = (u.ks + u.csize - 1) / u.csize;
+    const int rx_groups = u.csize == 2 ? bs_rx_groups(mt) : 0, kcta = (u.ks + u.csize - 1) / u.csize;
     // Half an SM (shared memory and tensor memory) when the tokens are few and the CTA's whole share of
     // the weights fits such a ring (TP-8 shards): the next step's CTA is then resident beside this one
     // (one CTA per SM and step) and loads all of its weights under this step's exchange and exit.
@@ -513,7 +513,7 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         const int accs = (u.slabs_per_stage + chain - 1) / chain;  // accumulators of a stage
         u.nacc = std::min((int)kBsMaxAcc, u.wue ? (tmem - 16 * u.slabs_per_stage) / (accs * u.mp) : (tmem - 8) / (accs * (u.mp + 4)));
         auto total = [&](int ns) {
-            return bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, u.nslot_max, skb, u.mp, rx_rows, u.wue,
+            return bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, u.nslot_max, skb, u.mp, rx_groups, u.wue,
                                   u.inline_x ? kcta * x_slab : 0).total + 1024;
         };
         int ns = kMaxStages;  // the most stages whose layout fits

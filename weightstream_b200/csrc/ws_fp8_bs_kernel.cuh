@@ -170,11 +170,16 @@ struct alignas(64) BsParams {
     const uint8_t *xq[WS_MAX_WORLD];   // the prep kernel's activations and scale atoms
 };
 
+// Of a CTA pair, CTA r finishes the groups of four tokens 2 j + r: every epilogue thread then sends half of its columns and
+// keeps half, in 16-byte words and without a test per column (each CTA half of the tokens in one run, a float at a time,
+// took 4.6 us a tile at 96 rows and 1.0 at 19: 96 rows of K 8192 28.5 us a step, 25.5 now; 8 rows of K 1024 5.84, 5.28).
+__host__ __device__ constexpr int bs_rx_groups(int m) { return ((m + 3) / 4 + 1) / 2; }
+
 struct BsSmem {
     int32_t a, x, wsf, sw, cand, rx, bars, misc, total;
 };
 __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stage, int a_pitch, int x_pitch, int nslot_max,
-                                                 int skb, int mp, int rx_rows, bool wue, int x_resident) {
+                                                 int skb, int mp, int rx_groups, bool wue, int x_resident) {
     BsSmem s{};
     const int nsl = nstages * slabs_per_stage;
     const int x_bytes = x_resident > 0 ? (x_resident + 127) / 128 * 128 : nstages * x_pitch;  // inline: all of this K half
@@ -187,7 +192,7 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
     s.wsf = o;  o += wue ? nsl * kBsAtomBytes : kBsAtomBytes;  // the weights' scale atoms (fp32 scales: one atom of 2^0)
     s.sw = o;   o += wue ? 0 : (int)align_up((int64_t)nslot_max * skb * 4, 16);
     s.cand = o; o += bs_epi_warps(mp) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
-    s.rx = o;   o += rx_rows * kBsMmaRows * 4;           // CTA pairs: the partner's sums of one tile for this CTA's tokens, [token][row]
+    s.rx = o;   o += rx_groups * kBsMmaRows * 16;        // CTA pairs: the partner's sums of one tile for this CTA's tokens, [group of 4 tokens][row][4]
     s.bars = o; o += (2 * kMaxStages + kBsMaxAcc + 4) * 8;
     s.misc = o; o += 64;
     s.total = o;
@@ -196,7 +201,7 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
 
 template <int MP, bool WUE, bool INL>
 __device__ __forceinline__ BsSmem bs_layout(const BsParams &p) {
-    return bs_smem_layout(p.nstages, p.slabs_per_stage, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? (p.m + 1) / 2 : 0, WUE,
+    return bs_smem_layout(p.nstages, p.slabs_per_stage, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? bs_rx_groups(p.m) : 0, WUE,
                           INL ? (p.ks + p.csize - 1) / p.csize * (p.m * 128 + bs_atom_bytes(p.m)) : 0);
 }
 
@@ -333,6 +338,9 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t local_addr, uint32_t cta_r
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
+__device__ __forceinline__ void st_cluster_f32x4(uint32_t addr, float a, float b, float c, float d) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {  // releases this thread's earlier stores to the cluster
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
 }
@@ -434,9 +442,12 @@ __device__ __forceinline__ float order_value(uint32_t key) { return __uint_as_fl
 // waiting for each missing word in turn took a round trip per word (40 rows on eight ranks 198 us a step, 72 now; two
 // tokens at a time 87).  A rank that stays away is left to wait_word, which
 // gives up and records it.
+// Word i is that of token (i & 3) + (i >> 2) * gap of the T; those at or past `count` are not there.
 constexpr int kFoldTokens = 4, kFoldTries = 256;
 template <int T, int R>
-__device__ __forceinline__ void fold_words(const BsParams &p, const RankCtx &X, const uint64_t *src, size_t astride, uint32_t seq, int count, float (&sum)[T]) {
+__device__ __forceinline__ void fold_words(const BsParams &p, const RankCtx &X, const uint64_t *src, size_t astride, uint32_t seq, int count, int gap,
+                                           float (&sum)[T]) {
+    auto token = [&](int i) { return (i & 3) + (i >> 2) * gap; };
     const int ranks = R == 1 ? 1 : p.world;
     bool here = false;
 #pragma unroll 1
@@ -448,7 +459,7 @@ __device__ __forceinline__ void fold_words(const BsParams &p, const RankCtx &X, 
         for (int rr = 0; rr < R; ++rr) {
             if (R == 1 || rr < ranks) {
 #pragma unroll
-                for (int i = 0; i < T; ++i) w[rr][i] = ld_word_sys(at + (int64_t)min(i, count - 1) * p.n);
+                for (int i = 0; i < T; ++i) w[rr][i] = ld_word_sys(at + (int64_t)(token(i) < count ? token(i) : 0) * p.n);
             }
             at += astride;
         }
@@ -468,10 +479,10 @@ __device__ __forceinline__ void fold_words(const BsParams &p, const RankCtx &X, 
 #pragma unroll
     for (int i = 0; i < T; ++i) {
         sum[i] = 0.0f;
-        if (i < count)
+        if (token(i) < count)
 #pragma unroll 1
             for (int rr = 0; rr < ranks; ++rr) {
-                const float v = wait_word(src + rr * astride + (int64_t)i * p.n, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
+                const float v = wait_word(src + rr * astride + (int64_t)token(i) * p.n, seq, p.timeout_ns, X.status, kStatTimeoutPeerA);
                 sum[i] = rr == 0 ? v : sum[i] + v;
             }
     }
@@ -486,11 +497,11 @@ static __device__ __noinline__ void bs_fold(const BsParams &p, int ew, int cp) {
     const Fp8RankArgs &A = p.r[vr];
     const RankCtx &X = A.ctx;
     const uint32_t seq = step_begin(X), bank = seq & 1u;
-    const int TR = p.tile_rows, part = blockIdx.x >> pair, nparts = gridDim.x >> pair, half = (p.m + 1) / 2;
+    const int TR = p.tile_rows, part = blockIdx.x >> pair, nparts = gridDim.x >> pair;
     const int t_lo = (int)((int64_t)p.ntiles * part / nparts), t_hi = (int)((int64_t)p.ntiles * (part + 1) / nparts) - 1;
     const int warp = (int)(threadIdx.x >> 5), rc = (warp & 3) * 32 + (int)(threadIdx.x & 31), col0 = ((warp - 2) >> 2) * cp;
-    const bool upper = pair && (blockIdx.x & 1);
-    const int tbeg = max(upper ? half : 0, col0), tend = min(pair && !upper ? half : p.m, col0 + cp);
+    // this thread's tokens: all of its columns', or, of a pair, every other group of four
+    const int tbeg = col0 + (pair ? 4 * (int)(blockIdx.x & 1) : 0), tend = min(p.m, col0 + cp), gap = pair ? 8 : 4;
     if (warp < 2 || warp >= 2 + ew) return;
     const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
     const uint64_t *slots = reinterpret_cast<const uint64_t *>(X.sym[X.rank] + p.lay.slota_off) + (size_t)bank * p.world * astride;
@@ -507,18 +518,20 @@ static __device__ __noinline__ void bs_fold(const BsParams &p, int ew, int cp) {
             const uint64_t *src = slots + (size_t)tbeg * p.n + row;
             float *out = A.out + (size_t)tbeg * p.n + row;
             if (owner != X.rank) {
-                for (int tok = tbeg; tok < tend; tok += 8, src += 8 * (int64_t)p.n, out += 8 * (int64_t)p.n) {
+                for (int tok = tbeg; tok < tend; tok += 2 * gap, src += 2 * gap * (int64_t)p.n, out += 2 * gap * (int64_t)p.n) {
                     float sum[8];
-                    fold_words<8, 1>(p, X, src + owner * astride, astride, seq, min(8, tend - tok), sum);
+                    fold_words<8, 1>(p, X, src + owner * astride, astride, seq, tend - tok, gap, sum);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (tok + i < tend) out[(int64_t)i * p.n] = sum[i];
+                    for (int i = 0; i < 8; ++i) {
+                        const int o = (i & 3) + (i >> 2) * gap;
+                        if (tok + o < tend) out[(int64_t)o * p.n] = sum[i];
+                    }
                 }
                 continue;
             }
-            for (int tok = tbeg; tok < tend; tok += kFoldTokens, src += kFoldTokens * (int64_t)p.n, out += kFoldTokens * (int64_t)p.n) {
+            for (int tok = tbeg; tok < tend; tok += gap, src += gap * (int64_t)p.n, out += gap * (int64_t)p.n) {
                 float sum[kFoldTokens];
-                fold_words<kFoldTokens, WS_MAX_WORLD>(p, X, src, astride, seq, min(kFoldTokens, tend - tok), sum);
+                fold_words<kFoldTokens, WS_MAX_WORLD>(p, X, src, astride, seq, tend - tok, gap, sum);
 #pragma unroll
                 for (int i = 0; i < kFoldTokens; ++i)
                     if (tok + i < tend) out[(int64_t)i * p.n] = sum[i];
@@ -964,9 +977,8 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         bs_epi_bar();
         const int kofs = (int)(A.k0 - kcol0 * ((int64_t)1 << p.bk_shift));
         const bool solo = p.mode == kModeAllReduce && p.world == 1;
-        // tokens this CTA finishes: of a pair, the first CTA the lower half, the second the upper
-        const int split = p.csize == 2 ? (p.m + 1) / 2 : p.m;
-        const int tok_lo = crank == 0 ? 0 : split, tok_hi = crank == 0 ? split : p.m;
+        // tokens this CTA finishes: bit (t >> 2) & 1 set (of a pair, each CTA every other group of four)
+        const uint32_t groups = p.csize == 2 ? 1u << crank : 3u;
         const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
         const int nflag = kMaxCtas + kMaxShared;
         float *cv_s = reinterpret_cast<float *>(smem + S.cand);        // [EW warps][MP]; a warp fills its own columns
@@ -976,7 +988,8 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
 
         // A finished tile: its rows go to the output or to the peers; of an lm_head tile the candidates are
         // kept and, when the caller wants them, the logits stored.
-        auto finalize = [&](const float (&v)[CP], int tile, const int tok_lo, const int tok_hi) {  // v[i]: token col0 + i
+        auto finalize = [&](const float (&v)[CP], int tile, const int m, const uint32_t groups) {  // v[i]: token col0 + i
+            auto done = [&](int i) { return col0 + i < m && (groups >> ((i >> 2) & 1) & 1u) != 0u; };  // (col0 is a multiple of 16)
             const int row = tile * TR + rc;
             const bool mine = rc < TR && row < p.n;
             // element (token, row) of a float matrix with `ld` floats per token
@@ -987,7 +1000,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                 float *dst = base + col0 * ld + row;
 #pragma unroll
                 for (int i = 0; i < CP; ++i) {
-                    if (col0 + i >= tok_lo && col0 + i < tok_hi) *dst = v[i];
+                    if (done(i)) *dst = v[i];
                     dst += ld;
                 }
             };
@@ -1003,7 +1016,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                         uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) + ((size_t)bank * p.world + X.rank) * astride + col0 * ld + row;
 #pragma unroll
                         for (int i = 0; i < CP; ++i) {
-                            if (col0 + i >= tok_lo && col0 + i < tok_hi) st_word_sys(dst, seq, v[i]);
+                            if (done(i)) st_word_sys(dst, seq, v[i]);
                             dst += ld;
                         }
                     }
@@ -1029,7 +1042,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                 for (int h = 0; h < H; ++h) best[h] = who[h] = 0u;
 #pragma unroll
                 for (int g = 0; g < CP; g += 8) {
-                    if (col0 + g >= tok_hi) break;  // warp-uniform
+                    if (col0 + g >= m) break;  // warp-uniform
 #pragma unroll
                     for (int i = g; i < g + 8; ++i) {
                         const uint32_t key = mine ? order_key(v[i]) : 0u;
@@ -1041,7 +1054,7 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
 #pragma unroll
                 for (int h = 0; h < H; ++h) {
                     const int c = h * 32 + lane, t = col0 + c;
-                    if (c >= CP || t < tok_lo || t >= tok_hi || best[h] == 0u) continue;
+                    if (c >= CP || !done(c) || best[h] == 0u) continue;
                     const float top = order_value(best[h]);
                     if (cand_better(top, idx0 + who[h], cv_s[ew * MP + t], ci_s[ew * MP + t])) {
                         cv_s[ew * MP + t] = top;
@@ -1103,31 +1116,37 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                 if (accempty == acc_end) { accempty = accempty0; t_col = tlane + (uint32_t)col0; }
             }
             // what depends on the tile's end only is not worth registers in the main loop: hidden from the optimiser
-            int lo = tok_lo, hi = tok_hi, m = p.m;
-            asm volatile("" : "+r"(lo), "+r"(hi), "+r"(m));
+            int m = p.m, at = col0 / 8 * kBsMmaRows + rc;
+            uint32_t gr = groups;
+            asm volatile("" : "+r"(gr), "+r"(m), "+r"(at));
             if (p.csize == 2) {
                 // a pair swaps its sums: each CTA gets the partner's for the tokens it finishes, in its shared memory
                 if (ntile_done > 0) mbar_wait_cluster(rxempty, (uint32_t)(ntile_done - 1) & 1u, X.status);  // the partner has read the previous tile's
-                const uint32_t dst = mapa_u32(smem_u32(smem + S.rx) + (uint32_t)rc * 4u, crank ^ 1u);
-                const int base = crank == 0 ? hi : 0;  // the partner's first token
+                const uint32_t rx = smem_u32(smem + S.rx) + (uint32_t)at * 16u, dst = mapa_u32(rx, crank ^ 1u);
+                auto swap = [&](auto mine) {  // K half 0 + K half 1, in that order (the sum of two does not depend on it)
+                    constexpr int R = decltype(mine)::value;
 #pragma unroll
-                for (int i = 0; i < CP; ++i) {
-                    const int t = col0 + i;
-                    if (t < m && (t < lo || t >= hi)) st_cluster_f32(dst + (uint32_t)((t - base) * kBsMmaRows * 4), acc[i]);
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(mapa_u32(rxfull, crank ^ 1u));
-                mbar_wait_cluster(rxfull, (uint32_t)ntile_done & 1u, X.status);
-                const float *rx = reinterpret_cast<const float *>(smem + S.rx) + rc;
+                    for (int i = 4 * (R ^ 1); i < CP; i += 8)
+                        if (col0 + i < m) st_cluster_f32x4(dst + (uint32_t)(i / 8 * kBsMmaRows) * 16u, acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(mapa_u32(rxfull, crank ^ 1u));
+                    mbar_wait_cluster(rxfull, (uint32_t)ntile_done & 1u, X.status);
 #pragma unroll
-                for (int i = 0; i < CP; ++i) {  // K half 0 + K half 1, in that order (the sum of two does not depend on it)
-                    const int t = col0 + i;
-                    if (t >= lo && t < hi) acc[i] += rx[(t - lo) * kBsMmaRows];
-                }
+                    for (int i = 4 * R; i < CP; i += 8)
+                        if (col0 + i < m) {
+                            const uint4 v = lds_u128(rx + (uint32_t)(i / 8 * kBsMmaRows) * 16u);
+                            acc[i] += __uint_as_float(v.x);
+                            acc[i + 1] += __uint_as_float(v.y);
+                            acc[i + 2] += __uint_as_float(v.z);
+                            acc[i + 3] += __uint_as_float(v.w);
+                        }
+                };
+                if (gr == 1u) swap(std::integral_constant<int, 0>{});
+                else swap(std::integral_constant<int, 1>{});
                 __syncwarp();
                 if (lane == 0 && tile < t_hi) mbar_arrive_cluster(mapa_u32(rxempty, crank ^ 1u));  // nobody waits for the last one
             }
-            finalize(acc, tile, lo, hi);
+            finalize(acc, tile, m, gr);
             ++ntile_done;
         }
     }
