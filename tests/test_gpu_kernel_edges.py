@@ -37,6 +37,9 @@ FP8 = [
     (1040, 1056, 0, 1056, "ue8m0", (3, 12, 13, 64, 65)),  # 33 scale columns: exponents collected byte by byte
     (1040, 1056, 128, 1280, "ue8m0", (4, 40)),       # word loads with a K tail
     (5120, 2304, 0, 2304, "ue8m0", (6, 19, 128)),    # two CTAs per SM, word loads, K halves of nine slabs
+    # CTA pairs swap groups of four tokens: a group or a half alone, ragged last groups, every accumulator width
+    (2064, 1024, 0, 1024, "f32", (4, 5, 8, 9, 15, 20, 31, 36, 63, 66, 97, 127)),
+    (2064, 1056, 0, 1056, "ue8m0", (4, 5, 9, 20, 36, 66, 127)),
     (1040, 768, 0, 768, "f32", (129, 225, 449)),     # prefill tiles: last row tile of 16, token tiles of 1 and up
     (1040, 1056, 0, 1056, "ue8m0", (129, 449)),
     (1040, 1056, 128, 1280, "ue8m0", (200,)),
@@ -306,5 +309,28 @@ def test_lm_head_logits_of_a_lone_rank(dev, oracle, vocab, k, m):
         grp.check()
         check(logits[0], want, k)
         assert torch.equal(amax[0].cpu().long(), logits[0].argmax(dim=1).cpu())
+    finally:
+        grp.close()
+
+
+@pytest.mark.parametrize("world,m", [(1, 1), (1, 4), (1, 5), (1, 33), (1, 128), (2, 5), (2, 65)])
+def test_lm_head_equal_candidates_of_many_ctas(dev, world, m):
+    """Every row of the vocabulary returns in each 1024 rows, so that every token's largest logit is there in many tiles,
+    CTAs and ranks: the answer is the first of them (whole numbers, exact)."""
+    from weightstream_b200 import formats as F, synth, tp
+    rng = np.random.default_rng(synth.config_seed("head-ties", m, world))
+    vocab, k = 17 * 1024 * world, 2048
+    w, sc = synth.fp8_weight(rng, 1024, k)
+    x = torch.from_numpy(F.bf16_bits_to_f32(synth.activations_bf16(rng, m, k))).to(dev)
+    wd, sd = torch.from_numpy(np.tile(w, (17, 1))).to(dev), torch.from_numpy(np.tile(sc, (17, 1))).to(dev)
+    grp = tp.LocalGroup(world, max_m=128, max_n=16, max_vocab=vocab)
+    try:
+        logits, amax = grp.lm_head_allgather_argmax([x] * world, [wd] * world, [sd] * world, vocab=vocab,
+                                                    vocab_row0s=[r * 17 * 1024 for r in range(world)], row0s=[0] * world)
+        grp.check()
+        want = np.argmax(logits[0].cpu().numpy(), axis=1)  # the first of equals
+        assert want.max() < 1024
+        for r in range(world):
+            assert np.array_equal(amax[r].cpu().numpy().astype(np.int64), want)
     finally:
         grp.close()
