@@ -113,7 +113,7 @@ __device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
 #pragma unroll
     for (int i = 0; i < C; ++i) {
         const int k = ((slice * C + i) * 32 + lane) * 16;
-        if (k < p.k && grp < G)
+        if (k < p.k && grp < G && X.host_done == nullptr)  // (a host-buffer call's are fetched over the bus by the launch in front)
 #pragma unroll
             for (int t = 0; t < GT; ++t) prefetch_act(A.x, p.x_dtype, (int64_t)t * A.ldx + k);
     }
