@@ -989,7 +989,8 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         // A finished tile: its rows go to the output or to the peers; of an lm_head tile the candidates are
         // kept and, when the caller wants them, the logits stored.
         auto finalize = [&](const float (&v)[CP], int tile, const int m, const uint32_t groups) {  // v[i]: token col0 + i
-            auto done = [&](int i) { return col0 + i < m && (groups >> ((i >> 2) & 1) & 1u) != 0u; };  // (col0 is a multiple of 16)
+            const bool even = (groups & 1u) != 0u, odd = (groups & 2u) != 0u;
+            auto done = [&](int i) { return col0 + i < m && ((i & 4) ? odd : even); };  // (col0 is a multiple of 16)
             const int row = tile * TR + rc;
             const bool mine = rc < TR && row < p.n;
             // element (token, row) of a float matrix with `ld` floats per token
