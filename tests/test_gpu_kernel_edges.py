@@ -152,6 +152,72 @@ def test_fold_of_virtual_ranks(dev, oracle, world, m):
         grp.close()
 
 
+def _ranks_one_after_another(grp, order, xs, ws, sd, k0s):
+    """One step of every rank, each on its own and after the one before has ended: all but the last give up on the words
+    that are not there yet (their own have been sent).  The last one's endpoint and output."""
+    from weightstream_b200 import tp
+    for r in order[:-1]:
+        grp.eps[r].fp8_rowpar_gemm_allreduce(xs[r], ws[r], sd, k0=k0s[r])
+        with pytest.raises(tp.WsError) as ei:
+            grp.eps[r].check()
+        assert ei.value.status == tp._lib.WS_ERR_TIMEOUT
+    r = order[-1]
+    return grp.eps[r], grp.eps[r].fp8_rowpar_gemm_allreduce(xs[r], ws[r], sd, k0=k0s[r])
+
+
+def _shards(dev, oracle, n, k, m, world):
+    """K slices of a step, and the fold of the oracle's partial sums."""
+    from weightstream_b200 import formats as F, synth
+    rng = np.random.default_rng(synth.config_seed("pair-fold", m, world))
+    w, sc = synth.fp8_weight(rng, n, world * k)
+    x = F.bf16_bits_to_f32(synth.activations_bf16(rng, m, world * k))
+    wd, sd, xd = torch.from_numpy(w).to(dev), torch.from_numpy(sc).to(dev), torch.from_numpy(x).to(dev)
+    cut = [slice(r * k, (r + 1) * k) for r in range(world)]
+    parts = [oracle.fp8_gemv(w[:, c], sc, np.ascontiguousarray(x[:, c]), bn=128, bk=128, k0=c.start, threads=oracle.max_threads()) for c in cut]
+    return [xd[:, c].contiguous() for c in cut], [wd[:, c] for c in cut], sd, [c.start for c in cut], oracle.allreduce_fold(np.stack(parts))
+
+
+@pytest.mark.parametrize("m", [3, 4, 5, 8, 11, 12, 16, 33, 63, 128])
+def test_fold_of_cta_pairs(dev, oracle, m):
+    """The exchange as one rank per launch runs it, on CTA pairs (virtual ranks have none): ragged and lone groups of four
+    tokens, quantised in the main kernel and ahead of it.  The last rank finds the other's words and folds them."""
+    from weightstream_b200 import tp
+    n, k = 2064, 512
+    xs, ws, sd, k0s, want = _shards(dev, oracle, n, k, m, 2)
+    grp = tp.LocalGroup(2, max_m=m, max_n=n, wait_ms=20)
+    try:
+        outs = []
+        for order in ((1, 0), (0, 1), (1, 0)):  # both banks, and the first again
+            ep, out = _ranks_one_after_another(grp, order, xs, ws, sd, k0s)
+            ep.check()
+            check(out, want, 2 * k)
+            outs.append(out)
+        assert all(torch.equal(o.view(torch.int32), outs[0].view(torch.int32)) for o in outs)
+    finally:
+        grp.close()
+
+
+@pytest.mark.parametrize("world,m", [(4, 17), (4, 21), (4, 40), (4, 63), (8, 100), (8, 128)])
+def test_owners_of_void_sums_keep_them(dev, oracle, world, m):
+    """Sums by owners: the last rank folds the tiles it owns, but those of an owner that gave up on a rank never reach
+    it, so that its step fails, too, instead of returning what was folded without that rank."""
+    from weightstream_b200 import tp
+    n, k = 2064, 256
+    xs, ws, sd, k0s, want = _shards(dev, oracle, n, k, m, world)
+    grp = tp.LocalGroup(world, max_m=m, max_n=n, wait_ms=20)
+    try:
+        for last in (0, world - 1):
+            ep, out = _ranks_one_after_another(grp, [r for r in range(world) if r != last] + [last], xs, ws, sd, k0s)
+            with pytest.raises(tp.WsError) as ei:
+                ep.check()
+            assert ei.value.status == tp._lib.WS_ERR_TIMEOUT
+            tile_rows = -(-n // (ep.num_ctas // 2))  # a tile for every CTA pair
+            mine = np.arange(n) // tile_rows % world == last
+            check(out[:, torch.from_numpy(mine).to(dev)], want[:, mine], world * k)
+    finally:
+        grp.close()
+
+
 def test_step_behind_one_that_waits_longer_than_two_seconds(dev):
     """A step that starts early (programmatic dependent launch) behind one whose peer stays away: the time its
     predecessor spends waiting (wait_ms) is not its own.  Both take half an SM and the second has more stages to

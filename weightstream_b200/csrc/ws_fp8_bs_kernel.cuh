@@ -441,11 +441,11 @@ __device__ __forceinline__ float order_value(uint32_t key) { return __uint_as_fl
 // instead of one per rank (three rows on eight ranks: 29 of a 50 us step), and requested again while one is missing:
 // waiting for each missing word in turn took a round trip per word (40 rows on eight ranks 198 us a step, 72 now; two
 // tokens at a time 87).  A rank that stays away is left to wait_word, which
-// gives up and records it.
+// gives up and records it; false then: the sums are void.
 // Word i is that of token (i & 3) + (i >> 2) * gap of the T; those at or past `count` are not there.
 constexpr int kFoldTokens = 4, kFoldTries = 256;
 template <int T, int R>
-__device__ __forceinline__ void fold_words(const BsParams &p, const RankCtx &X, const uint64_t *src, size_t astride, uint32_t seq, int count, int gap,
+__device__ __forceinline__ bool fold_words(const BsParams &p, const RankCtx &X, const uint64_t *src, size_t astride, uint32_t seq, int count, int gap,
                                            float (&sum)[T]) {
     auto token = [&](int i) { return (i & 3) + (i >> 2) * gap; };
     const int ranks = R == 1 ? 1 : p.world;
@@ -475,7 +475,7 @@ __device__ __forceinline__ void fold_words(const BsParams &p, const RankCtx &X, 
                 }
             }
     }
-    if (here) return;
+    if (here) return true;
 #pragma unroll
     for (int i = 0; i < T; ++i) {
         sum[i] = 0.0f;
@@ -486,6 +486,7 @@ __device__ __forceinline__ void fold_words(const BsParams &p, const RankCtx &X, 
                 sum[i] = rr == 0 ? v : sum[i] + v;
             }
     }
+    return *(volatile uint32_t *)X.status == 0u;
 }
 
 // The exchange behind a CTA's finished tiles: fold its rows, in rank order, as the ranks' words arrive.  Thread
@@ -531,11 +532,11 @@ static __device__ __noinline__ void bs_fold(const BsParams &p, int ew, int cp) {
             }
             for (int tok = tbeg; tok < tend; tok += gap, src += gap * (int64_t)p.n, out += gap * (int64_t)p.n) {
                 float sum[kFoldTokens];
-                fold_words<kFoldTokens, WS_MAX_WORLD>(p, X, src, astride, seq, tend - tok, gap, sum);
+                const bool valid = fold_words<kFoldTokens, WS_MAX_WORLD>(p, X, src, astride, seq, tend - tok, gap, sum);
 #pragma unroll
                 for (int i = 0; i < kFoldTokens; ++i)
                     if (tok + i < tend) out[(int64_t)i * p.n] = sum[i];
-                if (p.owner_reduce)
+                if (p.owner_reduce && valid)  // (the others time out, too, rather than take what was folded without a rank)
                     for (int pr = 0; pr < p.world; ++pr) {
                         if (pr == X.rank) continue;
                         uint64_t *dst = reinterpret_cast<uint64_t *>(X.sym[pr] + p.lay.slota_off) +
