@@ -568,6 +568,11 @@ static ws_status_t zero_lone_shard(ws_tp *const *ranks, int n, const ws_lm_head_
     return WS_OK;
 }
 
+// Whether a step's CTAs may ask for their activations before the launch in front has ended: not where that launch is still
+// fetching them over the bus (a host-buffer call: 30.5 against 30.2 us), nor of virtual ranks, whose launch does not start
+// early.
+static bool asks_ahead(const ws_tp *t0, int n, bool same_device) { return !t0->host_done_arm && !(same_device && n > 1); }
+
 // One fused step over at most kBsMaxTokens activation rows on the block-scaled tcgen05 path: the prep
 // kernel (activation quantisation once per step) followed by the persistent MMA kernel.
 static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t *args, const ws_lm_head_args_t *lm,
@@ -812,6 +817,7 @@ static ws_status_t gemv_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_
     for (p.bn_shift = 0; (1 << p.bn_shift) < a0.block_n; ++p.bn_shift) {}
     p.nslot_max = u.nslot_max; p.skb = skb; p.slices = u.slices; p.rows_per_stage = u.rows_per_stage; p.nstages = u.nstages;
     p.rows_max = u.rows_max; p.stage_bytes = u.stage_bytes;
+    p.ahead = asks_ahead(t0, n, same_device) ? 1 : 0;
     p.timeout_ns = t0->timeout_ns;
     p.lay = t0->lay;
     for (int i = 0; i < n; ++i) {
