@@ -588,6 +588,10 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     p.tile_rows = u.tile_rows; p.ntiles = u.ntiles; p.a_pitch = u.a_pitch; p.x_pitch = u.x_pitch;
     p.slabs_per_stage = u.slabs_per_stage; p.nstages = u.nstages; p.nslot_max = u.nslot_max; p.skb = skb; p.nacc = u.nacc;
     p.csize = u.csize;
+    // More than 2048 values for a CTA to quantise: fewer are read as fast as they are asked for.  (Without and with: 768 and
+    // 1536 values, K 512 and 1024, 3 rows, 4.9 us a step, 5.0 and 5.3, 5.4; 2560, K 1024, 5 rows 6.0, 5.5; 3072, K 2048, 3 rows
+    // 9.4, 8.8; 4608, UE8M0 K 2304, 4 rows 8.7, 8.3; 6144, K 4096, 3 rows 13.2, 12.6; 8192, K 1024, 16 rows 7.9, 7.2.)
+    p.ahead = u.inline_x && mt * ((u.ks + u.csize - 1) / u.csize) * 128 > 2048 && asks_ahead(t0, n, same_device) ? 1 : 0;
     p.tmem_cols = u.tmem_cols;
     p.x_dtype = a0.x_dtype;
     // 17 rows and more (32 MMA columns) on four ranks and more: all-to-all of every partial sum costs more link time than

@@ -160,6 +160,7 @@ struct alignas(64) BsParams {
     int32_t world, mode, vocab, tmem_cols;  // tmem_cols: tensor-memory columns to allocate (512, or at most 256 when two CTAs share an SM)
     int32_t owner_reduce;              // all-reduce by owners: tile t is folded by rank t % world, which sends the sums back
     int32_t csize;                     // 1, or 2: CTA pairs (a cluster) share a tile, each streams half of K
+    int32_t ahead;                     // the CTA asks for its activations ahead of the wait on the predecessor (INL)
     int32_t tile_rows, ntiles;         // output rows per tile (<= 128) and tiles of the shard
     int32_t slabs_per_stage, nstages;
     int32_t a_pitch, x_pitch;          // bytes one slab's weights (a multiple of 1024) / one stage's activations and atoms (of 128) occupy
@@ -733,8 +734,8 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         }
         __syncwarp();
     }
-    if constexpr (INL) {  // (K 1024, 16 rows 7.9 us a step without, 7.3 with; 8 rows 6.4, 5.9; 3 rows 5.3, 5.5)
-        if (p.m > 4 && warp >= 2 && warp < 2 + EW)
+    if constexpr (INL) {
+        if (p.ahead && warp >= 2 && warp < 2 + EW)
             for (int c = tid - 64, chunks = (k_hi - k_lo) * 8; c < p.m * chunks; c += ET) {
                 const int tok = c / chunks, k = k_lo * 128 + (c - tok * chunks) * 16;
                 if (k < p.k) prefetch_act(A.x, p.x_dtype, (int64_t)tok * A.ldx + k);
