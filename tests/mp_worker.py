@@ -37,8 +37,10 @@ def main():
     # o_proj, K sliced
     n, k = 7168, 2048
     w, sc = synth.fp8_weight(rng, n, k)
-    for m in (1, 11, 40):  # 11 and 40 rows run on the tcgen05 kernel (CTA pairs sending tagged words to every rank)
-        xb = synth.activations_bf16(rng, m, k)
+    # from 3 rows on the tcgen05 kernel (CTA pairs sending tagged words to every rank, or to the owners of their tiles):
+    # lone and ragged groups of four tokens
+    for m, rows in [(1, rng), (11, rng), (40, rng)] + [(m, np.random.default_rng(m)) for m in (3, 5, 21, 63)]:
+        xb = synth.activations_bf16(rows, m, k)
         xf = F.bf16_bits_to_f32(xb)
         k0, kl = sh.slice_of(k)
         xd = torch.from_numpy(xb.view(np.int16)).to(dev).view(torch.bfloat16)[:, k0:k0 + kl].contiguous()

@@ -379,23 +379,50 @@ def test_lm_head_logits_of_a_lone_rank(dev, oracle, vocab, k, m):
         grp.close()
 
 
+@pytest.mark.parametrize("vocab,k,m", [(vocab, 1024, m) for vocab in (2064, 8192) for m in (4, 5, 9, 20, 36, 66, 127)] +
+                         [(9472, 2176, 12), (9488, 2176, 12)])  # the largest shard of CTA pairs on 148 SMs, and the first without
+def test_lm_head_of_cta_pairs(dev, oracle, vocab, k, m):
+    """Small shards run on CTA pairs, each finishing every other group of four tokens: logits, their argmax, and the
+    argmax by itself (ragged and lone groups, every accumulator width)."""
+    from weightstream_b200 import formats as F, synth, tp
+    rng = np.random.default_rng(synth.config_seed("head-pairs", m, 1))
+    w, sc = synth.fp8_weight(rng, vocab, k)
+    x = F.bf16_bits_to_f32(synth.activations_bf16(rng, m, k))
+    want = oracle.fp8_gemv(w, sc, x, bn=128, bk=128, threads=oracle.max_threads())
+    wd, sd, xd = torch.from_numpy(w).to(dev), torch.from_numpy(sc).to(dev), torch.from_numpy(x).to(dev)
+    ep = tp.Endpoint(max_m=128, max_n=16, max_vocab=vocab)
+    try:
+        for _ in range(2):  # both banks of the candidate table
+            logits, amax = ep.lm_head_allgather_argmax(xd, wd, sd, vocab_row0=0, vocab=vocab)
+            _, only = ep.lm_head_allgather_argmax(xd, wd, sd, vocab_row0=0, vocab=vocab, want_logits=False)
+            ep.check()
+            check(logits, want, k)
+            first = np.argmax(logits.cpu().numpy(), axis=1)  # the first of equals
+            assert np.array_equal(amax.cpu().numpy(), first) and np.array_equal(only.cpu().numpy(), first)
+    finally:
+        ep.close()
+
+
 @pytest.mark.parametrize("world,m", [(1, 1), (1, 4), (1, 5), (1, 33), (1, 128), (2, 5), (2, 65)])
-def test_lm_head_equal_candidates_of_many_ctas(dev, world, m):
+def test_lm_head_equal_candidates_of_many_ctas(dev, oracle, world, m):
     """Every row of the vocabulary returns in each 1024 rows, so that every token's largest logit is there in many tiles,
-    CTAs and ranks: the answer is the first of them (whole numbers, exact)."""
+    CTAs and ranks (equal rows have equal sums, bit for bit): the answer is the first of them, also by the oracle's logits."""
     from weightstream_b200 import formats as F, synth, tp
     rng = np.random.default_rng(synth.config_seed("head-ties", m, world))
     vocab, k = 17 * 1024 * world, 2048
     w, sc = synth.fp8_weight(rng, 1024, k)
-    x = torch.from_numpy(F.bf16_bits_to_f32(synth.activations_bf16(rng, m, k))).to(dev)
+    x = F.bf16_bits_to_f32(synth.activations_bf16(rng, m, k))
+    ref = oracle.fp8_gemv(w, sc, x, bn=128, bk=128, threads=oracle.max_threads())
+    x = torch.from_numpy(x).to(dev)
     wd, sd = torch.from_numpy(np.tile(w, (17, 1))).to(dev), torch.from_numpy(np.tile(sc, (17, 1))).to(dev)
     grp = tp.LocalGroup(world, max_m=128, max_n=16, max_vocab=vocab)
     try:
         logits, amax = grp.lm_head_allgather_argmax([x] * world, [wd] * world, [sd] * world, vocab=vocab,
                                                     vocab_row0s=[r * 17 * 1024 for r in range(world)], row0s=[0] * world)
         grp.check()
+        check(logits[0], np.tile(ref, (1, 17 * world)), k)
         want = np.argmax(logits[0].cpu().numpy(), axis=1)  # the first of equals
-        assert want.max() < 1024
+        assert want.max() < 1024 and np.array_equal(want, np.argmax(ref, axis=1))
         for r in range(world):
             assert np.array_equal(amax[r].cpu().numpy().astype(np.int64), want)
     finally:
