@@ -174,6 +174,9 @@ struct alignas(64) BsParams {
 // Of a CTA pair, CTA r finishes the groups of four tokens 2 j + r: every epilogue thread then sends half of its columns and
 // keeps half, in 16-byte words and without a test per column (each CTA half of the tokens in one run, a float at a time,
 // took 4.6 us a tile at 96 rows and 1.0 at 19: 96 rows of K 8192 28.5 us a step, 25.5 now; 8 rows of K 1024 5.84, 5.28).
+// Up to four rows are all CTA 0's, of twelve eight are: with peers its threads send and fold more words than equal halves
+// would.  A last rank's step, the words of eight ranks at hand, takes the same time either way (3, 4, 12 rows 19.5, 19.5,
+// 23.6 us); over NVLink it has not been timed.
 __host__ __device__ constexpr int bs_rx_groups(int m) { return ((m + 3) / 4 + 1) / 2; }
 
 struct BsSmem {
@@ -601,6 +604,7 @@ static __device__ __noinline__ void bs_lm_head(const BsParams &p) {
         // tokens before it looks at the first (one by one, the merge of 15 tokens was 10 us of a 30 us step).
         auto merge = [&](int count, auto entry, auto done) {
             constexpr int U = 4, J = kMaxCtas / 32;
+            static_assert(kMaxCtas % 32 == 0, "every entry has a lane");
             for (int t0 = ew; t0 < p.m; t0 += U * EW) {
                 uint64_t pr[U][J];
 #pragma unroll
@@ -982,7 +986,6 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
         // tokens this CTA finishes: bit (t >> 2) & 1 set (of a pair, each CTA every other group of four)
         const uint32_t groups = p.csize == 2 ? 1u << crank : 3u;
         const size_t astride = (size_t)p.lay.max_m * p.lay.max_n;
-        const int nflag = kMaxCtas + kMaxShared;
         float *cv_s = reinterpret_cast<float *>(smem + S.cand);        // [EW warps][MP]; a warp fills its own columns
         uint32_t *ci_s = reinterpret_cast<uint32_t *>(smem + S.cand) + EW * MP;
         if (p.mode == kModeLmHead)
@@ -1039,8 +1042,8 @@ __global__ void __launch_bounds__(bs_threads(MP, WUE)) __maxnreg__(bs_regs(MP, W
                 // lane that holds it by one ballot, column i's handed to lane i mod 32, so that the columns' chains
                 // overlap; each lane then merges its columns into the warp's running best.  (Merged column by column,
                 // each a shared-memory round trip behind the last, the accumulators were held up at a tile's end and
-                // HBM idled: 64 rows of 62944 x 4352 with logits 94.8 us a
-                // step, 82.0 now; 32 rows 67.2, 64.2; one row 51.5, 50.9)
+                // HBM idled: 64 rows of 62944 x 4352 with logits 94.8 us a step, 82.0 with this, ~65 with the exchange
+                // in a function of its own; 32 rows 67.2, 64.2; one row 51.5, 50.9)
                 const uint32_t idx0 = (uint32_t)(A.vocab_row0 + tile * TR + quad * 32);
                 constexpr int H = (CP + 31) / 32;
                 uint32_t best[H], who[H];

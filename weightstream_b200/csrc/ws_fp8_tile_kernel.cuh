@@ -12,8 +12,9 @@
 // setmaxnreg, 112 sums per thread do not fit an even share.  UE8M0 weight scales (WUE) are an MMA operand,
 // whose atoms warps 2 and 3 lay out; an accumulator takes two slabs (see bs_chain).
 //
-// Bound: tokens x (128 + tokens) per slab decide between the tensor pipe (N / 2 clocks per MMA) and what L2
-// hands an SM (16 KB + 128 bytes per token a slab); wide token tiles favour both.
+// Bound: with fp32 scales the hand-off and read-back of an accumulator per slab (2000 rows of K 8192 150 us a step, and no
+// faster without the activation loads; 9.7 TB/s out of L2, tensor pipe 41 %); with UE8M0 scales, half the read-backs, what
+// L2 hands the SMs (131 us, 12 TB/s).  Wide token tiles favour both: 16 KB + 128 bytes per token a slab.
 #pragma once
 
 #include "ws_fp8_bs_kernel.cuh"

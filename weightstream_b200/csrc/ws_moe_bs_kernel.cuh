@@ -90,6 +90,9 @@ __global__ void __launch_bounds__(256) moe_bs_prep_kernel(const __grid_constant_
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const MoePrepRank &A = p.r[blockIdx.y];
     const int NR = p.m * p.top_k, tid = threadIdx.x;
+    // The route's hidden row, asked for before it is known to be this rank's.  (Without and with, 48 of 384 experts on this
+    // rank: 8 tokens of 5120 x 2304 16.65 us a step, 16.3; 21 of 7168 x 2048 30.6, 30.3; 64 54.6, 54.2; all experts, no
+    // difference.)
     if ((int)blockIdx.x < NR)
         for (int c = tid; c < (p.k >> 4); c += blockDim.x) prefetch_act(A.h, p.h_dtype, (int64_t)blockIdx.x * A.ldh + c * 16);
     asm volatile("griddepcontrol.wait;" ::: "memory");
