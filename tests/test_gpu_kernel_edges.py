@@ -40,6 +40,11 @@ FP8 = [
     # CTA pairs swap groups of four tokens: a group or a half alone, ragged last groups, every accumulator width
     (2064, 1024, 0, 1024, "f32", (4, 5, 8, 9, 15, 20, 31, 36, 63, 66, 97, 127)),
     (2064, 1056, 0, 1056, "ue8m0", (4, 5, 9, 20, 36, 66, 127)),
+    # the partner's sums arrive behind the activations: half an SM, and the third stage of UE8M0 scales
+    (608, 7040, 0, 7040, "f32", (11, 12)),
+    (8432, 1408, 0, 1408, "f32", (14,)),
+    (8528, 1408, 0, 1408, "ue8m0", (3, 4)),
+    (8208, 1664, 0, 1664, "ue8m0", (61, 124)),
     (1040, 768, 0, 768, "f32", (129, 225, 449)),     # prefill tiles: last row tile of 16, token tiles of 1 and up
     (1040, 1056, 0, 1056, "ue8m0", (129, 449)),
     (1040, 1056, 128, 1280, "ue8m0", (200,)),

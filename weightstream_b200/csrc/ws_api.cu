@@ -460,6 +460,7 @@ static ws_status_t validate_fp8(ws_tp *tp, const ws_fp8_gemm_args_t &a, bool lm_
 struct BsPlan {
     bool ok, wue;
     int mp, ks, tile_rows, ntiles, a_pitch, x_pitch, slabs_per_stage, nstages, nslot_max, nacc, inline_x;
+    int rx_behind;  // CTA pairs: the partner's sums arrive behind the activations (bs_smem_layout)
     int csize;  // 2: CTA pairs share a tile, each CTA streams half of K (tiles of a lone CTA would fill under half of the MMA's rows)
     int ncta;   // CTAs the plan is for (even with pairs)
     int tmem_cols;  // tensor-memory columns the CTA allocates (a power of two)
@@ -512,13 +513,28 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         u.x_pitch = (int)align_up((int64_t)u.slabs_per_stage * x_slab, 128);
         const int accs = (u.slabs_per_stage + chain - 1) / chain;  // accumulators of a stage
         u.nacc = std::min((int)kBsMaxAcc, u.wue ? (tmem - 16 * u.slabs_per_stage) / (accs * u.mp) : (tmem - 8) / (accs * (u.mp + 4)));
-        auto total = [&](int ns) {
-            return bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, u.nslot_max, skb, u.mp, rx_groups, u.wue,
+        auto total = [&](int ns, int sum_groups, bool behind) {
+            return bs_smem_layout(ns, u.slabs_per_stage, u.a_pitch, u.x_pitch, u.nslot_max, skb, u.mp, sum_groups, behind, u.wue,
                                   u.inline_x ? kcta * x_slab : 0).total + 1024;
         };
-        int ns = kMaxStages;  // the most stages whose layout fits
-        while (ns >= 2 && total(ns) > budget) --ns;
+        auto most = [&](int sum_groups, bool behind, int spare) {  // stages whose layout fits
+            int ns = kMaxStages;
+            while (ns >= 2 && total(ns, sum_groups, behind) + spare > budget) --ns;
+            return ns;
+        };
         const int items = tiles_per_cta * groups;
+        int ns = most(rx_groups, false, 0);
+        u.rx_behind = 0;
+        // A pair's exchange goes behind the activations where beside them it would take half an SM from a step that has room
+        // for the sums of half of the tokens (12 rows of 608 x 7040 13.3 us a step on a whole SM, 11.8 on half of one; of
+        // 8736 x 1408 9.4, 8.6; UE8M0, 3 rows of 8528 x 1408 7.9, 7.1; not for fp32 inline steps: 10 rows of 8464 x 1408 8.0,
+        // 8.6) or the third stage from UE8M0 scales (124 rows of 8208 x 8064 34.5, 30.7; a fourth or later one, or fp32
+        // scales, were 0 to 4 % slower).
+        if (u.csize == 2 && (half ? items > ns && (u.wue || !u.inline_x) : u.wue && ns < 3)) {
+            // (what it then takes, at most 2 KB more than there is behind the activations anyway, is below that for half)
+            const int nb = half ? most(0, false, (mt + 1) / 2 * kBsMmaRows * 4) : most(rx_groups, true, 0);
+            if (half ? nb >= items : nb > ns) { ns = nb; u.rx_behind = 1; }
+        }
         ns = std::min(ns, std::max(2, items));
         u.nstages = ns;
         // the epilogue and the producer wait on the same per-stage barrier: the MMA thread must not get a whole lap
@@ -526,7 +542,7 @@ static BsPlan bs_plan(const ws_fp8_gemm_args_t &a, int mt, int skb, int ncta, bo
         u.nacc = std::max(1, std::min(u.nacc, ns));
         u.ok = ns >= 2;
         if (!u.ok || (half && items > ns)) continue;  // half an SM only when the CTA's whole share of the weights fits the ring
-        u.smem = (size_t)total(ns);
+        u.smem = (size_t)total(ns, rx_groups, u.rx_behind != 0);
         int cols = 32;
         // (the epilogue reads the accumulators of a group in batches, see fp8_bs_kernel)
         const int batch = bs_read_batch(u.mp, u.wue), read = (accs + batch - 1) / batch * batch;
@@ -588,6 +604,7 @@ static ws_status_t bs_step(ws_tp *const *ranks, int n, const ws_fp8_gemm_args_t 
     p.tile_rows = u.tile_rows; p.ntiles = u.ntiles; p.a_pitch = u.a_pitch; p.x_pitch = u.x_pitch;
     p.slabs_per_stage = u.slabs_per_stage; p.nstages = u.nstages; p.nslot_max = u.nslot_max; p.skb = skb; p.nacc = u.nacc;
     p.csize = u.csize;
+    p.rx_behind = u.rx_behind;
     // More than 2048 values for a CTA to quantise: fewer are read as fast as they are asked for.  (Without and with: 768 and
     // 1536 values, K 512 and 1024, 3 rows, 4.9 us a step, 5.0 and 5.3, 5.4; 2560, K 1024, 5 rows 6.0, 5.5; 3072, K 2048, 3 rows
     // 9.4, 8.8; 4608, UE8M0 K 2304, 4 rows 8.7, 8.3; 6144, K 4096, 3 rows 13.2, 12.6; 8192, K 1024, 16 rows 7.9, 7.2.)

@@ -161,6 +161,7 @@ struct alignas(64) BsParams {
     int32_t owner_reduce;              // all-reduce by owners: tile t is folded by rank t % world, which sends the sums back
     int32_t csize;                     // 1, or 2: CTA pairs (a cluster) share a tile, each streams half of K
     int32_t ahead;                     // the CTA asks for its activations ahead of the wait on the predecessor (INL)
+    int32_t rx_behind;                 // CTA pairs: where the partner's sums arrive, see bs_smem_layout
     int32_t tile_rows, ntiles;         // output rows per tile (<= 128) and tiles of the shard
     int32_t slabs_per_stage, nstages;
     int32_t a_pitch, x_pitch;          // bytes one slab's weights (a multiple of 1024) / one stage's activations and atoms (of 128) occupy
@@ -183,7 +184,7 @@ struct BsSmem {
     int32_t a, x, wsf, sw, cand, rx, bars, misc, total;
 };
 __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stage, int a_pitch, int x_pitch, int nslot_max,
-                                                 int skb, int mp, int rx_groups, bool wue, int x_resident) {
+                                                 int skb, int mp, int rx_groups, bool rx_behind, bool wue, int x_resident) {
     BsSmem s{};
     const int nsl = nstages * slabs_per_stage;
     const int x_bytes = x_resident > 0 ? (x_resident + 127) / 128 * 128 : nstages * x_pitch;  // inline: all of this K half
@@ -191,12 +192,14 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
     s.a = o;    o += nsl * a_pitch;
     s.x = o;    o += x_bytes;
     // an MMA reads 128 rows of its weight slab however many the tile holds, and up to 128 tokens and 32 atom
-    // rows whatever m is: keep 16 KB readable behind the last slab and 2 KB behind the last activations
-    o += x_bytes + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - x_bytes : 2048;
+    // rows whatever m is: keep 16 KB readable behind the last slab and 2 KB behind the last activations.  What is there
+    // goes into sums that nobody looks at: where room is short (bs_plan) a pair's exchange has its place there.
+    const int behind = x_bytes + 2048 < kBsMmaRows * 128 ? kBsMmaRows * 128 - x_bytes : 2048, rx_bytes = rx_groups * kBsMmaRows * 16;
+    s.rx = o;   o += rx_behind && rx_bytes > behind ? rx_bytes : behind;  // CTA pairs: the partner's sums of one tile for this CTA's tokens, [group of 4 tokens][row][4]
     s.wsf = o;  o += wue ? nsl * kBsAtomBytes : kBsAtomBytes;  // the weights' scale atoms (fp32 scales: one atom of 2^0)
     s.sw = o;   o += wue ? 0 : (int)align_up((int64_t)nslot_max * skb * 4, 16);
     s.cand = o; o += bs_epi_warps(mp) * mp * 8;          // lm_head: per epilogue warp and token (value, index)
-    s.rx = o;   o += rx_groups * kBsMmaRows * 16;        // CTA pairs: the partner's sums of one tile for this CTA's tokens, [group of 4 tokens][row][4]
+    if (!rx_behind) { s.rx = o; o += rx_bytes; }
     s.bars = o; o += (2 * kMaxStages + kBsMaxAcc + 4) * 8;
     s.misc = o; o += 64;
     s.total = o;
@@ -205,7 +208,7 @@ __host__ __device__ inline BsSmem bs_smem_layout(int nstages, int slabs_per_stag
 
 template <int MP, bool WUE, bool INL>
 __device__ __forceinline__ BsSmem bs_layout(const BsParams &p) {
-    return bs_smem_layout(p.nstages, p.slabs_per_stage, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? bs_rx_groups(p.m) : 0, WUE,
+    return bs_smem_layout(p.nstages, p.slabs_per_stage, p.a_pitch, p.x_pitch, p.nslot_max, p.skb, MP, p.csize == 2 ? bs_rx_groups(p.m) : 0, p.rx_behind != 0, WUE,
                           INL ? (p.ks + p.csize - 1) / p.csize * (p.m * 128 + bs_atom_bytes(p.m)) : 0);
 }
 
