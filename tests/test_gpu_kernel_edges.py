@@ -408,6 +408,36 @@ def test_lm_head_of_cta_pairs(dev, oracle, vocab, k, m):
         ep.close()
 
 
+@pytest.mark.parametrize("want_logits", [True, False])
+@pytest.mark.parametrize("m", [3, 5, 12, 40])
+def test_lm_head_of_cta_pairs_and_a_peer(dev, oracle, m, want_logits):
+    """The head as one rank per launch runs it: two ranks one after the other, each alone.  The first gives up on the flags of
+    the second, which finds the first's logits and candidates."""
+    from weightstream_b200 import formats as F, synth, tp
+    rows, k = 2064, 1024  # (not a multiple of the scale block)
+    rng = np.random.default_rng(synth.config_seed("head-pairs-peer", m, 2))
+    w, sc = synth.fp8_weight(rng, 2 * rows, k)
+    x = F.bf16_bits_to_f32(synth.activations_bf16(rng, m, k))
+    want = oracle.fp8_gemv(w, sc, x, bn=128, bk=128, threads=oracle.max_threads())
+    wd, sd, xd = torch.from_numpy(w).to(dev), torch.from_numpy(sc).to(dev), torch.from_numpy(x).to(dev)
+    grp = tp.LocalGroup(2, max_m=64, max_n=16, max_vocab=2 * rows, wait_ms=20)
+    step = lambda r: grp.eps[r].lm_head_allgather_argmax(xd, wd[r * rows:(r + 1) * rows], sd, vocab_row0=r * rows, vocab=2 * rows,
+                                                         row0=r * rows, want_logits=want_logits)
+    try:
+        for first in (1, 0, 1):
+            step(first)
+            with pytest.raises(tp.WsError) as ei:
+                grp.eps[first].check()
+            assert ei.value.status == tp._lib.WS_ERR_TIMEOUT
+            logits, amax = step(1 - first)
+            grp.eps[1 - first].check()
+            if want_logits:
+                check(logits, want, k)
+            assert np.array_equal(amax.cpu().numpy(), np.argmax(want, axis=1))
+    finally:
+        grp.close()
+
+
 @pytest.mark.parametrize("world,m", [(1, 1), (1, 4), (1, 5), (1, 33), (1, 128), (2, 5), (2, 65)])
 def test_lm_head_equal_candidates_of_many_ctas(dev, oracle, world, m):
     """Every row of the vocabulary returns in each 1024 rows, so that every token's largest logit is there in many tiles,
