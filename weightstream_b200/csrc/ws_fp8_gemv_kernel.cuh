@@ -29,7 +29,7 @@ struct alignas(64) Fp8GemvParams {
     int32_t m, n, k, x_dtype, scale_kind, world, mode, vocab;
     int32_t bk_shift, bn_shift, nslot_max, skb;
     int32_t slices, rows_per_stage, nstages, rows_max, stage_bytes, gather_logits;
-    int32_t ahead;  // activations are asked for ahead of the wait on the predecessor
+    int32_t ahead;  // groups of warps (0 or 1) that ask for the activations ahead of the wait on the predecessor
     uint64_t timeout_ns;
     SymLayout lay;
     Fp8RankArgs r[WS_MAX_WORLD];
@@ -113,15 +113,15 @@ __device__ __forceinline__ void fp8_gemv_body(const Fp8GemvParams &p) {
     }
     // One warp of each slice of K asks for its activations.  (All warps asking, 148 CTAs of them, queued at the few lines
     // that a small K is: two rows of 7168 x 512 4.8 us a step without, 5.9 with all eight, 4.6 with one; of 1024 x 512 3.7,
-    // 4.7, 3.5; of K 2048 and up, no difference.)
-    if (p.ahead && grp == 0)
+    // 4.7, 3.5; of K 2048 and up, no difference.  A branch around the loop instead of a test in it: 8 virtual ranks, one row
+    // of K 8192, which ask for nothing, 26.8 us, 25.8 so.)
 #pragma unroll
-        for (int i = 0; i < C; ++i) {
-            const int k = ((slice * C + i) * 32 + lane) * 16;
-            if (k < p.k)
+    for (int i = 0; i < C; ++i) {
+        const int k = ((slice * C + i) * 32 + lane) * 16;
+        if (k < p.k && grp < p.ahead)
 #pragma unroll
-                for (int t = 0; t < GT; ++t) prefetch_act(A.x, p.x_dtype, (int64_t)t * A.ldx + k);
-        }
+            for (int t = 0; t < GT; ++t) prefetch_act(A.x, p.x_dtype, (int64_t)t * A.ldx + k);
+    }
     consumer_bar();
     // Everything below may read what the previous kernel on the stream wrote (activations, the step
     // sequence, exchange slots).
